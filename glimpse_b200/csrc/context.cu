@@ -262,6 +262,11 @@ Context::~Context() {
   ckpt.release(); ckpt_sum.release(); ckpt_scratch.release(); loglik.release();
   for (DevBuf* b : learned.all()) b->release();
   if (phase_err_host) cudaFreeHost(phase_err_host);
+  for (SideStream& x : side) {
+    cudaEventDestroy(x.done);
+    cudaStreamDestroy(x.s);
+  }
+  if (fork_event) cudaEventDestroy(fork_event);
   if (stream) cudaStreamDestroy(stream);
 }
 
@@ -484,6 +489,37 @@ int Context::check_phase_errors() {
   return GP_OK;
 }
 
+// Side streams 0 .. n - 1 start after the work queued on the context's stream so
+// far (fork) and the context's stream waits for them (join). Streams are made
+// when first needed and kept; only this context's kernels run on them.
+cudaError_t Context::fork_streams(int n) {
+  cudaError_t e = cudaSuccess;
+  if (n <= 0) return e;
+  if (!fork_event && (e = cudaEventCreateWithFlags(&fork_event, cudaEventDisableTiming)) != cudaSuccess) return e;
+  while ((int)side.size() < n) {
+    SideStream x;
+    if ((e = cudaStreamCreateWithFlags(&x.s, cudaStreamNonBlocking)) != cudaSuccess) return e;
+    if ((e = cudaEventCreateWithFlags(&x.done, cudaEventDisableTiming)) != cudaSuccess) {
+      cudaStreamDestroy(x.s);
+      return e;
+    }
+    side.push_back(x);
+  }
+  if ((e = cudaEventRecord(fork_event, stream)) != cudaSuccess) return e;
+  for (int i = 0; i < n; ++i)
+    if ((e = cudaStreamWaitEvent(side[i].s, fork_event, 0)) != cudaSuccess) return e;
+  return e;
+}
+
+cudaError_t Context::join_streams(int n) {
+  cudaError_t e = cudaSuccess;
+  for (int i = 0; i < n; ++i) {
+    if ((e = cudaEventRecord(side[i].done, side[i].s)) != cudaSuccess) return e;
+    if ((e = cudaStreamWaitEvent(stream, side[i].done, 0)) != cudaSuccess) return e;
+  }
+  return e;
+}
+
 // Phasing for nb entries of the current conditioning sets (tsel: device list of
 // entry indices or null for 0..nb-1; target_ids: device stream targets or null).
 int Context::run_phase(const int32_t* d_tsel, const std::vector<int32_t>& tsel_host, int nb, uint8_t* d_h0,
@@ -499,6 +535,7 @@ int Context::run_phase(const int32_t* d_tsel, const std::vector<int32_t>& tsel_h
   if ((e = p.code.ensure((size_t)nb * lv)) != cudaSuccess) return cuda_fail(e, "alloc vars");
   if ((e = p.seg.ensure((size_t)nb * lv * 4)) != cudaSuccess) return cuda_fail(e, "alloc vars");
   if ((e = p.miss.ensure((size_t)nb * lv * 4)) != cudaSuccess) return cuda_fail(e, "alloc vars");
+  if ((e = p.miss_rel.ensure((size_t)nb * lv * 4)) != cudaSuccess) return cuda_fail(e, "alloc vars");
   if ((e = p.seg_start.ensure((size_t)nb * (lv + 2) * 4)) != cudaSuccess) return cuda_fail(e, "alloc vars");
   if ((e = p.counts.ensure((size_t)nb * 3 * 4)) != cudaSuccess) return cuda_fail(e, "alloc vars");
   if ((e = p.ytp.ensure((size_t)nb * lv * 4)) != cudaSuccess) return cuda_fail(e, "alloc vars");
@@ -511,6 +548,7 @@ int Context::run_phase(const int32_t* d_tsel, const std::vector<int32_t>& tsel_h
   V.code = p.code.as<uint8_t>();
   V.seg = p.seg.as<int32_t>();
   V.miss = p.miss.as<int32_t>();
+  V.miss_rel = p.miss_rel.as<int32_t>();
   V.seg_start = p.seg_start.as<int32_t>();
   V.yt_prev = p.ytp.as<float>();
   V.yt_next = p.ytn.as<float>();
@@ -539,85 +577,78 @@ int Context::run_phase(const int32_t* d_tsel, const std::vector<int32_t>& tsel_h
     Kmax = std::max(Kmax, host_nstates[t]);
   }
   std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost[x] > cost[y]; });
-  // Placement 2, for batches of one to two entries per SM: the CTAs at grid
-  // positions i and S + i share an SM (S SMs, two CTAs per SM), so the heaviest
-  // 2S - nb entries take positions nb - S .. S - 1 and run alone, and the rest
-  // are paired heaviest with lightest.
-  if (sm_count == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
-  }
-  const int S_sm = sm_count;
-  std::vector<int32_t> order_paired;
-  if (nb > S_sm && nb <= 2 * S_sm) {
-    const int npair = nb - S_sm, nsolo = S_sm - npair;
-    order_paired.assign(nb, 0);
-    for (int j = 0; j < nsolo; ++j) order_paired[npair + j] = order[j];
-    for (int j = 0; j < npair; ++j) {
-      order_paired[j] = order[nsolo + j];
-      order_paired[S_sm + j] = order[nb - 1 - j];
-    }
-  }
-  // The per-entry buffers of fixed size come first, so that the budget below
+  // The packed segment and flat-het arrays come first, so that the budget below
   // sees the memory they leave.
-  if ((e = p.offs.ensure((size_t)nb * 2 * 8)) != cudaSuccess) return cuda_fail(e, "alloc offs");
-  if ((e = p.pprob_sum.ensure((size_t)nb * (lv + 2) * 8 * 4)) != cudaSuccess) return cuda_fail(e, "alloc psum");
-  if ((e = p.pprob_sumsum.ensure((size_t)nb * (lv + 2) * 4)) != cudaSuccess) return cuda_fail(e, "alloc pss");
-  if ((e = p.iprob_sum.ensure((size_t)nb * lv * 8 * 4)) != cudaSuccess) return cuda_fail(e, "alloc isum");
-  if ((e = p.of1.ensure((size_t)nb * lv * 8 * 4)) != cudaSuccess) return cuda_fail(e, "alloc of1");
-  if ((e = p.dip.ensure((size_t)nb * (lv + 2) * 4)) != cudaSuccess) return cuda_fail(e, "alloc dip");
+  std::vector<int64_t> offs((size_t)3 * nb);  // pool, segment and flat-het offsets
+  int64_t seg_total = 0, miss_total = 0;
+  for (int b = 0; b < nb; ++b) {
+    offs[nb + b] = seg_total;
+    offs[2 * nb + b] = miss_total;
+    seg_total += cnt[nb + b];
+    miss_total += cnt[2 * nb + b];
+  }
+  const size_t sg = (size_t)std::max<int64_t>(seg_total, 1), ms = (size_t)std::max<int64_t>(miss_total, 1);
+  if ((e = p.offs.ensure(offs.size() * 8)) != cudaSuccess) return cuda_fail(e, "alloc offs");
+  if ((e = p.seg_sum.ensure(2 * sg * 8 * 4)) != cudaSuccess) return cuda_fail(e, "alloc segment sums");
+  if ((e = p.seg_tot.ensure(2 * sg * 4)) != cudaSuccess) return cuda_fail(e, "alloc segment sums");
+  if ((e = p.miss_sum.ensure(2 * ms * 8 * 4)) != cudaSuccess) return cuda_fail(e, "alloc flat-het sums");
+  if ((e = p.of1.ensure(ms * 8 * 4)) != cudaSuccess) return cuda_fail(e, "alloc of1");
+  if ((e = p.next.ensure(sg * 4)) != cudaSuccess) return cuda_fail(e, "alloc draws");
+  if ((e = p.dip.ensure(sg * 4)) != cudaSuccess) return cuda_fail(e, "alloc dip");
   if ((e = p.err.ensure((size_t)nb * 4)) != cudaSuccess) return cuda_fail(e, "alloc err");
   if ((e = p.order.ensure((size_t)nb * 4)) != cudaSuccess) return cuda_fail(e, "alloc order");
-  // The stored segment-start and flat-het messages of every entry, its two
-  // regions side by side in one pool, packed per chunk of that order: chunks
-  // run one after another when all entries' stores do not fit the memory
-  // budget together (low coverage makes many flat hets).
+  // The stored messages of every entry (backward and forward, at segment
+  // boundaries and flat hets) side by side in one pool, packed per chunk of that
+  // order: chunks run one after another when all entries' stores do not fit the
+  // memory budget together (low coverage makes many flat hets).
   size_t need_all = 0;
   for (int b = 0; b < nb; ++b) {
     const int K = host_nstates[tsel_host.empty() ? b : tsel_host[b]];
-    need_all += ((size_t)cnt[nb + b] + (size_t)cnt[2 * nb + b]) * K * 8 * 4;
+    need_all += 2 * ((size_t)cnt[nb + b] + (size_t)cnt[2 * nb + b]) * K * 8 * 4;
   }
   const size_t budget = store_budget(p.pool.cap, need_all);
-  std::vector<int64_t> poff(nb), ioff(nb);
   std::vector<int> chunk_start(1, 0);
   int64_t tot = 0, need = 0;
   for (int j = 0; j < nb; ++j) {
     const int b = order[j];
     const int t = tsel_host.empty() ? b : tsel_host[b];
-    const int K = host_nstates[t];
-    const int64_t pb = (int64_t)cnt[nb + b] * K * 8, ib = (int64_t)cnt[2 * nb + b] * K * 8;
-    if (j > chunk_start.back() && (size_t)(tot + pb + ib) * 4 > budget) {
+    const int64_t rows = 2 * ((int64_t)cnt[nb + b] + cnt[2 * nb + b]) * host_nstates[t] * 8;
+    if (j > chunk_start.back() && (size_t)(tot + rows) * 4 > budget) {
       chunk_start.push_back(j);
       tot = 0;
     }
-    poff[b] = tot;
-    ioff[b] = tot + pb;
-    tot += pb + ib;
+    offs[b] = tot;
+    tot += rows;
     need = std::max(need, tot);
   }
   chunk_start.push_back(nb);
   if ((e = p.pool.ensure((size_t)std::max<int64_t>(need, 1) * 4)) != cudaSuccess) return cuda_fail(e, "alloc phasing store");
-  std::vector<int64_t> offs(poff);
-  offs.insert(offs.end(), ioff.begin(), ioff.end());
   cudaMemcpyAsync(p.offs.ptr, offs.data(), offs.size() * 8, cudaMemcpyHostToDevice, stream);
-  const int porder = fixed_porder ? fixed_porder : 1;
-  const bool paired_ok = !order_paired.empty() && chunk_start.size() == 2;
-  cudaMemcpyAsync(p.order.ptr, (paired_ok && porder == 2 ? order_paired : order).data(), (size_t)nb * 4,
-                  cudaMemcpyHostToDevice, stream);
+  // Within a chunk: the classes of 256 (J - 1) < K <= 256 J states, largest J
+  // first, each still in decreasing order of work.
+  auto class_of = [&](int b) {
+    return std::max(1, (host_nstates[tsel_host.empty() ? b : tsel_host[b]] + kPhaseThreads - 1) / kPhaseThreads);
+  };
+  for (size_t c = 0; c + 1 < chunk_start.size(); ++c)
+    std::stable_sort(order.begin() + chunk_start[c], order.begin() + chunk_start[c + 1],
+                     [&](int x, int y) { return class_of(x) > class_of(y); });
+  cudaMemcpyAsync(p.order.ptr, order.data(), (size_t)nb * 4, cudaMemcpyHostToDevice, stream);
   PhaseStore S;
-  S.pprob = p.pool.as<float>();
-  S.pprob_off = p.offs.as<int64_t>();
-  S.pprob_sum = p.pprob_sum.as<float>();
-  S.pprob_sumsum = p.pprob_sumsum.as<float>();
-  S.iprob = p.pool.as<float>();
-  S.iprob_off = p.offs.as<int64_t>() + nb;
-  S.iprob_sum = p.iprob_sum.as<float>();
+  S.pool = p.pool.as<float>();
+  S.pool_off = p.offs.as<int64_t>();
+  S.seg_off = S.pool_off + nb;
+  S.miss_off = S.pool_off + 2 * nb;
+  S.seg_total = seg_total;
+  S.miss_total = miss_total;
+  S.seg_sum = p.seg_sum.as<float>();
+  S.seg_tot = p.seg_tot.as<float>();
+  S.miss_sum = p.miss_sum.as<float>();
   S.of1 = p.of1.as<float>();
+  S.next = p.next.as<uint32_t>();
   S.dip = p.dip.as<int32_t>();
   S.err = p.err.as<int32_t>();
   S.order = p.order.as<int32_t>();
-  const int J = std::max(1, (Kmax + kPhaseThreads - 1) / kPhaseThreads);
+  if (Kmax > kMaxStates) return (fail(GP_E_ARG, "phasing: too many states"), GP_E_ARG);
   double pcells = 0;
   for (int b = 0; b < nb; ++b) {
     const int t = tsel_host.empty() ? b : tsel_host[b];
@@ -627,13 +658,33 @@ int Context::run_phase(const int32_t* d_tsel, const std::vector<int32_t>& tsel_h
   cudaEvent_t ea;
   prof_begin(ea);
   for (size_t c = 0; c + 1 < chunk_start.size(); ++c) {
+    const int c0 = chunk_start[c], c1 = chunk_start[c + 1];
+    // One chain launch per class, side by side on the context's streams: the
+    // instance for J states per thread takes only the registers that J needs, so
+    // that the chains of all classes are resident together.
+    std::vector<int> cls(1, c0);
+    int units = 0;
+    for (int j = c0; j < c1; ++j) {
+      if (j > c0 && class_of(order[j]) != class_of(order[j - 1])) cls.push_back(j);
+      units = std::max(units, cnt[nb + order[j]] - 1 + cnt[2 * nb + order[j]]);
+    }
+    cls.push_back(c1);
+    const int nside = (int)cls.size() - 2;
+    if ((e = fork_streams(nside)) != cudaSuccess) return cuda_fail(e, "phasing streams");
+    for (int i = 0; i <= nside; ++i) {
+      PhaseStore Sc = S;
+      Sc.order = S.order + cls[i];
+      if (launch_phase_chain(class_of(order[cls[i]]), d_tsel, cls[i + 1] - cls[i], w.nstates.as<int32_t>(),
+                             w.hvar.as<uint32_t>(), w.WB, w.Kp, w.npoly.as<int32_t>(), V, Sc, mc,
+                             i == 0 ? stream : side[i - 1].s) != GP_OK)
+        return (fail(GP_E_ARG, "phasing: too many states"), GP_E_ARG);
+    }
+    if ((e = join_streams(nside)) != cudaSuccess) return cuda_fail(e, "phasing streams");
     PhaseStore Sc = S;
-    Sc.order = S.order + chunk_start[c];
-    if (launch_phase(J, d_tsel, chunk_start[c + 1] - chunk_start[c], w.nstates.as<int32_t>(), w.hvar.as<uint32_t>(),
-                     w.WB, w.Kp, w.poly.as<int32_t>(), w.npoly.as<int32_t>(), L, panel.cm, V, Sc, mc, cfg.seed,
-                     iteration, d_target_ids, stream) != GP_OK)
-      return (fail(GP_E_ARG, "phasing: too many states"), GP_E_ARG);
-    prof.kernel_launches += 1;
+    Sc.order = S.order + c0;
+    launch_phase_units(units, d_tsel, c1 - c0, w.nstates.as<int32_t>(), w.hvar.as<uint32_t>(), w.WB, w.Kp, V, Sc,
+                       cfg.seed, iteration, d_target_ids, stream);
+    prof.kernel_launches += nside + 3;
   }
   prof_end(ea, 1, pcells);
   phase_chunks = (int)chunk_start.size() - 1;

@@ -113,12 +113,18 @@ struct Context {
   // large enough to tell them apart; fixed_* (gp_tuning_set) override it.
   int tune_cpc = 0, tune_hpw = 0;     // chosen chains per CTA / haplotypes per sweep warp (0: not yet)
   int fixed_cpc = 0, fixed_hpw = 0;
-  // k_phase placement (1, the default: entries in decreasing order of work; 2:
-  // the heaviest alone on an SM, the others paired heavy with light)
-  int fixed_porder = 0;
+  int fixed_porder = 0;  // the caller's phasing placement, reported back; every placement runs the same launches
   // phase-1 ms for 1, 2, 4 chains per CTA; sweep ms for 1, 2, 4, 8; k_phase ms for placements 1, 2
   float tune_ms[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  int sm_count = 0;
+  // streams beside `stream` for launches that run together (fork_streams / join_streams)
+  struct SideStream {
+    cudaStream_t s = nullptr;
+    cudaEvent_t done = nullptr;
+  };
+  std::vector<SideStream> side;
+  cudaEvent_t fork_event = nullptr;
+  cudaError_t fork_streams(int n);
+  cudaError_t join_streams(int n);
   DevBuf tune_tarhap;
   // --state-list: per target the sorted union of its haplotypes' rows (empty: no lists)
   std::vector<int32_t> list_len;

@@ -129,12 +129,12 @@ struct ImputeWork {
 
 // Scratch of the phasing HMM.
 struct PhaseWork {
-  DevBuf rel, code, seg, miss, seg_start, counts, ytp, ytn, vflags, recb, recf;
-  DevBuf pool;  // the stored segment-start and flat-het messages of one chunk of entries
-  DevBuf offs, pprob_sum, pprob_sumsum, iprob_sum, of1, dip, err, order;
+  DevBuf rel, code, seg, miss, miss_rel, seg_start, counts, ytp, ytn, vflags, recb, recf;
+  DevBuf pool;  // the stored messages of one chunk of entries
+  DevBuf offs, seg_sum, seg_tot, miss_sum, of1, next, dip, err, order;
   std::vector<DevBuf*> all() {
-    return {&rel, &code, &seg, &miss, &seg_start, &counts, &ytp, &ytn, &vflags, &recb, &recf, &pool, &offs,
-            &pprob_sum, &pprob_sumsum, &iprob_sum, &of1, &dip, &err, &order};
+    return {&rel, &code, &seg, &miss, &miss_rel, &seg_start, &counts, &ytp, &ytn, &vflags, &recb, &recf, &pool,
+            &offs, &seg_sum, &seg_tot, &miss_sum, &of1, &next, &dip, &err, &order};
   }
 };
 

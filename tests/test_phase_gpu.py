@@ -131,3 +131,45 @@ def test_chunked_phasing_matches_single_launch(small_workload, monkeypatch):
         assert np.array_equal(a0, b0) and np.array_equal(a1, b1)
     finally:
         ctx.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("edges", [(1, 31, 32, 33, 64, 65), (255, 256, 257, 319, 321), (511, 512, 513, 767, 769, 1023),
+                                   (1024, 1025, 1535, 1537, 1791, 1793, 2047, 2048)])
+def test_state_count_edges_and_mixed_classes(edges):
+    """The chain kernel has an instance per 256 states, its last two register slots
+    may be partly empty, and a batch runs its instances side by side: every
+    target of a mixed batch must get the haplotypes it gets alone, at state
+    counts around the warp and class boundaries, and (where it is built) those
+    of rephaseHaplotypes."""
+    from glimpse_b200 import native, synth
+    w = synth.make_panel_and_targets(2048, 1500, 0.3, 0.5, 2, ("uniform", 0.3, 1.5), ("fixed", 200), seed=61,
+                                     sparse_maf=0.005)
+    P, T = w.panel, w.targets
+    rng = np.random.default_rng(edges[0])
+    cases = []
+    for i, K in enumerate(edges):
+        t = i % T.n
+        s = np.sort(rng.choice(P.n_ref_haps, size=K, replace=False)).astype(np.uint32)
+        flat = T.flat[t].copy()
+        if i % 3 == 1:
+            flat[:] = 1  # flat hets only: the first VAR site starts the recursion without a sum
+        if i % 3 == 2:
+            flat[40:1400] = 1  # most 32-site blocks without a VAR site but flat hets
+        cases.append((s, _noisy_haps(rng, T.truth[t, 0]), _noisy_haps(rng, T.truth[t, 1]), flat, i))
+    ctx = native.Context(P)
+    try:
+        it = 3
+        args = ([c[0] for c in cases], np.stack([c[1] for c in cases]), np.stack([c[2] for c in cases]),
+                np.stack([c[3] for c in cases]), it)
+        g0, g1 = ctx.rephase_batch(*args, target_ids=[c[4] for c in cases])
+        for i, (s, h0, h1, fl, tid) in enumerate(cases):
+            a0, a1 = ctx.rephase_batch([s], h0[None], h1[None], fl[None], it, target_ids=[tid])
+            assert np.array_equal(a0[0], g0[i]) and np.array_equal(a1[0], g1[i]), edges[i]
+        O = ref_oracle_or_skip()
+        orc = O.RefOracle(P, T, kinit=200, kpbwt=150)
+        for i, (s, h0, h1, fl, tid) in enumerate(cases):
+            r0, r1, _ = orc.rephase(s, h0, h1, fl, it, tid)
+            assert np.array_equal(g0[i], r0) and np.array_equal(g1[i], r1), edges[i]
+    finally:
+        ctx.close()
