@@ -246,7 +246,7 @@ Context::~Context() {
   impute.states.release(); impute.nstates.release(); impute.states_off.release();
   impute.mark.release(); impute.polyidx.release(); impute.poly.release(); impute.npoly.release();
   impute.hvar.release(); impute.em.release(); impute.tr.release(); impute.fl.release();
-  impute.alpha.release(); impute.alpha_off.release(); impute.split.release(); impute.split_scr.release();
+  impute.rows.release(); impute.row_off.release(); impute.fac.release();
   impute.hl.release(); impute.hp.release(); impute.flat.release();
   prof_resolve();
   for (DevBuf* b : phase.all()) b->release();
@@ -342,6 +342,37 @@ size_t Context::store_budget(size_t held, size_t need) {
   return b;
 }
 
+// Side streams 0 .. n - 1 start after the work queued on the context's stream so
+// far (fork) and the context's stream waits for them (join). Streams are made
+// when first needed and kept; only this context's kernels run on them.
+cudaError_t Context::fork_streams(int n) {
+  cudaError_t e = cudaSuccess;
+  if (n <= 0) return e;
+  if (!fork_event && (e = cudaEventCreateWithFlags(&fork_event, cudaEventDisableTiming)) != cudaSuccess) return e;
+  while ((int)side.size() < n) {
+    SideStream x;
+    if ((e = cudaStreamCreateWithFlags(&x.s, cudaStreamNonBlocking)) != cudaSuccess) return e;
+    if ((e = cudaEventCreateWithFlags(&x.done, cudaEventDisableTiming)) != cudaSuccess) {
+      cudaStreamDestroy(x.s);
+      return e;
+    }
+    side.push_back(x);
+  }
+  if ((e = cudaEventRecord(fork_event, stream)) != cudaSuccess) return e;
+  for (int i = 0; i < n; ++i)
+    if ((e = cudaStreamWaitEvent(side[i].s, fork_event, 0)) != cudaSuccess) return e;
+  return e;
+}
+
+cudaError_t Context::join_streams(int n) {
+  cudaError_t e = cudaSuccess;
+  for (int i = 0; i < n; ++i) {
+    if ((e = cudaEventRecord(side[i].done, side[i].s)) != cudaSuccess) return e;
+    if ((e = cudaStreamWaitEvent(stream, side[i].done, 0)) != cudaSuccess) return e;
+  }
+  return e;
+}
+
 // Forward-backward over the current conditioning sets. The haplotypes run in
 // decreasing order of polymorphic sites; when their stores do not fit the
 // budget together, they run in consecutive chunks of that order, each chunk's
@@ -354,64 +385,83 @@ int Context::run_impute(const float* d_hl, const uint8_t* d_flat, float* d_hp) {
   if ((e = w.tr.ensure((size_t)n * L * 8)) != cudaSuccess) return cuda_fail(e, "alloc tr");
   if ((e = w.fl.ensure((size_t)n * L)) != cudaSuccess) return cuda_fail(e, "alloc fl");
   if (precision_mode != GP_PRECISION_FULL) return run_impute_ckpt(d_hl, d_flat, d_hp);
-  if ((e = w.alpha_off.ensure((size_t)n * 8)) != cudaSuccess) return cuda_fail(e, "alloc alpha_off");
-  int Kmax = 0;
-  for (int i = 0; i < n; ++i) Kmax = std::max(Kmax, host_nstates[i]);
-  w.Ks = impute_store_stride(Kmax);
+  if ((e = w.row_off.ensure((size_t)n * 8)) != cudaSuccess) return cuda_fail(e, "alloc row offsets");
   // Chains of the longest haplotypes (most poly sites) are launched first.
   std::vector<int32_t> order(n);
   for (int i = 0; i < n; ++i) order[i] = i;
   std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return impute_np[x] > impute_np[y]; });
-  // chunks of the order whose stores fit the budget
+  // chunks of the order whose kept rows (two per kRowSites sites) fit the budget
+  auto row_bytes = [&](int i) {
+    return (int64_t)2 * ((impute_np[i] + kRowSites - 1) / kRowSites) * 128 * impute_groups(host_nstates[i]) * 4;
+  };
   size_t need_all = 0;
-  for (int i = 0; i < n; ++i) need_all += (size_t)impute_np[i] * w.Ks * 4;
-  const size_t budget = store_budget(w.alpha.cap, need_all);
-  std::vector<int64_t> aoff(n);
-  std::vector<int32_t> split(n);
+  for (int i = 0; i < n; ++i) need_all += (size_t)row_bytes(i);
+  const size_t budget = store_budget(w.rows.cap, need_all);
+  std::vector<int64_t> roff(n);
   std::vector<int> chunk_start(1, 0);
   int64_t tot = 0, need = 0;
   for (int j = 0; j < n; ++j) {
     const int i = order[j];
-    const int64_t bytes = (int64_t)impute_np[i] * w.Ks * 4;
+    const int64_t bytes = row_bytes(i);
     if (j > chunk_start.back() && (size_t)(tot + bytes) > budget) {
       chunk_start.push_back(j);
       tot = 0;
     }
-    aoff[i] = tot / 4;
+    roff[i] = tot / 4;
     tot += bytes;
     need = std::max(need, tot);
-    split[i] = (impute_np[i] / 2) & ~31;  // forward/backward meeting point, a multiple of 32
   }
   chunk_start.push_back(n);
-  if ((e = w.alpha.ensure((size_t)std::max<int64_t>(need, 4))) != cudaSuccess) return cuda_fail(e, "alloc alpha");
-  if ((e = w.split.ensure((size_t)n * 4)) != cudaSuccess) return cuda_fail(e, "alloc split");
-  if ((e = w.split_scr.ensure(((size_t)((2 * n + 3) & ~3) + (size_t)n * w.Ks) * 4)) != cudaSuccess)
-    return cuda_fail(e, "alloc split");
-  cudaMemcpyAsync(w.alpha_off.ptr, aoff.data(), n * 8, cudaMemcpyHostToDevice, stream);
-  cudaMemcpyAsync(w.split.ptr, split.data(), n * 4, cudaMemcpyHostToDevice, stream);
+  if ((e = w.rows.ensure((size_t)std::max<int64_t>(need, 4))) != cudaSuccess) return cuda_fail(e, "alloc rows");
+  if ((e = w.fac.ensure((size_t)2 * n * w.WB * 32 * 4)) != cudaSuccess) return cuda_fail(e, "alloc factors");
   if ((e = w.order.ensure((size_t)n * 4)) != cudaSuccess) return cuda_fail(e, "alloc order");
+  // Within a chunk: the classes of 128 (J - 1) < K <= 128 J states, largest J first.
+  auto class_of = [&](int i) { return impute_groups(host_nstates[i]); };
+  for (size_t c = 0; c + 1 < chunk_start.size(); ++c)
+    std::stable_sort(order.begin() + chunk_start[c], order.begin() + chunk_start[c + 1],
+                     [&](int x, int y) { return class_of(x) > class_of(y); });
+  cudaMemcpyAsync(w.row_off.ptr, roff.data(), n * 8, cudaMemcpyHostToDevice, stream);
   cudaMemcpyAsync(w.order.ptr, order.data(), (size_t)n * 4, cudaMemcpyHostToDevice, stream);
   launch_site_records(panel, mc, w, d_hl, d_flat, stream);
   double cells = 0;
   for (int i = 0; i < n; ++i) cells += (double)impute_np[i] * (double)host_nstates[i];
-  // one warp per chain: lane-owned states in groups of 8 per lane
-  const int J = impute_groups(Kmax);
+  // The chains of one chunk: a launch per class, side by side on the context's streams.
+  auto run_chains = [&](size_t c, int cpc) -> int {
+    const int c0 = chunk_start[c], c1 = chunk_start[c + 1];
+    std::vector<int> cls(1, c0);
+    for (int j = c0 + 1; j < c1; ++j)
+      if (class_of(order[j]) != class_of(order[j - 1])) cls.push_back(j);
+    cls.push_back(c1);
+    const int nc = (int)cls.size() - 1, nside = std::min(nc - 1, kMaxSideStreams);
+    if (fork_streams(nside) != cudaSuccess) return GP_E_CUDA;
+    int rc = GP_OK;
+    for (int i = 0; i < nc && rc == GP_OK; ++i) {
+      const int q = i % (nside + 1);
+      rc = launch_impute_chain(class_of(order[cls[i]]), w, q == 0 ? stream : side[q - 1].s, cls[i],
+                               cls[i + 1] - cls[i], cpc);
+      prof.kernel_launches += 1;
+    }
+    if (join_streams(nside) != cudaSuccess) return GP_E_CUDA;
+    return rc;
+  };
   cudaEvent_t ea;
   prof_begin(ea);
   int cpc = fixed_cpc ? fixed_cpc : tune_cpc;
   if (!cpc) {
-    // Autotune chains per CTA on this batch's first chunk: phase 1 only writes
-    // the store, so the runs repeat the same work; the real run follows.
-    cpc = 2;
+    // Autotune chains per CTA on this batch's first chunk: the chains only write
+    // their rows and factors, so the runs repeat the same work; the real run
+    // follows. A run before the first timed one loads the kernels.
+    cpc = 1;
     if (chunk_start[1] >= 16) {
       const int cand[3] = {1, 2, 4};
       cudaEvent_t e0, e1;
       cudaEventCreate(&e0);
       cudaEventCreate(&e1);
       float best = 1e30f;
+      run_chains(0, 1);
       for (int ci = 0; ci < 3; ++ci) {
         cudaEventRecord(e0, stream);
-        const int lrc = launch_impute_warp(1, J, mc, w, d_hp, stream, 0, chunk_start[1], cand[ci]);
+        const int lrc = run_chains(0, cand[ci]);
         cudaEventRecord(e1, stream);
         float ms = 1e30f;
         if (lrc == GP_OK && cudaEventSynchronize(e1) == cudaSuccess) cudaEventElapsedTime(&ms, e0, e1);
@@ -425,16 +475,17 @@ int Context::run_impute(const float* d_hl, const uint8_t* d_flat, float* d_hp) {
       cudaEventDestroy(e0);
       cudaEventDestroy(e1);
       tune_cpc = cpc;
-      prof.kernel_launches += 3;
     }
   }
   for (size_t c = 0; c + 1 < chunk_start.size(); ++c) {
-    const int j0 = chunk_start[c], nc = chunk_start[c + 1] - j0;
-    int lrc = launch_impute_warp(1, J, mc, w, d_hp, stream, j0, nc, cpc);
-    if (lrc == GP_OK) lrc = launch_impute_warp(2, J, mc, w, d_hp, stream, j0, nc, cpc);
-    if (lrc == GP_E_CUDA) return cuda_fail(cudaGetLastError(), "imputation: shared-memory attribute");
+    const int c0 = chunk_start[c], c1 = chunk_start[c + 1];
+    int lrc = run_chains(c, cpc);
+    int np_max = 0;
+    for (int j = c0; j < c1; ++j) np_max = std::max(np_max, impute_np[order[j]]);
+    if (lrc == GP_OK) lrc = launch_impute_block(np_max, w, d_hp, stream, c0, c1 - c0);
+    if (lrc == GP_E_CUDA) return cuda_fail(cudaGetLastError(), "imputation: launch");
     if (lrc != GP_OK) return (fail(GP_E_ARG, "imputation: too many states"), GP_E_ARG);
-    prof.kernel_launches += 2;
+    prof.kernel_launches += 1;
   }
   prof_end(ea, 0, cells);
   impute_chunks = (int)chunk_start.size() - 1;
@@ -487,37 +538,6 @@ int Context::check_phase_errors() {
                                   std::to_string(phase_err_ids[b])),
               GP_E_DATA);
   return GP_OK;
-}
-
-// Side streams 0 .. n - 1 start after the work queued on the context's stream so
-// far (fork) and the context's stream waits for them (join). Streams are made
-// when first needed and kept; only this context's kernels run on them.
-cudaError_t Context::fork_streams(int n) {
-  cudaError_t e = cudaSuccess;
-  if (n <= 0) return e;
-  if (!fork_event && (e = cudaEventCreateWithFlags(&fork_event, cudaEventDisableTiming)) != cudaSuccess) return e;
-  while ((int)side.size() < n) {
-    SideStream x;
-    if ((e = cudaStreamCreateWithFlags(&x.s, cudaStreamNonBlocking)) != cudaSuccess) return e;
-    if ((e = cudaEventCreateWithFlags(&x.done, cudaEventDisableTiming)) != cudaSuccess) {
-      cudaStreamDestroy(x.s);
-      return e;
-    }
-    side.push_back(x);
-  }
-  if ((e = cudaEventRecord(fork_event, stream)) != cudaSuccess) return e;
-  for (int i = 0; i < n; ++i)
-    if ((e = cudaStreamWaitEvent(side[i].s, fork_event, 0)) != cudaSuccess) return e;
-  return e;
-}
-
-cudaError_t Context::join_streams(int n) {
-  cudaError_t e = cudaSuccess;
-  for (int i = 0; i < n; ++i) {
-    if ((e = cudaEventRecord(side[i].done, side[i].s)) != cudaSuccess) return e;
-    if ((e = cudaStreamWaitEvent(stream, side[i].done, 0)) != cudaSuccess) return e;
-  }
-  return e;
 }
 
 // Phasing for nb entries of the current conditioning sets (tsel: device list of

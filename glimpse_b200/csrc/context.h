@@ -50,6 +50,9 @@ void unphred_table(float* out);
 
 ModelConst model_constants(const gp_config& c, int n_ref_haps);
 
+// Streams beside a context's own: with it, no more than the device's default hardware queues.
+constexpr int kMaxSideStreams = 7;
+
 struct Context {
   gp_config cfg{};
   ModelConst mc{};

@@ -49,10 +49,10 @@ size_t round256(size_t x) { return (x + 255) & ~size_t(255); }
 
 // Byte offsets of every buffer of a one-haplotype imputation inside the region.
 // The per-site buffers are sized on all L sites; the forward-backward store
-// starts at `alpha` and may use the region up to its end.
+// starts at `store` and may use the region up to its end.
 struct StaticLayout {
-  size_t states, nstates, mark, polyidx, poly, npoly, hvar, em, tr, fl, alpha_off, split, split_scr, hl, hp, flat,
-      alpha;
+  size_t states, nstates, mark, polyidx, poly, npoly, hvar, em, tr, fl, row_off, reserve, hl, hp, flat,
+      store;
 };
 
 StaticLayout static_layout(int L, int Kp, int Ks) {
@@ -74,13 +74,12 @@ StaticLayout static_layout(int L, int Kp, int Ks) {
   s.em = take((size_t)L * 16);
   s.tr = take((size_t)L * 8);
   s.fl = take((size_t)L);
-  s.alpha_off = take(8);
-  s.split = take(4);
-  s.split_scr = take((size_t)(4 + Ks) * 4);
+  s.row_off = take(8);
+  s.reserve = take(256 + (size_t)(4 + Ks) * 4);  // counted in the limits below, not used
   s.hl = take((size_t)L * 2 * 4);
   s.hp = take((size_t)L * 2 * 4);
   s.flat = take((size_t)L);
-  s.alpha = o;
+  s.store = o;
   return s;
 }
 
@@ -108,14 +107,14 @@ extern "C" int gp_impute_one_static(gp_ctx* ctx, int32_t k, const uint32_t* stat
   }
   const int L = c.panel.L;
   const int Kp = (k + 31) / 32 * 32;
-  const int Ks = gp::impute_store_stride(k);
+  const int Ks = 128 * gp::impute_groups(k);
   const gp::StaticLayout lay = gp::static_layout(L, Kp, Ks);
-  if (lay.alpha + (size_t)Ks * 4 * 32 > gp::kStaticScratchBytes)
+  if (lay.store + (size_t)Ks * 4 * 32 > gp::kStaticScratchBytes)
     return (c.fail(GP_E_ARG, "impute_one_static: the per-site buffers of " + std::to_string(L) + " sites x " +
-                                 std::to_string(k) + " states need " + std::to_string(lay.alpha >> 20) +
+                                 std::to_string(k) + " states need " + std::to_string(lay.store >> 20) +
                                  " MiB of scratch, above the fixed 64 MiB"),
             GP_E_ARG);
-  const size_t store_cap = gp::kStaticScratchBytes - lay.alpha;
+  const size_t store_cap = gp::kStaticScratchBytes - lay.store;
   const int dev = c.cfg.device;
   if (dev < 0 || dev >= gp::kMaxDevices) return (c.fail(GP_E_ARG, "impute_one_static: device ordinal"), GP_E_ARG);
 
@@ -142,7 +141,6 @@ extern "C" int gp_impute_one_static(gp_ctx* ctx, int32_t k, const uint32_t* stat
   w.L = L;
   w.Kp = Kp;
   w.WB = (L + 31) / 32;
-  w.Ks = Ks;
   gp::point(w.states, base, lay.states, (size_t)Kp * 4);
   gp::point(w.nstates, base, lay.nstates, 4);
   gp::point(w.mark, base, lay.mark, L);
@@ -153,10 +151,7 @@ extern "C" int gp_impute_one_static(gp_ctx* ctx, int32_t k, const uint32_t* stat
   gp::point(w.em, base, lay.em, (size_t)L * 16);
   gp::point(w.tr, base, lay.tr, (size_t)L * 8);
   gp::point(w.fl, base, lay.fl, L);
-  gp::point(w.alpha_off, base, lay.alpha_off, 8);
-  gp::point(w.split, base, lay.split, 4);
-  gp::point(w.split_scr, base, lay.split_scr, (size_t)(4 + Ks) * 4);
-  gp::point(w.alpha, base, lay.alpha, store_cap);
+  gp::point(w.row_off, base, lay.row_off, 8);
   gp::point(w.hl, base, lay.hl, (size_t)L * 8);
   gp::point(w.hp, base, lay.hp, (size_t)L * 8);
   gp::point(w.flat, base, lay.flat, L);
@@ -183,14 +178,16 @@ extern "C" int gp_impute_one_static(gp_ctx* ctx, int32_t k, const uint32_t* stat
                                         " MiB forward-backward store; the fixed 64 MiB region has " +
                                         std::to_string(store_cap >> 20) + " MiB left for it"),
                    GP_E_ARG));
-  const int32_t split = (np / 2) & ~31;  // forward/backward meeting point, a multiple of 32
-  cudaMemcpyAsync(w.alpha_off.ptr, &zero64, 8, cudaMemcpyHostToDevice, s);
-  cudaMemcpyAsync(w.split.ptr, &split, 4, cudaMemcpyHostToDevice, s);
+  // Two kept rows per kRowSites sites, then two factors a site: well within np rows of Ks floats, or the 32
+  // rows that the first check leaves.
+  const size_t nrow = ((size_t)np + gp::kRowSites - 1) / gp::kRowSites, nblk = ((size_t)np + 31) / 32;
+  gp::point(w.rows, base, lay.store, 2 * nrow * Ks * 4);
+  gp::point(w.fac, base, lay.store + 2 * nrow * Ks * 4, 2 * nblk * 32 * 4);
+  w.WB = (int)nblk;  // of one haplotype, only the factors' stride depends on it from here on
+  cudaMemcpyAsync(w.row_off.ptr, &zero64, 8, cudaMemcpyHostToDevice, s);
   gp::launch_site_records(c.panel, c.mc, w, w.hl.as<float>(), w.flat.as<uint8_t>(), s);
-  const int J = gp::impute_groups(k);
-  int lrc = gp::launch_impute_warp(1, J, c.mc, w, w.hp.as<float>(), s);
-  if (lrc == GP_OK) lrc = gp::launch_impute_warp(2, J, c.mc, w, w.hp.as<float>(), s);
-  if (lrc == GP_E_CUDA) return finish(c.cuda_fail(cudaGetLastError(), "impute_one_static: shared-memory attribute"));
+  int lrc = gp::launch_impute_chain(gp::impute_groups(k), w, s);
+  if (lrc == GP_OK) lrc = gp::launch_impute_block(np, w, w.hp.as<float>(), s);
   if (lrc != GP_OK) return finish((c.fail(GP_E_ARG, "impute_one_static: too many states"), GP_E_ARG));
   gp::launch_impute_finish(c.panel, c.mc, w, w.hl.as<float>(), w.flat.as<uint8_t>(), w.hp.as<float>(), s);
   c.prof.kernel_launches += 9;

@@ -118,11 +118,10 @@ struct DevPanel {
 // Per-batch scratch for the imputation path (sized for n haplotypes).
 struct ImputeWork {
   int n = 0, L = 0, Kp = 0, WB = 0;  // WB: 32-site blocks per haplotype (upper bound)
-  int Ks = 0;                         // row stride of the forward-backward store (padded state coordinates)
   DevBuf states, nstates, states_off;
   DevBuf mark, polyidx, poly, npoly;
   DevBuf hvar, em, tr, fl;
-  DevBuf alpha, alpha_off, split, split_scr;
+  DevBuf rows, row_off, fac;  // kept rows of the chains and their offsets, the factors of every site
   DevBuf order;  // [n] haplotypes in decreasing order of poly sites (chain launch order); ptr null: identity
   DevBuf hl, hp, flat;
 };
@@ -151,16 +150,16 @@ void launch_compact_poly(const DevPanel& P, ImputeWork& w, cudaStream_t s);
 void launch_build_hvar(const DevPanel& P, ImputeWork& w, cudaStream_t s);
 void launch_site_records(const DevPanel& P, const ModelConst& mc, ImputeWork& w, const float* hl,
                          const uint8_t* flat, cudaStream_t s);
-// Chains of the haplotypes order[first .. first + count) (count < 0: all n),
-// cpc chains per CTA (1, 2 or 4; GP_E_ARG when their shared memory does not fit).
-int launch_impute_warp(int phase, int J, const ModelConst& mc, ImputeWork& w, float* hp, cudaStream_t s,
-                       int first = 0, int count = -1, int cpc = 2);
-// Register groups per lane of the imputation chain kernel for at most Kmax
-// states (the J of launch_impute_warp).
-int impute_groups(int Kmax);
-// Row stride (floats) of the forward-backward store for at most Kmax states; the
-// scratch split_scr holds round_up(2 n, 4) + n * stride floats.
-int impute_store_stride(int Kmax);
+// Sites between kept rows of a chain (a divisor of 32): two rows, one per direction.
+constexpr int kRowSites = 16;
+// Forward and backward chains of the haplotypes order[first .. first + count)
+// (count < 0: all n), all with impute_groups(K) = J, cpc chains per CTA (1, 2 or 4).
+int launch_impute_chain(int J, ImputeWork& w, cudaStream_t s, int first = 0, int count = -1, int cpc = 1);
+// After the chains, for haplotypes of any K with at most max_poly polymorphic
+// sites: prob_hid of every site into hp.
+int launch_impute_block(int max_poly, ImputeWork& w, float* hp, cudaStream_t s, int first = 0, int count = -1);
+// Rows of 128 states that a chain of K states runs (the J of launch_impute_chain).
+int impute_groups(int K);
 // The checkpointed forward-backward (kernels_impute_ckpt.cu) over the batch's
 // conditioning sets: leaves prob_hid pairs in hp for k_impute_finish.
 int launch_impute_ckpt(ImputeWork& w, bool bf16, void* ckpt, float* csum, float* scratch, double* loglik, float* hp,

@@ -1,38 +1,30 @@
-// Imputation HMM forward-backward with W warps per chain and 4 states per lane
-// per quad.
+// Imputation HMM forward-backward: sequential chains that keep a row every 16
+// sites, and a parallel pass over the blocks of 16 that forms the posteriors.
 //
 // The haploid Li-Stephens recursion (phase/src/models/imputation_hmm.cpp:143-416)
-// is sequential over sites with a sum over all K states at every site. A chain
-// (one haplotype in one direction) is run by W warps of one CTA. The states are
-// padded in front to the launch's 128 W J states (J quads per warp, from the
-// largest K of the call) and warp w, lane `lane`, local quad j owns the 4
-// consecutive padded states 128 (W j + w) + 4 lane + c, c = 0..3 (state k =
-// padded index - pad). Every chain runs all J quads, so a site is one
-// straight-line block for the scheduler; padded states are held at 0, and quads
-// without a state are neither stored nor fetched. Rows of
-// the store are kept in padded coordinates with stride Ks, so a lane's 4 values
-// of a row are one aligned 16-byte vector: phase 1 writes a row with one 16-byte
-// store per lane and quad, phase 2 stages rows with 16-byte cp.async. The
-// per-site sums are warp butterflies followed, for W > 1, by an exchange of the
-// W partial sums through shared memory behind a named barrier of the chain.
-// Hvar words of the next 32-site block and the stored rows of the next D sites
-// go through a per-warp shared-memory ring filled by cp.async; per-site records
-// (emissions, transitions, flags) of the next block are loaded one block ahead.
+// is sequential over sites only through one number a site: the sum over all K
+// states that scales the next site's factor (1 - t) / sum. Given those factors,
+// every state's recursion runs by itself. So
+//   k_impute_chain  runs both directions of a haplotype, each over all its sites,
+//                   as two concurrent chains; it keeps the factor of every site
+//                   and the row entering every block of 16 sites;
+//   k_impute_block  runs one block of one haplotype per CTA: each thread repeats
+//                   its states' forward steps from the kept row into registers and
+//                   then the backward steps, multiplies the two and sums. The steps
+//                   are the chain's own operations on the same numbers, so the
+//                   rows it forms are the chain's, bit for bit.
+// Measured, both kernels (K = 1,000, 62,700 polymorphic sites): one haplotype 11.6 ms,
+// 256 haplotypes 25.8; with every row stored and read back by the chains, split in
+// the middle of the haplotype, 16.3 and 33 ms.
+// Nothing of the size (sites x states) goes through memory: 4 bytes per 16 cells
+// and direction are written and read, where storing every row takes 8 bytes a cell.
 //
-// Each haplotype is split at M (a multiple of 32) into two chains that run
-// concurrently and meet in the middle (no waiting between them):
-//   phase 1  forward  [0, M)       stores alpha rows
-//            backward [np-1, M]    stores the pre-emission backward rows (prob_curr,
-//                                  1 at the last site) and leaves Beta at M
-//   phase 2  forward  [M, np)      alpha from row M-1; posteriors from alpha x prob_curr
-//            backward [M-1, 0]     Beta from site M; posteriors from stored alpha x prob_curr
-// Rows [0, M) of the store hold alpha and rows [M, np) prob_curr: one 4-byte
-// write and one read per (site, state), plus 1/8 byte of Hvar per pass.
-//
-// Sums follow a fixed order (per lane over quads and components, then a lane
-// butterfly, then the warps in order), so results are deterministic. Every fused
-// multiply-add is an explicit fmaf where the reference's compiled arithmetic has
-// one (build with --fmad=false).
+// The states are padded in front to 128 J (J exact: 128 (J - 1) < K <= 128 J, so
+// only row 0 holds padding, kept at 0). Sums follow a fixed tree: padded state
+// 128 j + 4 l + c belongs to lane l and component c; each (l, c) adds its j in
+// increasing order, then (c0 + c1) + (c2 + c3), then the lanes pairwise at
+// distances 16, 8, 4, 2, 1. Every fused multiply-add is an explicit one where the
+// reference's compiled arithmetic has one (build with --fmad=false).
 #include <algorithm>
 #include <type_traits>
 
@@ -42,161 +34,13 @@ namespace gp {
 
 namespace {
 
-constexpr int kMaxChainsPerCta = 4;     // chains per CTA: 1, 2 or 4 (the autotuner's choice)
-constexpr int kWarpsPerChain = 1;       // W
-constexpr int kRowDepth = 3;         // stored rows fetched this many sites ahead
-constexpr int kRing = kRowDepth + 1;      // ring slots
+constexpr int kMaxChainsPerCta = 4;  // chains per CTA: 1, 2 or 4 (the autotuner's choice)
+constexpr int kChainThreads = 64;
+static_assert(32 % kRowSites == 0, "kept rows at the starts of equal parts of a 32-site block");
 
-__device__ __forceinline__ unsigned smem_addr(const void* p) {
-  return static_cast<unsigned>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(smem_addr(smem)), "l"(gmem));
-}
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(smem_addr(smem)), "l"(gmem));
-}
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-template <int N>
-__device__ __forceinline__ void cp_wait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
-}
-
-__device__ __forceinline__ float warp_sum(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
-}
-
-struct WarpScratch {
-  float* asum;          // [n] AlphaSum at site M-1
-  float* bsum;          // [n] betaSum at site M
-  float* brow;          // [n][Ks] Beta at site M, padded coordinates
-  const int32_t* split; // [n] M
-};
-
-// Per-warp shared memory: records (2 blocks), Hvar words (2 blocks) and a row
-// ring, both holding the warp's own states: [buffer][quad j][lane] x 16 bytes.
-struct WarpSmem {
-  float4* em;       // [2][32]
-  float2* tr;       // [2][32]
-  int32_t* pl;      // [2][32] site of the poly index
-  uint4* words;     // [2][J][32]
-  float4* ring;     // [kRing][J][32]
-  uint8_t* fl;      // [2][32]
-};
-
-__host__ __device__ __forceinline__ size_t warp_smem_bytes(int J) {
-  return 2 * 32 * 16 + 2 * 32 * 8 + 2 * 32 * 4 + (size_t)(2 + kRing) * J * 32 * 16 + 2 * 32;
-}
-
-__device__ __forceinline__ WarpSmem carve(char* base, int J) {
-  WarpSmem m;
-  size_t o = 0;
-  m.em = reinterpret_cast<float4*>(base + o);
-  o += 2 * 32 * 16;
-  m.tr = reinterpret_cast<float2*>(base + o);
-  o += 2 * 32 * 8;
-  m.pl = reinterpret_cast<int32_t*>(base + o);
-  o += 2 * 32 * 4;
-  m.words = reinterpret_cast<uint4*>(base + o);
-  o += (size_t)2 * J * 32 * 16;
-  m.ring = reinterpret_cast<float4*>(base + o);
-  o += (size_t)kRing * J * 32 * 16;
-  m.fl = reinterpret_cast<uint8_t*>(base + o);
-  return m;
-}
-
-// Sum over the W warps of a chain of each warp's partial sums (x, y, z), in
-// warp order, through a double-buffered exchange slot and a named barrier of
-// the chain's 32 W threads.
-template <int W>
-__device__ __forceinline__ float3 chain_sum(float x, float y, float z, float4* xch, int parity, int wi, int lane,
-                                            int bar_id) {
-  if (W == 1) return make_float3(x, y, z);
-  float4* slot = xch + parity * W;
-  if (lane == 0) slot[wi] = make_float4(x, y, z, 0.f);
-  asm volatile("bar.sync %0, %1;" ::"r"(bar_id), "r"(32 * W) : "memory");
-  float4 s = slot[0];
-#pragma unroll
-  for (int i = 1; i < W; ++i) {
-    const float4 v = slot[i];
-    s.x = __fadd_rn(s.x, v.x);
-    s.y = __fadd_rn(s.y, v.y);
-    s.z = __fadd_rn(s.z, v.z);
-  }
-  return make_float3(s.x, s.y, s.z);
-}
-
-__device__ __forceinline__ float& comp(float4& v, int c) { return c == 0 ? v.x : c == 1 ? v.y : c == 2 ? v.z : v.w; }
-__device__ __forceinline__ uint32_t compu(const uint4& v, int c) { return c == 0 ? v.x : c == 1 ? v.y : c == 2 ? v.z : v.w; }
-__device__ __forceinline__ float compf(const float4& v, int c) { return c == 0 ? v.x : c == 1 ? v.y : c == 2 ? v.z : v.w; }
-
-// One site of a chain for the owned states, specialised at compile time:
-//   FWD   forward (alpha) or backward (Beta) recursion
-//   POST  phase 2: form prob_hid from the stored row instead of storing a row
-//   INIT  first forward / last backward site: the pre-emission value is 1/K
-// Flat or low-quality sites pass emissions (1, 1): the product by 1.0 is exact,
-// so the same loop serves both kinds of site.
-// At the last site the forward posterior uses alpha alone and the stored
-// prob_curr is 1 there, so alpha x 1 is used unchanged (imputation_hmm.cpp:337-368).
-// m selects the current site's bit in the Hvar words; rowl points at this lane's
-// staged row vector of local quad 0 (shared, quad j at offset 32 j) and srowl at
-// its stored row vector (global, quad j at offset 32 W j). Every chain of a
-// launch runs the launch's J quads, so a site is one straight-line block; the
-// padded states (vf = 0) are kept at 0, and the vectors are written whole.
-template <int J, int W, bool FWD, bool POST, bool INIT>
-__device__ __forceinline__ void chain_step(float4 (&x)[J], const uint4 (&w)[J], uint32_t m, float (&q0)[4],
-                                           float (&q1)[4], float (&q2)[4], const float4 (&vf)[J], uint32_t qmask,
-                                           float fact1,
-                                           float fact2, float ex, float ey, const float4* rowl, float4* srowl) {
-  // components (0, 1) and (2, 3) of a quad are processed as packed pairs
-  const f2 fact1p = f2_pack(fact1, fact1), fact2p = f2_pack(fact2, fact2);
-  f2 q0p[2] = {f2_pack(q0[0], q0[1]), f2_pack(q0[2], q0[3])};
-#pragma unroll
-  for (int j = 0; j < J; ++j) {
-    float4 r4 = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (POST) r4 = rowl[32 * j];
-    float4 st;
-    bool bit[4];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) bit[c] = (compu(w[j], c) & m) != 0u;
-    const f2 xp[2] = {f2_pack(x[j].x, x[j].y), f2_pack(x[j].z, x[j].w)};
-    const f2 vp[2] = {f2_pack(vf[j].x, vf[j].y), f2_pack(vf[j].z, vf[j].w)};
-    float pcv[4], nx[4];
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const f2 pc = INIT ? fact1p : f2_fma(xp[h], fact2p, fact1p);
-      const f2 e = f2_pack(bit[2 * h] ? ey : ex, bit[2 * h + 1] ? ey : ex);
-      // padded states are multiplied by 0, valid ones by 1 (exact)
-      const f2 n2 = f2_mul(f2_mul(pc, e), vp[h]);
-      q0p[h] = f2_add(q0p[h], n2);
-      f2_unpack(pc, pcv[2 * h], pcv[2 * h + 1]);
-      f2_unpack(n2, nx[2 * h], nx[2 * h + 1]);
-    }
-    x[j] = make_float4(nx[0], nx[1], nx[2], nx[3]);
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      if (POST) {
-        const float r = compf(r4, c);
-        float d;
-        if (FWD) d = __fmul_rn(nx[c], r);           // alpha x stored prob_curr (1 at the last site)
-        else d = INIT ? r : __fmul_rn(r, pcv[c]);  // stored alpha x prob_curr; alpha alone at the last site
-        if (bit[c]) q2[c] = __fadd_rn(q2[c], d);
-        else q1[c] = __fadd_rn(q1[c], d);
-      } else {
-        comp(st, c) = FWD ? nx[c] : (INIT ? 1.0f : pcv[c]);
-      }
-    }
-    if (!POST && ((qmask >> j) & 1u)) srowl[32 * W * j] = st;
-  }
-  f2_unpack(q0p[0], q0[0], q0[1]);
-  f2_unpack(q0p[1], q0[2], q0[3]);
-}
-
-// Arguments of one launch, shared by the forward and backward chains.
+// Arguments of the chains and blocks of a launch.
 struct ChainArgs {
-  int nchains;
+  int count;                          // haplotypes
   const int32_t* __restrict__ poly;
   const int32_t* __restrict__ npoly;
   const int32_t* __restrict__ nstates;
@@ -204,299 +48,380 @@ struct ChainArgs {
   const float4* __restrict__ em;
   const float2* __restrict__ tr;
   const uint8_t* __restrict__ fl;
-  const int64_t* __restrict__ store_off;
-  float* __restrict__ store_pool;
-  WarpScratch sc;
-  int L, WB, Kp, Ks;
-  ModelConst mc;
+  const int64_t* __restrict__ row_off;  // [n] first kept row (floats): forward rows of the blocks, then backward rows
+  float* __restrict__ rows;
+  float* __restrict__ fac;              // [2][n][32 WB] (1 - t) / sum into every site, forward and backward
+  int n, L, WB, Kp;
   float* __restrict__ hp;
-  const int32_t* __restrict__ order;  // [n] haplotype of chain pair c (longest first), or null for the identity
+  const int32_t* __restrict__ order;    // [count] haplotype of each chain pair (longest first), or null for the identity
 };
 
-// Hvar words of this lane's states (state index kb + 128 W j + c) of one block
-// row, into dst[32 j] (dst already offset by the lane); padded states skipped.
-template <int J, int W>
-__device__ __forceinline__ void fetch_words(uint4* dst, const uint32_t* row, int kb) {
-#pragma unroll
-  for (int j = 0; j < J; ++j) {
-    uint32_t* d = reinterpret_cast<uint32_t*>(dst + 32 * j);
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const int k = kb + 128 * W * j + c;
-      if (k >= 0) cp_async4(d + c, row + k);
-    }
-  }
-}
+// ---------------------------------------------------------------------------
+// k_impute_chain: 64 threads per chain; thread `tid` owns the padded states
+// 128 j + 2 tid and + 1 of every row j as a packed pair. A chain is bound by the
+// latency of a site (division, state loop, sum) with one to two warps per
+// scheduler, and a full batch by its instructions: four warps of half the rows
+// measured the same for one haplotype (K = 1,000: 209 against 213 ns a site) and
+// more for a batch (K = 400, 256 haplotypes: 439 against 358), as every warp
+// repeats the division and the sum. The threads' sums meet in shared memory behind
+// the site's only barrier, where every lane adds the eight partial sums of its
+// group (components and distances 16 and 8) from two 16-byte loads, so that three
+// shuffles finish the sum. Records and Hvar words are loaded a block ahead.
+// ---------------------------------------------------------------------------
 
-// This lane's vectors of a stored row (padded coordinates; quad j at vector
-// offset 32 W j from the lane's quad 0) into dst[32 j].
-template <int J, int W>
-__device__ __forceinline__ void fetch_row(float4* dst, const float4* rowl, uint32_t qmask) {
-#pragma unroll
-  for (int j = 0; j < J; ++j)
-    if ((qmask >> j) & 1u) cp_async16(dst + 32 * j, rowl + 32 * W * j);
-}
+// Partial sums of the threads: lane l's pair p (components 2p, 2p + 1) at
+// 12 (l & 7) + 4 (l >> 4) + 2 p + (l >> 3 & 1): the eight values of l & 7 are two
+// aligned 16-byte vectors, whose halves add as packed pairs, and neither the
+// stores nor the loads conflict.
+constexpr int kRedStride = 12;
 
-template <int J, int W, bool FWD, bool POST>
-__device__ __forceinline__ void run_chain(const ChainArgs& A, char* smem, float4* xch, int t, int wi, int lane,
-                                          int bar_id) {
+struct ChainSmem {
+  float red[2][8 * kRedStride];
+  // per block of 32 sites: emission of allele 0 and 1, t / K and 1 - t into this site; a record
+  // past either end of a block is read and not used
+  float4 rec[1 + 4 * 32 + 1];
+};
+
+// SOLO: one chain per CTA (its barrier is the CTA's), else a named barrier per chain.
+template <int J, bool FWD, bool SOLO>
+__device__ __forceinline__ void run_chain(const ChainArgs& A, ChainSmem& S, int t, int tid, int bar_id) {
+  constexpr int Ks = 128 * J;
   const int np = A.npoly[t];
   const int K = A.nstates[t];
-  const int M = A.sc.split[t];
   if (np == 0 || K == 0) return;
-  const int lo = (FWD == POST) ? M : 0;   // phase 1: forward [0, M), backward [M, np)
-  const int hi = (FWD == POST) ? np : M;  // phase 2: forward [M, np), backward [0, M)
-  if (lo >= hi) return;
-  const int Kp = A.Kp, Ks = A.Ks;
-  const int pad = 128 * W * J - K;    // every chain is padded in front to the launch's 128 W J states
-  const int pb = 128 * wi + 4 * lane;  // padded index of this lane's quad 0
-  const int kb = pb - pad;             // its state index
-  float4 vf[J];                        // 1 for a state, 0 for padding
-  uint32_t qmask = 0u;                 // bit j: quad j holds at least one state (is stored and fetched)
-#pragma unroll
-  for (int j = 0; j < J; ++j) {
-    const int q = pb + 128 * W * j;
-    vf[j] = make_float4(q >= pad ? 1.f : 0.f, q + 1 >= pad ? 1.f : 0.f, q + 2 >= pad ? 1.f : 0.f,
-                        q + 3 >= pad ? 1.f : 0.f);
-    if (q + 3 >= pad) qmask |= 1u << j;
-  }
-  WarpSmem S = carve(smem, J);
-  float* store = A.store_pool + A.store_off[t];
-  const uint32_t* hv = A.hvar + (size_t)t * A.WB * Kp;
+  const int lane = tid & 31, wi = tid >> 5;
+  const int kb = 2 * tid - (Ks - K);  // state of this thread's first element in row 0
+  const f2 exists0 = f2_pack(kb >= 0 ? 1.f : 0.f, kb >= -1 ? 1.f : 0.f);
+  const int nrow = (np + kRowSites - 1) / kRowSites;
+  float* rows = A.rows + A.row_off[t] + (FWD ? 0 : (size_t)nrow * Ks) + 2 * tid;
+  float* fac = A.fac + ((size_t)(FWD ? 0 : A.n) + t) * 32 * A.WB;
+  const uint32_t* hv = A.hvar + (size_t)t * A.WB * A.Kp + kb;
   const float4* E = A.em + (size_t)t * A.L;
   const float2* T = A.tr + (size_t)t * A.L;
   const uint8_t* F = A.fl + (size_t)t * A.L;
-  float* HP = A.hp + (size_t)t * 2 * A.L;
-  const int32_t* PL = A.poly + (size_t)t * A.L;
-  const int n = hi - lo;
-  const float Kf = (float)K;
-  auto site_of = [&](int s) { return FWD ? lo + s : hi - 1 - s; };
-  auto row_vec = [&](int l) { return reinterpret_cast<float4*>(store + (size_t)l * Ks + pb); };
   constexpr int dir = FWD ? 1 : -1;
-  uint4* wl = S.words + lane;   // this lane's words; block buffer (b & 1) at offset 32 J (b & 1)
-  float4* rl = S.ring + lane;   // this lane's staged row vectors; slot s at offset 32 J s
-
-  // Ring entries of fully padded quads are never fetched; they hold 0.
-  if (POST) {
-#pragma unroll
-    for (int d = 0; d < kRing; ++d)
-#pragma unroll
-      for (int j = 0; j < J; ++j)
-        if (!((qmask >> j) & 1u)) rl[(d * J + j) * 32] = make_float4(0.f, 0.f, 0.f, 0.f);
-  }
-
-  // ---- prologue: records and Hvar words of the first two blocks, first rows ----
-  const int b_first = site_of(0) >> 5;
-  const int b_last = site_of(n - 1) >> 5;
-  {
-    const int l = (b_first << 5) + lane;
-    if (l < np) {
-      S.em[(b_first & 1) * 32 + lane] = E[l];
-      S.tr[(b_first & 1) * 32 + lane] = T[l];
-      S.fl[(b_first & 1) * 32 + lane] = F[l];
-      S.pl[(b_first & 1) * 32 + lane] = PL[l];
-    }
-    fetch_words<J, W>(wl + (b_first & 1) * 32 * J, hv + (size_t)b_first * Kp, kb);
-    if (b_first != b_last) {
-      const int b2 = b_first + dir;
-      fetch_words<J, W>(wl + (b2 & 1) * 32 * J, hv + (size_t)b2 * Kp, kb);
-    }
-  }
-  cp_commit();
-  if (POST) {
-#pragma unroll
-    for (int d = 0; d < kRowDepth; ++d) {
-      if (d < n) fetch_row<J, W>(rl + (d % kRing) * 32 * J, row_vec(site_of(d)), qmask);
-      cp_commit();
-    }
-  }
-
-  float4 x[J];  // alpha (forward) or Beta (backward)
-  uint4 w[J];   // Hvar words of the current block
-#pragma unroll
-  for (int j = 0; j < J; ++j) {
-    x[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-    w[j] = make_uint4(0u, 0u, 0u, 0u);
-  }
-  float acc = 0.f;  // AlphaSum / betaSum of the previous step
-  float2 t_prev = make_float2(0.f, 0.f);
-  if (FWD && lo > 0) {
-    const float4* r = row_vec(lo - 1);
-#pragma unroll
-    for (int j = 0; j < J; ++j)
-      if ((qmask >> j) & 1u) x[j] = r[32 * W * j];
-    acc = A.sc.asum[t];
-    t_prev = T[lo - 1];
-  }
-  if (!FWD && hi < np) {
-    const float4* r = reinterpret_cast<const float4*>(A.sc.brow + (size_t)t * Ks + pb);
-#pragma unroll
-    for (int j = 0; j < J; ++j)
-      x[j] = r[32 * W * j];
-    acc = A.sc.bsum[t];
-  }
-  float4 pe = make_float4(0.f, 0.f, 0.f, 0.f);
-  float2 pt = make_float2(0.f, 0.f);
-  uint8_t pf = 0;
-  int32_t pp = 0;
-  if (b_first != b_last) {
-    const int ln = ((b_first + dir) << 5) + lane;
-    if (ln < np) { pe = E[ln]; pt = T[ln]; pf = F[ln]; pp = PL[ln]; }
-  }
-  int cur_block = b_first;
-  if (!POST) cp_wait<0>();  // words of the first block (phase 2 waits per site below)
-
-  auto step = [&](int s, auto init_tag) {
-    constexpr bool INIT = decltype(init_tag)::value;
-    const int l = site_of(s);
-    const int b = l >> 5;
-    const int i = l & 31;
-    const bool new_block = INIT || (s == 0) || (b != cur_block);
-    if (b != cur_block) {
-      S.em[(b & 1) * 32 + lane] = pe;
-      S.tr[(b & 1) * 32 + lane] = pt;
-      S.fl[(b & 1) * 32 + lane] = pf;
-      S.pl[(b & 1) * 32 + lane] = pp;
-      cur_block = b;
-      if (b != b_last) {
-        const int bn = b + dir;
-        const int ln = (bn << 5) + lane;
-        if (ln < np) { pe = E[ln]; pt = T[ln]; pf = F[ln]; pp = PL[ln]; }
-        fetch_words<J, W>(wl + (bn & 1) * 32 * J, hv + (size_t)bn * Kp, kb);
-      }
-      if (!POST) {
-        cp_commit();
-        cp_wait<1>();  // this block's words; the next block's may still be in flight
-      }
-    }
-    if (POST) {
-      if (s + kRowDepth < n)
-        fetch_row<J, W>(rl + ((s + kRowDepth) % kRing) * 32 * J, row_vec(site_of(s + kRowDepth)), qmask);
-      cp_commit();
-      cp_wait<kRowDepth>();
-    }
-    __syncwarp();
-    if (new_block) {
-      const uint4* wb = wl + (b & 1) * 32 * J;
-#pragma unroll
-      for (int j = 0; j < J; ++j)
-        w[j] = wb[32 * j];
-    }
-    const uint32_t m = 1u << i;
-    const uint8_t f = S.fl[(b & 1) * 32 + i];
-    const float4 e = S.em[(b & 1) * 32 + i];
-    const float4* rowl = rl + (s % kRing) * 32 * J;
-    float4* srowl = row_vec(l);
-    float q0[4] = {0.f, 0.f, 0.f, 0.f}, q1[4] = {0.f, 0.f, 0.f, 0.f}, q2[4] = {0.f, 0.f, 0.f, 0.f};
-    float fact1, fact2;
-    if (INIT) {
-      fact1 = 1.0f / Kf;
-      fact2 = 0.f;
-    } else if (FWD) {
-      fact1 = t_prev.x;  // t / K of the previous site
-      fact2 = t_prev.y / acc;
-    } else {
-      const float2 tt = S.tr[(b & 1) * 32 + i];
-      fact1 = tt.x;
-      fact2 = tt.y / acc;
-    }
-    const float ex = f ? 1.0f : e.x, ey = f ? 1.0f : e.y;
-    chain_step<J, W, FWD, POST, INIT>(x, w, m, q0, q1, q2, vf, qmask, fact1, fact2, ex, ey, rowl, srowl);
-    const float v0 = warp_sum(__fadd_rn(__fadd_rn(q0[0], q0[1]), __fadd_rn(q0[2], q0[3])));
-    float v1 = 0.f, v2 = 0.f;
-    if (POST) {
-      v1 = warp_sum(__fadd_rn(__fadd_rn(q1[0], q1[1]), __fadd_rn(q1[2], q1[3])));
-      v2 = warp_sum(__fadd_rn(__fadd_rn(q2[0], q2[1]), __fadd_rn(q2[2], q2[3])));
-    }
-    const float3 tot = chain_sum<W>(v0, v1, v2, xch, s & 1, wi, lane, bar_id);
-    // AlphaSum = 1 at a flat first site, betaSum = 1 at a flat last site (imputation_hmm.cpp:156,285)
-    acc = (INIT && f) ? 1.0f : tot.x;
-    if (FWD) t_prev = S.tr[(b & 1) * 32 + i];
-    // prob_hid of the two alleles; k_impute_finish turns them into HP
-    if (POST && wi == 0 && lane == 0)
-      *reinterpret_cast<float2*>(HP + 2 * S.pl[(b & 1) * 32 + i]) = make_float2(tot.y, tot.z);
-    __syncwarp();
+  auto barrier = [&]() {
+    if (SOLO) __syncthreads();
+    else asm volatile("bar.sync %0, %1;" ::"r"(bar_id), "r"(kChainThreads) : "memory");
   };
 
-  // The recursion starts at site 0 (forward) or np - 1 (backward) with 1/K.
-  const bool starts = FWD ? (lo == 0) : (hi == np);
-  int s0 = 0;
-  if (starts) {
-    step(0, std::integral_constant<bool, true>());
-    s0 = 1;
-  }
-  for (int s = s0; s < n; ++s) step(s, std::integral_constant<bool, false>());
-
-  cp_wait<0>();
-  if (!POST) {
-    if (FWD) {
-      if (wi == 0 && lane == 0) A.sc.asum[t] = acc;
-    } else {
-      float4* r = reinterpret_cast<float4*>(A.sc.brow + (size_t)t * Ks + pb);
+  // Records of a block, loaded a block ahead by the first warp; Hvar words likewise, each thread its own.
+  float4 pe = make_float4(0.f, 0.f, 0.f, 0.f);
+  auto load_recs = [&](int b) {
+    const int l = (b << 5) + lane;
+    if (wi != 0 || l >= np) return;
+    const float4 e = E[l];
+    const bool f = F[l] != 0;  // flat and low-quality sites: emissions (1, 1), an exact factor
+    const float2 tt = FWD ? (l > 0 ? T[l - 1] : make_float2(0.f, 0.f)) : T[l];
+    pe = make_float4(f ? 1.0f : e.x, f ? 1.0f : e.y, tt.x, tt.y);
+  };
+  uint32_t w[2 * J], wn[2 * J];
+  auto load_words = [&](int b) {
+    const uint32_t* r = hv + (size_t)b * A.Kp;
 #pragma unroll
-      for (int j = 0; j < J; ++j)
-        r[32 * W * j] = x[j];
-      if (wi == 0 && lane == 0) A.sc.bsum[t] = acc;
+    for (int j = 0; j < J; ++j) {
+      wn[2 * j] = j > 0 || kb >= 0 ? r[128 * j] : 0u;
+      wn[2 * j + 1] = j > 0 || kb >= -1 ? r[128 * j + 1] : 0u;
     }
+  };
+
+  const int b_first = FWD ? 0 : (np - 1) >> 5;
+  const int b_last = FWD ? (np - 1) >> 5 : 0;
+  load_recs(b_first);
+  if (wi == 0) S.rec[1 + (b_first & 3) * 32 + lane] = pe;
+  load_words(b_first);
+  f2 x[J];  // alpha (forward) or Beta (backward)
+#pragma unroll
+  for (int j = 0; j < J; ++j) x[j] = f2_pack(0.f, 0.f);
+  float acc = 1.f;  // AlphaSum / betaSum of the previous step
+  barrier();
+  const int l_first = FWD ? 0 : np - 1;
+  float* const rout = &S.red[0][kRedStride * ((tid >> 1) & 7) + 4 * (tid >> 5) + 2 * (tid & 1) + ((tid >> 4) & 1)];
+  const ulonglong2* const rin = reinterpret_cast<const ulonglong2*>(&S.red[0][kRedStride * (lane & 7)]);
+  int parity = 0;
+  float keep = 0.f;  // lane i: the factor of the block's site i
+  int i = l_first & 31;
+  uint32_t m = 1u << i;
+  const float4* rp = nullptr;
+  float4 rec;
+
+  // Site i of the block; INIT: the first one of the chain, whose pre-emission value is 1/K.
+  auto step = [&](auto init_tag) {
+    constexpr bool INIT = decltype(init_tag)::value;
+    const float fact1 = INIT ? 1.0f / (float)K : rec.z;
+    const float fact2 = INIT ? 0.f : rec.w / acc;
+    const f2 f1 = f2_pack(fact1, fact1), f2v = f2_pack(fact2, fact2);
+    const float ex = rec.x, ey = rec.y;
+    if (lane == i) keep = fact2;
+    f2 q = f2_pack(0.f, 0.f);
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
+      const bool b0 = (w[2 * j] & m) != 0u, b1 = (w[2 * j + 1] & m) != 0u;
+      f2 nx = f2_mul(f2_fma(x[j], f2v, f1), f2_pack(b0 ? ey : ex, b1 ? ey : ex));
+      if (j == 0) nx = f2_mul(nx, exists0);  // padding is multiplied by 0, states by 1 (exact)
+      q = j == 0 ? nx : f2_add(q, nx);
+      x[j] = nx;
+    }
+    float v0, v1;
+    f2_unpack(q, v0, v1);
+    rout[parity] = __fadd_rn(v0, v1);
+    i += dir;
+    m = FWD ? m << 1 : m >> 1;
+    rp += dir;
+    rec = *rp;
+    barrier();
+    const ulonglong2 a = rin[parity >> 2], c = rin[(parity >> 2) + 1];
+    f2_unpack(f2_add(f2_add(a.x, a.y), f2_add(c.x, c.y)), v0, v1);
+    float v = __fadd_rn(v0, v1);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, o));
+    // AlphaSum = 1 at a flat first site, betaSum = 1 at a flat last site (imputation_hmm.cpp:156,285)
+    acc = INIT && F[l_first] != 0 ? 1.0f : v;
+    parity ^= 8 * kRedStride;
+  };
+
+  for (int b = b_first;; b += dir) {
+    // the block's records and words are in place; request the next block's
+#pragma unroll
+    for (int j = 0; j < 2 * J; ++j) w[j] = wn[j];
+    rp = &S.rec[1 + (b & 3) * 32 + i];
+    rec = *rp;
+    if (b != b_last) {
+      load_recs(b + dir);
+      load_words(b + dir);
+    }
+    if (b == b_first) step(std::integral_constant<bool, true>());
+    const int end = FWD ? min(np - (b << 5), 32) : -1;  // i after the block
+    while (i != end) {
+      const int part = i / kRowSites;
+      if (FWD ? i == part * kRowSites : i == (part + 1) * kRowSites - 1) {
+        // the row entering this part of the block
+        float* r = rows + (size_t)(b * (32 / kRowSites) + part) * Ks;
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+          float o0, o1;
+          f2_unpack(x[j], o0, o1);
+          *reinterpret_cast<float2*>(r + 128 * j) = make_float2(o0, o1);
+        }
+      }
+      const int stop = FWD ? min(end, (part + 1) * kRowSites) : part * kRowSites - 1;
+      while (i != stop) step(std::integral_constant<bool, false>());
+    }
+    if (wi == 0) fac[(b << 5) + lane] = keep;
+    if (b == b_last) break;
+    if (wi == 0) S.rec[1 + ((b + dir) & 3) * 32 + lane] = pe;
+    i = FWD ? 0 : 31;
+    m = FWD ? 1u : 1u << 31;
+    barrier();
   }
 }
 
-// Chain c = blockIdx.x * (chains per CTA) + (warp / W) is run by the W warps
-// (warp % W = 0..W-1) of its slot: haplotype order[c / 2] (c / 2 without an
-// order), forward for even chains and backward for odd ones. Every warp of a chain takes the same branches, so the
-// chain's named barrier (id 1 + slot) always sees all 32 W threads.
-template <int J, int W, bool POST>
-__global__ void __launch_bounds__(32 * W * kMaxChainsPerCta) k_impute_warp(ChainArgs A) {
-  extern __shared__ __align__(16) char smem_raw[];
-  __shared__ float4 xch[kMaxChainsPerCta][2 * W];
-  const int warp = threadIdx.x >> 5;
-  const int lane = threadIdx.x & 31;
-  const int slot = warp / W, wi = warp % W;
-  const int chain = blockIdx.x * (int)(blockDim.x / (32 * W)) + slot;
-  if (chain >= A.nchains) return;
-  char* smem = smem_raw + (size_t)warp * warp_smem_bytes(J);
+// Chain c = blockIdx.x * (chains per CTA) + slot is run by the 64 threads of its
+// slot: haplotype order[c / 2] (c / 2 without an order), forward for even chains
+// and backward for odd ones. Both warps of a chain take the same branches, so the
+// chain's barrier always sees all 64 threads.
+template <int J, bool SOLO>
+__global__ void __launch_bounds__(SOLO ? kChainThreads : kChainThreads * kMaxChainsPerCta, 1)
+    k_impute_chain(ChainArgs A) {
+  __shared__ ChainSmem S[SOLO ? 1 : kMaxChainsPerCta];
+  const int slot = SOLO ? 0 : threadIdx.x / kChainThreads, tid = threadIdx.x % kChainThreads;
+  const int chain = SOLO ? blockIdx.x : blockIdx.x * (int)(blockDim.x / kChainThreads) + slot;
+  if (chain >= 2 * A.count) return;
   const int t = A.order ? A.order[chain >> 1] : chain >> 1;
-  if ((chain & 1) == 0) run_chain<J, W, true, POST>(A, smem, xch[slot], t, wi, lane, 1 + slot);
-  else run_chain<J, W, false, POST>(A, smem, xch[slot], t, wi, lane, 1 + slot);
+  if ((chain & 1) == 0) run_chain<J, true, SOLO>(A, S[slot], t, tid, 1 + slot);
+  else run_chain<J, false, SOLO>(A, S[slot], t, tid, 1 + slot);
+}
+
+// ---------------------------------------------------------------------------
+// k_impute_block: posteriors of kRowSites sites, 128 threads. Thread tid = 4 l + c
+// takes its padded states 128 j + tid two rows j at a time, as a packed pair (rows
+// -1 and 0 first when J is odd): the forward steps, whose values stay in
+// registers, then the backward steps, the products added to the thread's two sums
+// per site (one per allele). All site data is uniform and comes from shared memory;
+// the loop over rows needs no communication. Bound by issue, about 11 instructions
+// per (site, state). One lane tree per site and allele ends it.
+// ---------------------------------------------------------------------------
+constexpr int kBlockThreads = 128;
+constexpr int RS = kRowSites;
+
+struct BlockSmem {
+  float4 fwd[RS];  // t / K twice, (1 - t) / sum twice, into the site from the left
+  float4 bwd[RS];  // the same from the right
+  float2 em[RS];   // emissions of allele 0 and 1
+  float part[32][2 * RS + 4];  // [lane l][value 2 site + allele]
+};
+
+// Shared-memory loads that stay where they are: moved out of the loop over rows,
+// as plain loads of the same addresses would be, they do not fit the registers.
+__device__ __forceinline__ void lds(unsigned addr, f2& a, f2& b) {
+  asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "r"(addr));
+}
+__device__ __forceinline__ void lds(unsigned addr, float& a, float& b) {
+  asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(a), "=f"(b) : "r"(addr));
+}
+
+// A pair of rows over the block. MASK: states that do not exist are held at 0 by a
+// factor (1 elsewhere, exact). LAST: the haplotype's last block, where the site
+// `last` starts the backward recursion and its posterior uses alpha alone
+// (imputation_hmm.cpp:268-300).
+template <bool MASK, bool LAST>
+__device__ __forceinline__ void block_pair(unsigned fwd, unsigned bwd, unsigned em, uint32_t w0, uint32_t w1, f2 x,
+                                           f2 y, f2 exists, int last, float (&q0)[RS], float (&q1)[RS]) {
+  f2 alpha[RS];
+#pragma unroll
+  for (int i = 0; i < RS; ++i) {
+    f2 f1, fac;
+    float ea, eb;
+    lds(fwd + 16 * i, f1, fac);
+    lds(em + 8 * i, ea, eb);
+    x = f2_mul(f2_fma(x, fac, f1), f2_pack((w0 >> i) & 1u ? eb : ea, (w1 >> i) & 1u ? eb : ea));
+    if (MASK) x = f2_mul(x, exists);
+    alpha[i] = x;
+  }
+  // the same words as new values: tests kept from the loop above would take registers
+  asm volatile("" : "+r"(w0), "+r"(w1));
+#pragma unroll
+  for (int i = RS - 1; i >= 0; --i) {
+    f2 f1, fac;
+    float ea, eb;
+    lds(bwd + 16 * i, f1, fac);
+    lds(em + 8 * i, ea, eb);
+    const bool b0 = (w0 >> i) & 1u, b1 = (w1 >> i) & 1u;
+    const f2 pc = f2_fma(y, fac, f1);
+    const f2 d = LAST && i == last ? alpha[i] : f2_mul(alpha[i], pc);
+    y = f2_mul(pc, f2_pack(b0 ? eb : ea, b1 ? eb : ea));
+    float d0, d1;
+    f2_unpack(d, d0, d1);
+    if (b0) q1[i] = __fadd_rn(q1[i], d0);
+    else q0[i] = __fadd_rn(q0[i], d0);
+    if (b1) q1[i] = __fadd_rn(q1[i], d1);
+    else q0[i] = __fadd_rn(q0[i], d1);
+  }
+}
+
+template <bool LAST>
+__device__ __forceinline__ void block_rows(const BlockSmem& S, const float* __restrict__ arow,
+                                           const float* __restrict__ brow, const uint32_t* __restrict__ hv, int shift,
+                                           int J, int pad, int last, float (&q0)[RS], float (&q1)[RS]) {
+  const int tid = threadIdx.x;
+  const unsigned fwd = static_cast<unsigned>(__cvta_generic_to_shared(S.fwd));
+  const unsigned bwd = static_cast<unsigned>(__cvta_generic_to_shared(S.bwd));
+  const unsigned em = static_cast<unsigned>(__cvta_generic_to_shared(S.em));
+  // rows j and j + 1 of this thread: words and the kept values entering from both sides
+  struct Pair {
+    uint32_t w0, w1;
+    float a0, a1, b0, b1;
+  };
+  auto load = [&](int j) {
+    Pair p;
+    const int o = 128 * j + tid;
+    const bool e0 = j > 0 || (j == 0 && tid >= pad), e1 = j >= 0 || tid >= pad;
+    p.w0 = e0 ? hv[o] >> shift : 0u;
+    p.w1 = e1 ? hv[o + 128] >> shift : 0u;
+    p.a0 = arow && e0 ? arow[o] : 0.f;
+    p.a1 = arow && e1 ? arow[o + 128] : 0.f;
+    p.b0 = brow && e0 ? brow[o] : 0.f;
+    p.b1 = brow && e1 ? brow[o + 128] : 0.f;
+    return p;
+  };
+  int j = -(J & 1);
+  Pair p = load(j), n;
+  const f2 exists = f2_pack(j == 0 && tid >= pad ? 1.f : 0.f, j == 0 || tid >= pad ? 1.f : 0.f);
+  if (j + 2 < J) n = load(j + 2);
+  block_pair<true, LAST>(fwd, bwd, em, p.w0, p.w1, f2_pack(p.a0, p.a1), f2_pack(p.b0, p.b1), exists, last, q0, q1);
+#pragma unroll 1
+  for (j += 2; j < J; j += 2) {
+    p = n;
+    if (j + 2 < J) n = load(j + 2);
+    block_pair<false, LAST>(fwd, bwd, em, p.w0, p.w1, f2_pack(p.a0, p.a1), f2_pack(p.b0, p.b1), 0, last, q0, q1);
+  }
+}
+
+__global__ void __launch_bounds__(kBlockThreads, 4) k_impute_block(ChainArgs A) {
+  __shared__ BlockSmem S;
+  const int t = A.order ? A.order[blockIdx.y] : blockIdx.y;
+  const int np = A.npoly[t], K = A.nstates[t];
+  const int nrow = (np + RS - 1) / RS;
+  const int b = blockIdx.x;
+  if (b >= nrow || K == 0) return;
+  const int J = (K + 127) >> 7, Ks = 128 * J, pad = Ks - K;
+  const int tid = threadIdx.x;
+  const int l0 = b * RS, n = min(RS, np - l0);
+  if (tid < RS) {
+    const int l = l0 + tid;
+    // past the last site: the identity step
+    float4 f = make_float4(0.f, 0.f, 1.f, 1.f), g = f;
+    float2 e = make_float2(1.f, 1.f);
+    if (l < np) {
+      const float2* T = A.tr + (size_t)t * A.L;
+      const float* fac = A.fac + (size_t)t * 32 * A.WB + l;
+      const float init = 1.0f / (float)K;
+      const float fa = fac[0], fb = fac[(size_t)A.n * 32 * A.WB];
+      const float ta = l > 0 ? T[l - 1].x : init, tb = l < np - 1 ? T[l].x : init;
+      f = make_float4(ta, ta, fa, fa);
+      g = make_float4(tb, tb, fb, fb);
+      const float4 ee = A.em[(size_t)t * A.L + l];
+      if (A.fl[(size_t)t * A.L + l] == 0) e = make_float2(ee.x, ee.y);
+    }
+    S.fwd[tid] = f;
+    S.bwd[tid] = g;
+    S.em[tid] = e;
+  }
+  __syncthreads();
+  float q0[RS], q1[RS];
+#pragma unroll
+  for (int i = 0; i < RS; ++i) q0[i] = q1[i] = 0.f;
+  const float* base = A.rows + A.row_off[t];
+  const float* arow = b > 0 ? base + (size_t)b * Ks : nullptr;
+  const float* brow = b < nrow - 1 ? base + ((size_t)nrow + b) * Ks : nullptr;
+  const uint32_t* hv = A.hvar + ((size_t)t * A.WB + (l0 >> 5)) * A.Kp - pad;
+  if (b == nrow - 1) block_rows<true>(S, arow, brow, hv, l0 & 31, J, pad, n - 1, q0, q1);
+  else block_rows<false>(S, arow, brow, hv, l0 & 31, J, pad, -1, q0, q1);
+  // Components of a lane l = tid / 4: reduce-scatter over thread distances 1 and 2.
+  const int c = tid & 3;
+  const bool up1 = c & 1, up2 = c & 2;
+#pragma unroll
+  for (int i = 0; i < RS / 2; ++i) {
+    const float s0 = up1 ? q0[i] : q0[i + RS / 2], k0 = up1 ? q0[i + RS / 2] : q0[i];
+    const float s1 = up1 ? q1[i] : q1[i + RS / 2], k1 = up1 ? q1[i + RS / 2] : q1[i];
+    q0[i] = __fadd_rn(k0, __shfl_xor_sync(0xffffffffu, s0, 1));
+    q1[i] = __fadd_rn(k1, __shfl_xor_sync(0xffffffffu, s1, 1));
+  }
+#pragma unroll
+  for (int i = 0; i < RS / 4; ++i) {
+    const float s0 = up2 ? q0[i] : q0[i + RS / 4], k0 = up2 ? q0[i + RS / 4] : q0[i];
+    const float s1 = up2 ? q1[i] : q1[i + RS / 4], k1 = up2 ? q1[i + RS / 4] : q1[i];
+    const int site = RS / 2 * (c & 1) + RS / 4 * (c >> 1) + i;
+    const float v0 = __fadd_rn(k0, __shfl_xor_sync(0xffffffffu, s0, 2));
+    const float v1 = __fadd_rn(k1, __shfl_xor_sync(0xffffffffu, s1, 2));
+    *reinterpret_cast<float2*>(&S.part[tid >> 2][2 * site]) = make_float2(v0, v1);
+  }
+  __syncthreads();
+  if (tid < 2 * RS) {
+    float v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      v[i] = __fadd_rn(__fadd_rn(S.part[i][tid], S.part[i + 16][tid]),
+                       __fadd_rn(S.part[i + 8][tid], S.part[i + 24][tid]));
+#pragma unroll
+    for (int h = 4; h > 0; h >>= 1)
+#pragma unroll
+      for (int i = 0; i < h; ++i) v[i] = __fadd_rn(v[i], v[i + h]);
+    // prob_hid of the two alleles; k_impute_finish turns them into HP
+    const int i = tid >> 1;
+    if (i < n) A.hp[(size_t)t * 2 * A.L + 2 * A.poly[(size_t)t * A.L + l0 + i] + (tid & 1)] = v[0];
+  }
 }
 
 }  // namespace
 
-size_t impute_warp_smem(int J, int cpc) { return (size_t)kWarpsPerChain * cpc * warp_smem_bytes(J); }
+// Rows of 128 states for K states (the J of launch_impute_chain).
+int impute_groups(int K) { return std::max(1, (K + 127) / 128); }
 
-// Local quads per warp for at most Kmax states (the J of launch_impute_warp).
-int impute_groups(int Kmax) {
-  const int W = kWarpsPerChain;
-  return std::max(1, ((Kmax + 127) / 128 + W - 1) / W);
-}
-
-// Row stride of the store in padded coordinates for at most Kmax states.
-int impute_store_stride(int Kmax) { return 128 * kWarpsPerChain * impute_groups(Kmax); }
-
-template <int J, bool POST>
-static int launch_chains(const ChainArgs& a, int cpc, cudaStream_t s) {
-  constexpr int W = kWarpsPerChain;
-  if (cpc < 1 || cpc > kMaxChainsPerCta) return GP_E_ARG;
-  const size_t sm = impute_warp_smem(J, cpc);
-  if (sm > 200 * 1024) return GP_E_ARG;
-  if (set_smem_limit_once<k_impute_warp<J, W, POST>>(200 * 1024) != cudaSuccess)
-    return GP_E_CUDA;
-  const dim3 g((a.nchains + cpc - 1) / cpc);
-  k_impute_warp<J, W, POST><<<g, 32 * W * cpc, sm, s>>>(a);
-  return GP_OK;
-}
-
-int launch_impute_warp(int phase, int J, const ModelConst& mc, ImputeWork& w, float* hp, cudaStream_t s, int first,
-                       int count, int cpc) {
-  ChainArgs a;
-  a.sc.asum = w.split_scr.as<float>();
-  a.sc.bsum = a.sc.asum + w.n;
-  a.sc.brow = a.sc.asum + ((2 * w.n + 3) & ~3);  // 16-byte aligned rows of Ks floats
-  a.sc.split = w.split.as<int32_t>();
+static int chain_args(ImputeWork& w, float* hp, int first, int count, ChainArgs& a) {
   if (count < 0) count = w.n;
   if (first < 0 || first + count > w.n || (first > 0 && !w.order.ptr)) return GP_E_ARG;
-  if (count == 0) return GP_OK;
-  a.nchains = 2 * count;
+  a.count = count;
   a.poly = w.poly.as<int32_t>();
   a.npoly = w.npoly.as<int32_t>();
   a.nstates = w.nstates.as<int32_t>();
@@ -504,23 +429,43 @@ int launch_impute_warp(int phase, int J, const ModelConst& mc, ImputeWork& w, fl
   a.em = w.em.as<float4>();
   a.tr = w.tr.as<float2>();
   a.fl = w.fl.as<uint8_t>();
-  a.store_off = w.alpha_off.as<int64_t>();
-  a.store_pool = w.alpha.as<float>();
+  a.row_off = w.row_off.as<int64_t>();
+  a.rows = w.rows.as<float>();
+  a.fac = w.fac.as<float>();
+  a.n = w.n;
   a.L = w.L;
   a.WB = w.WB;
   a.Kp = w.Kp;
-  a.Ks = w.Ks;
-  a.mc = mc;
   a.hp = hp;
   a.order = w.order.ptr ? w.order.as<int32_t>() + first : nullptr;
-#define GP_WARP(JJ) \
-  case JJ: return phase == 2 ? launch_chains<JJ, true>(a, cpc, s) : launch_chains<JJ, false>(a, cpc, s);
+  return GP_OK;
+}
+
+int launch_impute_chain(int J, ImputeWork& w, cudaStream_t s, int first, int count, int cpc) {
+  ChainArgs a;
+  if (chain_args(w, nullptr, first, count, a) != GP_OK || cpc < 1 || cpc > kMaxChainsPerCta) return GP_E_ARG;
+  if (a.count == 0) return GP_OK;
+  const int g = (2 * a.count + cpc - 1) / cpc, threads = kChainThreads * cpc;
+#define GP_CHAIN(JJ)                                           \
+  case JJ:                                                     \
+    if (cpc == 1) k_impute_chain<JJ, true><<<g, threads, 0, s>>>(a);  \
+    else k_impute_chain<JJ, false><<<g, threads, 0, s>>>(a);   \
+    return GP_OK;
   switch (J) {
-    GP_WARP(1) GP_WARP(2) GP_WARP(3) GP_WARP(4) GP_WARP(5) GP_WARP(6) GP_WARP(7) GP_WARP(8)
-    GP_WARP(9) GP_WARP(10) GP_WARP(11) GP_WARP(12) GP_WARP(13) GP_WARP(14) GP_WARP(15) GP_WARP(16)
+    GP_CHAIN(1) GP_CHAIN(2) GP_CHAIN(3) GP_CHAIN(4) GP_CHAIN(5) GP_CHAIN(6) GP_CHAIN(7) GP_CHAIN(8)
+    GP_CHAIN(9) GP_CHAIN(10) GP_CHAIN(11) GP_CHAIN(12) GP_CHAIN(13) GP_CHAIN(14) GP_CHAIN(15) GP_CHAIN(16)
     default: return GP_E_ARG;
   }
-#undef GP_WARP
+#undef GP_CHAIN
+}
+
+int launch_impute_block(int max_poly, ImputeWork& w, float* hp, cudaStream_t s, int first, int count) {
+  ChainArgs a;
+  if (chain_args(w, hp, first, count, a) != GP_OK) return GP_E_ARG;
+  const int blocks = (max_poly + kRowSites - 1) / kRowSites;
+  if (a.count == 0 || blocks == 0) return GP_OK;
+  k_impute_block<<<dim3(blocks, a.count), kBlockThreads, 0, s>>>(a);
+  return GP_OK;
 }
 
 }  // namespace gp

@@ -91,3 +91,46 @@ def test_chunked_store_matches_single_launch(small_workload, monkeypatch):
         assert np.array_equal(whole, chunked)
     finally:
         ctx.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sites", [1, 2, 15, 16, 17, 31, 32, 33, 48, 64, 65, 200])
+def test_block_and_state_count_edges_match_fp64(sites):
+    """The chains keep a row every 16 sites of 32-site blocks and the block kernel
+    takes rows of 128 states in pairs: site counts around the block boundaries and
+    state counts around the row boundaries, odd and even numbers of rows in one
+    batch, against the FP64 restatement; chains per CTA 1, 2 and 4 give the same
+    bits."""
+    from oracle import oracle as O
+    from glimpse_b200 import native, synth
+    w = synth.make_panel_and_targets(2050, 260, 0.2, 0.0, 2, ("uniform", 0.4, 2.0), ("fixed", 200), seed=67,
+                                     sparse_maf=0.005)
+    P, T = w.panel, w.targets
+    keep = slice(0, sites)
+    import dataclasses
+    P = dataclasses.replace(P, n_sites=sites, bp=P.bp[keep], cm=P.cm[keep], cref=P.cref[keep], calt=P.calt[keep],
+                            lq=P.lq[keep], flag_common=P.flag_common[keep], major=P.major[keep],
+                            hvar=np.ascontiguousarray(P.hvar[keep]))
+    rng = np.random.default_rng(sites)
+    states, hls, flats = [], [], []
+    for i, K in enumerate((1, 2, 3, 127, 128, 129, 255, 256, 257, 384, 640, 1023, 1025, 1920, 2047, 2048)):
+        t = i % T.n
+        flat = T.flat[t][keep].copy()
+        if i % 4 == 3:
+            flat[[0, -1]] = 1  # AlphaSum and betaSum of 1 at flat end sites
+        states.append(_random_states(rng, P.n_ref_haps, K))
+        hls.append(init_hl(T.gl[t][keep], flat))
+        flats.append(flat)
+    ctx = native.Context(P)
+    try:
+        got = []
+        for cpc in (1, 2, 4):
+            ctx.tuning_set(cpc, 0, 0)
+            got.append(ctx.impute_batch(states, np.stack(hls), np.stack(flats)))
+        assert np.array_equal(got[0], got[1]) and np.array_equal(got[0], got[2])
+        for i in range(len(states)):
+            ref, _ = O.restate_impute(P, states[i], hls[i], flats[i], precision=64)
+            err = float(np.abs(got[0][i] - ref).max())
+            assert err <= TOL, f"K={states[i].size}: max |dHP| = {err:.3e}"
+    finally:
+        ctx.close()
