@@ -5,7 +5,7 @@
 // state union of conditioning_set::compactSelection (conditioning_set.cpp:96-104).
 //
 // Given the panel-side prefix/rank arrays (decoded once), every target haplotype's
-// sweep over the sites depends only on its own alleles, so one thread runs one
+// sweep over the sites depends only on its own alleles, so a group of lanes runs one
 // haplotype. Each selectK push is recorded with the key (site << 1 | phase) so
 // that the union can rebuild the per-sample, per-level lists in the reference's
 // push order (sites in order, init_common before select_common, haplotypes in
@@ -13,15 +13,20 @@
 #include <algorithm>
 
 #include "select.h"
+#include "tc.h"
 
 namespace gp {
 
 namespace {
 
+// Ones before position x: bits and prefix counts in arrays of their own (small
+// columns), or as pairs {bits, prefix count} (rank rows).
 __device__ __forceinline__ int rank_v(const uint32_t* __restrict__ bits, const uint32_t* __restrict__ pref, int x) {
-  const uint32_t w = bits[x >> 5];
-  const uint32_t m = (x & 31) ? (w & ((1u << (x & 31)) - 1u)) : 0u;
-  return (int)(pref[x >> 5] + __popc(m));
+  return (int)(pref[x >> 5] + __popc(bits[x >> 5] & ((1u << (x & 31)) - 1u)));
+}
+__device__ __forceinline__ int rank_row(const uint2* row, int x) {
+  const uint2 v = row[x >> 5];
+  return (int)v.y + __popc(v.x & ~__funnelshift_l(0u, ~0u, x));  // ~0 << (x & 31)
 }
 
 // number of entries of the sorted array a[0..n) that are < x (std::lower_bound distance)
@@ -34,49 +39,47 @@ __device__ __forceinline__ int lower_count(const int32_t* __restrict__ a, int n,
   return lo;
 }
 
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(smem))),
-               "l"(gmem));
-}
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-__device__ __forceinline__ void cp_wait_all_but(int n) {
-  // wait until at most n of this thread's cp.async groups are pending (n < 8)
-  switch (n) {
-    case 0: asm volatile("cp.async.wait_group 0;\n" ::); break;
-    case 1: asm volatile("cp.async.wait_group 1;\n" ::); break;
-    case 2: asm volatile("cp.async.wait_group 2;\n" ::); break;
-    case 3: asm volatile("cp.async.wait_group 3;\n" ::); break;
-    case 4: asm volatile("cp.async.wait_group 4;\n" ::); break;
-    case 5: asm volatile("cp.async.wait_group 5;\n" ::); break;
-    case 6: asm volatile("cp.async.wait_group 6;\n" ::); break;
-    default: asm volatile("cp.async.wait_group 7;\n" ::); break;
-  }
+// One bulk copy (TMA) of n bytes, a multiple of 16, global to shared memory, both
+// 16-byte aligned; completes on the mbarrier.
+__device__ __forceinline__ void bulk_load(void* smem, const void* gmem, uint32_t n, uint64_t* bar) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tc::smem_u32(bar)), "r"(n) : "memory");
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                   tc::smem_u32(smem)),
+               "l"(gmem), "r"(n), "r"(tc::smem_u32(bar))
+               : "memory");
 }
 
-// Warp-cooperative copy of one vrow row (R words, R a multiple of 4, 16-byte
-// aligned) into a ring slot, spread over the live lanes of the warp.
-__device__ __forceinline__ void stage_row(uint32_t* slot, const uint32_t* row, int R, int rank, int nlive) {
-  for (int c = rank; c < (R >> 2); c += nlive) cp_async16(slot + 4 * c, row + 4 * c);
-}
-
-// Per-level push lists of one target haplotype. The counts live in shared
-// memory (level-major, one column per lane) while the sweep runs and are
-// written back to push_cnt at its end.
+// Per-level push lists of one target haplotype, run by the G lanes of its group:
+// lane gl owns the levels gl, gl + G, ... The counts live in shared memory while
+// the sweep runs and are written back to push_cnt at its end. A lane's pushes to
+// its first level wait in registers until the next call, so that the loads of the
+// ids are not waited for.
+template <int G>
 struct Pusher {
   uint32_t* key;
   uint32_t* id;
-  int32_t* cnt;  // shared: cnt[level * 32]
+  int32_t* cnt;  // shared: cnt[level]
   int cap;
   int32_t* overflow;
+  int gl;
+  uint32_t pend_key;
+  uint32_t pend_id0, pend_id1;
+  int npend;  // pending pushes of level gl
+
   __device__ __forceinline__ void push(int level, uint32_t k, uint32_t h) {
-    const int c = cnt[level * 32];
+    const int c = cnt[level];
     if (c >= cap) {
       *overflow = 1;
       return;
     }
     key[(size_t)level * cap + c] = k;
     id[(size_t)level * cap + c] = h;
-    cnt[level * 32] = c + 1;
+    cnt[level] = c + 1;
+  }
+  __device__ __forceinline__ void flush() {
+    if (npend > 0) push(gl, pend_key, pend_id0);
+    if (npend > 1) push(gl, pend_key, pend_id1);
+    npend = 0;
   }
 };
 
@@ -85,9 +88,10 @@ struct Pusher {
 // (pbwt_idx - 1, ...) one level at a time and stops a side at its first position
 // outside [0, N) or on the other side of ref_rac than allele a; positions on the
 // allowed side of ref_rac form an interval, so each side pushes a run whose
-// length is known up front, and the loads of the run are independent.
-__device__ void select_k(int pbwt_idx, int f, int g, int ref_rac, const uint32_t* __restrict__ arr, int a, int K,
-                         int N, uint32_t key, Pusher& P) {
+// length is known up front, level o from the group's lane o % G (down before up).
+template <int G>
+__device__ __forceinline__ void select_k(int pbwt_idx, int f, int g, int ref_rac, const uint32_t* __restrict__ arr, int a,
+                                      int K, int N, uint32_t key, Pusher<G>& P) {
   int nh_up = 0, nh_down = 0;
   const int d_up = pbwt_idx - f;
   const int d_down = g - pbwt_idx;
@@ -114,11 +118,21 @@ __device__ void select_k(int pbwt_idx, int f, int g, int ref_rac, const uint32_t
     const int lo = alt ? max(ref_rac, 0) : 0;
     cu = min(nh_up, p - lo + 1);
   }
-  const int n = max(cd, cu);
-#pragma unroll 4
-  for (int o = 0; o < n; ++o) {
-    if (o < cd) P.push(o, key, arr ? arr[pbwt_idx + o] : (uint32_t)(pbwt_idx + o));
-    if (o < cu) P.push(o, key, arr ? arr[p - o] : (uint32_t)(p - o));
+  P.flush();
+  int o = P.gl;
+  if (o < max(cd, cu)) {
+    P.pend_key = key;
+    const bool down = o < cd, up = o < cu;
+    const int i0 = down ? pbwt_idx + o : p - o;
+    P.pend_id0 = arr ? arr[i0] : (uint32_t)i0;
+    if (down && up) P.pend_id1 = arr ? arr[p - o] : (uint32_t)(p - o);
+    P.npend = (int)down + (int)up;
+  }
+  for (o += G; o < max(cd, cu); o += G) {
+    const uint32_t hd = o < cd ? (arr ? arr[pbwt_idx + o] : (uint32_t)(pbwt_idx + o)) : 0u;
+    const uint32_t hu = o < cu ? (arr ? arr[p - o] : (uint32_t)(p - o)) : 0u;
+    if (o < cd) P.push(o, key, hd);
+    if (o < cu) P.push(o, key, hu);
   }
 }
 
@@ -198,183 +212,209 @@ __global__ void k_event_bits(PbwtSelectArgs a) {
   }
 }
 
-// Haplotypes per sweep warp (hpw, a power of two, chosen by the autotuner).
-// Lane l runs haplotype l % hpw of its warp's group: lanes l, l + hpw, ... run
-// the same haplotype, take the same branches and write the same values to the
-// same addresses, so a warp diverges only over hpw haplotypes while all 32
-// lanes share the row staging.
+// The sweep: one warp per HPW target haplotypes (1, 2, 4 or 8, chosen by the
+// autotuner), G = 32 / HPW lanes per haplotype. A haplotype's chain over the events
+// (non-LQ common sites and runs of rare sites, in site order) is bound by the
+// latency of its dependent integer instructions: each event's interval depends on
+// the previous one's. All lanes of a group run the chain (the three rank lookups
+// of an event are independent of one another); the levels of a selectK are spread
+// over the group's lanes, and their loads are not waited for.
 //
-// One warp per block; lane l runs target haplotype blockIdx.x * hpw + l % hpw
-// (measured at 256 targets: 39 ms per sweep with 32 haplotypes per warp, 33 ms
-// with 2, as a warp runs every branch any of its haplotypes takes).
-// The lanes of a warp walk the event list (non-LQ common sites and runs of rare sites) in step: every branch
-// that skips work is warp-uniform. Shared memory per warp holds
-//   ring    D slots, one per HQ common site l, filled by cp.async D common sites
-//           ahead with the rank row of l (R words: the V ranks of
-//           select_common_pd_fg and the small-PBWT position ranks of init_common);
+// The haplotypes of a warp walk the event list in step; what only some of them do
+// (an empty interval, a stored site, a carried rare run) branches per group.
+// Shared memory per warp holds
+//   ring    kRankStages stages of rows_per consecutive rank rows, one bulk copy
+//           each, kRankStages - 1 stages ahead (row l: pairs {bits, prefix count} of
+//           the V ranks of select_common_pd_fg, then of the small-PBWT position
+//           ranks of init_common), and an mbarrier per stage;
 //   evbuf   two chunks of 32 event records (the next chunk is loaded one chunk ahead);
-//   scnt    the per-level push counts, one column per lane.
-// D = 0 reads the rows from global memory (panels whose rows do not fit in
-// shared memory).
-__global__ void __launch_bounds__(32) k_pbwt_sweep(PbwtSelectArgs a, int D, int hpw) {
-  extern __shared__ __align__(16) uint32_t smem[];
-  const int lane = threadIdx.x & 31;
-  const int hp = blockIdx.x * hpw + (lane & (hpw - 1));
-  const unsigned live = __ballot_sync(0xffffffffu, hp < a.n_haps);
-  if (hp >= a.n_haps) return;
-  const int rank = __popc(live & ((1u << lane) - 1u)), nlive = __popc(live);
-  const DevPbwt& P = a.P;
-  const int R = P.R, Wv = P.Wv, ncom = P.n_com_hq, nev = P.n_events;
-  const int N = a.N, K = a.depth;
-  uint32_t* ring = smem;
-  int4* evbuf = reinterpret_cast<int4*>(smem + (size_t)D * R);  // [2][32][2]
-  int32_t* scnt = reinterpret_cast<int32_t*>(evbuf + 2 * 32 * 2) + lane;  // [K][32]
+//   scnt    the per-level push counts of each haplotype.
+// Without RING the rows are read from global memory (panels whose rows do not fit
+// in shared memory). Waits are bounded; a time-out sets the overflow flag to 2.
+// Measured per sweep: 20,000 events, 1,000 haplotypes, one target 11.0 -> 4.1 ms;
+// 54,000 events, 10,000 haplotypes, 256 targets 25.8 -> 10.6 ms (2 per warp; 18.3, 11.2
+// and 12.2 ms for 1, 4 and 8, as every warp reads all rank rows once). Before, the rows
+// came by one 16-byte copy per lane and 512 bytes, addresses and shapes were run-time
+// values, and a selectK waited for its ids.
+constexpr int kRankStages = 3;
 
-  if (D > 0) {
-    for (int j = 0; j < D; ++j) {
-      if (j < ncom) stage_row(ring + (size_t)j * R, P.vrow + (size_t)j * R, R, rank, nlive);
-      cp_commit();
-    }
+template <int HPW, bool RING>
+__global__ void __launch_bounds__(32, 1) k_pbwt_sweep(PbwtSelectArgs a, int rows_per) {
+  constexpr int G = 32 / HPW;
+  extern __shared__ __align__(16) uint32_t smem[];
+  __shared__ uint64_t bars[kRankStages];
+  const int lane = threadIdx.x & 31;
+  const int grp = lane / G, gl = lane % G;
+  const bool act = blockIdx.x * HPW + grp < a.n_haps;  // idle groups repeat the last haplotype and record nothing
+  const int hp = min((int)(blockIdx.x * HPW + grp), a.n_haps - 1);
+  const DevPbwt& P = a.P;
+  const int R = P.R, ncom = P.n_com_hq, nev = P.n_events;
+  const int N = a.N, K = a.depth;
+  const int stage_words = RING ? rows_per * R : 0;
+  uint32_t* ring = smem;
+  int4* evbuf = reinterpret_cast<int4*>(smem + kRankStages * stage_words);  // [2][32][2]
+  int32_t* scnt = reinterpret_cast<int32_t*>(evbuf + 2 * 32 * 2) + grp * K;  // [HPW][K]
+
+  // stage st takes the rows [rows_per * g, rows_per * (g + 1)) of group g = st modulo kRankStages
+  auto load_rows = [&](int first, int st) {
+    if (first < ncom)
+      bulk_load(ring + st * stage_words, P.vrow + (size_t)first * R, (uint32_t)(min(rows_per, ncom - first) * R * 4),
+                &bars[st]);
+  };
+  if (RING && lane == 0) {
+    for (int st = 0; st < kRankStages; ++st) tc::mbar_init(&bars[st], 1);
+    tc::fence_mbar_init();
+    for (int st = 0; st < kRankStages; ++st) load_rows(st * rows_per, st);
   }
-  int ri = 0;  // ring slot of the next HQ common site
-  // Event chunk c (32 records) goes to evbuf[c & 1], spread over the live lanes
-  // (the last warp of the grid may have fewer than 32); chunk c + 1 is loaded
-  // when chunk c starts.
+  // Event chunk c (32 records) goes to evbuf[c & 1]; chunk c + 1 is loaded when chunk c starts.
   auto load_chunk = [&](int c) {
-    for (int i = rank; i < 32; i += nlive) {
-      const int en = (c << 5) + i;
-      if (en < nev) {
-        evbuf[((c & 1) * 32 + i) * 2] = P.events[2 * en];
-        evbuf[((c & 1) * 32 + i) * 2 + 1] = P.events[2 * en + 1];
-      }
+    const int en = (c << 5) + lane;
+    if (en < nev) {
+      evbuf[((c & 1) * 32 + lane) * 2] = P.events[2 * en];
+      evbuf[((c & 1) * 32 + lane) * 2 + 1] = P.events[2 * en + 1];
     }
   };
   load_chunk(0);
   load_chunk(1);
-  __syncwarp(live);
 
-  const int L = a.L;
   const int t = a.hap_target[hp];
-  const uint8_t* H = (a.hap_which[hp] ? a.h1 : a.h0) + (size_t)t * L;
+  const uint8_t* H = (a.hap_which[hp] ? a.h1 : a.h0) + (size_t)t * a.L;
   // event bits of the current chunk and of the next one
   const uint32_t* eb = a.ebits + (size_t)hp * a.We;
   uint32_t ebw = a.We > 0 ? eb[0] : 0u;
   uint32_t ebn = a.We > 1 ? eb[1] : 0u;
-  Pusher pu{a.push_key + (size_t)hp * K * a.cap, a.push_id + (size_t)hp * K * a.cap, scnt, a.cap, a.overflow};
-  for (int o = 0; o < K; ++o) scnt[o * 32] = 0;
+  // stored sites l & ~31 .. and the next 32
+  uint32_t sbw = 0u, sbn = a.stored_bits[0];
+  Pusher<G> pu;
+  pu.key = a.push_key + (size_t)hp * K * a.cap;
+  pu.id = a.push_id + (size_t)hp * K * a.cap;
+  pu.cnt = scnt;
+  pu.cap = a.cap;
+  pu.overflow = a.overflow;
+  pu.gl = gl;
+  pu.pend_key = pu.pend_id0 = pu.pend_id1 = 0u;
+  pu.npend = 0;
+  for (int o = gl; o < K; o += G) scnt[o] = 0;
   int idx = a.start_idx[hp], f = 0, g = N;
-  int sidx = 0, fs = 0, gs = 0;
+  int sidx = 0, fs = 0, gs = 0;  // the same in the run's small PBWT
   int last_reset = 0, last_rare = 0;
   int tar = a.tar_hap[hp];
   bool in_rare = false;
   int prev_ref_com = 0;
   const float half_mod = a.modulo / 2.0f;
   const float fifth_mod = a.modulo / 5.0f;
+  const int half = R >> 1;
+  const uint32_t* row = RING ? smem : P.vrow;  // rank row of the next HQ common site
+  int in_stage = rows_per - 1;                // its place in its stage
+  int stage = kRankStages - 1;                // its stage, and the parity to wait for
+  uint32_t parity = 1u;
+  int next_rows = (kRankStages - 1) * rows_per;  // first row of the stage to request next
+  bool failed = false;
+  __syncwarp();
+  int4 r0 = evbuf[0], r1 = evbuf[1];
 
+#pragma unroll 2
   for (int e = 0; e < nev; ++e) {
-    const int c = e >> 5;
     if ((e & 31) == 0 && e > 0) {
-      __syncwarp(live);  // chunk c - 1 is no longer read
-      load_chunk(c + 1);
+      const int c = e >> 5;
+      load_chunk(c + 1);  // chunk c - 1 is no longer read: its last record was read before the last __syncwarp
       ebw = ebn;
       ebn = c + 1 < a.We ? eb[c + 1] : 0u;
     }
     const bool ebit = (ebw >> (e & 31)) & 1u;
-    const int4 r0 = evbuf[((c & 1) * 32 + (e & 31)) * 2];
-    const int4 r1 = evbuf[((c & 1) * 32 + (e & 31)) * 2 + 1];
-    const int sn = r1.x;
-    if (!(r0.x & (1 << 30))) {
+    const int4 q0 = r0, q1 = r1;
+    __syncwarp();
+    {
+      const int4* nx = evbuf + (((e + 1) & 63) * 2);  // the record after the last one is read and not used
+      r0 = nx[0];
+      r1 = nx[1];
+    }
+    if (!(q0.x & (1 << 30))) {
       // ---------------- HQ common site ----------------
-      const int k = r0.x, l = r0.y, ref = r0.z;
-      const uint32_t* a_pre = l > 0 ? P.a_after + (size_t)(l - 1) * N : nullptr;
-      // rank row of l: the ring slot, or global memory without a ring
-      const uint32_t* row = P.vrow + (size_t)l * R;
-      uint32_t* slot = nullptr;
-      if (D > 0) {
-        slot = ring + (size_t)ri * R;
-        row = slot;
-        cp_wait_all_but(D - 1);  // this lane's part of slot l has landed
-        __syncwarp(live);        // and every other lane's
+      const int k = q0.x, l = q0.y, ref = q0.z;
+      if (RING && ++in_stage == rows_per) {
+        // The stage before is free: every lane is past its last row (the __syncwarp above).
+        if (lane == 0 && l > 0) load_rows(next_rows, stage);
+        next_rows += rows_per;
+        in_stage = 0;
+        if (++stage == kRankStages) {
+          stage = 0;
+          parity ^= 1u;
+        }
+        if (!tc::mbar_wait(&bars[stage], parity)) {
+          failed = true;
+          break;
+        }
+        row = smem + stage * stage_words;
       }
-      if (r1.z) {  // init_common
+      if (q1.z) {  // init_common
+        const int sn = q1.x;
+        const uint2* srow = reinterpret_cast<const uint2*>(row + half);
         int nidx, nf, ng;
         if (in_rare) {
           nidx = N - sn + sidx;
           nf = last_reset >= last_rare ? 0 : N - sn + fs;
           ng = N - sn + gs;
-          if (ng <= nf) {
-            select_k(idx, f, g, prev_ref_com, a_pre, tar, K, N, (uint32_t)(k << 1), pu);
-            nf = 0;
-            ng = N;
-            last_reset = k - 1;
-          }
         } else {
-          // numbers of small-PBWT positions below f, g and idx: ranks in the row's second bit vector
-          const uint32_t* sb = row + 2 * Wv + 1;
-          const int c0 = rank_v(sb, sb + Wv, f), c1 = rank_v(sb, sb + Wv, g), c2 = rank_v(sb, sb + Wv, idx);
-          nidx = idx - c2;
-          nf = f - c0;
-          ng = g - c1;
-          if (ng <= nf) {
-            const int prev_site = r1.w;  // common2tot indexed by the HQ count, as the reference does
-            if (__fsub_rn(P.cm_pos[prev_site], P.cm_pos[last_reset]) > fifth_mod)
-              select_k(idx, f, g, prev_ref_com, a_pre, tar, K, N, (uint32_t)(k << 1), pu);
-            nf = 0;
-            ng = N - sn;
-            last_reset = prev_site;
-          }
+          // numbers of small-PBWT positions below f, g and idx: ranks in the row's second part
+          nidx = idx - rank_row(srow, idx);
+          nf = f - rank_row(srow, f);
+          ng = g - rank_row(srow, g);
+        }
+        if (ng <= nf) {
+          const uint32_t* a_pre = l > 0 ? P.a_after + (size_t)(l - 1) * N : nullptr;
+          const int prev_site = q1.w;  // common2tot indexed by the HQ count, as the reference does
+          if (act && (in_rare || __fsub_rn(P.cm_pos[prev_site], P.cm_pos[last_reset]) > fifth_mod))
+            select_k<G>(idx, f, g, prev_ref_com, a_pre, tar, K, N, (uint32_t)(k << 1), pu);
+          nf = 0;
+          ng = in_rare ? N : N - sn;
+          last_reset = in_rare ? k - 1 : prev_site;
         }
         idx = nidx;
         f = nf;
         g = ng;
       }
       // select_common_pd_fg at HQ common site l
-      const int prev_hap = tar;
+      const uint2* vrow = reinterpret_cast<const uint2*>(row);
+      row += R;
+      const int vi = rank_row(vrow, idx), vf = rank_row(vrow, f), vg = rank_row(vrow, g);
       const int al = ebit ? 1 : 0;  // H[k]
-      tar = al;
-      const int vi = rank_v(row, row + Wv, idx), vf = rank_v(row, row + Wv, f), vg = rank_v(row, row + Wv, g);
-      if (D > 0) {
-        __syncwarp(live);  // the slot is free again
-        if (l + D < ncom) stage_row(slot, P.vrow + (size_t)(l + D) * R, R, rank, nlive);
-        cp_commit();
-        ri = (ri + 1 == D) ? 0 : ri + 1;
+      if ((l & 31) == 0) {
+        sbw = sbn;
+        if (l + 32 < ncom) sbn = a.stored_bits[(l >> 5) + 1];
       }
-      int nidx = al ? ref + vi : idx - vi;
+      const bool stored = (sbw >> (l & 31)) & 1u;
+      const int nidx = al ? ref + vi : idx - vi;
       int nf = al ? ref + vf : f - vf;
       int ng = al ? ref + vg : g - vg;
-      const bool stored = (a.stored_bits[l >> 5] >> (l & 31)) & 1u;
-      bool reset = false;
-      if (ng <= nf) {
-        const int km1 = k > 0 ? k - 1 : 0;
-        if (stored || __fsub_rn(P.cm_pos[km1], P.cm_pos[last_reset]) > half_mod) {
-          const int bid = r1.y;
-          const uint32_t* b_arr = bid >= 0 ? P.merged + (size_t)bid * N : (bid == -1 ? a_pre : nullptr);
-          select_k(idx, f, g, prev_ref_com, b_arr, prev_hap, K, N, (uint32_t)((k << 1) | 1), pu);
+      if (ng <= nf || stored) {
+        if (ng <= nf) {
+          const int km1 = k > 0 ? k - 1 : 0;
+          if (act && (stored || __fsub_rn(P.cm_pos[km1], P.cm_pos[last_reset]) > half_mod)) {
+            const int bid = q1.y;
+            const uint32_t* a_pre = l > 0 ? P.a_after + (size_t)(l - 1) * N : nullptr;
+            const uint32_t* b_arr = bid >= 0 ? P.merged + (size_t)bid * N : (bid == -1 ? a_pre : nullptr);
+            select_k<G>(idx, f, g, prev_ref_com, b_arr, tar, K, N, (uint32_t)((k << 1) | 1), pu);
+          }
+        } else if (act) {
+          select_k<G>(nidx, nf, ng, ref, P.a_after + (size_t)l * N, al, K, N, (uint32_t)((k << 1) | 1), pu);
         }
         nf = al * ref;
         ng = al * N + (1 - al) * ref;
         last_reset = k;
-        reset = true;
       }
       idx = nidx;
       f = nf;
       g = ng;
-      if (!reset && stored) {
-        select_k(idx, f, g, ref, P.a_after + (size_t)l * N, al, K, N, (uint32_t)((k << 1) | 1), pu);
-        f = al * ref;
-        g = al * N + (1 - al) * ref;
-        last_reset = k;
-      }
+      tar = al;
       prev_ref_com = ref;
     } else {
       // ---------------- run of rare sites [k0, kend] ----------------
-      const int k0 = r0.x & ~(1 << 30), kend = r0.z, so = r0.w;
       // init_rare: is this haplotype in rareTarHaps for the run?
       in_rare = ebit;  // sn > 0 and a carrier bit in [k0, kend]
-      // Nothing happens at the run's sites for a haplotype outside rareTarHaps;
-      // when no haplotype of the warp is in it, the warp goes on to the next event.
-      if (__all_sync(live, !in_rare)) continue;
+      // Nothing happens at the run's sites for a haplotype outside rareTarHaps.
       if (in_rare) {
+        const int k0 = q0.x & ~(1 << 30), kend = q0.z, so = q0.w, sn = q1.x;
         const int32_t* sm = P.asidx + so;
         int fsn = lower_count(sm, sn, f);
         int gsn = lower_count(sm, sn, g);
@@ -386,46 +426,38 @@ __global__ void __launch_bounds__(32) k_pbwt_sweep(PbwtSelectArgs a, int D, int 
         sidx = lower_count(sm, sn, idx);
         fs = fsn;
         gs = gsn;
-      }
-      for (int k = k0; k <= kend; ++k) {
-        const int info = P.site_info[k];
-        if ((info & 3) == SK_LQ) continue;
-        if (!in_rare) continue;
-        const int r = info >> 2;
-        const int ref = a.major[k] ? (int)P.cref[k] : sn - (int)a.calt[k];
-        const uint32_t* vb = P.svbits + P.svoff[r];
-        const uint32_t* vp = P.svpref + (P.svoff[r] + r);
-        const int vi = rank_v(vb, vp, sidx), vf = rank_v(vb, vp, fs), vg = rank_v(vb, vp, gs);
-        int ns, nfs, ngs;
-        if (H[k] != a.major[k]) {
-          last_rare = k;
-          ns = ref + vi;
-          nfs = ref + vf;
-          ngs = ref + vg;
-          if (ngs <= nfs) {
-            nfs = ref;
-            ngs = sn;
-            last_reset = k;
-          }
-        } else {
-          ns = sidx - vi;
-          nfs = fs - vf;
-          ngs = gs - vg;
-          if (ngs <= nfs) {
-            nfs = 0;
-            ngs = ref;
+        for (int k = k0; k <= kend; ++k) {
+          const int info = P.site_info[k];
+          if ((info & 3) == SK_LQ) continue;
+          const int r = info >> 2;
+          const int ref = a.major[k] ? (int)P.cref[k] : sn - (int)a.calt[k];
+          const uint32_t* vb = P.svbits + P.svoff[r];
+          const uint32_t* vp = P.svpref + (P.svoff[r] + r);
+          const int vi = rank_v(vb, vp, sidx), vf = rank_v(vb, vp, fs), vg = rank_v(vb, vp, gs);
+          const bool car = H[k] != a.major[k];
+          if (car) last_rare = k;
+          sidx = car ? ref + vi : sidx - vi;
+          fs = car ? ref + vf : fs - vf;
+          gs = car ? ref + vg : gs - vg;
+          if (gs <= fs) {
+            fs = car ? ref : 0;
+            gs = car ? sn : ref;
             last_reset = k;
           }
         }
-        sidx = ns;
-        fs = nfs;
-        gs = ngs;
       }
     }
   }
-  if (D > 0) cp_wait_all_but(0);
-  for (int o = 0; o < K; ++o) a.push_cnt[(size_t)hp * K + o] = scnt[o * 32];
-  a.tar_hap[hp] = (uint8_t)tar;
+  if (failed) {
+    // the other stages' copies may still be under way: wait for each, bounded as well, before the memory is given up
+    if (lane == 0) *a.overflow = 2;
+    for (int st = 0; st < kRankStages; ++st) tc::mbar_wait(&bars[st], st <= stage ? parity : parity ^ 1u);
+    return;
+  }
+  if (!act) return;
+  pu.flush();
+  for (int o = gl; o < K; o += G) a.push_cnt[(size_t)hp * K + o] = scnt[o];
+  if (gl == 0) a.tar_hap[hp] = (uint8_t)tar;
 }
 
 // conditioning_set::compactSelection union (conditioning_set.cpp:96-104): levels
@@ -479,19 +511,27 @@ __global__ void k_pbwt_union(PbwtSelectArgs a) {
 
 }  // namespace
 
-static size_t sweep_smem(const PbwtSelectArgs& a, int& D) {
-  // Ring of D rank rows, D <= 8, within 96 KB.
-  const size_t slot_bytes = (size_t)a.P.R * 4;
-  D = (int)std::min<size_t>(8, (96u << 10) / slot_bytes);
-  if (D < 2) D = 0;
-  return (size_t)D * slot_bytes + 2 * 32 * 2 * 16 + (size_t)a.depth * 32 * 4;
+template <int HPW>
+static void launch_sweep(const PbwtSelectArgs& a, cudaStream_t s) {
+  // Stages of 4, 2 or 1 rank rows, within 96 KB.
+  const size_t row_bytes = (size_t)a.P.R * 4, fixed = 2 * 32 * 2 * 16 + (size_t)a.depth * HPW * 4;
+  int rows = 4;
+  while (rows > 0 && kRankStages * rows * row_bytes > (96u << 10)) rows >>= 1;
+  const int grid = (a.n_haps + HPW - 1) / HPW;
+  if (rows > 0) {
+    const size_t smem = kRankStages * rows * row_bytes + fixed;
+    if (smem > (48u << 10)) set_smem_limit_once<k_pbwt_sweep<HPW, true>>(200 << 10);
+    k_pbwt_sweep<HPW, true><<<grid, 32, smem, s>>>(a, rows);
+  } else {
+    k_pbwt_sweep<HPW, false><<<grid, 32, fixed, s>>>(a, 1);
+  }
 }
 
 void launch_pbwt_sweep(const PbwtSelectArgs& a, int hpw, cudaStream_t s) {
-  int D = 0;
-  const size_t smem = sweep_smem(a, D);
-  if (smem > (48u << 10)) set_smem_limit_once<k_pbwt_sweep>(200 << 10);
-  k_pbwt_sweep<<<(a.n_haps + hpw - 1) / hpw, 32, smem, s>>>(a, D, hpw);
+  if (hpw == 1) launch_sweep<1>(a, s);
+  else if (hpw == 2) launch_sweep<2>(a, s);
+  else if (hpw == 4) launch_sweep<4>(a, s);
+  else launch_sweep<8>(a, s);
 }
 
 void launch_pbwt_select(const PbwtSelectArgs& a, int hpw, cudaStream_t s) {

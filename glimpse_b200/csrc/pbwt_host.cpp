@@ -214,10 +214,10 @@ int Context::pbwt_prepare_panel() {
   const int n_com_hq = host.n_com_hq;
   D.n_com_hq = n_com_hq;
   D.Wv = (N + 1 + 31) / 32;
-  // Row l: V bits and their prefix counts (select_common_pd_fg), then the bits and
-  // prefix counts of the small-PBWT positions merged at l (init_common); 16-byte
-  // rows, staged by the sweep with cp.async.
-  D.R = (4 * D.Wv + 2 + 3) / 4 * 4;
+  // Row l: pairs of V bits and their prefix count (select_common_pd_fg), then the
+  // same of the small-PBWT positions merged at l (init_common); both parts whole
+  // multiples of 16 bytes, staged by the sweep with cp.async.
+  D.R = 2 * ((2 * D.Wv + 3) / 4 * 4);
   const int Wv = D.Wv, R = D.R;
   cudaError_t e;
   if ((e = dev_alloc(&D.a_after, (size_t)n_com_hq * N, owned)) != cudaSuccess) return cuda_fail(e, "alloc pbwt");
@@ -231,7 +231,7 @@ int Context::pbwt_prepare_panel() {
   std::vector<int32_t> site_info(L, 0), site_run(L, 0), run_end(L, -1), common2tot;
   std::vector<uint32_t> A(N), B(N);
   std::iota(A.begin(), A.end(), 0u);
-  std::vector<uint32_t> sA, sB;
+  std::vector<uint32_t> sA, sB, vbits(Wv), vpref(Wv + 1);
   // staged upload of a_after / V rows
   const int chunk = std::max(1, (int)std::min<int64_t>(4096, (512ll << 20) / ((int64_t)N * 4 + 1)));
   std::vector<uint32_t> stage_a((size_t)chunk * N), stage_vr((size_t)chunk * R, 0u);
@@ -301,20 +301,22 @@ int Context::pbwt_prepare_panel() {
         before_id[l_hq] = (l_hq == 0) ? -2 : -1;
       }
       if (stage_n == chunk && (e = flush()) != cudaSuccess) return cuda_fail(e, "pbwt upload");
-      uint32_t* vb = stage_vr.data() + (size_t)stage_n * R;
-      uint32_t* vp = vb + Wv;
-      if (!decode(A, B, N, (int)host.cref[k], vb, vp, Wv))
+      uint32_t* row = stage_vr.data() + (size_t)stage_n * R;
+      std::fill(row, row + R, 0u);
+      if (!decode(A, B, N, (int)host.cref[k], vbits.data(), vpref.data(), Wv))
         return (fail(GP_E_DATA, "sparse PBWT stream is malformed at site " + std::to_string(k)), GP_E_DATA);
       {
-        uint32_t* sb = vb + 2 * Wv + 1;
-        uint32_t* sp = sb + Wv;
-        std::fill(sb, sb + 2 * Wv + 1, 0u);
+        for (int w = 0; w < Wv; ++w) {
+          row[2 * w] = vbits[w];
+          row[2 * w + 1] = vpref[w];
+        }
+        uint32_t* sb = row + R / 2;
         if (initc[l_hq])
           for (int64_t i = 0; i < sn; ++i) {
             const int32_t q = sparse.asmall[so + i];
-            sb[q >> 5] |= 1u << (q & 31);
+            sb[2 * (q >> 5)] |= 1u << (q & 31);
           }
-        for (int w = 0; w < Wv; ++w) sp[w + 1] = sp[w] + (uint32_t)__builtin_popcount(sb[w]);
+        for (int w = 1; w < Wv; ++w) sb[2 * w + 1] = sb[2 * w - 1] + (uint32_t)__builtin_popcount(sb[2 * w - 2]);
       }
       std::copy(A.begin(), A.end(), stage_a.begin() + (size_t)stage_n * N);
       ++stage_n;
@@ -546,7 +548,7 @@ int Context::pbwt_select_states(int stage, int iteration, int Kp) {
   cudaMemsetAsync(T.overflow.ptr, 0, 4, stream);
   int hpw = fixed_hpw ? fixed_hpw : tune_hpw;
   if (!hpw) {
-    hpw = 2;
+    hpw = 1;
     if (a.n_haps >= 32) {
       // Autotune haplotypes per sweep warp: the sweep's only state carried across
       // iterations is tar_hap, restored before every candidate run.
@@ -585,6 +587,7 @@ int Context::pbwt_select_states(int stage, int iteration, int Kp) {
   cudaMemcpyAsync(&ovf, T.overflow.ptr, 4, cudaMemcpyDeviceToHost, stream);
   cudaError_t e = cudaStreamSynchronize(stream);
   if (e != cudaSuccess) return cuda_fail(e, "pbwt selection");
+  if (ovf == 2) return (fail(GP_E_CUDA, "PBWT selection: a copy into shared memory timed out"), GP_E_CUDA);
   if (ovf) return (fail(GP_E_DATA, "PBWT selection: per-level state list exceeded its capacity"), GP_E_DATA);
   (void)stage;
   return GP_OK;

@@ -43,7 +43,7 @@ struct DevPbwt {
   uint32_t* a_after = nullptr;   // [n_com_hq][N]
   int32_t* before_id = nullptr;  // [n_com_hq]: -2 iota, -1 a_after[l-1], >= 0 merged[id]
   uint32_t* merged = nullptr;    // [n_merged][N]
-  uint32_t* vrow = nullptr;      // [n_com_hq][R]: V bits (Wv words), then their prefix counts (Wv + 1 words)
+  uint32_t* vrow = nullptr;      // [n_com_hq][R]: {V bits, prefix count} pairs, at R / 2 those of the small-PBWT positions
   int64_t* svoff = nullptr;      // [n_rare_hq + 1] word offsets of small columns
   uint32_t* svbits = nullptr;    // small-column bits
   uint32_t* svpref = nullptr;    // small-column prefix counts (one more entry per column)
@@ -105,7 +105,7 @@ struct PbwtSelectArgs {
 };
 
 // The whole selection: prepare (stream starts, carrier bits, event bits),
-// sweep with hpw haplotypes per warp (1, 2, 4, 8 or 16), union.
+// sweep with hpw haplotypes per warp (1, 2, 4 or 8), union.
 void launch_pbwt_select(const PbwtSelectArgs& a, int hpw, cudaStream_t s);
 void launch_pbwt_prepare(const PbwtSelectArgs& a, cudaStream_t s);
 void launch_pbwt_sweep(const PbwtSelectArgs& a, int hpw, cudaStream_t s);

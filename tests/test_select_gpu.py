@@ -138,3 +138,42 @@ def test_selection_with_capped_grid_matches_reference(small_workload, monkeypatc
         assert float(np.abs(got - ref).max()) <= 1e-5
     finally:
         ctx.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("N,L", [(1500, 900), (20000, 90), (40000, 70), (70000, 60)])
+def test_sweep_shapes_and_panel_sizes_give_the_same_selection(N, L):
+    """The sweep stages 4, 2 or 1 rank rows per copy, or none where a panel's rows
+    do not fit shared memory (N above about 65,000), for 1, 2, 4 or 8 haplotypes
+    per warp, the last warp partly idle (7 haplotypes). Every shape must select
+    the same level lists and states, and (where it is built) the reference's."""
+    from glimpse_b200 import native, synth
+    from oracle import oracle as O
+    w = synth.make_panel_and_targets(N, L, 0.2, 0.4, 4, ("uniform", 0.5, 2.0), ("fixed", 90), seed=71,
+                                     sparse_maf=max(0.001, 4.5 / N))
+    T = dataclasses.replace(w.targets, ploidy=w.targets.ploidy.copy())
+    T.ploidy[2] = 1
+    kw = dict(kinit=60, kpbwt=90, pbwt_depth=7, pbwt_modulo_cm=0.05)
+    rng = np.random.default_rng(N)
+    h0 = np.stack([_noisy(rng, T.truth[t, 0], 0.03) for t in range(T.n)])
+    h1 = np.stack([_noisy(rng, T.truth[t, 1], 0.03) for t in range(T.n)])
+    ctx = native.Context(w.panel, **kw)
+    got = []
+    try:
+        for hpw in (1, 2, 4, 8):
+            ctx.tuning_set(0, hpw, 0)
+            ctx.set_targets(T, kpbwt=T.kpbwt)
+            ctx.set_haps(h0, h1)
+            ctx.select(O.STAGE_BURN, 3)
+            got.append([([x.tolist() for x in ctx.pbwt_states(t, depth=7)], ctx.states(t).tolist()) for t in range(T.n)])
+        assert got[0] == got[1] == got[2] == got[3]
+        assert all(0 < len(s) <= 90 for _, s in got[0])
+        orc = ref_oracle_or_skip().RefOracle(w.panel, T, kpbwt_target=T.kpbwt, **kw)
+        for t in range(T.n):
+            orc.set_haps(t, h0[t], h1[t])
+        orc.pbwt_select(3, main_iteration=False)
+        for t in range(T.n):
+            assert [x.tolist() for x in orc.pbwt_states(t)] == got[0][t][0]
+            assert orc.select(t, O.STAGE_BURN).tolist() == got[0][t][1]
+    finally:
+        ctx.close()
