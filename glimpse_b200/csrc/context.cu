@@ -702,8 +702,9 @@ int Context::run_phase(const int32_t* d_tsel, const std::vector<int32_t>& tsel_h
     if ((e = join_streams(nside)) != cudaSuccess) return cuda_fail(e, "phasing streams");
     PhaseStore Sc = S;
     Sc.order = S.order + c0;
-    launch_phase_units(units, d_tsel, c1 - c0, w.nstates.as<int32_t>(), w.hvar.as<uint32_t>(), w.WB, w.Kp, V, Sc,
-                       cfg.seed, iteration, d_target_ids, stream);
+    if (launch_phase_units(units, d_tsel, c1 - c0, w.nstates.as<int32_t>(), w.hvar.as<uint32_t>(), w.WB, w.Kp, V, Sc,
+                           cfg.seed, iteration, d_target_ids, stream) != GP_OK)
+      return cuda_fail(cudaGetLastError(), "phasing: shared-memory attribute");
     prof.kernel_launches += nside + 3;
   }
   prof_end(ea, 1, pcells);

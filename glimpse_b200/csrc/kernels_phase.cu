@@ -535,52 +535,35 @@ __global__ void __launch_bounds__(CT, J <= 2 ? 5 : J <= 4 ? 4 : J <= 5 ? 3 : 2)
 }
 
 // ---------------------------------------------------------------------------
-// k_phase_units: the sums that combine a forward and a backward message, one CTA
-// of 8 warps (a virtual warp each) per unit. Unit u < nseg - 1 of an entry is the
-// boundary between segments u and u + 1 (TRANS_HAP, phasing_hmm.h:376-397): the 8 x 8
-// transition sums and, for every diplotype the chain could arrive with, the
-// diplotype that SAMPLE_DIP (:400-411) draws next. The others are its flat hets
-// (IMPUTE_FLAT_HET, :414-447). Units are independent, so this is bound by
-// reading the stored messages (64 bytes a state and unit).
+// k_phase_units: the sums that combine a forward and a backward message. Unit
+// u < nseg - 1 of an entry is the boundary between segments u and u + 1 (TRANS_HAP,
+// phasing_hmm.h:376-397): the 8 x 8 transition sums and, for every diplotype the
+// chain could arrive with, the diplotype that SAMPLE_DIP (:400-411) draws next. The
+// others are its flat hets (IMPUTE_FLAT_HET, :414-447). Units are independent; the
+// work is reading two stored messages (64 bytes a state and unit) and 64 (or 16)
+// multiply-adds a state.
+//
+// A CTA of 8 warps (a virtual warp each) takes every gridDim.x-th unit of one entry.
+// Thread tid owns the states tid + 256 j; the values of the next steps (a step: one j
+// of a unit) are always in flight, copied by cp.async into slots that only its warp
+// reads, also while a unit is summed up, so that memory does not idle. Messages stay in the
+// chain's slot order (h -> h ^ f within the halves, f & 3 of the lane); the sums over
+// the lanes go through shared memory, where writing a value to the row of its
+// hypothesis pair undoes the permutation at no cost, 16 rows at a time; two lanes
+// add a row's 32 values in the fixed tree. One barrier a unit; a unit's last steps
+// and draws fall to one warp, the next unit's to the next warp.
 // ---------------------------------------------------------------------------
-// Reduce-scatter of N values over the lanes (distances 16, 8, 4, 2, 1); a lane
-// keeps the upper half of the values where its bit of the distance is set, so
-// lane l ends with values 2 l and 2 l + 1 of 64, or value l >> 1 of 16.
-template <int N>
-__device__ __forceinline__ void lane_scatter(float (&v)[N], int lane) {
-  int n = N;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    if (n > 1) {
-      n >>= 1;
-      const bool up = lane & o;
-#pragma unroll
-      for (int i = 0; i < N / 2; ++i) {
-        if (i >= n) break;
-        const float send = up ? v[i] : v[i + n];
-        const float keep = up ? v[i + n] : v[i];
-        v[i] = __fadd_rn(keep, shfl_x(send, o));
-      }
-    } else {
-      v[0] = __fadd_rn(v[0], shfl_x(v[0], o));
-    }
-  }
-}
+constexpr int kUnitStages = 4;
+constexpr int kUnitsPerCta = 8;  // at least, where an entry has that many
 
-// A stored row of state k in natural hypothesis order: position p of a half holds
-// hypothesis p ^ (f & 3) of that half, f the class of the state's lane in the chain.
-__device__ __forceinline__ void load_row(const float* row, int f, float (&v)[8]) {
-  const float4* r4 = reinterpret_cast<const float4*>(row);
-  const float4 a = r4[0], b = r4[1];
-  const bool x1 = f & 1, x2 = f & 2;
-  float u[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-#pragma unroll
-  for (int h = 0; h < 8; ++h) v[h] = x1 ? u[h ^ 1] : u[h];
-#pragma unroll
-  for (int h = 0; h < 8; ++h) u[h] = x2 ? v[h ^ 2] : v[h];
-#pragma unroll
-  for (int h = 0; h < 8; ++h) v[h] = u[h];
-}
+struct UnitSmem {
+  float4 row[kUnitStages][4][256];     // two messages of a thread's state
+  uint32_t word[kUnitStages][256];     // its Hvar word (flat hets)
+  float tr[NW][16][36];                // values of 16 hypothesis pairs by lane (lanes 2i + p at 16 p + i)
+  float red[2][NW][64];                // the warps' sums
+  float hp[64];
+  float sc[2][16];                     // a unit's factors
+};
 
 __device__ __forceinline__ float warps_sum(const float (*red)[64], int i) {
   const float a = __fadd_rn(red[0][i], red[1][i]), b = __fadd_rn(red[2][i], red[3][i]);
@@ -588,63 +571,176 @@ __device__ __forceinline__ float warps_sum(const float (*red)[64], int i) {
   return __fadd_rn(__fadd_rn(a, b), __fadd_rn(c, d));
 }
 
+// The sums over the lanes of the 16 rows that the warp wrote to tr: row lane / 2,
+// valid in both lanes of a pair.
+__device__ __forceinline__ float rows_sum(const float (*tr)[36], int lane) {
+  const ulonglong2* r = reinterpret_cast<const ulonglong2*>(&tr[lane >> 1][16 * (lane & 1)]);
+  const ulonglong2 v0 = r[0], v1 = r[1], v2 = r[2], v3 = r[3];  // lanes 2i + p, i = 0-3, 4-7, 8-11, 12-15
+  const f2 a = f2_add(f2_add(v0.x, v2.x), f2_add(v1.x, v3.x));  // distances 16 and 8
+  const f2 b = f2_add(f2_add(v0.y, v2.y), f2_add(v1.y, v3.y));
+  float x, y;
+  f2_unpack(f2_add(a, b), x, y);                                // distance 4
+  x = __fadd_rn(x, y);                                          // distance 2
+  return __fadd_rn(x, shfl_x(x, 1));
+}
+
 __global__ void __launch_bounds__(256, 2) k_phase_units(const int32_t* __restrict__ tsel,
                                                         const int32_t* __restrict__ nstates,
                                                         const uint32_t* __restrict__ hvar, int WB, int Kp, PhaseVars P,
                                                         PhaseStore S, uint64_t seed, int iteration,
                                                         const int32_t* __restrict__ target_ids) {
-  __shared__ float red[NW][64];
-  __shared__ float hp[64];
+  extern __shared__ __align__(16) char smem_raw[];
+  UnitSmem& sm = *reinterpret_cast<UnitSmem*>(smem_raw);
   const int b = S.order[blockIdx.y];
   const int t = tsel ? tsel[b] : b;
   const int K = nstates[t];
   const int nv = P.nvar[b];
   const int nseg = P.nseg[b], nmiss = P.nmiss[b];
-  const int nb = nv > 0 ? nseg - 1 : 0;
+  const int nb = nv > 0 ? nseg - 1 : 0;  // boundaries
+  const int nu = nb + nmiss;
+  if ((int)blockIdx.x >= nu) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int f = (lane >> 1) & 7;
+  const int f = (lane >> 1) & 3;  // the chain's slot s of a half holds hypothesis s ^ f
   const float* pool = S.pool + S.pool_off[b];
-  const size_t fbase = (size_t)(nseg + nmiss) * K * 8;
+  const size_t rowf = (size_t)K * 8, fbase = (size_t)(nseg + nmiss) * rowf;
+  const int64_t so = S.seg_off[b], mo = S.miss_off[b];
+  const int32_t* mrel = P.miss_rel + (size_t)b * P.lv;
   const uint32_t rng_target = target_ids ? (uint32_t)target_ids[b] : (uint32_t)t;
-  for (int u = blockIdx.x; u < nb + nmiss; u += gridDim.x) {
+  const int nj = (K + 255) >> 8;
+
+  // Steps in flight. A warp's states are 1 KB of either row, copied in whole 512-byte
+  // pieces: lane l takes the 16-byte chunks l and l + 32, half l & 1 of state l >> 1 (+ 16).
+  int iu = blockIdx.x, ij = 0, istage = 0;
+  const int kl = 32 * warp + (lane >> 1);
+  const uint32_t* hv = hvar + (size_t)t * WB * Kp + tid;
+  const float *px = pool, *py = pool;
+  const uint32_t* pw = nullptr;  // Hvar words of the unit's site, null at boundaries
+  auto site_of = [&](int u) { return u >= nb && u < nu ? mrel[u - nb] : 0; };
+  int site = site_of(iu);  // of the unit begun next
+  auto begin_unit = [&]() {
+    if (iu >= nu) return;
+    // boundary u: forward row at the end of segment u, backward row at the start of u + 1;
+    // flat het m: backward and forward row
+    const bool flat = iu >= nb;
+    px = (flat ? pool + (size_t)(nseg + iu - nb) * rowf : pool + fbase + (size_t)iu * rowf) + 256 * warp + 4 * lane;
+    py = flat ? px + fbase : pool + (size_t)(iu + 1) * rowf + 256 * warp + 4 * lane;
+    pw = flat ? hv + (size_t)(site >> 5) * Kp : nullptr;
+    site = site_of(iu + gridDim.x);
+  };
+  auto issue = [&]() {
+    if (iu < nu) {
+      const int k = kl + 256 * ij;
+      float4* d = &sm.row[istage][lane & 1][kl];
+      if (k < K) {
+        cp_async16(d, px);
+        cp_async16(d + 512, py);
+      }
+      if (k + 16 < K) {
+        cp_async16(d + 16, px + 128);
+        cp_async16(d + 528, py + 128);
+      }
+      if (pw && tid + 256 * ij < K) cp_async4(&sm.word[istage][tid], pw + 256 * ij);
+      px += 2048;
+      py += 2048;
+    }
+    asm volatile("cp.async.commit_group;\n" ::);
+    istage = istage + 1 == kUnitStages ? 0 : istage + 1;
+    if (++ij == nj) {
+      ij = 0;
+      iu += gridDim.x;
+      begin_unit();
+    }
+  };
+  begin_unit();
+  // A unit's factors, one per thread of the first 16. Boundary: fact1 of hypothesis h (8 of them) and fact2;
+  // flat het: the reciprocal sums of the backward and the forward message.
+  float s0 = 0.f, s1 = 1.f, s2 = 0.f;
+  auto load_factors = [&](int u) {
+    if (tid >= 16 || u >= nu) return;
     if (u < nb) {
-      const int64_t so = S.seg_off[b] + u;
-      const float* fsum = S.seg_sum + (S.seg_total + so) * 8;
-      const float sumT = S.seg_tot[S.seg_total + so];
-      const float yt = P.yt_next[(size_t)b * P.lv + P.seg_start[(size_t)b * (P.lv + 2) + u + 1] - 1];
-      const float fact2 = (1.0f - yt) / sumT;
+      s0 = S.seg_sum[(S.seg_total + so + u) * 8 + (tid & 7)];
+      s1 = S.seg_tot[S.seg_total + so + u];
+      s2 = P.yt_next[(size_t)b * P.lv + P.seg_start[(size_t)b * (P.lv + 2) + u + 1] - 1];
+    } else {
+      s0 = S.miss_sum[((tid < 8 ? 0 : S.miss_total) + mo + u - nb) * 8 + (tid & 7)];
+    }
+  };
+  auto put_factors = [&](int u, int par) {
+    if (tid >= 16 || u >= nu) return;
+    float v;
+    if (u >= nb) v = 1.0f / s0;
+    else if (tid < 8) v = __fmul_rn(s0 / s1, s2) / (float)K;
+    else v = (1.0f - s2) / s1;
+    sm.sc[par][tid] = v;
+  };
+#pragma unroll
+  for (int i = 0; i < kUnitStages - 1; ++i) issue();
+  load_factors(blockIdx.x);
+  put_factors(blockIdx.x, 0);
+  __syncthreads();
+  // where this lane writes value (s1, s2) (low two bits each) of 16 pairs: row (s1 ^ f) * 4 + (s2 ^ f)
+  float* const trp = &sm.tr[warp][0][16 * (lane & 1) + (lane >> 1)];
+  const int fx = 5 * f;
+  int cstage = 0, par = 0, owner = 0;
+  for (int u = blockIdx.x; u < nu; u += gridDim.x) {
+    load_factors(u + gridDim.x);
+    if (u < nb) {
+      const float4* c4 = reinterpret_cast<const float4*>(sm.sc[par]);
       float fact1[8];
 #pragma unroll
-      for (int h = 0; h < 8; ++h) fact1[h] = __fmul_rn(fsum[h] / sumT, yt) / (float)K;
-      float acc[64];
+      for (int h = 0; h < 8; ++h) fact1[h] = sm.sc[par][(h & 4) | ((h & 3) ^ f)];
+      const float fact2 = c4[2].x;
+      f2 acc[8][4];
 #pragma unroll
-      for (int i = 0; i < 64; ++i) acc[i] = 0.f;
-      const float* fr = pool + fbase + (size_t)u * K * 8;
-      const float* nr = pool + (size_t)(u + 1) * K * 8;
-      for (int k = tid; k < K; k += 256) {
-        float p[8], n[8];
-        load_row(fr + (size_t)k * 8, f, p);
-        load_row(nr + (size_t)k * 8, f, n);
+      for (int h = 0; h < 8; ++h)
 #pragma unroll
-        for (int h1 = 0; h1 < 8; ++h1) {
-          const float p0 = fmaf(p[h1], fact2, fact1[h1]);
+        for (int q = 0; q < 4; ++q) acc[h][q] = f2_pack(0.f, 0.f);
+      for (int j = 0; j < nj; ++j) {
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(kUnitStages - 2) : "memory");
+        __syncwarp();  // the other lanes' pieces have landed, and the slot issued next is no longer read
+        if (tid + 256 * j < K) {
+          const float4 x0 = sm.row[cstage][0][tid], x1 = sm.row[cstage][1][tid];
+          const float4 y0 = sm.row[cstage][2][tid], y1 = sm.row[cstage][3][tid];
+          const float p[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+          const f2 n[4] = {lo2(y0), hi2(y0), lo2(y1), hi2(y1)};
 #pragma unroll
-          for (int h2 = 0; h2 < 8; ++h2) acc[h1 * 8 + h2] = fmaf(p0, n[h2], acc[h1 * 8 + h2]);
+          for (int h = 0; h < 8; ++h) {
+            const float p0 = fmaf(p[h], fact2, fact1[h]);
+            const f2 pp = f2_pack(p0, p0);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) acc[h][q] = f2_fma(pp, n[q], acc[h][q]);
+          }
         }
+        issue();
+        cstage = cstage + 1 == kUnitStages ? 0 : cstage + 1;
       }
-      lane_scatter<64>(acc, lane);
-      red[warp][2 * lane] = acc[0];
-      red[warp][2 * lane + 1] = acc[1];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {  // rounds of 16 pairs: halves r / 2 of h1 and r % 2 of h2
+#pragma unroll
+        for (int i = 0; i < 16; i += 2) {
+          float lo, hi;
+          f2_unpack(acc[4 * (r >> 1) + (i >> 2)][2 * (r & 1) + ((i >> 1) & 1)], lo, hi);
+          trp[(i ^ fx) * 36] = lo;
+          trp[((i + 1) ^ fx) * 36] = hi;
+        }
+        __syncwarp();
+        const float v = rows_sum(sm.tr[warp], lane);
+        const int i = lane >> 1;
+        if ((lane & 1) == 0) sm.red[par][warp][(4 * (r >> 1) + (i >> 2)) * 8 + 4 * (r & 1) + (i & 3)] = v;
+        __syncwarp();
+      }
+      put_factors(u + gridDim.x, par ^ 1);
       __syncthreads();
-      if (tid < 64) hp[tid] = warps_sum(red, tid);
-      __syncthreads();
-      if (warp == 0) {
+      if (warp == owner) {
+        sm.hp[lane] = warps_sum(sm.red[par], lane);
+        sm.hp[lane + 32] = warps_sum(sm.red[par], lane + 32);
+        __syncwarp();
         float sumHP = 0.f;
 #pragma unroll
         for (int h1 = 0; h1 < 8; ++h1) {
           float v[8];
 #pragma unroll
-          for (int h2 = 0; h2 < 8; ++h2) v[h2] = hp[h1 * 8 + h2];
+          for (int h2 = 0; h2 < 8; ++h2) v[h2] = sm.hp[h1 * 8 + h2];
           sumHP = __fadd_rn(sumHP, hadd8(v));
         }
         const int prev = lane & 7;
@@ -652,7 +748,7 @@ __global__ void __launch_bounds__(256, 2) k_phase_units(const int32_t* __restric
         float dp[8], sd = 0.f;
 #pragma unroll
         for (int d = 0; d < 8; ++d) {
-          dp[d] = __fmul_rn(hp[prev * 8 + d] / sumHP, hp[(7 - prev) * 8 + (7 - d)] / sumHP);
+          dp[d] = __fmul_rn(sm.hp[prev * 8 + d] / sumHP, sm.hp[(7 - prev) * 8 + (7 - d)] / sumHP);
           sd = __fadd_rn(sd, dp[d]);
         }
         const bool bad = bad1 || isnan(sd) || isinf(sd) || sd < 1.17549435e-38f;
@@ -668,48 +764,56 @@ __global__ void __launch_bounds__(256, 2) k_phase_units(const int32_t* __restric
         if (bad) nd = prev;  // an invalid sum keeps the diplotype and raises the entry's error flag
         uint32_t mine = lane < 8 ? ((uint32_t)nd << (3 * prev)) | ((bad ? 1u : 0u) << (24 + prev)) : 0u;
         mine = __reduce_or_sync(kFull, mine);
-        if (lane == 0) S.next[so] = mine;
+        if (lane == 0) S.next[so + u] = mine;
       }
-      __syncthreads();
     } else {
       const int m = u - nb;
-      const int64_t mo = S.miss_off[b] + m;
-      const float* bsum = S.miss_sum + mo * 8;
-      const float* fsum = S.miss_sum + (S.miss_total + mo) * 8;
-      const int l = P.miss_rel[(size_t)b * P.lv + m];
-      const uint32_t* hv = hvar + ((size_t)t * WB + (l >> 5)) * Kp;
+      const uint32_t bit = 1u << (mrel[m] & 31);
       float sR[8], sL[8], v[16];
 #pragma unroll
       for (int h = 0; h < 8; ++h) {
-        sR[h] = 1.0f / bsum[h];
-        sL[h] = 1.0f / fsum[h];
+        sR[h] = sm.sc[par][(h & 4) | ((h & 3) ^ f)];
+        sL[h] = sm.sc[par][8 + ((h & 4) | ((h & 3) ^ f))];
         v[h] = v[h + 8] = 0.f;
       }
-      const float* br = pool + (size_t)(nseg + m) * K * 8;
-      const float* fr = br + fbase;
-      for (int k = tid; k < K; k += 256) {
-        const bool bit = (hv[k] >> (l & 31)) & 1u;
-        float ip[8], pr[8];
-        load_row(br + (size_t)k * 8, f, ip);
-        load_row(fr + (size_t)k * 8, f, pr);
+      for (int j = 0; j < nj; ++j) {
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(kUnitStages - 2) : "memory");
+        __syncwarp();  // the other lanes' pieces have landed, and the slot issued next is no longer read
+        if (tid + 256 * j < K) {
+          const float4 x0 = sm.row[cstage][0][tid], x1 = sm.row[cstage][1][tid];
+          const float4 y0 = sm.row[cstage][2][tid], y1 = sm.row[cstage][3][tid];
+          const bool alt = (sm.word[cstage][tid] & bit) != 0u;
+          const float ip[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+          const float pr[8] = {y0.x, y0.y, y0.z, y0.w, y1.x, y1.y, y1.z, y1.w};
 #pragma unroll
-        for (int h = 0; h < 8; ++h) {
-          const float p1 = __fmul_rn(ip[h], sR[h]);
-          const float p2 = __fmul_rn(pr[h], sL[h]);
-          if (bit) v[8 + h] = fmaf(p1, p2, v[8 + h]); else v[h] = fmaf(p1, p2, v[h]);
+          for (int h = 0; h < 8; ++h) {
+            const float p1 = __fmul_rn(ip[h], sR[h]);
+            const float p2 = __fmul_rn(pr[h], sL[h]);
+            if (alt) v[8 + h] = fmaf(p1, p2, v[8 + h]); else v[h] = fmaf(p1, p2, v[h]);
+          }
         }
+        issue();
+        cstage = cstage + 1 == kUnitStages ? 0 : cstage + 1;
       }
-      lane_scatter<16>(v, lane);
-      if ((lane & 1) == 0) red[warp][lane >> 1] = v[0];
+      // rows: allele * 8 + hypothesis
+#pragma unroll
+      for (int i = 0; i < 16; ++i) trp[(i ^ f) * 36] = v[i];
+      __syncwarp();
+      const float x = rows_sum(sm.tr[warp], lane);
+      if ((lane & 1) == 0) sm.red[par][warp][lane >> 1] = x;
+      __syncwarp();
+      put_factors(u + gridDim.x, par ^ 1);
       __syncthreads();
-      if (tid < 8) {
-        const float t0 = warps_sum(red, tid), t1 = warps_sum(red, tid + 8);
+      if (warp == owner && lane < 8) {
+        const float t0 = warps_sum(sm.red[par], lane), t1 = warps_sum(sm.red[par], lane + 8);
         const float r = t1 / __fadd_rn(t0, t1);
-        S.of1[mo * 8 + tid] = fmaxf(0.0f, fminf(1.0f, r));
+        S.of1[(mo + m) * 8 + lane] = fmaxf(0.0f, fminf(1.0f, r));
       }
-      __syncthreads();
     }
+    par ^= 1;
+    owner = (owner + 1) & (NW - 1);
   }
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
 }
 
 // The diplotype chain of one entry per warp: the first draw (phasing_hmm.cpp:249-256)
@@ -868,13 +972,17 @@ int launch_phase_chain(int J, const int32_t* tsel, int nb, const int32_t* nstate
 #undef GP_CHAIN
 }
 
-void launch_phase_units(int max_units, const int32_t* tsel, int nb, const int32_t* nstates, const uint32_t* hvar,
+int launch_phase_units(int max_units, const int32_t* tsel, int nb, const int32_t* nstates, const uint32_t* hvar,
                         int WB, int Kp, PhaseVars P, PhaseStore S, uint64_t seed, int iteration,
                         const int32_t* target_ids, cudaStream_t s) {
-  if (max_units > 0)
-    k_phase_units<<<dim3(max_units < 4096 ? max_units : 4096, nb), 256, 0, s>>>(tsel, nstates, hvar, WB, Kp, P, S, seed,
-                                                                               iteration, target_ids);
+  if (max_units > 0) {
+    if (set_smem_limit_once<k_phase_units>((int)sizeof(UnitSmem)) != cudaSuccess) return GP_E_CUDA;
+    const int g = (max_units + kUnitsPerCta - 1) / kUnitsPerCta;
+    k_phase_units<<<dim3(g, nb), 256, sizeof(UnitSmem), s>>>(tsel, nstates, hvar, WB, Kp, P, S, seed, iteration,
+                                                             target_ids);
+  }
   k_phase_draw<<<(nb + 3) / 4, 128, 0, s>>>(tsel, nb, P, S, seed, iteration, target_ids);
+  return GP_OK;
 }
 
 void launch_phase_writeback(const int32_t* tsel, int nb, const int32_t* poly, const int32_t* polyidx, int L,

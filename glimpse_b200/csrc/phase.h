@@ -66,9 +66,9 @@ int launch_phase_chain(int J, const int32_t* tsel, int nb, const int32_t* nstate
                        int Kp, const int32_t* npoly, PhaseVars P, PhaseStore S, const ModelConst& mc, cudaStream_t s);
 // After the chains, for entries of any K: the units and draws. max_units: the
 // largest count of segment boundaries and flat hets of an entry.
-void launch_phase_units(int max_units, const int32_t* tsel, int nb, const int32_t* nstates, const uint32_t* hvar,
-                        int WB, int Kp, PhaseVars P, PhaseStore S, uint64_t seed, int iteration,
-                        const int32_t* target_ids, cudaStream_t s);
+int launch_phase_units(int max_units, const int32_t* tsel, int nb, const int32_t* nstates, const uint32_t* hvar,
+                       int WB, int Kp, PhaseVars P, PhaseStore S, uint64_t seed, int iteration,
+                       const int32_t* target_ids, cudaStream_t s);
 void launch_phase_writeback(const int32_t* tsel, int nb, const int32_t* poly, const int32_t* polyidx, int L,
                             PhaseVars V, PhaseStore S, const ModelConst& mc, uint64_t seed, int iteration,
                             const int32_t* target_ids, uint8_t* h0, uint8_t* h1, cudaStream_t s);
