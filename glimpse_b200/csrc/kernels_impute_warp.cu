@@ -233,22 +233,25 @@ __global__ void __launch_bounds__(SOLO ? kChainThreads : kChainThreads * kMaxCha
 }
 
 // ---------------------------------------------------------------------------
-// k_impute_block: posteriors of kRowSites sites, 128 threads. Thread tid = 4 l + c
-// takes its padded states 128 j + tid two rows j at a time, as a packed pair (rows
-// -1 and 0 first when J is odd): the forward steps, whose values stay in
+// k_impute_block: posteriors, block by block of kRowSites sites, 128 threads. Thread
+// tid = 4 l + c takes its padded states 128 j + tid two rows j at a time, as a packed
+// pair (rows -1 and 0 first when J is odd): the forward steps, whose values stay in
 // registers, then the backward steps, the products added to the thread's two sums
 // per site (one per allele). All site data is uniform and comes from shared memory;
-// the loop over rows needs no communication. Bound by issue, about 11 instructions
-// per (site, state). One lane tree per site and allele ends it.
+// the loop over rows needs no communication. One lane tree per site and allele ends
+// a block. Bound by issue, about 14 instructions per (site, state); to keep it so, a
+// CTA takes several consecutive blocks and loads the next pair of rows and the next
+// block's site data while it works on the current ones.
 // ---------------------------------------------------------------------------
 constexpr int kBlockThreads = 128;
 constexpr int RS = kRowSites;
 
 struct BlockSmem {
-  float4 fwd[RS];  // t / K twice, (1 - t) / sum twice, into the site from the left
-  float4 bwd[RS];  // the same from the right
-  float2 em[RS];   // emissions of allele 0 and 1
-  float part[32][2 * RS + 4];  // [lane l][value 2 site + allele]
+  // site data of two blocks
+  float4 fwd[2][RS];  // t / K twice, (1 - t) / sum twice, into the site from the left
+  float4 bwd[2][RS];  // the same from the right
+  float2 em[2][RS];   // emissions of allele 0 and 1
+  float part[2][32][2 * RS + 4];  // [lane l][value 2 site + allele]
 };
 
 // Shared-memory loads that stay where they are: moved out of the loop over rows,
@@ -299,117 +302,137 @@ __device__ __forceinline__ void block_pair(unsigned fwd, unsigned bwd, unsigned 
   }
 }
 
-template <bool LAST>
-__device__ __forceinline__ void block_rows(const BlockSmem& S, const float* __restrict__ arow,
-                                           const float* __restrict__ brow, const uint32_t* __restrict__ hv, int shift,
-                                           int J, int pad, int last, float (&q0)[RS], float (&q1)[RS]) {
-  const int tid = threadIdx.x;
-  const unsigned fwd = static_cast<unsigned>(__cvta_generic_to_shared(S.fwd));
-  const unsigned bwd = static_cast<unsigned>(__cvta_generic_to_shared(S.bwd));
-  const unsigned em = static_cast<unsigned>(__cvta_generic_to_shared(S.em));
-  // rows j and j + 1 of this thread: words and the kept values entering from both sides
-  struct Pair {
-    uint32_t w0, w1;
-    float a0, a1, b0, b1;
-  };
-  auto load = [&](int j) {
-    Pair p;
-    const int o = 128 * j + tid;
-    const bool e0 = j > 0 || (j == 0 && tid >= pad), e1 = j >= 0 || tid >= pad;
-    p.w0 = e0 ? hv[o] >> shift : 0u;
-    p.w1 = e1 ? hv[o + 128] >> shift : 0u;
-    p.a0 = arow && e0 ? arow[o] : 0.f;
-    p.a1 = arow && e1 ? arow[o + 128] : 0.f;
-    p.b0 = brow && e0 ? brow[o] : 0.f;
-    p.b1 = brow && e1 ? brow[o + 128] : 0.f;
-    return p;
-  };
-  int j = -(J & 1);
-  Pair p = load(j), n;
-  const f2 exists = f2_pack(j == 0 && tid >= pad ? 1.f : 0.f, j == 0 || tid >= pad ? 1.f : 0.f);
-  if (j + 2 < J) n = load(j + 2);
-  block_pair<true, LAST>(fwd, bwd, em, p.w0, p.w1, f2_pack(p.a0, p.a1), f2_pack(p.b0, p.b1), exists, last, q0, q1);
-#pragma unroll 1
-  for (j += 2; j < J; j += 2) {
-    p = n;
-    if (j + 2 < J) n = load(j + 2);
-    block_pair<false, LAST>(fwd, bwd, em, p.w0, p.w1, f2_pack(p.a0, p.a1), f2_pack(p.b0, p.b1), 0, last, q0, q1);
-  }
-}
-
-__global__ void __launch_bounds__(kBlockThreads, 4) k_impute_block(ChainArgs A) {
+__global__ void __launch_bounds__(kBlockThreads, 4) k_impute_block(ChainArgs A, int blocks_per) {
   __shared__ BlockSmem S;
   const int t = A.order ? A.order[blockIdx.y] : blockIdx.y;
   const int np = A.npoly[t], K = A.nstates[t];
   const int nrow = (np + RS - 1) / RS;
-  const int b = blockIdx.x;
-  if (b >= nrow || K == 0) return;
+  int b = blockIdx.x * blocks_per;
+  const int bend = min(nrow, b + blocks_per);
+  if (b >= bend || K == 0) return;
   const int J = (K + 127) >> 7, Ks = 128 * J, pad = Ks - K;
-  const int tid = threadIdx.x;
-  const int l0 = b * RS, n = min(RS, np - l0);
-  if (tid < RS) {
-    const int l = l0 + tid;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const float* base = A.rows + A.row_off[t];
+  const uint32_t* hvt = A.hvar + (size_t)t * A.WB * A.Kp - pad;
+
+  // Rows j and j + 1 of this thread in block b: words and the kept values entering from both sides.
+  struct Pair {
+    uint32_t w0, w1;
+    float a0, a1, b0, b1;
+  };
+  auto load = [&](int b, int j) {
+    Pair p;
+    const int o = 128 * j + tid;
+    const bool e0 = j > 0 || (j == 0 && tid >= pad), e1 = j >= 0 || tid >= pad;
+    const uint32_t* hv = hvt + (size_t)((b * RS) >> 5) * A.Kp + o;
+    const float* ar = base + (size_t)b * Ks + o;
+    const float* br = ar + (size_t)nrow * Ks;
+    const bool left = b > 0, right = b < nrow - 1;
+    p.w0 = e0 ? hv[0] : 0u;
+    p.w1 = e1 ? hv[128] : 0u;
+    p.a0 = left && e0 ? ar[0] : 0.f;
+    p.a1 = left && e1 ? ar[128] : 0.f;
+    p.b0 = right && e0 ? br[0] : 0.f;
+    p.b1 = right && e1 ? br[128] : 0.f;
+    return p;
+  };
+  // Site data of a block, one site per thread of the first RS, and the site of this lane's output.
+  const float2* T = A.tr + (size_t)t * A.L;
+  const float* fac = A.fac + (size_t)t * 32 * A.WB;
+  const float init = 1.0f / (float)K;
+  float4 f = make_float4(0.f, 0.f, 0.f, 0.f), g = f;
+  float2 em = make_float2(0.f, 0.f);
+  int site = 0, next_site = 0;
+  auto load_sites = [&](int b) {
+    const int lo = b * RS + (lane >> 1);
+    if (lo < np) next_site = A.poly[(size_t)t * A.L + lo];
+    if (tid >= RS) return;
+    const int l = b * RS + tid;
     // past the last site: the identity step
-    float4 f = make_float4(0.f, 0.f, 1.f, 1.f), g = f;
-    float2 e = make_float2(1.f, 1.f);
+    f = g = make_float4(0.f, 0.f, 1.f, 1.f);
+    em = make_float2(1.f, 1.f);
     if (l < np) {
-      const float2* T = A.tr + (size_t)t * A.L;
-      const float* fac = A.fac + (size_t)t * 32 * A.WB + l;
-      const float init = 1.0f / (float)K;
-      const float fa = fac[0], fb = fac[(size_t)A.n * 32 * A.WB];
+      const float fa = fac[l], fb = fac[(size_t)A.n * 32 * A.WB + l];
       const float ta = l > 0 ? T[l - 1].x : init, tb = l < np - 1 ? T[l].x : init;
       f = make_float4(ta, ta, fa, fa);
       g = make_float4(tb, tb, fb, fb);
       const float4 ee = A.em[(size_t)t * A.L + l];
-      if (A.fl[(size_t)t * A.L + l] == 0) e = make_float2(ee.x, ee.y);
+      if (A.fl[(size_t)t * A.L + l] == 0) em = make_float2(ee.x, ee.y);
     }
-    S.fwd[tid] = f;
-    S.bwd[tid] = g;
-    S.em[tid] = e;
-  }
+  };
+  auto put_sites = [&](int par) {
+    if (tid >= RS) return;
+    S.fwd[par][tid] = f;
+    S.bwd[par][tid] = g;
+    S.em[par][tid] = em;
+  };
+  const int j0 = -(J & 1);
+  const f2 exists = f2_pack(j0 == 0 && tid >= pad ? 1.f : 0.f, j0 == 0 || tid >= pad ? 1.f : 0.f);
+  Pair n = load(b, j0);
+  load_sites(b);
+  put_sites(0);
   __syncthreads();
-  float q0[RS], q1[RS];
+  const unsigned fwd0 = static_cast<unsigned>(__cvta_generic_to_shared(&S.fwd[0][0]));
+  const unsigned bwd0 = static_cast<unsigned>(__cvta_generic_to_shared(&S.bwd[0][0]));
+  const unsigned em0 = static_cast<unsigned>(__cvta_generic_to_shared(&S.em[0][0]));
+  int par = 0;
+#pragma unroll 1
+  for (; b < bend; ++b) {
+    site = next_site;
+    if (b + 1 < bend) load_sites(b + 1);
+    const unsigned fwd = fwd0 + par * sizeof(S.fwd[0]), bwd = bwd0 + par * sizeof(S.bwd[0]);
+    const unsigned ems = em0 + par * sizeof(S.em[0]);
+    const int shift = (b * RS) & 31, last = np - 1 - b * RS;
+    float q0[RS], q1[RS];
 #pragma unroll
-  for (int i = 0; i < RS; ++i) q0[i] = q1[i] = 0.f;
-  const float* base = A.rows + A.row_off[t];
-  const float* arow = b > 0 ? base + (size_t)b * Ks : nullptr;
-  const float* brow = b < nrow - 1 ? base + ((size_t)nrow + b) * Ks : nullptr;
-  const uint32_t* hv = A.hvar + ((size_t)t * A.WB + (l0 >> 5)) * A.Kp - pad;
-  if (b == nrow - 1) block_rows<true>(S, arow, brow, hv, l0 & 31, J, pad, n - 1, q0, q1);
-  else block_rows<false>(S, arow, brow, hv, l0 & 31, J, pad, -1, q0, q1);
-  // Components of a lane l = tid / 4: reduce-scatter over thread distances 1 and 2.
-  const int c = tid & 3;
-  const bool up1 = c & 1, up2 = c & 2;
+    for (int i = 0; i < RS; ++i) q0[i] = q1[i] = 0.f;
+    const bool final_block = b == nrow - 1;
+#pragma unroll 1
+    for (int j = j0; j < J; j += 2) {
+      const Pair p = n;
+      if (j + 2 < J) n = load(b, j + 2);
+      else if (b + 1 < bend) n = load(b + 1, j0);
+      const f2 x = f2_pack(p.a0, p.a1), y = f2_pack(p.b0, p.b1);
+      const uint32_t w0 = p.w0 >> shift, w1 = p.w1 >> shift;
+      if (final_block) block_pair<true, true>(fwd, bwd, ems, w0, w1, x, y, j == j0 ? exists : f2_pack(1.f, 1.f), last, q0, q1);
+      else if (j == j0) block_pair<true, false>(fwd, bwd, ems, w0, w1, x, y, exists, -1, q0, q1);
+      else block_pair<false, false>(fwd, bwd, ems, w0, w1, x, y, 0, -1, q0, q1);
+    }
+    // Components of a lane l = tid / 4: reduce-scatter over thread distances 1 and 2.
+    const int c = tid & 3;
+    const bool up1 = c & 1, up2 = c & 2;
 #pragma unroll
-  for (int i = 0; i < RS / 2; ++i) {
-    const float s0 = up1 ? q0[i] : q0[i + RS / 2], k0 = up1 ? q0[i + RS / 2] : q0[i];
-    const float s1 = up1 ? q1[i] : q1[i + RS / 2], k1 = up1 ? q1[i + RS / 2] : q1[i];
-    q0[i] = __fadd_rn(k0, __shfl_xor_sync(0xffffffffu, s0, 1));
-    q1[i] = __fadd_rn(k1, __shfl_xor_sync(0xffffffffu, s1, 1));
-  }
+    for (int i = 0; i < RS / 2; ++i) {
+      const float s0 = up1 ? q0[i] : q0[i + RS / 2], k0 = up1 ? q0[i + RS / 2] : q0[i];
+      const float s1 = up1 ? q1[i] : q1[i + RS / 2], k1 = up1 ? q1[i + RS / 2] : q1[i];
+      q0[i] = __fadd_rn(k0, __shfl_xor_sync(0xffffffffu, s0, 1));
+      q1[i] = __fadd_rn(k1, __shfl_xor_sync(0xffffffffu, s1, 1));
+    }
 #pragma unroll
-  for (int i = 0; i < RS / 4; ++i) {
-    const float s0 = up2 ? q0[i] : q0[i + RS / 4], k0 = up2 ? q0[i + RS / 4] : q0[i];
-    const float s1 = up2 ? q1[i] : q1[i + RS / 4], k1 = up2 ? q1[i + RS / 4] : q1[i];
-    const int site = RS / 2 * (c & 1) + RS / 4 * (c >> 1) + i;
-    const float v0 = __fadd_rn(k0, __shfl_xor_sync(0xffffffffu, s0, 2));
-    const float v1 = __fadd_rn(k1, __shfl_xor_sync(0xffffffffu, s1, 2));
-    *reinterpret_cast<float2*>(&S.part[tid >> 2][2 * site]) = make_float2(v0, v1);
-  }
-  __syncthreads();
-  if (tid < 2 * RS) {
-    float v[8];
+    for (int i = 0; i < RS / 4; ++i) {
+      const float s0 = up2 ? q0[i] : q0[i + RS / 4], k0 = up2 ? q0[i + RS / 4] : q0[i];
+      const float s1 = up2 ? q1[i] : q1[i + RS / 4], k1 = up2 ? q1[i + RS / 4] : q1[i];
+      const int st = RS / 2 * (c & 1) + RS / 4 * (c >> 1) + i;
+      const float v0 = __fadd_rn(k0, __shfl_xor_sync(0xffffffffu, s0, 2));
+      const float v1 = __fadd_rn(k1, __shfl_xor_sync(0xffffffffu, s1, 2));
+      *reinterpret_cast<float2*>(&S.part[par][tid >> 2][2 * st]) = make_float2(v0, v1);
+    }
+    if (b + 1 < bend) put_sites(par ^ 1);
+    __syncthreads();
+    if (warp == (b & 3)) {  // the 2 RS = 32 sums of the block, the warps in turn
+      float v[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
-      v[i] = __fadd_rn(__fadd_rn(S.part[i][tid], S.part[i + 16][tid]),
-                       __fadd_rn(S.part[i + 8][tid], S.part[i + 24][tid]));
+      for (int i = 0; i < 8; ++i)
+        v[i] = __fadd_rn(__fadd_rn(S.part[par][i][lane], S.part[par][i + 16][lane]),
+                         __fadd_rn(S.part[par][i + 8][lane], S.part[par][i + 24][lane]));
 #pragma unroll
-    for (int h = 4; h > 0; h >>= 1)
+      for (int h = 4; h > 0; h >>= 1)
 #pragma unroll
-      for (int i = 0; i < h; ++i) v[i] = __fadd_rn(v[i], v[i + h]);
-    // prob_hid of the two alleles; k_impute_finish turns them into HP
-    const int i = tid >> 1;
-    if (i < n) A.hp[(size_t)t * 2 * A.L + 2 * A.poly[(size_t)t * A.L + l0 + i] + (tid & 1)] = v[0];
+        for (int i = 0; i < h; ++i) v[i] = __fadd_rn(v[i], v[i + h]);
+      // prob_hid of the two alleles; k_impute_finish turns them into HP
+      if ((lane >> 1) <= last) A.hp[(size_t)t * 2 * A.L + 2 * site + (lane & 1)] = v[0];
+    }
+    par ^= 1;
   }
 }
 
@@ -459,12 +482,17 @@ int launch_impute_chain(int J, ImputeWork& w, cudaStream_t s, int first, int cou
 #undef GP_CHAIN
 }
 
+static_assert(2 * kRowSites == 32, "k_impute_block: one lane per sum of a block");
+
 int launch_impute_block(int max_poly, ImputeWork& w, float* hp, cudaStream_t s, int first, int count) {
   ChainArgs a;
   if (chain_args(w, hp, first, count, a) != GP_OK) return GP_E_ARG;
   const int blocks = (max_poly + kRowSites - 1) / kRowSites;
   if (a.count == 0 || blocks == 0) return GP_OK;
-  k_impute_block<<<dim3(blocks, a.count), kBlockThreads, 0, s>>>(a);
+  // Blocks per CTA: enough to hide the loads of each, while some eight CTAs per SM are left.
+  const long long total = (long long)blocks * a.count;
+  const int per = (int)std::max(1ll, std::min(16ll, total / (8 * 148)));
+  k_impute_block<<<dim3((blocks + per - 1) / per, a.count), kBlockThreads, 0, s>>>(a, per);
   return GP_OK;
 }
 
