@@ -691,10 +691,24 @@ int Context::run_phase(const int32_t* d_tsel, const std::vector<int32_t>& tsel_h
     cls.push_back(c1);
     const int nside = (int)cls.size() - 2;
     if ((e = fork_streams(nside)) != cudaSuccess) return cuda_fail(e, "phasing streams");
+    // Classes whose chains run two warps instead of four (fewer instructions a
+    // site in all, a longer site). It pays where chains wait for issue slots, from
+    // about three chains per SM on: with 400 chains four warps were the faster
+    // (K 200-600: 29.9 against 31.7 ms). Chains of a mixed batch finish together when
+    // the heavy ones keep four: 512 chains at K 400-1,200 50.9 ms with classes 2 and
+    // 3 narrow, 60.8 with none, 56.8 with all. Where one class holds most chains, all
+    // of them: K 700-1,000 49.0 against 54.0 ms, K 1,000-1,200 61.9 against 81.3.
+    uint32_t narrow = 0;
+    if (2 * (c1 - c0) >= 3 * sm_count) {
+      int most = 0;
+      for (int i = 0; i <= nside; ++i) most = std::max(most, cls[i + 1] - cls[i]);
+      narrow = 4 * most >= 3 * (c1 - c0) ? (2u << kPhaseNarrowJ) - 1u : (1u << 2) | (1u << 3);
+    }
     for (int i = 0; i <= nside; ++i) {
       PhaseStore Sc = S;
       Sc.order = S.order + cls[i];
-      if (launch_phase_chain(class_of(order[cls[i]]), d_tsel, cls[i + 1] - cls[i], w.nstates.as<int32_t>(),
+      const int J = class_of(order[cls[i]]);
+      if (launch_phase_chain(J, J <= kPhaseNarrowJ && ((narrow >> J) & 1u), d_tsel, cls[i + 1] - cls[i], w.nstates.as<int32_t>(),
                              w.hvar.as<uint32_t>(), w.WB, w.Kp, w.npoly.as<int32_t>(), V, Sc, mc,
                              i == 0 ? stream : side[i - 1].s) != GP_OK)
         return (fail(GP_E_ARG, "phasing: too many states"), GP_E_ARG);
@@ -702,7 +716,7 @@ int Context::run_phase(const int32_t* d_tsel, const std::vector<int32_t>& tsel_h
     if ((e = join_streams(nside)) != cudaSuccess) return cuda_fail(e, "phasing streams");
     PhaseStore Sc = S;
     Sc.order = S.order + c0;
-    if (launch_phase_units(units, d_tsel, c1 - c0, w.nstates.as<int32_t>(), w.hvar.as<uint32_t>(), w.WB, w.Kp, V, Sc,
+    if (launch_phase_units(units, narrow, d_tsel, c1 - c0, w.nstates.as<int32_t>(), w.hvar.as<uint32_t>(), w.WB, w.Kp, V, Sc,
                            cfg.seed, iteration, d_target_ids, stream) != GP_OK)
       return cuda_fail(cudaGetLastError(), "phasing: shared-memory attribute");
     prof.kernel_launches += nside + 3;
@@ -766,6 +780,7 @@ int gp_ctx_create(const gp_panel_desc* panel, const gp_config* cfg, gp_ctx** out
     const long v = std::strtol(cap, nullptr, 10);
     if (v >= 1 && v <= 65535) c->grid_y_cap = (int)v;
   }
+  if (cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, cfg->device) != cudaSuccess) return GP_E_CUDA;
   if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) return GP_E_CUDA;
   int rc = c->create_panel(*panel);
   if (rc != GP_OK) {

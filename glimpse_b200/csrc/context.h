@@ -119,6 +119,7 @@ struct Context {
   int fixed_porder = 0;  // the caller's phasing placement, reported back; every placement runs the same launches
   // phase-1 ms for 1, 2, 4 chains per CTA; sweep ms for 1, 2, 4, 8; k_phase ms for placements 1, 2
   float tune_ms[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+  int sm_count = 0;
   // streams beside `stream` for launches that run together (fork_streams / join_streams)
   struct SideStream {
     cudaStream_t s = nullptr;

@@ -143,7 +143,7 @@ __device__ __forceinline__ void run_chain(const ChainArgs& A, ChainSmem& S, int 
   int i = l_first & 31;
   uint32_t m = 1u << i;
   const float4* rp = nullptr;
-  float4 rec;
+  float4 rec = make_float4(1.f, 1.f, 0.f, 0.f);
 
   // Site i of the block; INIT: the first one of the chain, whose pre-emission value is 1/K.
   auto step = [&](auto init_tag) {

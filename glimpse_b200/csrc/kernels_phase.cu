@@ -202,15 +202,16 @@ __device__ __forceinline__ float transition(const double* __restrict__ cm, int p
 // A chain is bound by the latency of one VAR site: totals -> two divisions ->
 // the state loop -> the sums over states -> totals, with about one warp per
 // scheduler, so every instruction of a site counts. The shape follows from that:
-//  - Four warps of two virtual warps each; a thread holds the 8 hypothesis
-//    messages of its 2 J states in registers, as packed pairs. J is exact: a
-//    launch holds the targets with 256 (J - 1) < K <= 256 J, so only the last
-//    two slots can be empty and the state loop is one straight-line block.
+//  - Four warps of V = 2 virtual warps each (two of V = 4 where many chains share an
+//    SM, Context::run_phase); a thread holds the 8 hypothesis messages of its V J
+//    states in registers, as packed pairs. J is exact: a launch holds the targets
+//    with 256 (J - 1) < K <= 256 J, so only the last V slots can be empty and the
+//    state loop is one straight-line block.
 //  - Register slot s of lane `lane` holds hypothesis s ^ f, f a function of the
 //    lane: the reduce-scatter over the lanes then always keeps its lower slots
-//    and sends its upper ones, with no selects. The upper half warp also holds
-//    the two virtual warps in swapped order, so the first level scatters the
-//    virtual warps and 17 shuffles reduce 16 values.
+//    and sends its upper ones, with no selects. The virtual warps are held in
+//    lane-swapped order too, so the first levels scatter them and 17 (V = 2) or 33
+//    (V = 4) shuffles reduce 16 or 32 values.
 //  - The warps' sums meet in shared memory behind the site's only barrier, in
 //    four copies (one per f % 4), so that every lane reads all 8 totals in its
 //    own slot order with 16-byte loads from one 128-byte row per warp.
@@ -227,11 +228,10 @@ __device__ __forceinline__ float transition(const double* __restrict__ cm, int p
 // site at J = 2; two warps of one virtual warp each instead of one of two: slower
 // at 11 targets (16.1 against 14.2 ms, first version) and at 256.
 // ---------------------------------------------------------------------------
-constexpr int CT = 128;       // threads of a chain
-constexpr int CW = CT / 32;   // warps
-
+// V virtual warps per warp: 8 / V warps, 256 / V threads a chain.
+template <int V>
 struct ChainShared {
-  float4 red[2][CW][4][2];  // [buffer][warp][copy][slots 0-3 / 4-7]
+  float4 red[2][8 / V][4][2];  // [buffer][warp][copy][slots 0-3 / 4-7]
   int4 rec[128];            // ring of four chunks of 32 records
   float* rows;     // the chain's stored messages: segments, then flat hets
   float* segsum;   // their sums and totals
@@ -243,23 +243,51 @@ struct ChainShared {
 __device__ __forceinline__ f2 lo2(float4 v) { return f2_pack(v.x, v.y); }
 __device__ __forceinline__ f2 hi2(float4 v) { return f2_pack(v.z, v.w); }
 
-// A warp's sums of its two virtual warps over the lanes, added: hypothesis
-// lane_class(lane) of the pair, the same in the four lanes of that class.
-__device__ __forceinline__ float warp_scatter(const f2 (&part)[2][4]) {
+// Set s of a lane's registers holds virtual warp V * warp + (s ^ set_swap), slot s
+// hypothesis s ^ lane_class.
+template <int V>
+__device__ __forceinline__ int set_swap(int lane) { return V == 2 ? lane >> 4 : lane >> 3; }
+template <int V>
+__device__ __forceinline__ int lane_class(int lane) { return V == 2 ? (lane >> 1) & 7 : lane & 7; }
+// The copy of the sums that a lane writes: the four lanes of a class write all four.
+template <int V>
+__device__ __forceinline__ int lane_copy(int lane) { return V == 2 ? (lane & 1) | ((lane >> 4) << 1) : lane >> 3; }
+
+// A warp's sums of its virtual warps over the lanes, added: hypothesis lane_class,
+// the same in the four lanes of that class.
+template <int V>
+__device__ __forceinline__ float warp_scatter(const f2 (&part)[V][4]) {
   f2 v[4];
   float x, y;
+  if constexpr (V == 2) {
 #pragma unroll
-  for (int q = 0; q < 4; ++q) v[q] = f2_add(part[0][q], shfl_x(part[1][q], 16));
-  v[0] = f2_add(v[0], shfl_x(v[2], 8));
-  v[1] = f2_add(v[1], shfl_x(v[3], 8));
-  v[0] = f2_add(v[0], shfl_x(v[1], 4));
-  f2_unpack(v[0], x, y);
-  x = __fadd_rn(x, shfl_x(y, 2));
-  x = __fadd_rn(x, shfl_x(x, 1));
-  return __fadd_rn(x, shfl_x(x, 16));
+    for (int q = 0; q < 4; ++q) v[q] = f2_add(part[0][q], shfl_x(part[1][q], 16));
+    v[0] = f2_add(v[0], shfl_x(v[2], 8));
+    v[1] = f2_add(v[1], shfl_x(v[3], 8));
+    v[0] = f2_add(v[0], shfl_x(v[1], 4));
+    f2_unpack(v[0], x, y);
+    x = __fadd_rn(x, shfl_x(y, 2));
+    x = __fadd_rn(x, shfl_x(x, 1));
+    return __fadd_rn(x, shfl_x(x, 16));
+  } else {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      v[q] = f2_add(part[0][q], shfl_x(part[2][q], 16));
+      const f2 u = f2_add(part[1][q], shfl_x(part[3][q], 16));
+      v[q] = f2_add(v[q], shfl_x(u, 8));
+    }
+    v[0] = f2_add(v[0], shfl_x(v[2], 4));
+    v[1] = f2_add(v[1], shfl_x(v[3], 4));
+    v[0] = f2_add(v[0], shfl_x(v[1], 2));
+    f2_unpack(v[0], x, y);
+    x = __fadd_rn(x, shfl_x(y, 1));
+    x = __fadd_rn(x, shfl_x(x, 8));
+    return __fadd_rn(x, shfl_x(x, 16));
+  }
 }
 
 // The totals over the warps, tot[q] = slots (2q, 2q + 1) of a lane of class f.
+template <int CW>
 __device__ __forceinline__ void read_totals(const float4 (*red)[4][2], int f, f2 (&tot)[4]) {
   f2 t[CW][4];
 #pragma unroll
@@ -272,7 +300,10 @@ __device__ __forceinline__ void read_totals(const float4 (*red)[4][2], int f, f2
     t[w][3] = hi2(b);
   }
 #pragma unroll
-  for (int q = 0; q < 4; ++q) tot[q] = f2_add(f2_add(t[0][q], t[1][q]), f2_add(t[2][q], t[3][q]));
+  for (int q = 0; q < 4; ++q) {
+    tot[q] = f2_add(t[0][q], t[1][q]);
+    if (CW == 4) tot[q] = f2_add(tot[q], f2_add(t[CW - 2][q], t[CW - 1][q]));
+  }
 }
 
 __device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
@@ -305,13 +336,13 @@ __device__ __forceinline__ void het_update(f2 (&prob)[NS][4], const uint32_t (&w
   }
 }
 
-template <int J>
-__global__ void __launch_bounds__(CT, J <= 2 ? 5 : J <= 4 ? 4 : J <= 5 ? 3 : 2)
+template <int J, int V>
+__global__ void __launch_bounds__(256 / V, V == 4 ? (J <= 3 ? 6 : 4) : J <= 2 ? 5 : J <= 4 ? 4 : J <= 5 ? 3 : 2)
     k_phase_chain(const int32_t* __restrict__ tsel, const int32_t* __restrict__ nstates,
                   const int32_t* __restrict__ npoly, const uint32_t* __restrict__ hvar, int WB, int Kp, PhaseVars P,
                   PhaseStore S, ModelConst mc) {
-  constexpr int NS = 2 * J;
-  __shared__ ChainShared sm;
+  constexpr int NS = V * J, CW = 8 / V, CT = 32 * CW;
+  __shared__ ChainShared<V> sm;
   __shared__ uint32_t words[2][NS][CT];  // Hvar words of two 32-site blocks, each thread's own
   const int b = S.order[blockIdx.x >> 1];
   const bool fwd = blockIdx.x & 1;
@@ -320,22 +351,21 @@ __global__ void __launch_bounds__(CT, J <= 2 ? 5 : J <= 4 ? 4 : J <= 5 ? 3 : 2)
   const int nv = P.nvar[b];
   if (nv == 0) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int f = (lane >> 1) & 7;                        // slot s holds hypothesis s ^ f
-  const int copy = (lane & 1) | ((lane >> 4) << 1);     // the copy of the sums that this lane writes
+  const int f = lane_class<V>(lane), copy = lane_copy<V>(lane);
   const uint32_t* hv = hvar + (size_t)t * WB * Kp;
   const int nblk_poly = (npoly[t] + 31) >> 5;
   const int4* recs = (fwd ? P.recf : P.recb) + (size_t)b * P.lv;
-  // slot (j, s): state k = 256 j + kb[s]; the virtual warps swapped in the upper half warp
-  int kb[2];
-  bool last[2];
-  f2 exists[2];
+  // slot i = V j + s: state k = 256 j + kb[s]
+  int kb[V];
+  bool last[V];
+  f2 exists[V];
 #pragma unroll
-  for (int s = 0; s < 2; ++s) {
-    kb[s] = 32 * (2 * warp + (s ^ (lane >> 4))) + lane;
+  for (int s = 0; s < V; ++s) {
+    kb[s] = 32 * (V * warp + (s ^ set_swap<V>(lane))) + lane;
     last[s] = 256 * (J - 1) + kb[s] < K;
     exists[s] = last[s] ? f2_pack(1.f, 1.f) : f2_pack(0.f, 0.f);
   }
-  auto has = [&](int i) { return i < 2 * J - 2 || last[i & 1]; };
+  auto has = [&](int i) { return i < NS - V || last[i % V]; };
 
   f2 prob[NS][4];
   uint32_t w[NS];
@@ -346,7 +376,7 @@ __global__ void __launch_bounds__(CT, J <= 2 ? 5 : J <= 4 ? 4 : J <= 5 ? 3 : 2)
     if (blk < 0 || blk >= nblk_poly) return;
 #pragma unroll
     for (int i = 0; i < NS; ++i)
-      if (has(i)) cp_async4(&words[blk & 1][i][tid], hv + (size_t)blk * Kp + 256 * (i >> 1) + kb[i & 1]);
+      if (has(i)) cp_async4(&words[blk & 1][i][tid], hv + (size_t)blk * Kp + 256 * (i / V) + kb[i % V]);
   };
   auto read_words = [&](int blk) {
 #pragma unroll
@@ -360,7 +390,7 @@ __global__ void __launch_bounds__(CT, J <= 2 ? 5 : J <= 4 ? 4 : J <= 5 ? 3 : 2)
       float v[8];
 #pragma unroll
       for (int q = 0; q < 4; ++q) f2_unpack(prob[i][q], v[2 * q], v[2 * q + 1]);
-      float4* d4 = reinterpret_cast<float4*>(dst + (size_t)(256 * (i >> 1) + kb[i & 1]) * 8);
+      float4* d4 = reinterpret_cast<float4*>(dst + (size_t)(256 * (i / V) + kb[i % V]) * 8);
       d4[f >> 2] = make_float4(v[0], v[1], v[2], v[3]);
       d4[(f >> 2) ^ 1] = make_float4(v[4], v[5], v[6], v[7]);
     }
@@ -485,7 +515,7 @@ __global__ void __launch_bounds__(CT, J <= 2 ? 5 : J <= 4 ? 4 : J <= 5 ? 3 : 2)
       const float np = (1.0f - yt) / sumT;
       const f2 scp = f2_pack(sc, sc);
       f2 ntp = f2_pack(np, np);
-      f2 tF[4], part[2][4];
+      f2 tF[4], part[V][4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) tF[q] = f2_mul(tot[q], scp);
       if (rx & collapse) {  // COLLAPSE: every message of a state becomes their sum (SUMK)
@@ -515,17 +545,17 @@ __global__ void __launch_bounds__(CT, J <= 2 ? 5 : J <= 4 ? 4 : J <= 5 ? 3 : 2)
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           prob[i][q] = f2_mul(f2_fma(prob[i][q], ntp, tF[q]), xx);
-          // the last two slots count by a factor of exactly 1 or 0
-          if (i < 2) part[i][q] = i < NS - 2 ? prob[i][q] : f2_mul(prob[i][q], exists[i]);
-          else part[i & 1][q] = i < NS - 2 ? f2_add(part[i & 1][q], prob[i][q])
-                                           : f2_fma(prob[i][q], exists[i & 1], part[i & 1][q]);
+          // the last V slots count by a factor of exactly 1 or 0
+          if (i < V) part[i][q] = i < NS - V ? prob[i][q] : f2_mul(prob[i][q], exists[i]);
+          else part[i % V][q] = i < NS - V ? f2_add(part[i % V][q], prob[i][q])
+                                           : f2_fma(prob[i][q], exists[i % V], part[i % V][q]);
         }
       }
-      rbase[buf * (CW * 32)] = warp_scatter(part);
+      rbase[buf * (CW * 32)] = warp_scatter<V>(part);
       const uint32_t cx = rx;
       read_rec(s + 1);
       __syncthreads();
-      read_totals(sm.red[buf], f, tot);
+      read_totals<CW>(sm.red[buf], f, tot);
       sumT = hadd8(tot);
       buf ^= 1;
       if (cx & keep) keep_messages(s, cx);
@@ -588,7 +618,8 @@ __global__ void __launch_bounds__(256, 2) k_phase_units(const int32_t* __restric
                                                         const int32_t* __restrict__ nstates,
                                                         const uint32_t* __restrict__ hvar, int WB, int Kp, PhaseVars P,
                                                         PhaseStore S, uint64_t seed, int iteration,
-                                                        const int32_t* __restrict__ target_ids) {
+                                                        const int32_t* __restrict__ target_ids,
+                                                        uint32_t narrow) {
   extern __shared__ __align__(16) char smem_raw[];
   UnitSmem& sm = *reinterpret_cast<UnitSmem*>(smem_raw);
   const int b = S.order[blockIdx.y];
@@ -600,13 +631,14 @@ __global__ void __launch_bounds__(256, 2) k_phase_units(const int32_t* __restric
   const int nu = nb + nmiss;
   if ((int)blockIdx.x >= nu) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int f = (lane >> 1) & 3;  // the chain's slot s of a half holds hypothesis s ^ f
+  const int nj = (K + 255) >> 8;
+  // the chain's slot s of a half holds hypothesis s ^ f
+  const int f = ((narrow >> nj) & 1u ? lane_class<4>(lane) : lane_class<2>(lane)) & 3;
   const float* pool = S.pool + S.pool_off[b];
   const size_t rowf = (size_t)K * 8, fbase = (size_t)(nseg + nmiss) * rowf;
   const int64_t so = S.seg_off[b], mo = S.miss_off[b];
   const int32_t* mrel = P.miss_rel + (size_t)b * P.lv;
   const uint32_t rng_target = target_ids ? (uint32_t)target_ids[b] : (uint32_t)t;
-  const int nj = (K + 255) >> 8;
 
   // Steps in flight. A warp's states are 1 KB of either row, copied in whole 512-byte
   // pieces: lane l takes the 16-byte chunks l and l + 32, half l & 1 of state l >> 1 (+ 16).
@@ -961,25 +993,40 @@ void launch_var_records(const int32_t* tsel, int nb, const int32_t* poly, int L,
   k_var_records<<<dim3(32, nb), 256, 0, s>>>(tsel, poly, L, cm, mc, V);
 }
 
-int launch_phase_chain(int J, const int32_t* tsel, int nb, const int32_t* nstates, const uint32_t* hvar, int WB,
-                       int Kp, const int32_t* npoly, PhaseVars P, PhaseStore S, const ModelConst& mc, cudaStream_t s) {
-#define GP_CHAIN(JJ) \
-  case JJ: k_phase_chain<JJ><<<2 * nb, CT, 0, s>>>(tsel, nstates, npoly, hvar, WB, Kp, P, S, mc); return GP_OK;
-  switch (J) {
-    GP_CHAIN(1) GP_CHAIN(2) GP_CHAIN(3) GP_CHAIN(4) GP_CHAIN(5) GP_CHAIN(6) GP_CHAIN(7) GP_CHAIN(8)
+int launch_phase_chain(int J, bool narrow, const int32_t* tsel, int nb, const int32_t* nstates, const uint32_t* hvar,
+                       int WB, int Kp, const int32_t* npoly, PhaseVars P, PhaseStore S, const ModelConst& mc,
+                       cudaStream_t s) {
+  if (narrow && J > kPhaseNarrowJ) return GP_E_ARG;
+#define GP_CHAIN(JJ, VV) \
+  k_phase_chain<JJ, VV><<<2 * nb, 256 / VV, 0, s>>>(tsel, nstates, npoly, hvar, WB, Kp, P, S, mc)
+  switch (J + (narrow ? 10 : 0)) {
+    case 1: GP_CHAIN(1, 2); break;
+    case 2: GP_CHAIN(2, 2); break;
+    case 3: GP_CHAIN(3, 2); break;
+    case 4: GP_CHAIN(4, 2); break;
+    case 5: GP_CHAIN(5, 2); break;
+    case 6: GP_CHAIN(6, 2); break;
+    case 7: GP_CHAIN(7, 2); break;
+    case 8: GP_CHAIN(8, 2); break;
+    case 11: GP_CHAIN(1, 4); break;
+    case 12: GP_CHAIN(2, 4); break;
+    case 13: GP_CHAIN(3, 4); break;
+    case 14: GP_CHAIN(4, 4); break;
+    case 15: GP_CHAIN(5, 4); break;
     default: return GP_E_ARG;
   }
 #undef GP_CHAIN
+  return GP_OK;
 }
 
-int launch_phase_units(int max_units, const int32_t* tsel, int nb, const int32_t* nstates, const uint32_t* hvar,
-                        int WB, int Kp, PhaseVars P, PhaseStore S, uint64_t seed, int iteration,
-                        const int32_t* target_ids, cudaStream_t s) {
+int launch_phase_units(int max_units, uint32_t narrow, const int32_t* tsel, int nb, const int32_t* nstates,
+                       const uint32_t* hvar, int WB, int Kp, PhaseVars P, PhaseStore S, uint64_t seed, int iteration,
+                       const int32_t* target_ids, cudaStream_t s) {
   if (max_units > 0) {
     if (set_smem_limit_once<k_phase_units>((int)sizeof(UnitSmem)) != cudaSuccess) return GP_E_CUDA;
     const int g = (max_units + kUnitsPerCta - 1) / kUnitsPerCta;
     k_phase_units<<<dim3(g, nb), 256, sizeof(UnitSmem), s>>>(tsel, nstates, hvar, WB, Kp, P, S, seed, iteration,
-                                                             target_ids);
+                                                             target_ids, narrow);
   }
   k_phase_draw<<<(nb + 3) / 4, 128, 0, s>>>(tsel, nb, P, S, seed, iteration, target_ids);
   return GP_OK;

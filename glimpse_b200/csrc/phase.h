@@ -61,13 +61,17 @@ void launch_build_vars(const int32_t* tsel, int nb, const int32_t* poly, const i
 void launch_var_records(const int32_t* tsel, int nb, const int32_t* poly, int L, const double* cm,
                         const ModelConst& mc, PhaseVars V, cudaStream_t s);
 // The backward and forward chains of the nb entries S.order[0 .. nb), all with
-// 256 (J - 1) < K <= 256 J states (S.order may point into a longer order).
-int launch_phase_chain(int J, const int32_t* tsel, int nb, const int32_t* nstates, const uint32_t* hvar, int WB,
-                       int Kp, const int32_t* npoly, PhaseVars P, PhaseStore S, const ModelConst& mc, cudaStream_t s);
+// 256 (J - 1) < K <= 256 J states (S.order may point into a longer order). narrow:
+// two warps a chain instead of four, for J <= kPhaseNarrowJ.
+constexpr int kPhaseNarrowJ = 5;
+int launch_phase_chain(int J, bool narrow, const int32_t* tsel, int nb, const int32_t* nstates, const uint32_t* hvar,
+                       int WB, int Kp, const int32_t* npoly, PhaseVars P, PhaseStore S, const ModelConst& mc,
+                       cudaStream_t s);
 // After the chains, for entries of any K: the units and draws. max_units: the
-// largest count of segment boundaries and flat hets of an entry.
-int launch_phase_units(int max_units, const int32_t* tsel, int nb, const int32_t* nstates, const uint32_t* hvar,
-                       int WB, int Kp, PhaseVars P, PhaseStore S, uint64_t seed, int iteration,
+// largest count of segment boundaries and flat hets of an entry; bit J of narrow: the
+// chains of class J ran narrow.
+int launch_phase_units(int max_units, uint32_t narrow, const int32_t* tsel, int nb, const int32_t* nstates,
+                       const uint32_t* hvar, int WB, int Kp, PhaseVars P, PhaseStore S, uint64_t seed, int iteration,
                        const int32_t* target_ids, cudaStream_t s);
 void launch_phase_writeback(const int32_t* tsel, int nb, const int32_t* poly, const int32_t* polyidx, int L,
                             PhaseVars V, PhaseStore S, const ModelConst& mc, uint64_t seed, int iteration,

@@ -134,6 +134,33 @@ def test_chunked_phasing_matches_single_launch(small_workload, monkeypatch):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("edges", [(40, 300, 600, 900, 1100, 1500), (250, 256), (700, 760, 768, 500), (1030, 1280, 1025)])
+def test_many_chains_match_single_calls(edges):
+    """From about three chains per SM on, the chains of some classes run two warps
+    instead of four (all classes where one holds most chains): 260 targets over
+    mixed and uniform state counts must get the haplotypes they get alone."""
+    from glimpse_b200 import native, synth
+    w = synth.make_panel_and_targets(1600, 500, 0.2, 0.4, 2, ("uniform", 0.3, 1.5), ("fixed", 200), seed=73,
+                                     sparse_maf=0.005)
+    P, T = w.panel, w.targets
+    rng = np.random.default_rng(edges[0])
+    n = 260
+    sets = [np.sort(rng.choice(P.n_ref_haps, size=edges[i % len(edges)], replace=False)).astype(np.uint32)
+            for i in range(n)]
+    h0 = np.stack([_noisy_haps(rng, T.truth[i % 2, 0]) for i in range(n)])
+    h1 = np.stack([_noisy_haps(rng, T.truth[i % 2, 1]) for i in range(n)])
+    flat = np.stack([T.flat[i % 2] for i in range(n)])
+    ctx = native.Context(P)
+    try:
+        g0, g1 = ctx.rephase_batch(sets, h0, h1, flat, 3)
+        for i in list(range(12)) + [100, 177, 259]:
+            a0, a1 = ctx.rephase_batch([sets[i]], h0[i][None], h1[i][None], flat[i][None], 3, target_ids=[i])
+            assert np.array_equal(a0[0], g0[i]) and np.array_equal(a1[0], g1[i]), (i, sets[i].size)
+    finally:
+        ctx.close()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("edges", [(1, 31, 32, 33, 64, 65), (255, 256, 257, 319, 321), (511, 512, 513, 767, 769, 1023),
                                    (1024, 1025, 1535, 1537, 1791, 1793, 2047, 2048)])
 def test_state_count_edges_and_mixed_classes(edges):
