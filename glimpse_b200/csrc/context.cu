@@ -258,6 +258,7 @@ Context::~Context() {
   lig_a.release(); lig_b.release(); lig_s.release(); lig_cnt.release();
   for (DevBuf* b : mlp.all()) b->release();
   tune_tarhap.release();
+  stage.release();
   list_off.release(); list_ids.release(); merged_states.release();
   ckpt.release(); ckpt_sum.release(); ckpt_scratch.release(); loglik.release();
   for (DevBuf* b : learned.all()) b->release();
@@ -864,12 +865,15 @@ int gp_impute_batch(gp_ctx* ctx, int32_t n, const int64_t* states_off, const uin
   if ((e = w.hl.ensure((size_t)n * 2 * L * 4)) != cudaSuccess) return c.cuda_fail(e, "alloc hl");
   if ((e = w.hp.ensure((size_t)n * 2 * L * 4)) != cudaSuccess) return c.cuda_fail(e, "alloc hp");
   if ((e = w.flat.ensure((size_t)n * L)) != cudaSuccess) return c.cuda_fail(e, "alloc flat");
-  cudaMemcpyAsync(w.hl.ptr, hl, (size_t)n * 2 * L * 4, cudaMemcpyHostToDevice, c.stream);
-  cudaMemcpyAsync(w.flat.ptr, flat, (size_t)n * L, cudaMemcpyHostToDevice, c.stream);
+  gp::Prefault pages;  // of the output, while the device works
+  pages.start(hp, (size_t)n * 2 * L * 4);
+  if ((e = c.copy_in(w.hl.ptr, hl, (size_t)n * 2 * L * 4)) != cudaSuccess) return c.cuda_fail(e, "copy hl");
+  if ((e = c.copy_in(w.flat.ptr, flat, (size_t)n * L)) != cudaSuccess) return c.cuda_fail(e, "copy flat");
   int rc = c.build_condsets(n, off, st);
   if (rc != GP_OK) return rc;
   rc = c.run_impute(w.hl.as<float>(), w.flat.as<uint8_t>(), w.hp.as<float>());
   if (rc != GP_OK) return rc;
+  pages.wait();
   cudaMemcpyAsync(hp, w.hp.ptr, (size_t)n * 2 * L * 4, cudaMemcpyDeviceToHost, c.stream);
   if ((e = cudaStreamSynchronize(c.stream)) != cudaSuccess) return c.cuda_fail(e, "impute");
   c.prof_resolve();
@@ -898,9 +902,9 @@ int gp_rephase_batch(gp_ctx* ctx, int32_t n, const int64_t* states_off, const ui
   if ((e = bid.ensure((size_t)n * 4)) != cudaSuccess) return c.cuda_fail(e, "alloc ids");
   std::vector<int32_t> ids(n);
   for (int i = 0; i < n; ++i) ids[i] = target_ids ? target_ids[i] : i;
-  cudaMemcpyAsync(bh0.ptr, h0, (size_t)n * L, cudaMemcpyHostToDevice, c.stream);
-  cudaMemcpyAsync(bh1.ptr, h1, (size_t)n * L, cudaMemcpyHostToDevice, c.stream);
-  cudaMemcpyAsync(bfl.ptr, flat, (size_t)n * L, cudaMemcpyHostToDevice, c.stream);
+  if ((e = c.copy_in(bh0.ptr, h0, (size_t)n * L)) != cudaSuccess) return c.cuda_fail(e, "copy h0");
+  if ((e = c.copy_in(bh1.ptr, h1, (size_t)n * L)) != cudaSuccess) return c.cuda_fail(e, "copy h1");
+  if ((e = c.copy_in(bfl.ptr, flat, (size_t)n * L)) != cudaSuccess) return c.cuda_fail(e, "copy flat");
   cudaMemcpyAsync(bid.ptr, ids.data(), (size_t)n * 4, cudaMemcpyHostToDevice, c.stream);
   rc = c.run_phase(nullptr, {}, n, bh0.as<uint8_t>(), bh1.as<uint8_t>(), bfl.as<uint8_t>(), iteration,
                    bid.as<int32_t>());

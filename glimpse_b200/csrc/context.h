@@ -3,6 +3,7 @@
 #include <string>
 #include <vector>
 
+#include "host_copy.h"
 #include "internal.h"
 #include "learned.h"
 #include "mlp.h"
@@ -62,6 +63,10 @@ struct Context {
   DevPanel panel;
   ImputeWork impute;
   PhaseWork phase;
+  HostStage stage;  // large copies from pageable host memory
+  cudaError_t copy_in(void* dst, const void* src, size_t bytes) {
+    return stage.copy_in(cfg.device, dst, src, bytes, stream);
+  }
   DevBuf scratch_h0, scratch_h1, scratch_ids;
   DevBuf glin_src, glin_nval, glin_ploidy, glin_gl, glin_flat, glin_err;  // gp_gl_from_pl / gp_gl_from_float
   DevBuf out_gp, out_site;                                                 // gp_output_records

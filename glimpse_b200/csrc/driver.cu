@@ -54,8 +54,8 @@ int Context::set_targets(int n, const uint8_t* gl, const uint8_t* flat, const in
   if ((e = T.dip_list.ensure(std::max<size_t>(1, T.diploid.size()) * 4)) != cudaSuccess)
     return cuda_fail(e, "alloc targets");
   if ((e = T.bitmap.ensure((size_t)n * ((panel.N + 31) / 32) * 4)) != cudaSuccess) return cuda_fail(e, "alloc");
-  cudaMemcpyAsync(T.gl.ptr, gl, nL * 3, cudaMemcpyHostToDevice, stream);
-  cudaMemcpyAsync(T.flat.ptr, flat, nL, cudaMemcpyHostToDevice, stream);
+  if ((e = copy_in(T.gl.ptr, gl, nL * 3)) != cudaSuccess) return cuda_fail(e, "copy targets");
+  if ((e = copy_in(T.flat.ptr, flat, nL)) != cudaSuccess) return cuda_fail(e, "copy targets");
   cudaMemcpyAsync(T.ploidy.ptr, ploidy, n * 4, cudaMemcpyHostToDevice, stream);
   if (!T.diploid.empty())
     cudaMemcpyAsync(T.dip_list.ptr, T.diploid.data(), T.diploid.size() * 4, cudaMemcpyHostToDevice, stream);
@@ -381,6 +381,11 @@ int gp_gp_get(gp_ctx* ctx, float* gp0, float* gp1, float* ds, uint8_t* gt0, uint
   Context& c = *C_(ctx);
   if (!c.tw.finalized) return (c.fail(GP_E_STATE, "gp_finalize has not run"), GP_E_STATE);
   const size_t nL = (size_t)c.tw.n * c.panel.L;
+  {
+    gp::Prefault pages;
+    for (void* p : {(void*)gp0, (void*)gp1, (void*)ds}) if (p) pages.start(p, nL * 4);
+    for (void* p : {(void*)gt0, (void*)gt1}) if (p) pages.start(p, nL);
+  }
   if (gp0) cudaMemcpyAsync(gp0, c.tw.gp0.ptr, nL * 4, cudaMemcpyDeviceToHost, c.stream);
   if (gp1) cudaMemcpyAsync(gp1, c.tw.gp1.ptr, nL * 4, cudaMemcpyDeviceToHost, c.stream);
   if (ds) cudaMemcpyAsync(ds, c.tw.ds.ptr, nL * 4, cudaMemcpyDeviceToHost, c.stream);

@@ -133,7 +133,11 @@ int gl_input(Context& c, int32_t n, int32_t L, const T* src, const int32_t* site
       (site_nval && (e = c.glin_nval.ensure((size_t)L * 4)) != cudaSuccess))
     return finish(c.cuda_fail(e, "gl input: alloc"));
   cudaStream_t s = c.stream;
-  cudaMemcpyAsync(c.glin_src.ptr, src, nent * P * sizeof(T), cudaMemcpyHostToDevice, s);
+  Prefault pages;  // of the outputs, while the input is copied
+  pages.start(gl, nent * 3);
+  pages.start(flat, nent);
+  if ((e = c.copy_in(c.glin_src.ptr, src, nent * P * sizeof(T))) != cudaSuccess)
+    return finish(c.cuda_fail(e, "gl input: copy in"));
   cudaMemcpyAsync(c.glin_ploidy.ptr, ploidy, (size_t)n * 4, cudaMemcpyHostToDevice, s);
   if (site_nval) cudaMemcpyAsync(c.glin_nval.ptr, site_nval, (size_t)L * 4, cudaMemcpyHostToDevice, s);
   cudaMemsetAsync(c.glin_err.ptr, 0xff, 8, s);
@@ -153,6 +157,7 @@ int gl_input(Context& c, int32_t n, int32_t L, const T* src, const int32_t* site
                                          std::to_string(sample) + "] at site [" + std::to_string(site) + "]"),
                    GP_E_DATA));
   }
+  pages.wait();
   cudaMemcpyAsync(gl, c.glin_gl.ptr, nent * 3, cudaMemcpyDeviceToHost, s);
   cudaMemcpyAsync(flat, c.glin_flat.ptr, nent, cudaMemcpyDeviceToHost, s);
   if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return finish(c.cuda_fail(e, "gl input: copy out"));

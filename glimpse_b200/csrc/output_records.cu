@@ -163,6 +163,10 @@ extern "C" int gp_output_records(gp_ctx* ctx, float* gp, float* raf, float* af, 
                                                      T.gpflags.as<uint8_t>(), T.gp0.as<float>(), T.gp1.as<float>(),
                                                      c.panel.cref, c.panel.calt, d_gp, d_raf, d_af, d_info);
   c.prof.kernel_launches += 1;
+  {
+    gp::Prefault pages;  // while the kernel runs
+    pages.start(gp, nL * 3 * 4);
+  }
   cudaMemcpyAsync(gp, d_gp, nL * 3 * 4, cudaMemcpyDeviceToHost, c.stream);
   cudaMemcpyAsync(raf, d_raf, (size_t)L * 4, cudaMemcpyDeviceToHost, c.stream);
   cudaMemcpyAsync(af, d_af, (size_t)L * 4, cudaMemcpyDeviceToHost, c.stream);

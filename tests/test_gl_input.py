@@ -144,3 +144,23 @@ def test_gl_input_batched_shape(small_workload):
         ctx.close()
     want_gl, want_flat = G.gl_input("PL", src, ploidy)
     assert np.array_equal(gl, want_gl) and np.array_equal(flat, want_flat)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,L", [(1, 699050), (1, 699051), (7, 250001)])
+def test_gl_input_staged_copy_edges(small_workload, n, L):
+    """Inputs just below and above 8 MiB, the size from which pageable memory is
+    copied through staging buffers (a last piece of 4 bytes), and one whose pieces
+    reuse the buffers. The second call on the context has other values."""
+    from glimpse_b200 import native
+    rng = np.random.default_rng(L)
+    ploidy = np.full(n, 2, np.int32)
+    ctx = native.Context(small_workload.panel)
+    try:
+        for _ in range(2):
+            src = rng.integers(0, 300, size=(L, n, 3), dtype=np.int32)
+            gl, flat = ctx.gl_from_format("PL", src, ploidy)
+            want_gl, want_flat = G.gl_input("PL", src, ploidy)
+            assert np.array_equal(gl, want_gl) and np.array_equal(flat, want_flat)
+    finally:
+        ctx.close()
