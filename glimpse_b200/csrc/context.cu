@@ -260,7 +260,7 @@ Context::~Context() {
   tune_tarhap.release();
   stage.release();
   list_off.release(); list_ids.release(); merged_states.release();
-  ckpt.release(); ckpt_sum.release(); ckpt_scratch.release(); loglik.release();
+  ckpt.release(); ckpt_sum.release(); loglik.release();
   for (DevBuf* b : learned.all()) b->release();
   if (phase_err_host) cudaFreeHost(phase_err_host);
   for (SideStream& x : side) {
@@ -385,7 +385,13 @@ int Context::run_impute(const float* d_hl, const uint8_t* d_flat, float* d_hp) {
   if ((e = w.em.ensure((size_t)n * L * 16)) != cudaSuccess) return cuda_fail(e, "alloc em");
   if ((e = w.tr.ensure((size_t)n * L * 8)) != cudaSuccess) return cuda_fail(e, "alloc tr");
   if ((e = w.fl.ensure((size_t)n * L)) != cudaSuccess) return cuda_fail(e, "alloc fl");
-  if (precision_mode != GP_PRECISION_FULL) return run_impute_ckpt(d_hl, d_flat, d_hp);
+  // The checkpointed modes (kernels_impute_ckpt.cu): chains of their own, the same blocks.
+  const bool ck = precision_mode != GP_PRECISION_FULL, bf16 = precision_mode == GP_PRECISION_CKPT_BF16;
+  if (ck) {
+    if (bf16 && (e = ckpt.ensure((size_t)2 * n * w.WB * w.Kp * 2)) != cudaSuccess) return cuda_fail(e, "alloc ckpt");
+    if ((e = ckpt_sum.ensure((size_t)n * w.WB * 32 * 4)) != cudaSuccess) return cuda_fail(e, "alloc ckpt");
+    if ((e = loglik.ensure((size_t)n * 8)) != cudaSuccess) return cuda_fail(e, "alloc loglik");
+  }
   if ((e = w.row_off.ensure((size_t)n * 8)) != cudaSuccess) return cuda_fail(e, "alloc row offsets");
   // Chains of the longest haplotypes (most poly sites) are launched first.
   std::vector<int32_t> order(n);
@@ -416,8 +422,8 @@ int Context::run_impute(const float* d_hl, const uint8_t* d_flat, float* d_hp) {
   if ((e = w.rows.ensure((size_t)std::max<int64_t>(need, 4))) != cudaSuccess) return cuda_fail(e, "alloc rows");
   if ((e = w.fac.ensure((size_t)2 * n * w.WB * 32 * 4)) != cudaSuccess) return cuda_fail(e, "alloc factors");
   if ((e = w.order.ensure((size_t)n * 4)) != cudaSuccess) return cuda_fail(e, "alloc order");
-  // Within a chunk: the classes of 128 (J - 1) < K <= 128 J states, largest J first.
-  auto class_of = [&](int i) { return impute_groups(host_nstates[i]); };
+  // Within a chunk: the classes of 128 (J - 1) < K <= 128 J states (256 in the checkpointed modes), largest J first.
+  auto class_of = [&](int i) { return ck ? (host_nstates[i] + 255) / 256 : impute_groups(host_nstates[i]); };
   for (size_t c = 0; c + 1 < chunk_start.size(); ++c)
     std::stable_sort(order.begin() + chunk_start[c], order.begin() + chunk_start[c + 1],
                      [&](int x, int y) { return class_of(x) > class_of(y); });
@@ -437,9 +443,16 @@ int Context::run_impute(const float* d_hl, const uint8_t* d_flat, float* d_hp) {
     if (fork_streams(nside) != cudaSuccess) return GP_E_CUDA;
     int rc = GP_OK;
     for (int i = 0; i < nc && rc == GP_OK; ++i) {
-      const int q = i % (nside + 1);
-      rc = launch_impute_chain(class_of(order[cls[i]]), w, q == 0 ? stream : side[q - 1].s, cls[i],
-                               cls[i + 1] - cls[i], cpc);
+      const int q = i % (nside + 1), J = class_of(order[cls[i]]), cnt = cls[i + 1] - cls[i];
+      cudaStream_t cs = q == 0 ? stream : side[q - 1].s;
+      if (ck) {
+        int np_max = 0;
+        for (int j = cls[i]; j < cls[i + 1]; ++j) np_max = std::max(np_max, impute_np[order[j]]);
+        rc = launch_impute_ckpt(J, bf16, np_max, w, ckpt.ptr, ckpt_sum.as<float>(), cs, cls[i], cnt);
+        prof.kernel_launches += bf16 ? 2 : 1;
+        continue;
+      }
+      rc = launch_impute_chain(J, w, cs, cls[i], cnt, cpc);
       prof.kernel_launches += 1;
     }
     if (join_streams(nside) != cudaSuccess) return GP_E_CUDA;
@@ -448,7 +461,7 @@ int Context::run_impute(const float* d_hl, const uint8_t* d_flat, float* d_hp) {
   cudaEvent_t ea;
   prof_begin(ea);
   int cpc = fixed_cpc ? fixed_cpc : tune_cpc;
-  if (!cpc) {
+  if (!cpc && !ck) {
     // Autotune chains per CTA on this batch's first chunk: the chains only write
     // their rows and factors, so the runs repeat the same work; the real run
     // follows. A run before the first timed one loads the kernels.
@@ -483,45 +496,20 @@ int Context::run_impute(const float* d_hl, const uint8_t* d_flat, float* d_hp) {
     int lrc = run_chains(c, cpc);
     int np_max = 0;
     for (int j = c0; j < c1; ++j) np_max = std::max(np_max, impute_np[order[j]]);
-    if (lrc == GP_OK) lrc = launch_impute_block(np_max, w, d_hp, stream, c0, c1 - c0);
+    if (lrc == GP_OK) lrc = launch_impute_block(ck, np_max, w, d_hp, stream, c0, c1 - c0);
     if (lrc == GP_E_CUDA) return cuda_fail(cudaGetLastError(), "imputation: launch");
     if (lrc != GP_OK) return (fail(GP_E_ARG, "imputation: too many states"), GP_E_ARG);
     prof.kernel_launches += 1;
   }
   prof_end(ea, 0, cells);
   impute_chunks = (int)chunk_start.size() - 1;
+  if (ck) {
+    launch_ckpt_loglik(w, ckpt_sum.as<float>(), loglik.as<double>(), stream);
+    prof.kernel_launches += 1;
+    loglik_n = n;
+  }
   launch_impute_finish(panel, mc, w, d_hl, d_flat, d_hp, stream);
   prof.kernel_launches += 2;
-  if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "imputation launch");
-  return GP_OK;
-}
-
-// The checkpointed variant (kernels_impute_ckpt.cu): checkpoint rows every 32
-// polymorphic sites (FP32 or BF16), recompute in the backward pass, FP64 chunk
-// log-likelihood per haplotype into d_loglik.
-int Context::run_impute_ckpt(const float* d_hl, const uint8_t* d_flat, float* d_hp) {
-  ImputeWork& w = impute;
-  const int n = w.n;
-  const bool bf16 = precision_mode == GP_PRECISION_CKPT_BF16;
-  cudaError_t e;
-  // alpha and beta checkpoints and their sums, one 32-row scratch per chain,
-  // the log-likelihood and its first half
-  if ((e = ckpt.ensure((size_t)2 * n * w.WB * w.Kp * (bf16 ? 2 : 4))) != cudaSuccess) return cuda_fail(e, "alloc ckpt");
-  if ((e = ckpt_sum.ensure((size_t)2 * n * w.WB * 4)) != cudaSuccess) return cuda_fail(e, "alloc ckpt");
-  if ((e = ckpt_scratch.ensure((size_t)2 * n * 32 * w.Kp * 4)) != cudaSuccess) return cuda_fail(e, "alloc ckpt");
-  if ((e = loglik.ensure((size_t)2 * n * 8)) != cudaSuccess) return cuda_fail(e, "alloc loglik");
-  launch_site_records(panel, mc, w, d_hl, d_flat, stream);
-  double cells = 0;
-  for (int i = 0; i < n; ++i) cells += (double)impute_np[i] * (double)host_nstates[i];
-  cudaEvent_t ea;
-  prof_begin(ea);
-  if (launch_impute_ckpt(w, bf16, ckpt.ptr, ckpt_sum.as<float>(), ckpt_scratch.as<float>(), loglik.as<double>(),
-                         d_hp, stream) != GP_OK)
-    return (fail(GP_E_ARG, "imputation: too many states"), GP_E_ARG);
-  prof_end(ea, 0, cells);
-  launch_impute_finish(panel, mc, w, d_hl, d_flat, d_hp, stream);
-  prof.kernel_launches += 4;
-  loglik_n = n;
   if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "imputation launch");
   return GP_OK;
 }

@@ -111,9 +111,8 @@ struct Context {
   int build_condsets(int n, const std::vector<int64_t>& off, const std::vector<uint32_t>& states);
   int run_impute(const float* d_hl, const uint8_t* d_flat, float* d_hp);
   size_t store_budget(size_t held, size_t need);
-  int run_impute_ckpt(const float* d_hl, const uint8_t* d_flat, float* d_hp);
   int precision_mode = GP_PRECISION_FULL;
-  DevBuf ckpt, ckpt_sum, ckpt_scratch, loglik;  // checkpointed imputation (kernels_impute_ckpt.cu)
+  DevBuf ckpt, ckpt_sum, loglik;  // checkpointed imputation: BF16 rows, AlphaSums, log-likelihoods
   int loglik_n = 0;                             // entries of the last checkpointed imputation call
   int impute_chunks = 0;  // launches pairs of the last run_impute (1 when the whole batch fit)
   int phase_chunks = 0;   // k_phase launches of the last run_phase

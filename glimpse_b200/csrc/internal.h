@@ -157,13 +157,17 @@ constexpr int kRowSites = 16;
 int launch_impute_chain(int J, ImputeWork& w, cudaStream_t s, int first = 0, int count = -1, int cpc = 1);
 // After the chains, for haplotypes of any K with at most max_poly polymorphic
 // sites: prob_hid of every site into hp.
-int launch_impute_block(int max_poly, ImputeWork& w, float* hp, cudaStream_t s, int first = 0, int count = -1);
+int launch_impute_block(bool ck, int max_poly, ImputeWork& w, float* hp, cudaStream_t s, int first = 0, int count = -1);
 // Rows of 128 states that a chain of K states runs (the J of launch_impute_chain).
 int impute_groups(int K);
-// The checkpointed forward-backward (kernels_impute_ckpt.cu) over the batch's
-// conditioning sets: leaves prob_hid pairs in hp for k_impute_finish.
-int launch_impute_ckpt(ImputeWork& w, bool bf16, void* ckpt, float* csum, float* scratch, double* loglik, float* hp,
-                       cudaStream_t s);
+// The chains of the checkpointed modes (kernels_impute_ckpt.cu) for the haplotypes
+// order[first .. first + count), all with 256 (J - 1) < K <= 256 J and at most
+// max_poly polymorphic sites; launch_impute_block follows. ckpt: [2][n][WB][Kp] BF16
+// rows (bf16 only); asum: [n][32 WB].
+int launch_impute_ckpt(int J, bool bf16, int max_poly, ImputeWork& w, void* ckpt, float* asum, cudaStream_t s,
+                       int first, int count);
+// The FP64 log-likelihood of every haplotype from its AlphaSums.
+void launch_ckpt_loglik(ImputeWork& w, const float* asum, double* loglik, cudaStream_t s);
 void launch_impute_finish(const DevPanel& P, const ModelConst& mc, ImputeWork& w, const float* hl,
                         const uint8_t* flat, float* hp, cudaStream_t s);
 

@@ -1,385 +1,315 @@
-// The precision variant of the imputation forward-backward: checkpointed
-// messages with recompute, and an FP64 chunk log-likelihood.
+// The precision variant of the imputation forward-backward: FP32 or BF16
+// checkpoints and an FP64 chunk log-likelihood.
 //
-// Same HMM and same per-site arithmetic as the full-store chains
-// (kernels_impute_warp.cu, after imputation_hmm.cpp:80-353): forward
-// alpha_l = (alpha_{l-1} (1 - t) / AlphaSum_{l-1} + t / K) e_l, backward
-// beta likewise with betaSum, prob_hid of each allele = sum over states of
-// alpha_l x (backward message before the emission at l, 1 at the last site).
-// What differs is what is kept between the passes. As in the full-store
-// chains, each haplotype is split at M (a multiple of 32, about np / 2) into a
-// forward and a backward chain that run concurrently, one CTA each:
-//   phase A  forward  [0, M)      keeps the alpha row after the last site of
-//                                 every block of 32 polymorphic sites, and its
-//                                 AlphaSum
-//            backward [np-1, M]   keeps the beta row after the first site of
-//                                 every block, and its betaSum
-//   phase B  forward  [M, np)     per block: the block's backward messages are
-//                                 recomputed from the next block's checkpoint
-//                                 into a 32-row scratch, then the forward steps
-//                                 form the posteriors from them
-//            backward [M-1, 0]    per block: the block's alpha rows are
-//                                 recomputed from the previous block's
-//                                 checkpoint into the scratch, then the
-//                                 backward steps form the posteriors
-// Checkpoints are FP32, or BF16 for the lower-memory variant; recomputed rows
-// are FP32 (with FP32 checkpoints they equal the first pass's bit for bit).
-// The log of every AlphaSum is accumulated in FP64: the chunk log-likelihood
-// sum_l log AlphaSum_l (the reference keeps no such value).
-// One CTA of 256 threads runs one chain; thread x owns states x + 256 j. The
-// per-site sums are block reductions in one fixed tree.
+// Same HMM, same per-site arithmetic and same division of the work as the full
+// precision path (kernels_impute_warp.cu, after imputation_hmm.cpp:80-353):
+// sequential chains keep the scaling factor of every site and a row per kRowSites
+// sites, and k_impute_block forms the posteriors. What differs:
+//   - The sums over states have another fixed tree (state k: lane k % 32 of virtual
+//     warp (k / 32) % 8; j in order, lanes at distances 16 .. 1, virtual warps at 1,
+//     2, 4), that of the AlphaSums whose logarithms make up the log-likelihood.
+//   - With BF16 checkpoints, each haplotype is split at M (a multiple of 32, about
+//     np / 2). On [0, M) the forward messages, and on [M, np) the backward ones, are
+//     those recomputed from a row rounded to BF16 at the start of each block of 32
+//     sites (k_ckpt_block, one CTA per block: its factors and rows replace the
+//     chain's there), and either chain goes on from a rounded row at M.
+//     Either kernel is bound by its chain of dependent steps: a site per step, of which
+//     the sum over 256 J states, its barrier and its five shuffles are most. A chain has
+//     two warps, so that a lane's states are independent work within a step and the
+//     barrier joins two warps only; with 256 threads and both half passes in sequence,
+//     each a chain of its own, 32 haplotypes (400 - 1,200 states) at 150,000 sites took
+//     65 ms a call, against 27.
+//   - The FP64 chunk log-likelihood sum_l log AlphaSum_l (the reference keeps no such
+//     value), from the AlphaSum of every site, off the chain.
 #include <cuda_bf16.h>
+
+#include <type_traits>
 
 #include "internal.h"
 
 namespace gp {
 namespace {
 
-constexpr int kCT = 256, kCW = kCT / 32;
+constexpr int kCkptThreads = 64;
 
 struct CkptArgs {
-  const int32_t* poly;
-  const int32_t* npoly;
-  const int32_t* nstates;
-  const uint32_t* hvar;
-  const float4* em;
-  const float2* tr;
-  const uint8_t* fl;
+  int count;                // haplotypes of the launch
+  const int32_t* __restrict__ order;
+  const int32_t* __restrict__ npoly;
+  const int32_t* __restrict__ nstates;
+  const uint32_t* __restrict__ hvar;
+  const float4* __restrict__ em;
+  const float2* __restrict__ tr;
+  const uint8_t* __restrict__ fl;
+  const int64_t* __restrict__ row_off;
+  float* __restrict__ rows;  // as k_impute_block reads them: front-padded to 128 ceil(K / 128)
+  float* __restrict__ fac;   // [2][n][32 WB]
+  float* __restrict__ asum;  // [n][32 WB] AlphaSum of every site
+  __nv_bfloat16* __restrict__ ckpt;  // [2][n][WB][Kp] rows entering a block, forward and backward
   int n, L, WB, Kp;
-  void* ckpt;       // [2][t][WB][Kp]: alpha after each block's last site, beta after its first (float or BF16)
-  float* csum;      // [2][t][WB]: AlphaSum / betaSum at those sites
-  float* scratch;   // [t][2][32][Kp]: the recomputed rows of one block, per chain
-  float* hp;        // [t][2L]: (prob_hid 0, prob_hid 1) at each polymorphic site
-  double* llpart;   // [t]: sum of log AlphaSum over [0, M)
-  double* loglik;   // [t]: sum of log AlphaSum over the polymorphic sites
 };
 
-// Sums of N values over the CTA: warp butterflies, then the warps in one tree.
-// The partials alternate between two buffers, so one barrier per reduction
-// suffices: a reduction's writes go to the buffer that the previous one did
-// not read, and the one before that was read before the previous barrier.
-template <int N>
-__device__ __forceinline__ void cta_sum(float (&v)[N], float (*red)[3][kCW], int& buf) {
+// Partial sums: virtual warp v's lane at 32 v + 8 (lane & 3) + (lane >> 2), so that
+// lane 4 v + r of either warp adds the eight lanes = r (mod 4) of v, distances 16, 8
+// and 4, from two 16-byte loads.
+struct CkptSmem {
+  float red[2][256];
+  float4 rec[1 + 4 * 32 + 1];  // emission of allele 0 and 1, t / K and 1 - t into the site
+};
+
+// Steps through the blocks b_first .. b_last (in the direction of the chain).
+// SEG: one block, from its BF16 checkpoint. J: 256 (J - 1) < K <= 256 J.
+template <int J, bool FWD, bool SEG, bool BF16>
+__device__ __forceinline__ void ckpt_run(const CkptArgs& A, CkptSmem& S, int t, int b_first, int b_last) {
+  constexpr int NP = 2 * J;  // packed pairs of states: virtual warps (0, 1) and (2, 3) of the warp, per j
+  const int np = A.npoly[t], K = A.nstates[t];
+  const int tid = threadIdx.x, lane = tid & 31, wi = tid >> 5;
+  const int mblk = ((np / 2) & ~31) >> 5;  // M = 32 mblk
+  const int nrow = (np + kRowSites - 1) / kRowSites;
+  const int Ks = (K + 127) / 128 * 128;
+  // state of pair p: 256 (p / 2) + k0 + 64 (p & 1) (+ 32)
+  const int k0 = 128 * wi + lane;
+  auto state = [&](int p, int h) { return 256 * (p >> 1) + k0 + 64 * (p & 1) + 32 * h; };
+  float* rows = A.rows + A.row_off[t] + (FWD ? 0 : (size_t)nrow * Ks) + (Ks - K);
+  float* fac = A.fac + ((size_t)(FWD ? 0 : A.n) + t) * 32 * A.WB;
+  const uint32_t* hv = A.hvar + (size_t)t * A.WB * A.Kp;
+  __nv_bfloat16* ck = A.ckpt + ((size_t)(FWD ? 0 : A.n) + t) * A.WB * A.Kp;
+  const float4* E = A.em + (size_t)t * A.L;
+  const float2* T = A.tr + (size_t)t * A.L;
+  const uint8_t* F = A.fl + (size_t)t * A.L;
+  constexpr int dir = FWD ? 1 : -1;
+
+  float4 pe = make_float4(0.f, 0.f, 0.f, 0.f);
+  auto load_recs = [&](int b) {
+    const int l = (b << 5) + lane;
+    if (wi != 0 || l >= np) return;
+    const float4 e = E[l];
+    const bool f = F[l] != 0;
+    const float2 tt = FWD ? (l > 0 ? T[l - 1] : make_float2(0.f, 0.f)) : T[l];
+    pe = make_float4(f ? 1.0f : e.x, f ? 1.0f : e.y, tt.x, tt.y);
+  };
+  bool ok[4];  // the last four states
+  f2 exists[2];
 #pragma unroll
-  for (int i = 0; i < N; ++i)
+  for (int i = 0; i < 4; ++i) ok[i] = state(NP - 2 + (i >> 1), i & 1) < K;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v[i] = __fadd_rn(v[i], __shfl_xor_sync(0xFFFFFFFFu, v[i], o));
-  if ((threadIdx.x & 31) == 0)
+  for (int i = 0; i < 2; ++i) exists[i] = f2_pack(ok[2 * i] ? 1.f : 0.f, ok[2 * i + 1] ? 1.f : 0.f);
+  auto has = [&](int p, int h) { return p < NP - 2 || ok[2 * (p - (NP - 2)) + h]; };
+  uint32_t w[2 * NP], wn[2 * NP];
+  auto load_words = [&](int b) {
 #pragma unroll
-    for (int i = 0; i < N; ++i) red[buf][i][threadIdx.x >> 5] = v[i];
-  __syncthreads();
+    for (int p = 0; p < NP; ++p)
 #pragma unroll
-  for (int i = 0; i < N; ++i) {
-    const float4 p = reinterpret_cast<const float4*>(red[buf][i])[0], q = reinterpret_cast<const float4*>(red[buf][i])[1];
-    v[i] = __fadd_rn(__fadd_rn(__fadd_rn(p.x, p.y), __fadd_rn(p.z, p.w)),
-                     __fadd_rn(__fadd_rn(q.x, q.y), __fadd_rn(q.z, q.w)));
+      for (int h = 0; h < 2; ++h) wn[2 * p + h] = has(p, h) ? hv[(size_t)b * A.Kp + state(p, h)] : 0u;
+  };
+  f2 x[NP];
+  auto store_row = [&](int i) {
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+      float v[2];
+      f2_unpack(x[p], v[0], v[1]);
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        if (has(p, h)) rows[(size_t)i * Ks + state(p, h)] = v[h];
+    }
+  };
+  auto round_row = [&]() {
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+      float a, b;
+      f2_unpack(x[p], a, b);
+      x[p] = f2_pack(__bfloat162float(__float2bfloat16_rn(a)), __bfloat162float(__float2bfloat16_rn(b)));
+    }
+  };
+
+  const int l_first = FWD ? b_first << 5 : min(np, (b_first + 1) << 5) - 1;
+  const bool init = FWD ? l_first == 0 : l_first == np - 1;
+  load_recs(b_first);
+  if (wi == 0) S.rec[1 + (b_first & 3) * 32 + lane] = pe;
+  load_words(b_first);
+#pragma unroll
+  for (int p = 0; p < NP; ++p) {
+    float v[2] = {0.f, 0.f};
+    if (SEG && !init) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        if (has(p, h)) v[h] = __bfloat162float(ck[(size_t)b_first * A.Kp + state(p, h)]);
+    }
+    x[p] = f2_pack(v[0], v[1]);
   }
-  buf ^= 1;
+  float acc = 1.f;
+  __syncthreads();
+  const int wofs = 8 * (lane & 3) + (lane >> 2);
+  const ulonglong2* const rin = reinterpret_cast<const ulonglong2*>(&S.red[0][8 * lane]);
+  int parity = 0;
+  float keep = 0.f, keep_sum = 0.f;  // lane i: factor and sum of the block's site i
+  int i = l_first & 31;
+  uint32_t m = 1u << i;
+  const float4* rp = nullptr;
+  float4 rec = make_float4(1.f, 1.f, 0.f, 0.f);
+
+  auto step = [&](auto init_tag) {
+    constexpr bool INIT = decltype(init_tag)::value;
+    const float fact1 = INIT ? 1.0f / (float)K : rec.z;
+    const float fact2 = INIT ? 0.f : rec.w / acc;
+    const f2 f1 = f2_pack(fact1, fact1), f2v = f2_pack(fact2, fact2);
+    const float ex = rec.x, ey = rec.y;
+    if (lane == i) keep = fact2;
+    f2 q[2];
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+      const bool b0 = (w[2 * p] & m) != 0u, b1 = (w[2 * p + 1] & m) != 0u;
+      f2 nx = f2_mul(f2_fma(x[p], f2v, f1), f2_pack(b0 ? ey : ex, b1 ? ey : ex));
+      if (p >= NP - 2) nx = f2_mul(nx, exists[p - (NP - 2)]);  // absent states are multiplied by 0, others by 1
+      q[p & 1] = p < 2 ? nx : f2_add(q[p & 1], nx);
+      x[p] = nx;
+    }
+    float* ro = &S.red[0][parity + 128 * wi + wofs];
+    f2_unpack(q[0], ro[0], ro[32]);
+    f2_unpack(q[1], ro[64], ro[96]);
+    i += dir;
+    m = FWD ? m << 1 : m >> 1;
+    rp += dir;
+    rec = *rp;
+    __syncthreads();
+    const ulonglong2 a = rin[parity >> 2], c = rin[(parity >> 2) + 1];
+    float v0, v1;
+    f2_unpack(f2_add(f2_add(a.x, c.x), f2_add(a.y, c.y)), v0, v1);
+    float v = __fadd_rn(v0, v1);
+    v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 2));
+    v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 1));
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, o));
+    // AlphaSum = 1 at a flat first site, betaSum = 1 at a flat last site (imputation_hmm.cpp:156,285)
+    acc = INIT && F[l_first] != 0 ? 1.0f : v;
+    if (FWD && !SEG && lane == i - dir) keep_sum = acc;
+    parity ^= 256;
+  };
+
+  for (int b = b_first;; b += dir) {
+#pragma unroll
+    for (int p = 0; p < 2 * NP; ++p) w[p] = wn[p];
+    rp = &S.rec[1 + (b & 3) * 32 + i];
+    rec = *rp;
+    if (SEG && !init) rec.w = fac[(b << 5) + i];  // the chain's factor into the block, divided by acc = 1
+    if (b != b_last) {
+      load_recs(b + dir);
+      load_words(b + dir);
+    }
+    // Whether this block's rows are recomputed from its checkpoint (then only that is kept here).
+    const bool again = BF16 && !SEG && (FWD ? b < mblk : b >= mblk);
+    if (BF16 && !SEG && b != b_first) {
+      if (again) {
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+          float v[2];
+          f2_unpack(x[p], v[0], v[1]);
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+            if (has(p, h)) ck[(size_t)b * A.Kp + state(p, h)] = __float2bfloat16_rn(v[h]);
+        }
+      }
+      if (FWD ? b == mblk : b == mblk - 1) round_row();
+    }
+    if (b == b_first && init) step(std::integral_constant<bool, true>());
+    const int end = FWD ? min(np - (b << 5), 32) : -1;
+    while (i != end) {
+      const int part = i / kRowSites;
+      if (!again && (FWD ? i == part * kRowSites : i == (part + 1) * kRowSites - 1))
+        store_row(b * (32 / kRowSites) + part);
+      const int stop = FWD ? min(end, (part + 1) * kRowSites) : part * kRowSites - 1;
+      while (i != stop) step(std::integral_constant<bool, false>());
+    }
+    if (wi == 0) {
+      fac[(b << 5) + lane] = keep;
+      if (FWD && !SEG) A.asum[(size_t)t * 32 * A.WB + (b << 5) + lane] = keep_sum;
+    }
+    if (b == b_last) break;
+    if (wi == 0) S.rec[1 + ((b + dir) & 3) * 32 + lane] = pe;
+    i = FWD ? 0 : 31;
+    m = FWD ? 1u : 1u << 31;
+    __syncthreads();
+  }
 }
 
-// M of the meet-in-the-middle split (as the full-store chains take it).
-__device__ __forceinline__ int ckpt_split(int np) { return (np / 2) & ~31; }
+// Both chains of every haplotype: CTA 2 c forward, 2 c + 1 backward.
+template <int J, bool BF16>
+__global__ void __launch_bounds__(kCkptThreads, 1) k_ckpt_chain(CkptArgs A) {
+  __shared__ CkptSmem S;
+  const int t = A.order[blockIdx.x >> 1];
+  const int nblk = (A.npoly[t] + 31) >> 5;
+  if (nblk == 0 || A.nstates[t] == 0) return;
+  if ((blockIdx.x & 1) == 0) ckpt_run<J, true, false, BF16>(A, S, t, 0, nblk - 1);
+  else ckpt_run<J, false, false, BF16>(A, S, t, nblk - 1, 0);
+}
 
-// Phase A (PB = false) or phase B (PB = true) of one chain: CTA 2 t + role runs
-// haplotype t's forward (role 0) or backward (role 1) chain. J: states per
-// thread, from the launch's largest K.
-template <int J, bool BF16, bool PB>
-__global__ void __launch_bounds__(kCT) k_impute_ckpt(CkptArgs a) {
-  constexpr int kCJ = J;
-  static_assert(kCW == 8, "eight warps");
-  __shared__ __align__(16) float red[2][3][kCW];  // rows of 8 partials read as two float4
-  int buf = 0;
-  const int t = blockIdx.x >> 1, role = blockIdx.x & 1, tid = threadIdx.x;
-  const int np = a.npoly[t], K = a.nstates[t];
-  if (np <= 0 || K <= 0) return;
-  const int M = ckpt_split(np);
-  const int Kp = a.Kp;
-  const uint32_t* hv = a.hvar + (size_t)t * a.WB * Kp;
-  const float4* E = a.em + (size_t)t * a.L;
-  const float2* TR = a.tr + (size_t)t * a.L;
-  const uint8_t* F = a.fl + (size_t)t * a.L;
-  const int32_t* PL = a.poly + (size_t)t * a.L;
-  float* HP = a.hp + (size_t)t * 2 * a.L;
-  float* scr = a.scratch + ((size_t)t * 2 + role) * 32 * Kp;
-  const float invK = 1.0f / (float)K;
-  bool valid[kCJ];
-#pragma unroll
-  for (int j = 0; j < kCJ; ++j) valid[j] = tid + kCT * j < K;
-  uint32_t w[kCJ];
-  auto load_words = [&](int blk) {
-#pragma unroll
-    for (int j = 0; j < kCJ; ++j) w[j] = valid[j] ? hv[(size_t)blk * Kp + tid + kCT * j] : 0u;
-  };
-  // checkpoint d (0 alpha, 1 beta) of block blk
-  auto row_off = [&](int d, int blk, int j) {
-    return (((size_t)d * a.n + t) * a.WB + blk) * Kp + tid + kCT * j;
-  };
-  auto sum_off = [&](int d, int blk) { return ((size_t)d * a.n + t) * a.WB + blk; };
-  auto store_row = [&](int d, int blk, const float (&x)[kCJ]) {
-#pragma unroll
-    for (int j = 0; j < kCJ; ++j) {
-      if (!valid[j]) continue;
-      if (BF16) reinterpret_cast<__nv_bfloat16*>(a.ckpt)[row_off(d, blk, j)] = __float2bfloat16_rn(x[j]);
-      else reinterpret_cast<float*>(a.ckpt)[row_off(d, blk, j)] = x[j];
-    }
-  };
-  auto load_row = [&](int d, int blk, float (&x)[kCJ]) {
-#pragma unroll
-    for (int j = 0; j < kCJ; ++j) {
-      x[j] = 0.f;
-      if (!valid[j]) continue;
-      x[j] = BF16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(a.ckpt)[row_off(d, blk, j)])
-                  : reinterpret_cast<const float*>(a.ckpt)[row_off(d, blk, j)];
-    }
-  };
-  // one forward step at site l from (x, acc) of site l - 1
-  auto fwd_step = [&](int l, float (&x)[kCJ], float& acc) {
-    const uint8_t f = F[l];
-    const float4 e = E[l];
-    const float ex = f ? 1.0f : e.x, ey = f ? 1.0f : e.y;
-    float f1, f2 = 0.f;
-    if (l == 0) {
-      f1 = invK;
-    } else {
-      const float2 tp = TR[l - 1];
-      f1 = tp.x;
-      f2 = tp.y / acc;
-    }
-    const uint32_t m = 1u << (l & 31);
-    float s[1] = {0.f};
-#pragma unroll
-    for (int j = 0; j < kCJ; ++j) {
-      const float pc = l == 0 ? f1 : fmaf(x[j], f2, f1);
-      x[j] = valid[j] ? __fmul_rn(pc, (w[j] & m) ? ey : ex) : 0.f;
-      s[0] = __fadd_rn(s[0], x[j]);
-    }
-    cta_sum<1>(s, red, buf);
-    acc = (l == 0 && f) ? 1.0f : s[0];  // AlphaSum = 1 at a flat first site (imputation_hmm.cpp:156)
-  };
-  // one backward step at site l from (xb, bacc) of site l + 1; pc gets the
-  // message before the emission at l (1 at the last site), as the full store keeps it
-  auto bwd_step = [&](int l, float (&xb)[kCJ], float& bacc, float (&pc)[kCJ]) {
-    const uint8_t f = F[l];
-    const float4 e = E[l];
-    const float ex = f ? 1.0f : e.x, ey = f ? 1.0f : e.y;
-    const bool last = l == np - 1;
-    float f1 = invK, f2 = 0.f;
-    if (!last) {
-      const float2 tt = TR[l];
-      f1 = tt.x;
-      f2 = tt.y / bacc;
-    }
-    const uint32_t m = 1u << (l & 31);
-    float s[1] = {0.f};
-#pragma unroll
-    for (int j = 0; j < kCJ; ++j) {
-      pc[j] = 0.f;
-      if (!valid[j]) continue;
-      const float p = last ? f1 : fmaf(xb[j], f2, f1);
-      pc[j] = last ? 1.0f : p;
-      xb[j] = __fmul_rn(p, (w[j] & m) ? ey : ex);
-      s[0] = __fadd_rn(s[0], xb[j]);
-    }
-    cta_sum<1>(s, red, buf);
-    bacc = (last && f) ? 1.0f : s[0];  // betaSum = 1 at a flat last site (imputation_hmm.cpp:285)
-  };
+// The recomputed block blockIdx.x of haplotype order[blockIdx.y].
+template <int J>
+__global__ void __launch_bounds__(kCkptThreads, 1) k_ckpt_block(CkptArgs A) {
+  __shared__ CkptSmem S;
+  const int t = A.order[blockIdx.y], b = blockIdx.x;
+  const int np = A.npoly[t];
+  if (b >= (np + 31) >> 5 || A.nstates[t] == 0) return;
+  if (b < ((np / 2) & ~31) >> 5) ckpt_run<J, true, true, true>(A, S, t, b, b);
+  else ckpt_run<J, false, true, true>(A, S, t, b, b);
+}
 
-  float x[kCJ], pc[kCJ];
-  if (!PB) {
-    if (role == 0) {
-      // ---- phase A forward over [0, M): alpha checkpoints, log-likelihood ----
-      if (M == 0) return;
-      float acc = 0.f;
-      double ll = 0.0;
-#pragma unroll
-      for (int j = 0; j < kCJ; ++j) x[j] = 0.f;
-      for (int l = 0; l < M; ++l) {
-        if ((l & 31) == 0) load_words(l >> 5);
-        fwd_step(l, x, acc);
-        if (tid == 0) ll += log((double)acc);  // thread 0 alone keeps the FP64 sum
-        if ((l & 31) == 31) {
-          store_row(0, l >> 5, x);
-          if (tid == 0) a.csum[sum_off(0, l >> 5)] = acc;
-        }
-      }
-      if (tid == 0) a.llpart[t] = ll;
-    } else {
-      // ---- phase A backward over [np-1, M]: beta checkpoints ----
-      float bacc = 0.f;
-#pragma unroll
-      for (int j = 0; j < kCJ; ++j) x[j] = 0.f;
-      for (int l = np - 1; l >= M; --l) {
-        if (l == np - 1 || (l & 31) == 31) load_words(l >> 5);
-        bwd_step(l, x, bacc, pc);
-        if ((l & 31) == 0) {
-          store_row(1, l >> 5, x);
-          if (tid == 0) a.csum[sum_off(1, l >> 5)] = bacc;
-        }
-      }
-    }
-    return;
+// Sum of log AlphaSum over the sites of haplotype blockIdx.x, in FP64.
+__global__ void __launch_bounds__(256) k_ckpt_loglik(const float* __restrict__ asum, const int32_t* __restrict__ npoly,
+                                                     int WB, double* __restrict__ loglik) {
+  __shared__ double part[256];
+  const int t = blockIdx.x;
+  double s = 0.0;
+  for (int l = threadIdx.x; l < npoly[t]; l += 256) s += log((double)asum[(size_t)t * 32 * WB + l]);
+  part[threadIdx.x] = s;
+  __syncthreads();
+  for (int o = 128; o > 0; o >>= 1) {
+    if (threadIdx.x < o) part[threadIdx.x] += part[threadIdx.x + o];
+    __syncthreads();
   }
-
-  const int nblk = (np + 31) >> 5;
-  if (role == 0) {
-    // ---- phase B forward over [M, np): per block, the backward messages
-    // recomputed from the next block's checkpoint, then alpha and the posteriors ----
-    float acc = 0.f;
-    double ll = 0.0;
-    if (M > 0) {
-      load_row(0, (M >> 5) - 1, x);
-      acc = a.csum[sum_off(0, (M >> 5) - 1)];
-      ll = a.llpart[t];
-    } else {
-#pragma unroll
-      for (int j = 0; j < kCJ; ++j) x[j] = 0.f;
-    }
-    for (int b = M >> 5; b < nblk; ++b) {
-      const int s0 = b << 5, s1 = min(np, s0 + 32) - 1;
-      load_words(b);
-      float xb[kCJ];
-      float bacc = 0.f;
-      if (b + 1 < nblk) {
-        load_row(1, b + 1, xb);
-        bacc = a.csum[sum_off(1, b + 1)];
-      } else {
-#pragma unroll
-        for (int j = 0; j < kCJ; ++j) xb[j] = 0.f;
-      }
-      for (int l = s1; l >= s0; --l) {
-        bwd_step(l, xb, bacc, pc);
-#pragma unroll
-        for (int j = 0; j < kCJ; ++j)
-          if (valid[j]) scr[(size_t)(l - s0) * Kp + tid + kCT * j] = pc[j];
-      }
-      for (int l = s0; l <= s1; ++l) {
-        const uint8_t f = F[l];
-        const float4 e = E[l];
-        const float ex = f ? 1.0f : e.x, ey = f ? 1.0f : e.y;
-        float f1, f2 = 0.f;
-        if (l == 0) {
-          f1 = invK;
-        } else {
-          const float2 tp = TR[l - 1];
-          f1 = tp.x;
-          f2 = tp.y / acc;
-        }
-        const uint32_t m = 1u << (l & 31);
-        float v[3] = {0.f, 0.f, 0.f};  // AlphaSum, prob_hid 0, prob_hid 1
-#pragma unroll
-        for (int j = 0; j < kCJ; ++j) {
-          const float p = l == 0 ? f1 : fmaf(x[j], f2, f1);
-          const bool bit = (w[j] & m) != 0u;
-          x[j] = valid[j] ? __fmul_rn(p, bit ? ey : ex) : 0.f;
-          v[0] = __fadd_rn(v[0], x[j]);
-          if (!valid[j]) continue;
-          const float d = __fmul_rn(x[j], scr[(size_t)(l - s0) * Kp + tid + kCT * j]);  // alpha x message (1 at the last site)
-          if (bit) v[2] = __fadd_rn(v[2], d);
-          else v[1] = __fadd_rn(v[1], d);
-        }
-        cta_sum<3>(v, red, buf);
-        acc = (l == 0 && f) ? 1.0f : v[0];  // AlphaSum = 1 at a flat first site (imputation_hmm.cpp:156)
-        if (tid == 0) ll += log((double)acc);  // thread 0 alone keeps the FP64 sum
-        if (tid == 0) *reinterpret_cast<float2*>(HP + 2 * PL[l]) = make_float2(v[1], v[2]);
-      }
-    }
-    if (tid == 0) a.loglik[t] = ll;
-  } else {
-    // ---- phase B backward over [M-1, 0]: per block, the alpha rows recomputed
-    // from the previous block's checkpoint, then beta and the posteriors ----
-    if (M == 0) return;
-    float xb[kCJ];
-    load_row(1, M >> 5, xb);
-    float bacc = a.csum[sum_off(1, M >> 5)];
-    for (int b = (M >> 5) - 1; b >= 0; --b) {
-      const int s0 = b << 5, s1 = s0 + 31;
-      load_words(b);
-      float aacc = 0.f;
-      if (b > 0) {
-        load_row(0, b - 1, x);
-        aacc = a.csum[sum_off(0, b - 1)];
-      } else {
-#pragma unroll
-        for (int j = 0; j < kCJ; ++j) x[j] = 0.f;
-      }
-      for (int l = s0; l <= s1; ++l) {
-        fwd_step(l, x, aacc);
-#pragma unroll
-        for (int j = 0; j < kCJ; ++j)
-          if (valid[j]) scr[(size_t)(l - s0) * Kp + tid + kCT * j] = x[j];
-      }
-      for (int l = s1; l >= s0; --l) {  // l < M <= np - 1: never the last site
-        const uint8_t f = F[l];
-        const float4 e = E[l];
-        const float ex = f ? 1.0f : e.x, ey = f ? 1.0f : e.y;
-        const float2 tt = TR[l];
-        const float f1 = tt.x, f2 = tt.y / bacc;
-        const uint32_t m = 1u << (l & 31);
-        float v[3] = {0.f, 0.f, 0.f};  // betaSum, prob_hid 0, prob_hid 1
-#pragma unroll
-        for (int j = 0; j < kCJ; ++j) {
-          if (!valid[j]) continue;
-          const bool bit = (w[j] & m) != 0u;
-          const float al = scr[(size_t)(l - s0) * Kp + tid + kCT * j];
-          const float p = fmaf(xb[j], f2, f1);
-          const float d = __fmul_rn(al, p);
-          if (bit) v[2] = __fadd_rn(v[2], d);
-          else v[1] = __fadd_rn(v[1], d);
-          xb[j] = __fmul_rn(p, bit ? ey : ex);
-          v[0] = __fadd_rn(v[0], xb[j]);
-        }
-        cta_sum<3>(v, red, buf);
-        bacc = v[0];
-        if (tid == 0) *reinterpret_cast<float2*>(HP + 2 * PL[l]) = make_float2(v[1], v[2]);
-      }
-    }
-  }
+  if (threadIdx.x == 0) loglik[t] = part[0];
 }
 
 }  // namespace
 
-int launch_impute_ckpt(ImputeWork& w, bool bf16, void* ckpt, float* csum, float* scratch, double* loglik, float* hp,
-                       cudaStream_t s) {
+int launch_impute_ckpt(int J, bool bf16, int max_poly, ImputeWork& w, void* ckpt, float* asum, cudaStream_t s,
+                       int first, int count) {
   CkptArgs a;
-  a.poly = w.poly.as<int32_t>();
+  a.count = count;
+  a.order = w.order.as<int32_t>() + first;
   a.npoly = w.npoly.as<int32_t>();
   a.nstates = w.nstates.as<int32_t>();
   a.hvar = w.hvar.as<uint32_t>();
   a.em = w.em.as<float4>();
   a.tr = w.tr.as<float2>();
   a.fl = w.fl.as<uint8_t>();
+  a.row_off = w.row_off.as<int64_t>();
+  a.rows = w.rows.as<float>();
+  a.fac = w.fac.as<float>();
+  a.asum = asum;
+  a.ckpt = static_cast<__nv_bfloat16*>(ckpt);
   a.n = w.n;
   a.L = w.L;
   a.WB = w.WB;
   a.Kp = w.Kp;
-  a.ckpt = ckpt;
-  a.csum = csum;
-  a.scratch = scratch;
-  a.hp = hp;
-  a.loglik = loglik;
-  a.llpart = loglik + w.n;
-  if (w.Kp > kMaxStates) return GP_E_ARG;
-  const int grid = 2 * w.n;
-  const int jn = (w.Kp + kCT - 1) / kCT;  // states per thread; the smallest instantiated J >= jn
-#define GP_CK_LAUNCH(JJ)                                         \
-  if (jn <= JJ) {                                                \
-    if (bf16) {                                                  \
-      k_impute_ckpt<JJ, true, false><<<grid, kCT, 0, s>>>(a);    \
-      k_impute_ckpt<JJ, true, true><<<grid, kCT, 0, s>>>(a);     \
-    } else {                                                     \
-      k_impute_ckpt<JJ, false, false><<<grid, kCT, 0, s>>>(a);   \
-      k_impute_ckpt<JJ, false, true><<<grid, kCT, 0, s>>>(a);    \
-    }                                                            \
-    return GP_OK;                                                \
+  const dim3 blocks((max_poly + 31) / 32, count);
+#define GP_CK(JJ)                                                       \
+  case JJ:                                                              \
+    if (!bf16) k_ckpt_chain<JJ, false><<<2 * count, kCkptThreads, 0, s>>>(a); \
+    else {                                                              \
+      k_ckpt_chain<JJ, true><<<2 * count, kCkptThreads, 0, s>>>(a);     \
+      if (blocks.x > 0) k_ckpt_block<JJ><<<blocks, kCkptThreads, 0, s>>>(a); \
+    }                                                                   \
+    return GP_OK;
+  switch (J) {
+    GP_CK(1) GP_CK(2) GP_CK(3) GP_CK(4) GP_CK(5) GP_CK(6) GP_CK(7) GP_CK(8)
+    default: return GP_E_ARG;
   }
-  GP_CK_LAUNCH(2)
-  GP_CK_LAUNCH(3)
-  GP_CK_LAUNCH(4)
-  GP_CK_LAUNCH(5)
-  GP_CK_LAUNCH(6)
-  GP_CK_LAUNCH(8)
-#undef GP_CK_LAUNCH
-  return GP_OK;
+#undef GP_CK
+}
+
+void launch_ckpt_loglik(ImputeWork& w, const float* asum, double* loglik, cudaStream_t s) {
+  k_ckpt_loglik<<<w.n, 256, 0, s>>>(asum, w.npoly.as<int32_t>(), w.WB, loglik);
 }
 
 }  // namespace gp

@@ -242,16 +242,20 @@ __global__ void __launch_bounds__(SOLO ? kChainThreads : kChainThreads * kMaxCha
 // a block. Bound by issue, about 14 instructions per (site, state); to keep it so, a
 // CTA takes several consecutive blocks and loads the next pair of rows and the next
 // block's site data while it works on the current ones.
+//
+// CK, for the checkpointed modes: the same with 256 threads, thread tid taking the
+// states 256 j + tid, without padding (only the last pair has absent states), and the
+// sums of those modes: lanes at distances 16 .. 1, then warps at 1, 2, 4.
 // ---------------------------------------------------------------------------
-constexpr int kBlockThreads = 128;
 constexpr int RS = kRowSites;
 
+template <bool CK>
 struct BlockSmem {
   // site data of two blocks
   float4 fwd[2][RS];  // t / K twice, (1 - t) / sum twice, into the site from the left
   float4 bwd[2][RS];  // the same from the right
   float2 em[2][RS];   // emissions of allele 0 and 1
-  float part[2][32][2 * RS + 4];  // [lane l][value 2 site + allele]
+  float part[2][CK ? 8 : 32][2 * RS + 4];  // [lane l (CK: warp)][value 2 site + allele]
 };
 
 // Shared-memory loads that stay where they are: moved out of the loop over rows,
@@ -302,17 +306,20 @@ __device__ __forceinline__ void block_pair(unsigned fwd, unsigned bwd, unsigned 
   }
 }
 
-__global__ void __launch_bounds__(kBlockThreads, 4) k_impute_block(ChainArgs A, int blocks_per) {
-  __shared__ BlockSmem S;
+template <bool CK>
+__global__ void __launch_bounds__(CK ? 256 : 128, CK ? 2 : 4) k_impute_block(ChainArgs A, int blocks_per) {
+  constexpr int NT = CK ? 256 : 128;  // threads, states of a row
+  __shared__ BlockSmem<CK> S;
   const int t = A.order ? A.order[blockIdx.y] : blockIdx.y;
   const int np = A.npoly[t], K = A.nstates[t];
   const int nrow = (np + RS - 1) / RS;
   int b = blockIdx.x * blocks_per;
   const int bend = min(nrow, b + blocks_per);
   if (b >= bend || K == 0) return;
-  const int J = (K + 127) >> 7, Ks = 128 * J, pad = Ks - K;
+  const int J = (K + NT - 1) >> (CK ? 8 : 7), Ks = CK ? (K + 127) & ~127 : 128 * J;
+  const int pad = CK ? 0 : Ks - K;  // in front of row 0
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const float* base = A.rows + A.row_off[t];
+  const float* base = A.rows + A.row_off[t] + (CK ? Ks - K : 0);
   const uint32_t* hvt = A.hvar + (size_t)t * A.WB * A.Kp - pad;
 
   // Rows j and j + 1 of this thread in block b: words and the kept values entering from both sides.
@@ -322,18 +329,18 @@ __global__ void __launch_bounds__(kBlockThreads, 4) k_impute_block(ChainArgs A, 
   };
   auto load = [&](int b, int j) {
     Pair p;
-    const int o = 128 * j + tid;
-    const bool e0 = j > 0 || (j == 0 && tid >= pad), e1 = j >= 0 || tid >= pad;
+    const int o = NT * j + tid;
+    const bool e0 = CK ? o < K : j > 0 || (j == 0 && tid >= pad), e1 = CK ? o + NT < K : j >= 0 || tid >= pad;
     const uint32_t* hv = hvt + (size_t)((b * RS) >> 5) * A.Kp + o;
     const float* ar = base + (size_t)b * Ks + o;
     const float* br = ar + (size_t)nrow * Ks;
     const bool left = b > 0, right = b < nrow - 1;
     p.w0 = e0 ? hv[0] : 0u;
-    p.w1 = e1 ? hv[128] : 0u;
+    p.w1 = e1 ? hv[NT] : 0u;
     p.a0 = left && e0 ? ar[0] : 0.f;
-    p.a1 = left && e1 ? ar[128] : 0.f;
+    p.a1 = left && e1 ? ar[NT] : 0.f;
     p.b0 = right && e0 ? br[0] : 0.f;
-    p.b1 = right && e1 ? br[128] : 0.f;
+    p.b1 = right && e1 ? br[NT] : 0.f;
     return p;
   };
   // Site data of a block, one site per thread of the first RS, and the site of this lane's output.
@@ -366,8 +373,10 @@ __global__ void __launch_bounds__(kBlockThreads, 4) k_impute_block(ChainArgs A, 
     S.bwd[par][tid] = g;
     S.em[par][tid] = em;
   };
-  const int j0 = -(J & 1);
-  const f2 exists = f2_pack(j0 == 0 && tid >= pad ? 1.f : 0.f, j0 == 0 || tid >= pad ? 1.f : 0.f);
+  const int j0 = CK ? 0 : -(J & 1);
+  const int jm = CK ? (J - 1) & ~1 : j0;  // the pair with absent states
+  const f2 exists = CK ? f2_pack(NT * jm + tid < K ? 1.f : 0.f, NT * (jm + 1) + tid < K ? 1.f : 0.f)
+                       : f2_pack(j0 == 0 && tid >= pad ? 1.f : 0.f, j0 == 0 || tid >= pad ? 1.f : 0.f);
   Pair n = load(b, j0);
   load_sites(b);
   put_sites(0);
@@ -394,41 +403,70 @@ __global__ void __launch_bounds__(kBlockThreads, 4) k_impute_block(ChainArgs A, 
       else if (b + 1 < bend) n = load(b + 1, j0);
       const f2 x = f2_pack(p.a0, p.a1), y = f2_pack(p.b0, p.b1);
       const uint32_t w0 = p.w0 >> shift, w1 = p.w1 >> shift;
-      if (final_block) block_pair<true, true>(fwd, bwd, ems, w0, w1, x, y, j == j0 ? exists : f2_pack(1.f, 1.f), last, q0, q1);
-      else if (j == j0) block_pair<true, false>(fwd, bwd, ems, w0, w1, x, y, exists, -1, q0, q1);
+      if (final_block) block_pair<true, true>(fwd, bwd, ems, w0, w1, x, y, j == jm ? exists : f2_pack(1.f, 1.f), last, q0, q1);
+      else if (j == jm) block_pair<true, false>(fwd, bwd, ems, w0, w1, x, y, exists, -1, q0, q1);
       else block_pair<false, false>(fwd, bwd, ems, w0, w1, x, y, 0, -1, q0, q1);
     }
-    // Components of a lane l = tid / 4: reduce-scatter over thread distances 1 and 2.
-    const int c = tid & 3;
-    const bool up1 = c & 1, up2 = c & 2;
+    if constexpr (CK) {
+      // reduce-scatter over lane distances 16 .. 1: value 2 site + allele ends at lane 2 site + allele
+      float q[2 * RS];
 #pragma unroll
-    for (int i = 0; i < RS / 2; ++i) {
-      const float s0 = up1 ? q0[i] : q0[i + RS / 2], k0 = up1 ? q0[i + RS / 2] : q0[i];
-      const float s1 = up1 ? q1[i] : q1[i + RS / 2], k1 = up1 ? q1[i + RS / 2] : q1[i];
-      q0[i] = __fadd_rn(k0, __shfl_xor_sync(0xffffffffu, s0, 1));
-      q1[i] = __fadd_rn(k1, __shfl_xor_sync(0xffffffffu, s1, 1));
-    }
+      for (int i = 0; i < RS; ++i) {
+        q[2 * i] = q0[i];
+        q[2 * i + 1] = q1[i];
+      }
 #pragma unroll
-    for (int i = 0; i < RS / 4; ++i) {
-      const float s0 = up2 ? q0[i] : q0[i + RS / 4], k0 = up2 ? q0[i + RS / 4] : q0[i];
-      const float s1 = up2 ? q1[i] : q1[i + RS / 4], k1 = up2 ? q1[i + RS / 4] : q1[i];
-      const int st = RS / 2 * (c & 1) + RS / 4 * (c >> 1) + i;
-      const float v0 = __fadd_rn(k0, __shfl_xor_sync(0xffffffffu, s0, 2));
-      const float v1 = __fadd_rn(k1, __shfl_xor_sync(0xffffffffu, s1, 2));
-      *reinterpret_cast<float2*>(&S.part[par][tid >> 2][2 * st]) = make_float2(v0, v1);
+      for (int h = 16; h > 0; h >>= 1) {
+        const bool up = lane & h;
+#pragma unroll
+        for (int i = 0; i < h; ++i) {
+          const float send = up ? q[i] : q[i + h], keep = up ? q[i + h] : q[i];
+          q[i] = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, send, h));
+        }
+      }
+      S.part[par][warp][lane] = q[0];
+    } else {
+      // Components of a lane l = tid / 4: reduce-scatter over thread distances 1 and 2.
+      const int c = tid & 3;
+      const bool up1 = c & 1, up2 = c & 2;
+#pragma unroll
+      for (int i = 0; i < RS / 2; ++i) {
+        const float s0 = up1 ? q0[i] : q0[i + RS / 2], k0 = up1 ? q0[i + RS / 2] : q0[i];
+        const float s1 = up1 ? q1[i] : q1[i + RS / 2], k1 = up1 ? q1[i + RS / 2] : q1[i];
+        q0[i] = __fadd_rn(k0, __shfl_xor_sync(0xffffffffu, s0, 1));
+        q1[i] = __fadd_rn(k1, __shfl_xor_sync(0xffffffffu, s1, 1));
+      }
+#pragma unroll
+      for (int i = 0; i < RS / 4; ++i) {
+        const float s0 = up2 ? q0[i] : q0[i + RS / 4], k0 = up2 ? q0[i + RS / 4] : q0[i];
+        const float s1 = up2 ? q1[i] : q1[i + RS / 4], k1 = up2 ? q1[i + RS / 4] : q1[i];
+        const int st = RS / 2 * (c & 1) + RS / 4 * (c >> 1) + i;
+        const float v0 = __fadd_rn(k0, __shfl_xor_sync(0xffffffffu, s0, 2));
+        const float v1 = __fadd_rn(k1, __shfl_xor_sync(0xffffffffu, s1, 2));
+        *reinterpret_cast<float2*>(&S.part[par][tid >> 2][2 * st]) = make_float2(v0, v1);
+      }
     }
     if (b + 1 < bend) put_sites(par ^ 1);
     __syncthreads();
-    if (warp == (b & 3)) {  // the 2 RS = 32 sums of the block, the warps in turn
+    if (warp == (b & (NT / 32 - 1))) {  // the 2 RS = 32 sums of the block, the warps in turn
       float v[8];
+      if constexpr (CK) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
-        v[i] = __fadd_rn(__fadd_rn(S.part[par][i][lane], S.part[par][i + 16][lane]),
-                         __fadd_rn(S.part[par][i + 8][lane], S.part[par][i + 24][lane]));
+        for (int i = 0; i < 8; ++i) v[i] = S.part[par][i][lane];
 #pragma unroll
-      for (int h = 4; h > 0; h >>= 1)
+        for (int h = 1; h < 8; h <<= 1)
 #pragma unroll
-        for (int i = 0; i < h; ++i) v[i] = __fadd_rn(v[i], v[i + h]);
+          for (int i = 0; i < 8; i += 2 * h) v[i] = __fadd_rn(v[i], v[i + h]);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          v[i] = __fadd_rn(__fadd_rn(S.part[par][i][lane], S.part[par][i + 16][lane]),
+                           __fadd_rn(S.part[par][i + 8][lane], S.part[par][i + 24][lane]));
+#pragma unroll
+        for (int h = 4; h > 0; h >>= 1)
+#pragma unroll
+          for (int i = 0; i < h; ++i) v[i] = __fadd_rn(v[i], v[i + h]);
+      }
       // prob_hid of the two alleles; k_impute_finish turns them into HP
       if ((lane >> 1) <= last) A.hp[(size_t)t * 2 * A.L + 2 * site + (lane & 1)] = v[0];
     }
@@ -484,7 +522,7 @@ int launch_impute_chain(int J, ImputeWork& w, cudaStream_t s, int first, int cou
 
 static_assert(2 * kRowSites == 32, "k_impute_block: one lane per sum of a block");
 
-int launch_impute_block(int max_poly, ImputeWork& w, float* hp, cudaStream_t s, int first, int count) {
+int launch_impute_block(bool ck, int max_poly, ImputeWork& w, float* hp, cudaStream_t s, int first, int count) {
   ChainArgs a;
   if (chain_args(w, hp, first, count, a) != GP_OK) return GP_E_ARG;
   const int blocks = (max_poly + kRowSites - 1) / kRowSites;
@@ -492,7 +530,9 @@ int launch_impute_block(int max_poly, ImputeWork& w, float* hp, cudaStream_t s, 
   // Blocks per CTA: enough to hide the loads of each, while some eight CTAs per SM are left.
   const long long total = (long long)blocks * a.count;
   const int per = (int)std::max(1ll, std::min(16ll, total / (8 * 148)));
-  k_impute_block<<<dim3((blocks + per - 1) / per, a.count), kBlockThreads, 0, s>>>(a, per);
+  const dim3 g((blocks + per - 1) / per, a.count);
+  if (ck) k_impute_block<true><<<g, 256, 0, s>>>(a, per);
+  else k_impute_block<false><<<g, 128, 0, s>>>(a, per);
   return GP_OK;
 }
 

@@ -42,9 +42,9 @@ extern "C" {
 #define GP_MAX_BATCH 65535
 
 /* Precision modes of the imputation forward-backward (gp_set_precision). */
-#define GP_PRECISION_FULL 0       /* every forward row kept in FP32, as the reference keeps them */
-#define GP_PRECISION_CKPT_F32 1   /* FP32 checkpoints every 32 sites, FP32 recompute, FP64 log-likelihood */
-#define GP_PRECISION_CKPT_BF16 2  /* BF16 checkpoints every 32 sites, FP32 recompute, FP64 log-likelihood */
+#define GP_PRECISION_FULL 0       /* FP32, as the reference computes */
+#define GP_PRECISION_CKPT_F32 1   /* FP32, and an FP64 log-likelihood */
+#define GP_PRECISION_CKPT_BF16 2  /* one row in 32 sites rounded to BF16, and an FP64 log-likelihood */
 
 #define GP_STAGE_INIT 0
 #define GP_STAGE_BURN 1
@@ -223,13 +223,14 @@ int gp_impute_one_static(gp_ctx* ctx, int32_t k, const uint32_t* states, const f
 
 /* Precision of the imputation forward-backward for every later call (no
  * counterpart in the reference, which keeps every forward row,
- * imputation_hmm.cpp:53-59). GP_PRECISION_FULL (the default) keeps all rows in
- * FP32. The checkpointed modes keep the forward row after every 32nd
- * polymorphic site only (FP32 or BF16; about 1/32 or 1/64 of the memory),
- * recompute each block's rows in FP32 during the backward pass, and accumulate
- * the chunk log-likelihood sum_l log AlphaSum_l in FP64 (gp_loglik_get). With
- * FP32 checkpoints the posteriors are those of the same recursion without
- * checkpoints; BF16 checkpoints trade a small posterior error for memory. */
+ * imputation_hmm.cpp:53-59). GP_PRECISION_FULL (the default): FP32 throughout.
+ * The checkpointed modes add up the states in another fixed order and accumulate
+ * the chunk log-likelihood sum_l log AlphaSum_l in FP64 (gp_loglik_get). With FP32
+ * checkpoints the posteriors are those of the same recursion; with BF16 ones, the
+ * messages of one direction per half are recomputed in FP32 from a row rounded to
+ * BF16 every 32 polymorphic sites, at a small posterior error. Each mode keeps a row
+ * of either direction every 16 sites (half a byte per site and state, in chunks of
+ * haplotypes that fit); BF16 adds 1/8 byte per site and state for all haplotypes. */
 int gp_set_precision(gp_ctx* ctx, int32_t mode);
 
 /* The FP64 chunk log-likelihood of each haplotype of the last imputation call

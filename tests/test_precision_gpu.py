@@ -174,3 +174,33 @@ def test_checkpointed_bf16_full_run_r2():
     print(f"\nfull run r2: all rows {r2[native.PRECISION_FULL]:.5f}, BF16 checkpoints "
           f"{r2[native.PRECISION_CKPT_BF16]:.5f} (delta {d:+.5f})")
     assert abs(d) <= 0.002
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sites", [1, 16, 17, 32, 33, 63, 64, 65, 97, 200])
+def test_checkpointed_block_and_state_count_edges(sites):
+    """Site counts around the kept rows (16 sites), the blocks (32) and the split of
+    the BF16 rows (np / 2 rounded down to a block: none below 64 sites), and state
+    counts around the rows of 128 and 256, in one batch. FP32: HP within 1e-5 of
+    FP64, the log-likelihood within 1e-6 per site. BF16: rows rounded to 8 bits, a
+    relative error of 2^-9, at most two in a posterior and one in the likelihood: HP
+    within 5e-3, the log-likelihood within 2^-8 more."""
+    import dataclasses
+    from glimpse_b200 import native, synth
+    w = synth.make_panel_and_targets(2050, 260, 0.2, 0.0, 2, ("uniform", 0.4, 2.0), ("fixed", 200), seed=67,
+                                     sparse_maf=0.005)
+    P, T = w.panel, w.targets
+    keep = slice(0, sites)
+    P = dataclasses.replace(P, n_sites=sites, bp=P.bp[keep], cm=P.cm[keep], cref=P.cref[keep], calt=P.calt[keep],
+                            lq=P.lq[keep], flag_common=P.flag_common[keep], major=P.major[keep],
+                            hvar=np.ascontiguousarray(P.hvar[keep]))
+    T = dataclasses.replace(T, gl=np.ascontiguousarray(T.gl[:, keep]), flat=np.ascontiguousarray(T.flat[:, keep]))
+    Ks = [1, 31, 32, 33, 127, 128, 129, 255, 256, 257, 511, 513, 769, 1025, 1537, 2047, 2048]
+    out, ref = _impute_modes(dataclasses.replace(w, panel=P, targets=T), Ks, sites,
+                             [native.PRECISION_CKPT_F32, native.PRECISION_CKPT_BF16])
+    for m, tol, ll_tol in ((native.PRECISION_CKPT_F32, TOL, 0.0), (native.PRECISION_CKPT_BF16, 5e-3, 2.0 ** -8)):
+        hp, ll = out[m]
+        for i, (hr, llr) in enumerate(ref):
+            e = float(np.abs(hp[i].astype(np.float64) - hr.astype(np.float64)).max())
+            assert e <= tol, f"mode {m}, K={Ks[i]}: max |HP - HP_fp64| = {e:.3e}"
+            assert abs(ll[i] - llr) <= 1e-6 * sites + ll_tol, (m, Ks[i])
