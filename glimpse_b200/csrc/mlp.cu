@@ -13,7 +13,7 @@
 //   applies ReLU and takes the dot product with w3 in FP32: the score. Thread t
 //   of the CTA owns row t of the tile (tensor-memory lane t).
 // k_gemm_tn: D = A * B^T for the weight gradients (split over K) and for the
-//   layer-1 input gradient (masked by the ReLU of layer 1), two cp.async stages
+//   layer-1 input gradient (masked by the ReLU of layer 1), cp.async stages
 //   feeding tcgen05.mma.
 // Every wait on the tensor core is bounded (tc::mbar_wait); a time-out sets
 // the error flag, the CTA stops, frees its tensor memory and returns.
@@ -49,12 +49,18 @@ __device__ __forceinline__ void stage_kmajor(uint8_t* tile, const __nv_bfloat16*
                                              int nvalid, int k0, int kvalid) {
   const int chunks = rows * (kext >> 3);
   for (int c = threadIdx.x; c < chunks; c += blockDim.x) {
-    const int r = c / (kext >> 3), kc = c % (kext >> 3);
+    // 8 rows of a chunk column side by side: 128 bytes of the tile, no bank conflicts
+    const int u = c >> 3, r = u / (kext >> 3) * 8 + (c & 7), kc = u % (kext >> 3);
     const int k = k0 + kc * 8;
     const bool ok = r < nvalid && k < kvalid;
     const __nv_bfloat16* g = ok ? src + (size_t)r * ld + k : src;
     tc::cp_async16(tile + tc::kmajor_off(r, kc * 8, kext), g, ok ? 16u : 0u);
   }
+}
+
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
+  const __nv_bfloat162 b = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&b);
 }
 
 constexpr int kFwdThreads = 256;  // warps w and w + 4 share tensor-memory lanes 32 (w % 4) .. + 31 (the tile's
@@ -198,76 +204,93 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_mlp_fwd(MlpFwdArgs a) {
   if (warp == 0) tc::tmem_free(tbase, 512);
 }
 
-// D = A * B^T, M tile 128, N tile NT, K blocks of 64 in two cp.async stages.
+// D = A * B^T, M tile 128, N tile NT, K blocks of 64 in cp.async stages.
+// The K extents here are short (256, or a split of 2,048 rows): bound by the latency of
+// the loads and by the epilogue. So some 192 KB are kept in flight, and a thread writes
+// its row in 16-byte stores (the masked product of 16,384 rows: 76 us with two stages and
+// stores of single elements, 21 now).
+template <int NT>
+constexpr int kGemmStages = NT == 256 ? 4 : 8;
+
 template <int NT, int EPI>
 __global__ void __launch_bounds__(128) k_gemm_tn(GemmArgs g) {
   extern __shared__ __align__(1024) uint8_t sm[];
   constexpr uint32_t kA = kTileM * 64 * 2, kB = NT * 64 * 2, kStage = kA + kB;
-  uint64_t* bar = reinterpret_cast<uint64_t*>(sm + 2 * kStage);
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + 2 * kStage + 16);
-  int* abort_flag = reinterpret_cast<int*>(sm + 2 * kStage + 20);
+  constexpr int ST = kGemmStages<NT>;
+  uint64_t* bar = reinterpret_cast<uint64_t*>(sm + ST * kStage);
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + ST);
   const int tid = threadIdx.x, warp = tid >> 5;
-  const int m0 = blockIdx.x * kTileM, n0 = blockIdx.y * NT;
+  const bool second = EPI == 0 && (int)blockIdx.y * NT >= g.N;
+  const int m0 = blockIdx.x * kTileM, n0 = blockIdx.y * NT - (second ? g.N : 0);
+  const __nv_bfloat16* const ga = second ? g.a2 : g.a;
+  const __nv_bfloat16* const gb = second ? g.b2 : g.b;
+  const int N = second ? g.N2 : g.N;
   const int kbeg = blockIdx.z * g.kchunk, kend = min(g.K, kbeg + g.kchunk);
-  const int nkb = kend > kbeg ? (kend - kbeg + 63) / 64 : 0;
+  const int nkb = kend > kbeg ? (kend - kbeg) / 64 : 0;
   constexpr uint32_t ncols = NT < 32 ? 32 : NT;
   if (warp == 0) tc::tmem_alloc(tslot, ncols);
   if (tid == 0) {
-    tc::mbar_init(&bar[0], 1);
-    tc::mbar_init(&bar[1], 1);
+    for (int i = 0; i < ST; ++i) tc::mbar_init(&bar[i], 1);
     tc::fence_mbar_init();
-    *abort_flag = 0;
   }
+  // Chunks of 16 bytes, 8 rows of a chunk column side by side (128 bytes of the tile, no
+  // bank conflicts): this thread takes the rows r, r + 16, ... at one k of every block.
+  // With one warp per scheduler the address arithmetic counts, so it is kept out of
+  // the loop: tiles and blocks are whole.
+  const int r = (tid >> 6) * 8 + (tid & 7), k = (tid >> 3 & 7) * 8;
+  const __nv_bfloat16* pa = ga + (size_t)(m0 + r) * g.lda + kbeg + k;
+  const __nv_bfloat16* pb = gb + (size_t)(n0 + r) * g.ldb + kbeg + k;
+  const size_t sa16 = (size_t)16 * g.lda, sb16 = (size_t)16 * g.ldb;
+  uint8_t* const dst = sm + tc::kmajor_off(r, k, 64);
+  auto load = [&](int kb) {  // in order; one group per block, empty past the last
+    if (kb < nkb) {
+      uint8_t* d = dst + (kb % ST) * kStage;
+      const __nv_bfloat16* p = pa;
+#pragma unroll
+      for (int i = 0; i < kTileM / 16; ++i, p += sa16) tc::cp_async16(d + i * 2048, p, 16u);
+      p = pb;
+#pragma unroll
+      for (int i = 0; i < NT / 16; ++i, p += sb16) tc::cp_async16(d + kA + i * 2048, p, 16u);
+      pa += 64;
+      pb += 64;
+    }
+    tc::cp_async_commit();
+  };
+#pragma unroll
+  for (int kb = 0; kb < ST; ++kb) load(kb);
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tbase = *tslot;
   constexpr uint32_t idesc = tc::idesc_bf16(kTileM, NT);
-  uint32_t uses[2] = {0u, 0u};  // completed MMA batches per stage
-  auto load = [&](int kb) {
-    uint8_t* st = sm + (kb & 1) * kStage;
-    const int k0 = kbeg + kb * 64;
-    stage_kmajor(st, g.a + (size_t)m0 * g.lda, kTileM, 64, g.lda, g.M - m0, k0, kend);
-    stage_kmajor(st + kA, g.b + (size_t)n0 * g.ldb, NT, 64, g.ldb, g.N - n0, k0, kend);
-    tc::cp_async_commit();
-  };
-  if (nkb > 0) load(0);
+  bool late = false, stop = false;
   for (int kb = 0; kb < nkb; ++kb) {
-    if (kb + 1 < nkb) {
-      if (kb >= 1) {  // the stage about to be refilled was read by the MMAs of block kb - 1
-        const int s = (kb + 1) & 1;
-        if (!tc::mbar_wait(&bar[s], uses[s] & 1u)) *abort_flag = 1;
-        uses[s]++;
-      }
-      load(kb + 1);
-      tc::cp_async_wait<1>();
-    } else {
-      tc::cp_async_wait<0>();
-    }
+    tc::cp_async_wait<ST - 2>();
     tc::fence_proxy_async();
-    __syncthreads();
-    if (*abort_flag) break;
+    if ((stop = __syncthreads_or(late))) break;
     if (tid == 0) {
       tc::fence_after_sync();
-      const uint32_t sa = tc::smem_u32(sm + (kb & 1) * kStage), sb = sa + kA;
+      const uint32_t sa = tc::smem_u32(sm + (kb % ST) * kStage), sb = sa + kA;
 #pragma unroll
       for (int s = 0; s < 4; ++s)
         tc::mma_bf16(tbase, tc::smem_desc(sa + s * 256, 128, 1024), tc::smem_desc(sb + s * 256, 128, 1024), idesc,
                      kb > 0 || s > 0);
-      tc::commit(&bar[kb & 1]);
+      tc::commit(&bar[kb % ST]);
+    }
+    if (kb > 0) {  // the stage of block kb - 1, once its MMAs have read it
+      const int next = kb - 1 + ST;
+      if (next < nkb) late |= !tc::mbar_wait(&bar[(kb - 1) % ST], ((kb - 1) / ST) & 1u);
+      load(next);
     }
   }
   // the last commit covers every MMA issued before it
-  if (nkb > 0 && !*abort_flag) {
-    const int s = (nkb - 1) & 1;
-    if (!tc::mbar_wait(&bar[s], uses[s] & 1u)) *abort_flag = 1;
-  }
-  __syncthreads();
+  if (nkb > 0 && !stop)
+    late |= !tc::mbar_wait(&bar[(nkb - 1) % ST], ((nkb - 1) / ST) & 1u);
+  tc::cp_async_wait<0>();
+  stop = __syncthreads_or(late);
   tc::fence_after_sync();
   const int row = m0 + tid;
-  if (!*abort_flag) {
-    // every thread takes part in the warp-wide tensor-memory loads; only rows
-    // below M store
+  if (!stop) {
     const uint32_t lane_off = (uint32_t)(warp * 32) << 16;
 #pragma unroll 1
     for (int c = 0; c < NT / 32; ++c) {
@@ -279,22 +302,29 @@ __global__ void __launch_bounds__(128) k_gemm_tn(GemmArgs g) {
         for (int i = 0; i < 32; ++i) v[i] = 0.f;
       }
       const int nb = n0 + c * 32;
-      if (row >= g.M) continue;
       if (EPI == 0) {
-        float* o = g.out_f + ((size_t)blockIdx.z * g.M + row) * g.N;
+        float4* o = reinterpret_cast<float4*>((second ? g.out2 : g.out_f) + ((size_t)blockIdx.z * g.M + row) * N + nb);
 #pragma unroll
-        for (int i = 0; i < 32; ++i)
-          if (nb + i < g.N) o[nb + i] = v[i];
+        for (int i = 0; i < 8; ++i) o[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
       } else {
-        const __nv_bfloat16* mk = g.mask + (size_t)row * g.N;
-        __nv_bfloat16* o = g.out_b + (size_t)row * g.N;
+        const uint4* mk = reinterpret_cast<const uint4*>(g.mask + (size_t)row * N + nb);
+        uint4* o = reinterpret_cast<uint4*>(g.out_b + (size_t)row * N + nb);
 #pragma unroll
-        for (int i = 0; i < 32; ++i)
-          if (nb + i < g.N) o[nb + i] = __float2bfloat16_rn(__bfloat162float(mk[nb + i]) > 0.f ? v[i] : 0.f);
+        for (int i = 0; i < 4; ++i) {
+          const uint4 m = mk[i];
+          uint32_t mw[4] = {m.x, m.y, m.z, m.w};
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const float2 h = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&mw[k]));
+            const int q = 8 * i + 2 * k;
+            mw[k] = pack_bf16(h.x > 0.f ? v[q] : 0.f, h.y > 0.f ? v[q + 1] : 0.f);
+          }
+          o[i] = make_uint4(mw[0], mw[1], mw[2], mw[3]);
+        }
       }
     }
   }
-  if (*abort_flag && tid == 0) atomicExch(g.err, 1);
+  if (stop && tid == 0) atomicExch(g.err, 1);
   tc::fence_before_sync();
   __syncthreads();
   if (warp == 0) tc::tmem_free(tbase, ncols);
@@ -309,105 +339,163 @@ __global__ void k_feat_bf16(const float* __restrict__ x, int n, int rows, __nv_b
   }
 }
 
-// out[c][r] = in[r][c] for a [R][C] BF16 matrix, 32 x 32 tiles through shared memory.
-__global__ void k_transpose_bf16(const __nv_bfloat16* __restrict__ in, int R, int C, __nv_bfloat16* __restrict__ out) {
-  __shared__ __nv_bfloat16 t[32][33];
-  const int r0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
-  for (int i = threadIdx.y; i < 32; i += blockDim.y) {
-    const int r = r0 + i, c = c0 + threadIdx.x;
-    t[i][threadIdx.x] = (r < R && c < C) ? in[(size_t)r * C + c] : __float2bfloat16_rn(0.f);
-  }
-  __syncthreads();
-  for (int i = threadIdx.y; i < 32; i += blockDim.y) {
-    const int c = c0 + i, r = r0 + threadIdx.x;
-    if (c < C && r < R) out[(size_t)c * R + r] = t[threadIdx.x][i];
-  }
+// Columns of 64 rows of a BF16 matrix: the products over rows read their operands
+// with the rows contiguous. Thread j loads column j (a row of the matrix per request of
+// the block) and writes its 64 values, 128 bytes, in eight stores.
+constexpr int kColRows = 64;
+
+__device__ __forceinline__ void load_column(const __nv_bfloat16* __restrict__ m, int ld, int rb, int j,
+                                            uint32_t (&v)[kColRows / 2]) {
+  const unsigned short* p = reinterpret_cast<const unsigned short*>(m) + (size_t)rb * ld + j;
+#pragma unroll
+  for (int i = 0; i < kColRows / 2; ++i) v[i] = p[(size_t)(2 * i) * ld] | (uint32_t)p[(size_t)(2 * i + 1) * ld] << 16;
 }
 
+__device__ __forceinline__ void store_column(__nv_bfloat16* __restrict__ out, int rows, int rb, int j,
+                                             const uint32_t (&v)[kColRows / 2]) {
+  uint4* o = reinterpret_cast<uint4*>(out + (size_t)j * rows + rb);
+#pragma unroll
+  for (int i = 0; i < kColRows / 8; ++i) o[i] = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+}
+
+__device__ __forceinline__ float bf_lo(uint32_t v) { return __uint_as_float(v << 16); }
+__device__ __forceinline__ float bf_hi(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
+
 // Columns of the per-block partial sums (hpart rows): dL/dw3 | dL/db2 | dL/db3,
-// loss | dL/db1. They are added over the blocks in block order (k_sum_head), so
+// loss | dL/db1. They are added over the blocks in block order (k_step), so
 // a training step gives the same parameters on every run.
 constexpr int kHpW3 = 0, kHpB2 = kMlpHid, kHpB3 = 2 * kMlpHid, kHpLoss = 2 * kMlpHid + 1,
               kHpB1 = 2 * kMlpHid + 2, kHpCols = 3 * kMlpHid + 2;
 
-// Loss head and the gradients it feeds, for rows [blockIdx.x * rpb, ...):
+// Loss head and the gradients it feeds, for the rows [64 blockIdx.x, + 64):
 // p = sigmoid(score), loss = wt * BCE(p, y) / n, ds = (p - y) * wt / n;
-// dz2[r][j] = ds * w3[j] where h2[r][j] > 0; the block's sums of dL/dw3, dL/db2,
-// dL/db3 and the loss go to its row of hpart. Thread j owns hidden unit j.
-__global__ void k_bwd_head(const float* __restrict__ score, const float* __restrict__ y, const float* __restrict__ wt,
-                           const __nv_bfloat16* __restrict__ h2, const float* __restrict__ w3, int rows, int rpb,
-                           float inv_n, __nv_bfloat16* __restrict__ dz2, float* __restrict__ hpart) {
-  const int j = threadIdx.x;
-  const int rb = blockIdx.x * rpb, re = min(rows, rb + rpb);
+// dz2[r][j] = ds * w3[j] where h2[r][j] > 0, as rows and as columns; the columns of
+// h1; the block's sums of dL/dw3, dL/db2, dL/db3 and the loss go to its row of
+// hpart. Thread j owns hidden unit j; a row's scalars are formed by one thread.
+// Bound by the latency of its loads, 64 in flight per thread (16,384 rows: 42 us with
+// a row per iteration and 18 for the two transposes after it, 12 now).
+__global__ void __launch_bounds__(kMlpHid) k_bwd_head(
+    const float* __restrict__ score, const float* __restrict__ y, const float* __restrict__ wt,
+    const __nv_bfloat16* __restrict__ h1, const __nv_bfloat16* __restrict__ h2, const float* __restrict__ w3, int rows,
+    float inv_n, __nv_bfloat16* __restrict__ dz2, __nv_bfloat16* __restrict__ dz2t, __nv_bfloat16* __restrict__ h1t,
+    float* __restrict__ hpart) {
+  __shared__ float dss[kColRows], lss[kColRows];
+  const int j = threadIdx.x, rb = blockIdx.x * kColRows;
+  uint32_t v[kColRows / 2];
+  load_column(h2, kMlpHid, rb, j, v);
   const float w3j = w3[j];
-  float gw3 = 0.f, gb2 = 0.f, gb3 = 0.f, ls = 0.f;
-  for (int r = rb; r < re; ++r) {
-    const float s = score[r], yy = y[r], ww = wt[r];
+  if (j < kColRows) {
+    const float s = score[rb + j], yy = y[rb + j], ww = wt[rb + j];
     const float p = 1.f / (1.f + expf(-s));
-    const float ds = (p - yy) * ww * inv_n;
-    const float h = __bfloat162float(h2[(size_t)r * kMlpHid + j]);
-    const float dz = h > 0.f ? ds * w3j : 0.f;
-    dz2[(size_t)r * kMlpHid + j] = __float2bfloat16_rn(dz);
-    gw3 = fmaf(ds, h, gw3);
-    gb2 += dz;
-    if (j == 0) {
-      gb3 += ds;
-      ls += ww * inv_n * (fmaxf(s, 0.f) - s * yy + log1pf(expf(-fabsf(s))));
-    }
+    dss[j] = (p - yy) * ww * inv_n;
+    lss[j] = ww * inv_n * (fmaxf(s, 0.f) - s * yy + log1pf(expf(-fabsf(s))));
   }
+  __syncthreads();
+  float gw3 = 0.f, gb2 = 0.f;
+  unsigned short* o = reinterpret_cast<unsigned short*>(dz2) + (size_t)rb * kMlpHid + j;
+#pragma unroll
+  for (int i = 0; i < kColRows / 2; ++i) {
+    const float h0 = bf_lo(v[i]), hh = bf_hi(v[i]), d0 = dss[2 * i], d1 = dss[2 * i + 1];
+    const float z0 = h0 > 0.f ? d0 * w3j : 0.f, z1 = hh > 0.f ? d1 * w3j : 0.f;
+    gw3 = fmaf(d0, h0, gw3);
+    gb2 += z0;
+    gw3 = fmaf(d1, hh, gw3);
+    gb2 += z1;
+    v[i] = pack_bf16(z0, z1);
+    o[(size_t)(2 * i) * kMlpHid] = (unsigned short)(v[i] & 0xffffu);
+    o[(size_t)(2 * i + 1) * kMlpHid] = (unsigned short)(v[i] >> 16);
+  }
+  store_column(dz2t, rows, rb, j, v);
+  load_column(h1, kMlpHid, rb, j, v);
+  store_column(h1t, rows, rb, j, v);
   float* row = hpart + (size_t)blockIdx.x * kHpCols;
   row[kHpW3 + j] = gw3;
   row[kHpB2 + j] = gb2;
-  if (j == 0) {
-    row[kHpB3] = gb3;
-    row[kHpLoss] = ls;
-  }
-}
-
-// The block's sums over rows of m[r][j] (m: [rows][256] BF16) into its row of
-// hpart (dL/db1 columns), thread j per column.
-__global__ void k_colsum(const __nv_bfloat16* __restrict__ m, int rows, int rpb, float* __restrict__ hpart) {
-  const int j = threadIdx.x;
-  const int rb = blockIdx.x * rpb, re = min(rows, rb + rpb);
-  float acc = 0.f;
-  for (int r = rb; r < re; ++r) acc += __bfloat162float(m[(size_t)r * kMlpHid + j]);
-  hpart[(size_t)blockIdx.x * kHpCols + kHpB1 + j] = acc;
-}
-
-// The hpart columns added over the blocks in block order, into the gradient
-// vector and the loss.
-__global__ void k_sum_head(const float* __restrict__ hpart, int blocks, float* __restrict__ grad,
-                           float* __restrict__ loss) {
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < kHpCols; c += gridDim.x * blockDim.x) {
-    float v = 0.f;
-    for (int b = 0; b < blocks; ++b) v += hpart[(size_t)b * kHpCols + c];
-    if (c < kHpB2) grad[kOffW3 + c] = v;
-    else if (c < kHpB3) grad[kOffB2 + c - kHpB2] = v;
-    else if (c == kHpB3) grad[kOffB3] = v;
-    else if (c == kHpLoss) *loss = v;
-    else grad[kOffB1 + c - kHpB1] = v;
-  }
-}
-
-// dst[i] = sum over splits of part[z][i].
-__global__ void k_sum_splits(const float* __restrict__ part, int n, int splits, float* __restrict__ dst) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  if (j < 2) {
+    const float* t = j == 0 ? dss : lss;
     float acc = 0.f;
-    for (int z = 0; z < splits; ++z) acc += part[(size_t)z * n + i];
-    dst[i] = acc;
+    for (int r = 0; r < kColRows; ++r) acc += t[r];
+    row[j == 0 ? kHpB3 : kHpLoss] = acc;
   }
 }
 
-// Adam over the packed parameters (FP32 master copies), then the BF16 copies the GEMMs read.
-__global__ void k_adam(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
-                       int n, float lr, float b1, float b2, float eps, float c1, float c2) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const float gi = g[i];
-    const float mi = b1 * m[i] + (1.f - b1) * gi;
-    const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+// For the rows [64 blockIdx.x, + 64): the columns of dz1 and of x, and the block's
+// sums over rows of dz1 into its row of hpart (dL/db1), thread j per column.
+__global__ void __launch_bounds__(kMlpHid) k_dz1_columns(const __nv_bfloat16* __restrict__ dz1,
+                                                         const __nv_bfloat16* __restrict__ x, int rows,
+                                                         __nv_bfloat16* __restrict__ dz1t,
+                                                         __nv_bfloat16* __restrict__ xt, float* __restrict__ hpart) {
+  const int j = threadIdx.x, rb = blockIdx.x * kColRows;
+  uint32_t v[kColRows / 2];
+  load_column(dz1, kMlpHid, rb, j, v);
+  store_column(dz1t, rows, rb, j, v);
+  float acc = 0.f;
+#pragma unroll
+  for (int i = 0; i < kColRows / 2; ++i) {
+    acc += bf_lo(v[i]);
+    acc += bf_hi(v[i]);
+  }
+  hpart[(size_t)blockIdx.x * kHpCols + kHpB1 + j] = acc;
+  if (j < kMlpInP) {
+    load_column(x, kMlpInP, rb, j, v);
+    store_column(xt, rows, rb, j, v);
+  }
+}
+
+// The end of a step, a thread per parameter (and one for the loss): the gradient, from
+// the splits of the weight products or the blocks' sums, added in order; with lr > 0 the
+// Adam update of the FP32 master and the BF16 copies that the GEMMs read (16,384 rows:
+// 11 us, against 35 for a kernel per part).
+struct StepArgs {
+  const float* part1;  // [splits][256][64]
+  const float* part2;  // [splits][256][256]
+  const float* hpart;  // [blocks][kHpCols]
+  int splits, blocks;
+  float* grad;
+  float* loss;
+  float *p, *m, *v;
+  __nv_bfloat16 *w1, *w2, *w2t;
+  float lr, b1, b2, eps, c1, c2;
+};
+
+__device__ __forceinline__ float sum_strided(const float* __restrict__ p, int n, size_t stride) {
+  float acc = 0.f;
+#pragma unroll 16
+  for (int z = 0; z < n; ++z) acc += p[z * stride];
+  return acc;
+}
+
+__global__ void __launch_bounds__(256) k_step(StepArgs a) {
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i > kMlpParams) return;
+  if (i == kMlpParams) {
+    *a.loss = sum_strided(a.hpart + kHpLoss, a.blocks, kHpCols);
+    return;
+  }
+  const bool is1 = i < kOffB1, is2 = i >= kOffW2 && i < kOffB2;
+  float g;
+  if (is1) g = sum_strided(a.part1 + i - kOffW1, a.splits, kMlpHid * kMlpInP);
+  else if (is2) g = sum_strided(a.part2 + i - kOffW2, a.splits, kMlpHid * kMlpHid);
+  else {
+    const int col = i < kOffW2 ? kHpB1 + i - kOffB1
+                    : i < kOffW3 ? kHpB2 + i - kOffB2
+                    : i < kOffB3 ? kHpW3 + i - kOffW3 : kHpB3;
+    g = sum_strided(a.hpart + col, a.blocks, kHpCols);
+  }
+  a.grad[i] = g;
+  if (a.lr <= 0.f) return;
+  const float mi = a.b1 * a.m[i] + (1.f - a.b1) * g;
+  const float vi = a.b2 * a.v[i] + (1.f - a.b2) * g * g;
+  a.m[i] = mi;
+  a.v[i] = vi;
+  const float p = a.p[i] - a.lr * (mi / a.c1) / (sqrtf(vi / a.c2) + a.eps);
+  a.p[i] = p;
+  const __nv_bfloat16 b = __float2bfloat16_rn(p);
+  if (is1) a.w1[i - kOffW1] = b;
+  if (is2) {
+    const int e = i - kOffW2;
+    a.w2[e] = b;
+    a.w2t[(size_t)(e % kMlpHid) * kMlpHid + e / kMlpHid] = b;
   }
 }
 
@@ -438,17 +526,18 @@ cudaError_t launch_mlp_fwd(const MlpFwdArgs& a, int grid, cudaStream_t s) {
 
 template <int NT, int EPI>
 static cudaError_t gemm_launch(const GemmArgs& g, int splits, cudaStream_t s) {
-  constexpr size_t smem = 2 * (kTileM * 64 * 2 + NT * 64 * 2) + 64;
+  constexpr size_t smem = kGemmStages<NT> * (kTileM * 64 * 2 + NT * 64 * 2) + 128;
   cudaError_t e = set_smem_limit_once<k_gemm_tn<NT, EPI>>((int)smem);
   if (e != cudaSuccess) return e;
-  const dim3 grid((g.M + kTileM - 1) / kTileM, (g.N + NT - 1) / NT, splits);
+  const dim3 grid((g.M + kTileM - 1) / kTileM, (g.N + g.N2) / NT, splits);
   k_gemm_tn<NT, EPI><<<grid, 128, smem, s>>>(g);
   return cudaGetLastError();
 }
 
 cudaError_t launch_gemm_tn(const GemmArgs& g, int NT, int epi, int splits, cudaStream_t s) {
-  if ((g.K & 7) || (g.lda & 7) || (g.ldb & 7)) return cudaErrorInvalidValue;  // 16-byte rows of K chunks
-  if (NT == 256 && epi == 0) return gemm_launch<256, 0>(g, splits, s);
+  // whole tiles and blocks, rows of whole 16-byte chunks
+  if (g.M % kTileM || g.N % NT || g.N2 % NT || g.K % 64 || g.kchunk % 64 || (g.lda & 7) || (g.ldb & 7))
+    return cudaErrorInvalidValue;
   if (NT == 256 && epi == 1) return gemm_launch<256, 1>(g, splits, s);
   if (NT == 64 && epi == 0) return gemm_launch<64, 0>(g, splits, s);
   return cudaErrorInvalidValue;
@@ -548,21 +637,14 @@ int mlp_train_device(Context& c, int n, int rows, float lr, bool want_grad) {
   MlpState& M = c.mlp;
   cudaStream_t s = c.stream;
   auto bf = [](DevBuf& b) { return b.as<__nv_bfloat16>(); };
-  cudaMemsetAsync(M.grad.ptr, 0, (size_t)kMlpParams * 4, s);
-  cudaMemsetAsync(M.loss.ptr, 0, 4, s);
   int rc = mlp_forward_device(c, bf(M.x), rows, M.score.as<float>(), bf(M.h1), bf(M.h2));
   if (rc != GP_OK) return rc;
-  const int rpb = 64;
-  const int hb = (rows + rpb - 1) / rpb;
-  float* g = M.grad.as<float>();
+  const int hb = rows / kColRows;
   cudaError_t e;
   if ((e = M.hpart.ensure((size_t)hb * kHpCols * 4)) != cudaSuccess) return c.cuda_fail(e, "mlp partial");
-  k_bwd_head<<<hb, kMlpHid, 0, s>>>(M.score.as<float>(), M.y.as<float>(), M.wt.as<float>(), bf(M.h2),
-                                    params(M) + kOffW3, rows, rpb, 1.0f / (float)n, bf(M.dz2), M.hpart.as<float>());
-  const dim3 tb(32, 8);
-  k_transpose_bf16<<<dim3(rows / 32, kMlpHid / 32), tb, 0, s>>>(bf(M.dz2), rows, kMlpHid, bf(M.dz2t));
-  k_transpose_bf16<<<dim3(rows / 32, kMlpHid / 32), tb, 0, s>>>(bf(M.h1), rows, kMlpHid, bf(M.h1t));
-  k_transpose_bf16<<<dim3(rows / 32, kMlpInP / 32), tb, 0, s>>>(bf(M.x), rows, kMlpInP, bf(M.xt));
+  k_bwd_head<<<hb, kMlpHid, 0, s>>>(M.score.as<float>(), M.y.as<float>(), M.wt.as<float>(), bf(M.h1), bf(M.h2),
+                                    params(M) + kOffW3, rows, 1.0f / (float)n, bf(M.dz2), bf(M.dz2t), bf(M.h1t),
+                                    M.hpart.as<float>());
   // dL/dh1 = dz2 W2, masked by layer 1's ReLU: dz1 (rows x 256)
   GemmArgs ga{};
   ga.a = bf(M.dz2);
@@ -577,14 +659,16 @@ int mlp_train_device(Context& c, int n, int rows, float lr, bool want_grad) {
   ga.err = M.err.as<int>();
   e = launch_gemm_tn(ga, 256, 1, 1, s);
   if (e != cudaSuccess) return c.cuda_fail(e, "mlp dH1 launch");
-  k_transpose_bf16<<<dim3(rows / 32, kMlpHid / 32), tb, 0, s>>>(bf(M.dz1), rows, kMlpHid, bf(M.dz1t));
-  k_colsum<<<hb, kMlpHid, 0, s>>>(bf(M.dz1), rows, rpb, M.hpart.as<float>());
-  k_sum_head<<<(kHpCols + 255) / 256, 256, 0, s>>>(M.hpart.as<float>(), hb, g, M.loss.as<float>());
-  // weight gradients, split over rows: dW2 = dz2^T h1, dW1 = dz1^T x
+  k_dz1_columns<<<hb, kMlpHid, 0, s>>>(bf(M.dz1), bf(M.x), rows, bf(M.dz1t), bf(M.xt), M.hpart.as<float>());
+  // weight gradients, split over rows: dW2 = dz2^T h1 and dW1 = dz1^T x in one launch, of
+  // 128 x 64 tiles (ten CTAs per split; with tiles of 128 x 256 and a launch each, 16,384
+  // rows ran on 16 SMs: 93 and 46 us, against 36 for both)
   const int kchunk = 2048;
   const int splits = (rows + kchunk - 1) / kchunk;
-  if ((e = M.partial.ensure((size_t)splits * kMlpHid * kMlpHid * 4)) != cudaSuccess)
+  if ((e = M.partial.ensure((size_t)splits * kMlpHid * (kMlpHid + kMlpInP) * 4)) != cudaSuccess)
     return c.cuda_fail(e, "mlp partial");
+  float* part2 = M.partial.as<float>();
+  float* part1 = part2 + (size_t)splits * kMlpHid * kMlpHid;
   GemmArgs gw{};
   gw.a = bf(M.dz2t);
   gw.b = bf(M.h1t);
@@ -593,32 +677,39 @@ int mlp_train_device(Context& c, int n, int rows, float lr, bool want_grad) {
   gw.K = rows;
   gw.lda = gw.ldb = rows;
   gw.kchunk = kchunk;
-  gw.out_f = M.partial.as<float>();
+  gw.out_f = part2;
   gw.err = M.err.as<int>();
-  if ((e = launch_gemm_tn(gw, 256, 0, splits, s)) != cudaSuccess) return c.cuda_fail(e, "mlp dW2 launch");
-  k_sum_splits<<<256, 256, 0, s>>>(M.partial.as<float>(), kMlpHid * kMlpHid, splits, g + kOffW2);
-  GemmArgs g1{};
-  g1.a = bf(M.dz1t);
-  g1.b = bf(M.xt);
-  g1.M = kMlpHid;
-  g1.N = kMlpInP;
-  g1.K = rows;
-  g1.lda = g1.ldb = rows;
-  g1.kchunk = kchunk;
-  g1.out_f = M.partial.as<float>();
-  g1.err = M.err.as<int>();
-  if ((e = launch_gemm_tn(g1, 64, 0, splits, s)) != cudaSuccess) return c.cuda_fail(e, "mlp dW1 launch");
-  k_sum_splits<<<64, 256, 0, s>>>(M.partial.as<float>(), kMlpHid * kMlpInP, splits, g + kOffW1);
-  c.prof.kernel_launches += 12;
-  (void)want_grad;
+  gw.a2 = bf(M.dz1t);
+  gw.b2 = bf(M.xt);
+  gw.N2 = kMlpInP;
+  gw.out2 = part1;
+  if ((e = launch_gemm_tn(gw, 64, 0, splits, s)) != cudaSuccess) return c.cuda_fail(e, "mlp weight gradient launch");
+  StepArgs st{};
+  st.part1 = part1;
+  st.part2 = part2;
+  st.hpart = M.hpart.as<float>();
+  st.splits = splits;
+  st.blocks = hb;
+  st.grad = M.grad.as<float>();
+  st.loss = M.loss.as<float>();
+  st.p = params(M);
+  st.m = M.m.as<float>();
+  st.v = M.v.as<float>();
+  st.w1 = bf(M.w1);
+  st.w2 = bf(M.w2);
+  st.w2t = bf(M.w2t);
+  st.lr = lr;
   if (lr > 0.f) {
     M.step++;
-    const float b1 = 0.9f, b2 = 0.999f;
-    const float c1 = 1.f - std::pow(b1, (float)M.step), c2 = 1.f - std::pow(b2, (float)M.step);
-    k_adam<<<256, 256, 0, s>>>(params(M), g, M.m.as<float>(), M.v.as<float>(), kMlpParams, lr, b1, b2, 1e-8f, c1, c2);
-    pack(c);
-    c.prof.kernel_launches += 1;
+    st.b1 = 0.9f;
+    st.b2 = 0.999f;
+    st.eps = 1e-8f;
+    st.c1 = 1.f - std::pow(st.b1, (float)M.step);
+    st.c2 = 1.f - std::pow(st.b2, (float)M.step);
   }
+  k_step<<<(kMlpParams + 256) / 256, 256, 0, s>>>(st);
+  c.prof.kernel_launches += 5;
+  (void)want_grad;
   return GP_OK;
 }
 

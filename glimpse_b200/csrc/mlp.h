@@ -69,7 +69,8 @@ cudaError_t launch_mlp_fwd(const MlpFwdArgs& a, int grid, cudaStream_t s);
 
 // D = A * B^T over a K range per grid.z slice: A [M][lda], B [N][ldb] (BF16,
 // K contiguous). epi 0: FP32 partial sums out_f[z][M][N]; epi 1: BF16
-// out_b[M][N] = D * (mask[M][N] > 0).
+// out_b[M][N] = D * (mask[M][N] > 0). N2 > 0 (epi 0): a second product of the same M, K
+// and strides, a2 [M] times b2 [N2], into out2[z][M][N2], in the same launch.
 struct GemmArgs {
   const __nv_bfloat16* a;
   const __nv_bfloat16* b;
@@ -78,6 +79,10 @@ struct GemmArgs {
   __nv_bfloat16* out_b;
   const __nv_bfloat16* mask;
   int* err;
+  const __nv_bfloat16* a2;
+  const __nv_bfloat16* b2;
+  int N2;
+  float* out2;
 };
 cudaError_t launch_gemm_tn(const GemmArgs& g, int NT, int epi, int splits, cudaStream_t s);
 

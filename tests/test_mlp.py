@@ -114,6 +114,30 @@ def test_backward_matches_cpu_oracle(ctx, n):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 128, 129, 1984, 2048, 2049, 4200])
+def test_weight_gradient_split_edges(ctx, n):
+    """Row counts around the 128-row tiles and the 2,048-row splits of the weight
+    gradients (a last split of one 128-row tile, a split filled exactly, all eight
+    stages in use once or reused), as the test above; then the Adam step it feeds."""
+    x, y, wt = _problem(n, 31 + n)
+    wt[0] = 1.0  # at least one weighted row
+    p = M.init_params(9)
+    p[M.OFF_B1:M.OFF_W2] = 0.02
+    p[M.OFF_B2:M.OFF_W3] = 0.02
+    ctx.mlp_set_params(p)
+    loss, g = ctx.mlp_train_step(x, y, wt, lr=1e-3, grad=True)
+    loss_ref, g_ref = M.loss_and_grad(p, x, y, wt)
+    assert abs(loss - loss_ref) <= 1e-4 * max(1.0, abs(loss_ref)), (loss, loss_ref)
+    for name, a, b in _blocks():
+        d = np.linalg.norm(g[a:b] - g_ref[a:b])
+        r = np.linalg.norm(g_ref[a:b])
+        assert d <= 1e-2 * r + 1e-7, f"{name}: |dg| {d:.3e} vs |g| {r:.3e}"
+    # Adam's first step: m / c1 = g and v / c2 = g^2, up to the rounding of c1 and c2 (2^-24 / 1e-3)
+    want = p - 1e-3 * g / (np.abs(g) + 1e-8)
+    assert np.abs(ctx.mlp_params() - want).max() <= 1e-3 * 1e-4 + 1e-7
+
+
+@pytest.mark.gpu
 def test_training_reduces_loss(ctx):
     x, y, wt = _problem(8192, 21)
     ctx.mlp_init(3)
