@@ -177,3 +177,36 @@ def test_sweep_shapes_and_panel_sizes_give_the_same_selection(N, L):
             assert orc.select(t, O.STAGE_BURN).tolist() == got[0][t][1]
     finally:
         ctx.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kpbwt", [1, 31, 32, 33, 64, 500, 1500])
+def test_union_order_and_limits(kpbwt):
+    """The union takes 32 pushes at a time: limits inside, at the end of and past a
+    group, and many groups, for diploid targets (two merged lists) and a haploid one,
+    against the level lists walked one push at a time from the last. A limit of the
+    panel's size takes the whole panel instead, without lists."""
+    from glimpse_b200 import native, synth
+    from oracle import oracle as O
+    w = synth.make_panel_and_targets(1500, 900, 0.2, 0.4, 4, ("uniform", 0.5, 2.0), ("fixed", 90), seed=71,
+                                     sparse_maf=0.003)
+    T = dataclasses.replace(w.targets, ploidy=w.targets.ploidy.copy(), kpbwt=np.full(4, kpbwt, np.int32))
+    T.ploidy[2] = 1
+    rng = np.random.default_rng(kpbwt)
+    ctx = native.Context(w.panel, kinit=60, kpbwt=kpbwt, pbwt_depth=7, pbwt_modulo_cm=0.05)
+    try:
+        ctx.set_targets(T, kpbwt=T.kpbwt)
+        ctx.set_haps(np.stack([_noisy(rng, T.truth[t, 0], 0.03) for t in range(T.n)]),
+                     np.stack([_noisy(rng, T.truth[t, 1], 0.03) for t in range(T.n)]))
+        ctx.select(O.STAGE_BURN, 3)
+        for t in range(T.n):
+            want = set()
+            for level in ctx.pbwt_states(t, depth=7):
+                for h in level[::-1].tolist():
+                    if len(want) < kpbwt:
+                        want.add(h)
+            if kpbwt >= w.panel.n_ref_haps:
+                want = range(w.panel.n_ref_haps)
+            assert sorted(want) == ctx.states(t).tolist()
+    finally:
+        ctx.close()
