@@ -329,25 +329,26 @@ def run_ours(args):
     r2 = synth.dosage_r2(ds_h.numpy(), T.truth.sum(1))
 
     peak, peak_kind = load_peaks()
-    # algorithmic bytes per cell: full store 4 B written + 4 B read + 2 x 1/8 B Hvar;
-    # checkpoints 2 x 4/32 (FP32) or 2 x 2/32 (BF16) B + 3 x 1/8 B Hvar (forward, recompute, backward)
-    bpc = {"full": 8.25, "f32": 0.625, "bf16": 0.5}[args.precision]
-    kname = "k_impute_warp" if args.precision == "full" else "k_impute_ckpt"
+    # algorithmic bytes per cell: a row of either direction per 16 sites, written and read, and
+    # 1/8 B Hvar for each chain and the blocks; BF16 checkpoints: 2 B per 32 sites written and
+    # read, and Hvar once more for the recomputed half
+    bpc = {"full": 1.375, "f32": 1.375, "bf16": 1.625}[args.precision]
+    kname = "k_impute_chain" if args.precision == "full" else "k_ckpt_chain"
     achieved = prof["impute_cells"] * bpc / (prof["impute_ms"] / 1000.0) / 1e9 if prof["impute_ms"] > 0 else 0.0
     per_launch_cells = prof["impute_cells"] / max(1, prof["impute_launches"])
     tpc = read_traffic(kname)
-    roofline = {"bound": "hbm", "kernel": kname + " (imputation forward-backward)", "achieved": achieved,
+    roofline = {"bound": "latency", "kernel": kname + " + k_impute_block (imputation forward-backward)", "achieved": achieved,
                 "peak": peak, "unit": "GB/s", "frac": achieved / peak, "peak_kind": peak_kind,
                 "algorithmic_bytes_per_cell": bpc, "cells_per_launch": per_launch_cells,
                 "launch_ms": prof["impute_ms"] / max(1, prof["impute_launches"]),
                 "traffic": (tpc * per_launch_cells) if tpc is not None else None}
-    # Phasing (k_phase) is bound by its per-site dependent chain, not by HBM: its
-    # messages live in registers. Reported against the FP32 issue rate at the
+    # Phasing (k_phase_chain, k_phase_units, k_phase_draw) is bound by its per-site dependent
+    # chain, not by HBM: its messages live in registers. Reported against the FP32 issue rate at the
     # sampled clock: 148 SMs x 128 lanes x 2 flop per FMA.
     sm_mhz = clk.get("sm_mhz") or 1965.0
     fp32_peak = 148 * 128 * 2 * sm_mhz * 1e6 / 1e12
     phase_cells_s = prof["phase_cells"] / (prof["phase_ms"] / 1000.0) if prof["phase_ms"] > 0 else 0.0
-    phase = {"kernel": "k_phase (phasing backward + forward with diplotype sampling)", "bound": "latency",
+    phase = {"kernel": "k_phase_chain + k_phase_units + k_phase_draw (phasing passes and diplotype sampling)", "bound": "latency",
              "cells_per_s": phase_cells_s, "launch_ms": prof["phase_ms"] / max(1, prof["phase_launches"]),
              "share_of_step": prof["phase_ms"] / args.steps / ms, "flops_per_cell": 4,
              "fp32_tflops": phase_cells_s * 4 / 1e12, "fp32_peak_tflops": fp32_peak,
@@ -361,11 +362,11 @@ def run_ours(args):
             "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True, "scaling": "weak",
             "vs_baseline": None, "dtype": "f32", "data": "synthetic",
             "config": {"workload": workload_label(args.config), "targets_per_gpu": T.n, "iterations_per_step": N_ITER,
-                       "l2": "no flush: per-step working set (alpha store, prefix arrays) is tens of GB >> 126 MB L2",
+                       "l2": "no flush: per-step working set (kept rows, phasing messages, prefix arrays) is tens of GB >> 126 MB L2",
                        "parallelism": f"targets per GPU, {world} rank(s), no collective on the data path"},
-            "precision": {"full": "every forward row in FP32 (as the reference)",
-                          "f32": "FP32 checkpoints every 32 sites, recompute",
-                          "bf16": "BF16 checkpoints every 32 sites, FP32 recompute"}[args.precision],
+            "precision": {"full": "FP32 (as the reference)",
+                          "f32": "FP32, FP64 log-likelihood",
+                          "bf16": "a row rounded to BF16 every 32 sites, FP32 recompute, FP64 log-likelihood"}[args.precision],
             "autotuned": dict(zip(("chains_per_cta", "sweep_haps_per_warp", "phase_placement", "ms"),
                                   (lambda tu: (*tu[:3], [round(float(x), 3) for x in tu[3]]))(ctx.tuning()))),
             "hmm_cells_per_s": world * hmm_cells / (ms / 1000.0),

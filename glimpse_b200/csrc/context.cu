@@ -72,7 +72,7 @@ void Context::prof_resolve() {
       if (p.kind == 0) {
         prof.impute_ms += ms;
         prof.impute_cells += p.cells;
-        prof.impute_bytes += p.cells * 8.25;  // 1/8 B Hvar + 4 B alpha, forward and backward
+        prof.impute_bytes += p.cells * 1.375;  // two rows per 16 sites, written and read, 1/8 B Hvar three times
         prof.impute_launches++;
       } else if (p.kind == 1) {
         prof.phase_ms += ms;
