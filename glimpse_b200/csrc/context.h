@@ -115,13 +115,13 @@ struct Context {
   DevBuf ckpt, ckpt_sum, loglik;  // checkpointed imputation: BF16 rows, AlphaSums, log-likelihoods
   int loglik_n = 0;                             // entries of the last checkpointed imputation call
   int impute_chunks = 0;  // launches pairs of the last run_impute (1 when the whole batch fit)
-  int phase_chunks = 0;   // k_phase launches of the last run_phase
+  int phase_chunks = 0;   // chunks of the last run_phase
   // Autotuner: launch shapes picked by timing every candidate on the first batch
   // large enough to tell them apart; fixed_* (gp_tuning_set) override it.
   int tune_cpc = 0, tune_hpw = 0;     // chosen chains per CTA / haplotypes per sweep warp (0: not yet)
   int fixed_cpc = 0, fixed_hpw = 0;
   int fixed_porder = 0;  // the caller's phasing placement, reported back; every placement runs the same launches
-  // phase-1 ms for 1, 2, 4 chains per CTA; sweep ms for 1, 2, 4, 8; k_phase ms for placements 1, 2
+  // ms of the chains for 1, 2, 4 chains per CTA; sweep ms for 1, 2, 4, 8; two unused
   float tune_ms[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
   int sm_count = 0;
   // streams beside `stream` for launches that run together (fork_streams / join_streams)

@@ -343,11 +343,11 @@ int gp_learned_train(gp_ctx* ctx, int32_t kcand, float kpos, int32_t steps, int3
  * enough to tell them apart (16 haplotypes for the imputation chains, 32 target
  * haplotypes for the PBWT sweep): chains per CTA of the imputation
  * forward-backward (1, 2 or 4: how many sequential chains share an SM's
- * shared memory and schedulers) and target haplotypes per warp of the PBWT
+ * schedulers) and target haplotypes per warp of the PBWT
  * sweep (1, 2, 4 or 8: lockstep lanes against divergence). Results do not
  * depend on either. gp_tuning_set fixes them (0: tune again on next use);
  * gp_tuning_get reports the shapes in use (0: not tuned yet) and, in ms[7],
- * the measured times (phase-1 chains for 1, 2, 4 chains per CTA, then the sweep
+ * the measured times (the chains for 1, 2, 4 chains per CTA, then the sweep
  * for 1, 2, 4, 8 haplotypes per warp; -1 where a shape did not fit, 0 where
  * not measured). phase_placement (1, the default, or 2) is kept and reported
  * back; the chains of a phasing launch are all resident together, so it no
