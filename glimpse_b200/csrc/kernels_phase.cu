@@ -1028,8 +1028,12 @@ int launch_phase_units(int max_units, uint32_t narrow, const int32_t* tsel, int 
     k_phase_units<<<dim3(g, nb), 256, sizeof(UnitSmem), s>>>(tsel, nstates, hvar, WB, Kp, P, S, seed, iteration,
                                                              target_ids, narrow);
   }
-  k_phase_draw<<<(nb + 3) / 4, 128, 0, s>>>(tsel, nb, P, S, seed, iteration, target_ids);
   return GP_OK;
+}
+
+void launch_phase_draw(const int32_t* tsel, int nb, PhaseVars P, PhaseStore S, uint64_t seed, int iteration,
+                       const int32_t* target_ids, cudaStream_t s) {
+  k_phase_draw<<<(nb + 3) / 4, 128, 0, s>>>(tsel, nb, P, S, seed, iteration, target_ids);
 }
 
 void launch_phase_writeback(const int32_t* tsel, int nb, const int32_t* poly, const int32_t* polyidx, int L,

@@ -67,11 +67,14 @@ constexpr int kPhaseNarrowJ = 5;
 int launch_phase_chain(int J, bool narrow, const int32_t* tsel, int nb, const int32_t* nstates, const uint32_t* hvar,
                        int WB, int Kp, const int32_t* npoly, PhaseVars P, PhaseStore S, const ModelConst& mc,
                        cudaStream_t s);
-// After the chains, for entries of any K: the units and draws. max_units: the
-// largest count of segment boundaries and flat hets of an entry; bit J of narrow: the
-// chains of class J ran narrow.
+// After the chains, for entries of any K: the units. max_units: the largest count of
+// segment boundaries and flat hets of an entry; bit J of narrow: the chains of class J
+// ran narrow.
 int launch_phase_units(int max_units, uint32_t narrow, const int32_t* tsel, int nb, const int32_t* nstates,
                        const uint32_t* hvar, int WB, int Kp, PhaseVars P, PhaseStore S, uint64_t seed, int iteration,
+                       const int32_t* target_ids, cudaStream_t s);
+// After the units: the diplotype chains.
+void launch_phase_draw(const int32_t* tsel, int nb, PhaseVars P, PhaseStore S, uint64_t seed, int iteration,
                        const int32_t* target_ids, cudaStream_t s);
 void launch_phase_writeback(const int32_t* tsel, int nb, const int32_t* poly, const int32_t* polyidx, int L,
                             PhaseVars V, PhaseStore S, const ModelConst& mc, uint64_t seed, int iteration,
