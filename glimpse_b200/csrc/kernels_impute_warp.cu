@@ -14,7 +14,7 @@
 //                   are the chain's own operations on the same numbers, so the
 //                   rows it forms are the chain's, bit for bit.
 // Measured, both kernels (K = 1,000, 62,700 polymorphic sites): one haplotype 11.6 ms,
-// 256 haplotypes 25.8; with every row stored and read back by the chains, split in
+// 256 haplotypes 23.6; with every row stored and read back by the chains, split in
 // the middle of the haplotype, 16.3 and 33 ms.
 // Nothing of the size (sites x states) goes through memory: 4 bytes per 16 cells
 // and direction are written and read, where storing every row takes 8 bytes a cell.
