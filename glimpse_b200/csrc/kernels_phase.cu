@@ -355,14 +355,18 @@ __global__ void __launch_bounds__(256 / V, V == 4 ? (J <= 3 ? 6 : 4) : J <= 2 ? 
   const uint32_t* hv = hvar + (size_t)t * WB * Kp;
   const int nblk_poly = (npoly[t] + 31) >> 5;
   const int4* recs = (fwd ? P.recf : P.recb) + (size_t)b * P.lv;
-  // slot i = V j + s: state k = 256 j + kb[s]
-  int kb[V];
+  // slot i = V j + s: state k = 256 j + kb[s]. A slot without a state (of the last V)
+  // repeats the last state, words and all, and does not count in the sums: its messages
+  // are those of a state. (As a state of its own, with allele 0 everywhere, it would grow by
+  // ee / ed at every hom that all real states mismatch, and overflow.)
+  int kb[V], kw[V];
   bool last[V];
   f2 exists[V];
 #pragma unroll
   for (int s = 0; s < V; ++s) {
     kb[s] = 32 * (V * warp + (s ^ set_swap<V>(lane))) + lane;
     last[s] = 256 * (J - 1) + kb[s] < K;
+    kw[s] = min(256 * (J - 1) + kb[s], K - 1);
     exists[s] = last[s] ? f2_pack(1.f, 1.f) : f2_pack(0.f, 0.f);
   }
   auto has = [&](int i) { return i < NS - V || last[i % V]; };
@@ -376,11 +380,12 @@ __global__ void __launch_bounds__(256 / V, V == 4 ? (J <= 3 ? 6 : 4) : J <= 2 ? 
     if (blk < 0 || blk >= nblk_poly) return;
 #pragma unroll
     for (int i = 0; i < NS; ++i)
-      if (has(i)) cp_async4(&words[blk & 1][i][tid], hv + (size_t)blk * Kp + 256 * (i / V) + kb[i % V]);
+      cp_async4(&words[blk & 1][i][tid],
+                hv + (size_t)blk * Kp + (i < NS - V ? 256 * (i / V) + kb[i % V] : kw[i % V]));
   };
   auto read_words = [&](int blk) {
 #pragma unroll
-    for (int i = 0; i < NS; ++i) w[i] = has(i) ? words[blk & 1][i][tid] : 0u;
+    for (int i = 0; i < NS; ++i) w[i] = words[blk & 1][i][tid];
   };
   // Rows in slot order, only the halves back in place; k_phase_units undoes the rest of h -> h ^ f.
   auto store_rows = [&](float* dst) {

@@ -351,6 +351,12 @@ def restate_lib():
                                       C.POINTER(C.c_int64), C.POINTER(C.c_int32), C.POINTER(C.c_uint32), C.c_int,
                                       C.c_double, C.c_float, C.c_float, C.POINTER(C.c_float), C.POINTER(C.c_uint8),
                                       C.POINTER(C.c_int32), C.c_int, C.POINTER(C.c_double), C.POINTER(C.c_int32)]
+        lib.rs_rephase.restype = C.c_int
+        lib.rs_rephase.argtypes = [C.c_int, C.POINTER(C.c_uint8), C.POINTER(C.c_uint8), C.POINTER(C.c_uint8),
+                                   C.POINTER(C.c_double), C.POINTER(C.c_int32), C.POINTER(C.c_uint8), C.c_int,
+                                   C.POINTER(C.c_int64), C.POINTER(C.c_int32), C.POINTER(C.c_uint32), C.c_int,
+                                   C.c_double, C.c_float, C.c_float, C.POINTER(C.c_uint8), C.POINTER(C.c_float),
+                                   C.POINTER(C.c_uint8), C.POINTER(C.c_uint8)]
         _restate = lib
     return _restate
 
@@ -416,3 +422,39 @@ def restate_state_post(panel, states, HL, flat, ne=100000, err_imp=1e-12):
                       _p(keep[9], C.c_float), _p(keep[10], C.c_uint8), _p(keep[11], C.c_int32), nwin,
                       _p(mass, C.c_double), _p(ns, C.c_int32))
     return mass.reshape(nwin, K), ns
+
+
+def stream_floats(seed, purpose, iteration, target, n):
+    """The first n words of a random stream (replay_rng.h) as floats in [0, 1)."""
+    lo, s32 = np.uint64(0xFFFFFFFF), np.uint64(32)
+    q = np.arange((n + 3) // 4, dtype=np.uint64)
+    c = [q, np.full_like(q, target), np.full_like(q, iteration), np.full_like(q, purpose)]
+    k0, k1 = seed & 0xFFFFFFFF, seed >> 32
+    for _ in range(10):
+        p0, p1 = c[0] * np.uint64(0xD2511F53), c[2] * np.uint64(0xCD9E8D57)
+        c = [(p1 >> s32) ^ c[1] ^ np.uint64(k0), p1 & lo, (p0 >> s32) ^ c[3] ^ np.uint64(k1), p0 & lo]
+        k0, k1 = (k0 + 0x9E3779B9) & 0xFFFFFFFF, (k1 + 0xBB67AE85) & 0xFFFFFFFF
+    w = np.stack(c, 1).ravel()[:n].astype(np.float32) * np.float32(2.0 ** -32)
+    return np.minimum(w, np.nextafter(np.float32(1), np.float32(0)))
+
+
+def restate_rephase(panel, states, h0, h1, flat, iteration, target, seed=15052011, ne=100000, err_phase=1e-4):
+    """FP32 restatement of phasing_hmm::rephaseHaplotypes for one target: (H0, H1, invalid sums seen)."""
+    L = panel.n_sites
+    comrow = np.full(L, -1, np.int32)
+    com = np.flatnonzero(panel.flag_common)
+    comrow[com] = np.arange(com.size, dtype=np.int32)
+    keep = [np.ascontiguousarray(x) for x in (panel.flag_common.astype(np.uint8), panel.lq.astype(np.uint8),
+                                              panel.major.astype(np.uint8), panel.cm.astype(np.float64), comrow,
+                                              panel.hvar.astype(np.uint8), panel.shap_off.astype(np.int64),
+                                              panel.shap_sites.astype(np.int32), np.asarray(states, np.uint32),
+                                              np.asarray(flat, np.uint8), stream_floats(seed, 4, iteration, target, L + 1))]
+    g0, g1 = np.array(h0, np.uint8), np.array(h1, np.uint8)
+    ed = np.float32(err_phase)
+    bad = restate_lib().rs_rephase(L, _p(keep[0], C.c_uint8), _p(keep[1], C.c_uint8), _p(keep[2], C.c_uint8),
+                                   _p(keep[3], C.c_double), _p(keep[4], C.c_int32), _p(keep[5], C.c_uint8),
+                                   (panel.n_ref_haps + 7) // 8, _p(keep[6], C.c_int64), _p(keep[7], C.c_int32),
+                                   _p(keep[8], C.c_uint32), keep[8].size, (-0.04 * ne) / panel.n_ref_haps, float(ed),
+                                   float(np.float32(1.0 - float(ed))), _p(keep[9], C.c_uint8), _p(keep[10], C.c_float),
+                                   _p(g0, C.c_uint8), _p(g1, C.c_uint8))
+    return g0, g1, bool(bad)

@@ -200,3 +200,40 @@ def test_state_count_edges_and_mixed_classes(edges):
             assert np.array_equal(g0[i], r0) and np.array_equal(g1[i], r1), edges[i]
     finally:
         ctx.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("K", [1, 2, 3, 40, 300])
+def test_small_sets_on_long_chunks_match_restatement(K):
+    """Register slots without a state must stay at 0 however long the chunk is: the
+    homs that all states mismatch (here all sites where they agree on alt, the
+    targets being ref) scale whatever sits there by ee / ed each, so that a small
+    set overflowed it within a chunk. 20,000 sites, three targets, one of them with
+    flat sites at the ends: the haplotypes of the FP32 restatement, bit for bit."""
+    from oracle import oracle as O
+    from glimpse_b200 import native, synth
+    w = synth.make_panel_and_targets(1000, 20000, 0.5, 0.0, 3, ("uniform", 0.5, 2.0), ("fixed", 100), seed=83,
+                                     sparse_maf=0.005, alt_major_frac=0.1)
+    P, T = w.panel, w.targets
+    rng = np.random.default_rng(K)
+    cases = []
+    for t in range(3):
+        s = np.sort(rng.choice(P.n_ref_haps, size=K, replace=False)).astype(np.uint32)
+        h0, h1, flat = _noisy_haps(rng, T.truth[t, 0]), _noisy_haps(rng, T.truth[t, 1]), T.flat[t].copy()
+        alleles = (P.hvar[:, s >> 3] >> (7 - (s & 7)).astype(np.uint8)) & 1
+        alt = np.flatnonzero(P.flag_common)[alleles.all(axis=1)]
+        assert K == 300 or alt.size > 100
+        h0[alt] = h1[alt] = 0
+        if t == 1:
+            flat[:500] = flat[-500:] = 1
+        cases.append((s, h0, h1, flat))
+    ctx = native.Context(P)
+    try:
+        g0, g1 = ctx.rephase_batch([c[0] for c in cases], np.stack([c[1] for c in cases]),
+                                   np.stack([c[2] for c in cases]), np.stack([c[3] for c in cases]), 3)
+    finally:
+        ctx.close()
+    for t, (s, h0, h1, flat) in enumerate(cases):
+        r0, r1, invalid = O.restate_rephase(P, s, h0, h1, flat, 3, t)
+        assert not invalid
+        assert np.array_equal(g0[t], r0) and np.array_equal(g1[t], r1), t
