@@ -267,8 +267,8 @@ __device__ __forceinline__ void lds(unsigned addr, float& a, float& b) {
   asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(a), "=f"(b) : "r"(addr));
 }
 
-// A pair of rows over the block. MASK: states that do not exist are held at 0 by a
-// factor (1 elsewhere, exact). LAST: the haplotype's last block, where the site
+// A pair of rows over the block. MASK: forward values of states that do not exist are
+// held at 0 by a factor (1 elsewhere, exact). LAST: the haplotype's last block, where the site
 // `last` starts the backward recursion and its posterior uses alpha alone
 // (imputation_hmm.cpp:268-300).
 template <bool MASK, bool LAST>
@@ -322,7 +322,10 @@ __global__ void __launch_bounds__(CK ? 256 : 128, CK ? 2 : 4) k_impute_block(Cha
   const float* base = A.rows + A.row_off[t] + (CK ? Ks - K : 0);
   const uint32_t* hvt = A.hvar + (size_t)t * A.WB * A.Kp - pad;
 
-  // Rows j and j + 1 of this thread in block b: words and the kept values entering from both sides.
+  // Rows j and j + 1 of this thread in block b: words and the kept values entering from both
+  // sides. A state that does not exist takes those of the nearest one, so that its backward
+  // values are a state's: from 0, with allele 0 everywhere, they would grow by up to 1 / min_gl
+  // at each site that all states mismatch, and 0 * inf would enter the sums.
   struct Pair {
     uint32_t w0, w1;
     float a0, a1, b0, b1;
@@ -330,17 +333,17 @@ __global__ void __launch_bounds__(CK ? 256 : 128, CK ? 2 : 4) k_impute_block(Cha
   auto load = [&](int b, int j) {
     Pair p;
     const int o = NT * j + tid;
-    const bool e0 = CK ? o < K : j > 0 || (j == 0 && tid >= pad), e1 = CK ? o + NT < K : j >= 0 || tid >= pad;
-    const uint32_t* hv = hvt + (size_t)((b * RS) >> 5) * A.Kp + o;
-    const float* ar = base + (size_t)b * Ks + o;
+    const int o0 = CK ? min(o, K - 1) : max(o, pad), o1 = CK ? min(o + NT, K - 1) : max(o + NT, pad);
+    const uint32_t* hv = hvt + (size_t)((b * RS) >> 5) * A.Kp;
+    const float* ar = base + (size_t)b * Ks;
     const float* br = ar + (size_t)nrow * Ks;
     const bool left = b > 0, right = b < nrow - 1;
-    p.w0 = e0 ? hv[0] : 0u;
-    p.w1 = e1 ? hv[NT] : 0u;
-    p.a0 = left && e0 ? ar[0] : 0.f;
-    p.a1 = left && e1 ? ar[NT] : 0.f;
-    p.b0 = right && e0 ? br[0] : 0.f;
-    p.b1 = right && e1 ? br[NT] : 0.f;
+    p.w0 = hv[o0];
+    p.w1 = hv[o1];
+    p.a0 = left ? ar[o0] : 0.f;
+    p.a1 = left ? ar[o1] : 0.f;
+    p.b0 = right ? br[o0] : 0.f;
+    p.b1 = right ? br[o1] : 0.f;
     return p;
   };
   // Site data of a block, one site per thread of the first RS, and the site of this lane's output.

@@ -204,3 +204,42 @@ def test_checkpointed_block_and_state_count_edges(sites):
             e = float(np.abs(hp[i].astype(np.float64) - hr.astype(np.float64)).max())
             assert e <= tol, f"mode {m}, K={Ks[i]}: max |HP - HP_fp64| = {e:.3e}"
             assert abs(ll[i] - llr) <= 1e-6 * sites + ll_tol, (m, Ks[i])
+
+
+@pytest.mark.gpu
+def test_confident_likelihoods_against_all_states():
+    """Forty sites where every panel haplotype carries alt and the target is ref for
+    certain (likelihoods 1 and 1e-10, the clamp): each scales by up to 1e10 what is
+    not a state, so that four of a block's 16 sites would overflow an unused slot.
+    State counts with unused slots in either kernel, all precision modes: finite HP
+    within 1e-5 of FP64 (BF16 rows: 5e-3), the log-likelihood within 1e-6 per site
+    (BF16: 2^-8 more)."""
+    from glimpse_b200 import native, synth
+    from oracle import oracle as O
+    L, run = 260, slice(90, 130)
+    w = synth.make_panel_and_targets(1000, L, 0.2, 0.0, 2, ("uniform", 0.4, 2.0), ("fixed", 200), seed=67,
+                                     sparse_maf=0.005)
+    P, T = w.panel, w.targets
+    P.hvar[run], P.calt[run], P.cref[run], P.major[run] = 255, 1000, 0, 1
+    rng = np.random.default_rng(3)
+    Ks = [1, 2, 3, 127, 130, 255, 257, 520]
+    states = [np.sort(rng.choice(1000, size=K, replace=False)).astype(np.uint32) for K in Ks]
+    flats = np.stack([T.flat[i % 2] for i in range(len(Ks))])
+    flats[:, run] = 0
+    hls = np.stack([init_hl(T.gl[i % 2], flats[i]) for i in range(len(Ks))])
+    hls[:, 2 * run.start:2 * run.stop:2], hls[:, 2 * run.start + 1:2 * run.stop:2] = 1.0, 1e-10
+    ref = [O.restate_impute(P, s, hl, fl, precision=64) for s, hl, fl in zip(states, hls, flats)]
+    ctx = native.Context(P)
+    try:
+        for m, tol, ll_tol in ((native.PRECISION_FULL, TOL, None), (native.PRECISION_CKPT_F32, TOL, 0.0),
+                               (native.PRECISION_CKPT_BF16, 5e-3, 2.0 ** -8)):
+            ctx.set_precision(m)
+            hp = ctx.impute_batch(states, hls, flats)
+            assert np.isfinite(hp).all(), m
+            for i, (hr, llr) in enumerate(ref):
+                e = float(np.abs(hp[i].astype(np.float64) - hr.astype(np.float64)).max())
+                assert e <= tol, f"mode {m}, K={Ks[i]}: max |HP - HP_fp64| = {e:.3e}"
+                if ll_tol is not None:
+                    assert abs(ctx.loglik(len(Ks))[i] - llr) <= 1e-6 * L + ll_tol, (m, Ks[i])
+    finally:
+        ctx.close()
