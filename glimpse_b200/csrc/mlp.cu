@@ -483,7 +483,7 @@ __global__ void __launch_bounds__(256) k_step(StepArgs a) {
     g = sum_strided(a.hpart + col, a.blocks, kHpCols);
   }
   a.grad[i] = g;
-  if (a.lr <= 0.f) return;
+  if (!(a.lr > 0.f)) return;  // no update with a NaN rate either, as on the host
   const float mi = a.b1 * a.m[i] + (1.f - a.b1) * g;
   const float vi = a.b2 * a.v[i] + (1.f - a.b2) * g * g;
   a.m[i] = mi;

@@ -149,3 +149,19 @@ def test_training_reduces_loss(ctx):
     # the oracle agrees on the trained parameters' loss
     lr_, _ = M.loss_and_grad(ctx.mlp_params(), x, y, wt)
     assert abs(lr_ - l1) <= 1e-3 * max(1.0, abs(l1))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lr", [float("nan"), -1e-3, 0.0])
+def test_no_update_without_a_positive_rate(ctx, lr):
+    """A rate that is not above 0, NaN included, gives loss and gradient and leaves
+    the parameters and Adam's moments: the step after it is Adam's first."""
+    x, y, wt = _problem(200, 5)
+    p = M.init_params(9)
+    ctx.mlp_set_params(p)
+    _, g0 = ctx.mlp_train_step(x, y, wt, lr=0.0, grad=True)
+    _, g1 = ctx.mlp_train_step(x, y, wt, lr=lr, grad=True)
+    assert np.array_equal(g0, g1) and np.array_equal(ctx.mlp_params(), p)
+    ctx.mlp_train_step(x, y, wt, lr=1e-3)
+    want = p - 1e-3 * g0 / (np.abs(g0) + 1e-8)
+    assert np.abs(ctx.mlp_params() - want).max() <= 1e-3 * 1e-4 + 1e-7
