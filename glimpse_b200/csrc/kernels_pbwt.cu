@@ -238,6 +238,30 @@ __global__ void k_event_bits(PbwtSelectArgs a) {
 // values, and a selectK waited for its ids.
 constexpr int kRankStages = 3;
 
+// Group q of rank rows goes to stage q % kRankStages and completes the phase of this
+// parity there. While group g is waited for, the groups g .. g + kRankStages - 1 are
+// requested and not waited for (as far as there are any).
+__host__ __device__ constexpr uint32_t rank_parity(int q) { return (uint32_t)(q / kRankStages) & 1u; }
+
+// The sweep's own stage and parity, and its requests, over n groups.
+constexpr bool ring_agrees(int n) {
+  int stage = kRankStages - 1, requested[kRankStages] = {};
+  uint32_t parity = 1u;
+  for (int st = 0; st < kRankStages && st < n; ++st) requested[st] = 1;
+  for (int g = 0; g < n; ++g) {
+    if (g > 0 && g + kRankStages - 1 < n) ++requested[stage];
+    if (++stage == kRankStages) {
+      stage = 0;
+      parity ^= 1u;
+    }
+    if (stage != g % kRankStages || parity != rank_parity(g)) return false;
+    for (int q = g; q < g + kRankStages && q < n; ++q)  // what a time-out has to wait for: every stage's last request
+      if (rank_parity(q) != ((uint32_t)(requested[q % kRankStages] - 1) & 1u)) return false;
+  }
+  return true;
+}
+static_assert(ring_agrees(1) && ring_agrees(2) && ring_agrees(3) && ring_agrees(4) && ring_agrees(17), "rank row stages");
+
 template <int HPW, bool RING>
 __global__ void __launch_bounds__(32, 1) k_pbwt_sweep(PbwtSelectArgs a, int rows_per) {
   constexpr int G = 32 / HPW;
@@ -448,10 +472,12 @@ __global__ void __launch_bounds__(32, 1) k_pbwt_sweep(PbwtSelectArgs a, int rows
       }
     }
   }
-  if (failed) {
-    // the other stages' copies may still be under way: wait for each, bounded as well, before the memory is given up
+  if (RING && failed) {
+    // The copies requested and not waited for may still be under way: wait for each, bounded
+    // as well, before the memory is given up.
     if (lane == 0) *a.overflow = 2;
-    for (int st = 0; st < kRankStages; ++st) tc::mbar_wait(&bars[st], st <= stage ? parity : parity ^ 1u);
+    for (int q = next_rows / rows_per - kRankStages; q * rows_per < min(next_rows, ncom); ++q)
+      tc::mbar_wait(&bars[q % kRankStages], rank_parity(q));
     return;
   }
   if (!act) return;
