@@ -474,11 +474,10 @@ __global__ void __launch_bounds__(32, 1) k_pbwt_sweep(PbwtSelectArgs a, int rows
   }
   if (RING && failed) {
     // The copies requested and not waited for may still be under way: wait for each, bounded
-    // as well, before the memory is given up.
-    if (lane == 0) *a.overflow = 2;
+    // as well, before the memory is given up. The lists so far are in order for the union.
+    *a.overflow = 2;
     for (int q = next_rows / rows_per - kRankStages; q * rows_per < min(next_rows, ncom); ++q)
       tc::mbar_wait(&bars[q % kRankStages], rank_parity(q));
-    return;
   }
   if (!act) return;
   pu.flush();
