@@ -595,17 +595,20 @@ static void launch_sweep(const PbwtSelectArgs& a, cudaStream_t s) {
   }
 }
 
-void launch_pbwt_sweep(const PbwtSelectArgs& a, int hpw, cudaStream_t s) {
+cudaError_t launch_pbwt_sweep(const PbwtSelectArgs& a, int hpw, cudaStream_t s) {
   if (hpw == 1) launch_sweep<1>(a, s);
   else if (hpw == 2) launch_sweep<2>(a, s);
   else if (hpw == 4) launch_sweep<4>(a, s);
   else launch_sweep<8>(a, s);
+  return cudaGetLastError();
 }
 
-void launch_pbwt_select(const PbwtSelectArgs& a, int hpw, cudaStream_t s) {
+cudaError_t launch_pbwt_select(const PbwtSelectArgs& a, int hpw, cudaStream_t s) {
   launch_pbwt_prepare(a, s);
-  launch_pbwt_sweep(a, hpw, s);
+  const cudaError_t e = launch_pbwt_sweep(a, hpw, s);
+  if (e != cudaSuccess) return e;  // without the sweep there are no lists to unite
   k_pbwt_union<<<a.n_targets, 32, 0, s>>>(a);
+  return cudaGetLastError();
 }
 
 void launch_pbwt_prepare(const PbwtSelectArgs& a, cudaStream_t s) {

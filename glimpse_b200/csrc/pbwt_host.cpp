@@ -564,11 +564,11 @@ int Context::pbwt_select_states(int stage, int iteration, int Kp) {
       for (int ci = 0; ci < 4; ++ci) {
         cudaMemcpyAsync(a.tar_hap, tune_tarhap.ptr, (size_t)a.n_haps, cudaMemcpyDeviceToDevice, stream);
         cudaEventRecord(e0, stream);
-        launch_pbwt_sweep(a, cand[ci], stream);
+        const cudaError_t el = launch_pbwt_sweep(a, cand[ci], stream);
         cudaEventRecord(e1, stream);
         float ms = 1e30f;
-        if (cudaEventSynchronize(e1) == cudaSuccess) cudaEventElapsedTime(&ms, e0, e1);
-        tune_ms[3 + ci] = ms;
+        if (cudaEventSynchronize(e1) == cudaSuccess && el == cudaSuccess) cudaEventElapsedTime(&ms, e0, e1);
+        tune_ms[3 + ci] = el == cudaSuccess ? ms : -1.f;
         if (ms < best) {
           best = ms;
           hpw = cand[ci];
@@ -581,11 +581,12 @@ int Context::pbwt_select_states(int stage, int iteration, int Kp) {
       prof.kernel_launches += 7;
     }
   }
-  launch_pbwt_select(a, hpw, stream);
+  cudaError_t e = launch_pbwt_select(a, hpw, stream);
+  if (e != cudaSuccess) return cuda_fail(e, "pbwt selection launch");
   prof.kernel_launches += 5;
   int32_t ovf = 0;
   cudaMemcpyAsync(&ovf, T.overflow.ptr, 4, cudaMemcpyDeviceToHost, stream);
-  cudaError_t e = cudaStreamSynchronize(stream);
+  e = cudaStreamSynchronize(stream);
   if (e != cudaSuccess) return cuda_fail(e, "pbwt selection");
   if (ovf == 2) return (fail(GP_E_CUDA, "PBWT selection: a copy into shared memory timed out"), GP_E_CUDA);
   if (ovf) return (fail(GP_E_DATA, "PBWT selection: per-level state list exceeded its capacity"), GP_E_DATA);

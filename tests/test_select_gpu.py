@@ -210,3 +210,30 @@ def test_union_order_and_limits(kpbwt):
             assert sorted(want) == ctx.states(t).tolist()
     finally:
         ctx.close()
+
+
+@pytest.mark.gpu
+def test_deep_lists_on_a_panel_without_staged_rows():
+    """6,500 levels do not fit the SM for 8 haplotypes: an error, not a union of lists
+    that no sweep wrote."""
+    from glimpse_b200 import native, synth
+    from oracle import oracle as O
+    w = synth.make_panel_and_targets(70000, 60, 0.2, 0.4, 2, ("uniform", 0.5, 2.0), ("fixed", 90), seed=71,
+                                     sparse_maf=0.001)
+    T = w.targets
+    got = []
+    for depth, hpw in ((6500, 1), (6500, 8)):
+        ctx = native.Context(w.panel, kinit=60, kpbwt=90, pbwt_depth=depth, pbwt_modulo_cm=0.05)
+        try:
+            ctx.tuning_set(0, hpw, 0)
+            ctx.set_targets(T, kpbwt=T.kpbwt)
+            ctx.set_haps(T.truth[:, 0], T.truth[:, 1])
+            if (depth, hpw) == (6500, 8):
+                with pytest.raises(native.GpError, match="selection launch"):
+                    ctx.select(O.STAGE_BURN, 3)
+                ctx.tuning_set(0, 1, 0)  # the context stays usable
+            ctx.select(O.STAGE_BURN, 3)
+            got.append([ctx.states(t).tolist() for t in range(T.n)])
+        finally:
+            ctx.close()
+    assert got[0] == got[1] and all(0 < len(s) <= 90 for g in got for s in g)
