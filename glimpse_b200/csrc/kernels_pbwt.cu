@@ -581,16 +581,20 @@ __global__ void __launch_bounds__(32) k_pbwt_union(PbwtSelectArgs a) {
 
 template <int HPW>
 static void launch_sweep(const PbwtSelectArgs& a, cudaStream_t s) {
-  // Stages of 4, 2 or 1 rank rows, within 96 KB.
+  // Stages of 4, 2 or 1 rank rows, within 96 KB. Larger panels (above some 65,000 haplotypes)
+  // read from memory: there three longer rows a stage leave one warp per SM, and 256 targets of
+  // 80,000 haplotypes took 3.3, 2.0 or 1.27 ms (1, 2, 4 per warp) against 0.94, 1.08 or 1.22.
+  constexpr int kLimit = 200 << 10;
   const size_t row_bytes = (size_t)a.P.R * 4, fixed = 2 * 32 * 2 * 16 + (size_t)a.depth * HPW * 4;
   int rows = 4;
   while (rows > 0 && kRankStages * rows * row_bytes > (96u << 10)) rows >>= 1;
   const int grid = (a.n_haps + HPW - 1) / HPW;
   if (rows > 0) {
     const size_t smem = kRankStages * rows * row_bytes + fixed;
-    if (smem > (48u << 10)) set_smem_limit_once<k_pbwt_sweep<HPW, true>>(200 << 10);
+    if (smem > (48u << 10)) set_smem_limit_once<k_pbwt_sweep<HPW, true>>(kLimit);
     k_pbwt_sweep<HPW, true><<<grid, 32, smem, s>>>(a, rows);
   } else {
+    if (fixed > (48u << 10)) set_smem_limit_once<k_pbwt_sweep<HPW, false>>(kLimit);  // very deep lists
     k_pbwt_sweep<HPW, false><<<grid, 32, fixed, s>>>(a, 1);
   }
 }

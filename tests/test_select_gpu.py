@@ -214,7 +214,9 @@ def test_union_order_and_limits(kpbwt):
 
 @pytest.mark.gpu
 def test_deep_lists_on_a_panel_without_staged_rows():
-    """6,500 levels do not fit the SM for 8 haplotypes: an error, not a union of lists
+    """1,450 levels: the push counts of 8 haplotypes per warp pass the default 48 KB
+    of shared memory also where no rank rows are staged, and all shapes select alike.
+    6,500 levels do not fit the SM for 8 haplotypes: an error, not a union of lists
     that no sweep wrote."""
     from glimpse_b200 import native, synth
     from oracle import oracle as O
@@ -222,7 +224,7 @@ def test_deep_lists_on_a_panel_without_staged_rows():
                                      sparse_maf=0.001)
     T = w.targets
     got = []
-    for depth, hpw in ((6500, 1), (6500, 8)):
+    for depth, hpw in ((1450, 1), (1450, 8), (6500, 1), (6500, 8)):
         ctx = native.Context(w.panel, kinit=60, kpbwt=90, pbwt_depth=depth, pbwt_modulo_cm=0.05)
         try:
             ctx.tuning_set(0, hpw, 0)
@@ -236,4 +238,4 @@ def test_deep_lists_on_a_panel_without_staged_rows():
             got.append([ctx.states(t).tolist() for t in range(T.n)])
         finally:
             ctx.close()
-    assert got[0] == got[1] and all(0 < len(s) <= 90 for g in got for s in g)
+    assert got[0] == got[1] and got[2] == got[3] and all(0 < len(s) <= 90 for g in got for s in g)
