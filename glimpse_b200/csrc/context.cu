@@ -696,28 +696,30 @@ int Context::run_phase(const int32_t* d_tsel, const std::vector<int32_t>& tsel_h
       for (int i = 0; i <= nside; ++i) most = std::max(most, cls[i + 1] - cls[i]);
       narrow = 4 * most >= 3 * (c1 - c0) ? (2u << kPhaseNarrowJ) - 1u : (1u << 2) | (1u << 3);
     }
-    for (int i = 0; i <= nside; ++i) {
+    int lrc = GP_OK;
+    for (int i = 0; i <= nside && lrc == GP_OK; ++i) {
       PhaseStore Sc = S;
       Sc.order = S.order + cls[i];
       const int J = class_of(order[cls[i]]);
-      if (launch_phase_chain(J, J <= kPhaseNarrowJ && ((narrow >> J) & 1u), d_tsel, cls[i + 1] - cls[i], w.nstates.as<int32_t>(),
+      lrc = launch_phase_chain(J, J <= kPhaseNarrowJ && ((narrow >> J) & 1u), d_tsel, cls[i + 1] - cls[i], w.nstates.as<int32_t>(),
                              w.hvar.as<uint32_t>(), w.WB, w.Kp, w.npoly.as<int32_t>(), V, Sc, mc,
-                             i == 0 ? stream : side[i - 1].s) != GP_OK)
-        return (fail(GP_E_ARG, "phasing: too many states"), GP_E_ARG);
+                             i == 0 ? stream : side[i - 1].s);
     }
     // Each class's units follow its chains, beside the chains of the heavier classes
     // (256 targets at K 400-1,200: 55.3 ms, 61.0 with all units after all chains).
-    for (int i = 0; i <= nside; ++i) {
+    for (int i = 0; i <= nside && lrc == GP_OK; ++i) {
       PhaseStore Sc = S;
       Sc.order = S.order + cls[i];
       int units = 0;
       for (int j = cls[i]; j < cls[i + 1]; ++j)
         units = std::max(units, cnt[nb + order[j]] - 1 + cnt[2 * nb + order[j]]);
-      if (launch_phase_units(units, narrow, d_tsel, cls[i + 1] - cls[i], w.nstates.as<int32_t>(), w.hvar.as<uint32_t>(),
-                             w.WB, w.Kp, V, Sc, cfg.seed, iteration, d_target_ids, i == 0 ? stream : side[i - 1].s) != GP_OK)
-        return cuda_fail(cudaGetLastError(), "phasing: shared-memory attribute");
+      lrc = launch_phase_units(units, narrow, d_tsel, cls[i + 1] - cls[i], w.nstates.as<int32_t>(), w.hvar.as<uint32_t>(),
+                             w.WB, w.Kp, V, Sc, cfg.seed, iteration, d_target_ids, i == 0 ? stream : side[i - 1].s);
     }
+    // joined on an error too: the next call's work on the context's stream uses the same buffers
     if ((e = join_streams(nside)) != cudaSuccess) return cuda_fail(e, "phasing streams");
+    if (lrc == GP_E_CUDA) return cuda_fail(cudaGetLastError(), "phasing: shared-memory attribute");
+    if (lrc != GP_OK) return (fail(GP_E_ARG, "phasing: too many states"), GP_E_ARG);
     PhaseStore Sc = S;
     Sc.order = S.order + c0;
     launch_phase_draw(d_tsel, c1 - c0, V, Sc, cfg.seed, iteration, d_target_ids, stream);
