@@ -683,18 +683,29 @@ int Context::run_phase(const int32_t* d_tsel, const std::vector<int32_t>& tsel_h
     cls.push_back(c1);
     const int nside = (int)cls.size() - 2;
     if ((e = fork_streams(nside)) != cudaSuccess) return cuda_fail(e, "phasing streams");
-    // Classes whose chains run two warps instead of four (fewer instructions a
-    // site in all, a longer site). It pays where chains wait for issue slots, from
-    // about three chains per SM on: with 400 chains four warps were the faster
-    // (K 200-600: 29.9 against 31.7 ms). Chains of a mixed batch finish together when
-    // the heavy ones keep four: 512 chains at K 400-1,200 50.9 ms with classes 2 and
-    // 3 narrow, 60.8 with none, 56.8 with all. Where one class holds most chains, all
-    // of them: K 700-1,000 49.0 against 54.0 ms, K 1,000-1,200 61.9 against 81.3.
+    // Classes whose chains run two warps instead of four: fewer instructions a site in all and
+    // fewer registers, a longer site. From three chains per SM on:
+    //  - Where one class holds most chains, all of them, as they wait for issue slots (512
+    //    chains of 10,000 x 150,000: K = 1,000 51.7 against 53.7 ms, K = 500 30.4 against 31.8;
+    //    with 400 chains four warps were the faster, K 200-600 29.9 against 31.7 ms).
+    //  - In a mixed batch, classes 2 and 3, whose narrow instances fit six chains on an SM
+    //    instead of five and four (class 4 none more, and the heaviest chains last longest),
+    //    where the wide chains do not fit the SMs together. 600 chains at K 400-1,200, 1.05
+    //    times what fits: 57.0 against 58.7 ms (5,000 x 60,000: 25.9 against 27.0); 700 at
+    //    K 250-800, 1.07 times: 20.1 against 22.0. Where all fit, every chain wide: 512 at
+    //    K 400-1,200, 0.90: 46.6 against 47.4 ms (24.0 against 24.8); at K 100-900, 0.78: 17.2
+    //    against 19.9.
     uint32_t narrow = 0;
     if (2 * (c1 - c0) >= 3 * sm_count) {
       int most = 0;
-      for (int i = 0; i <= nside; ++i) most = std::max(most, cls[i + 1] - cls[i]);
-      narrow = 4 * most >= 3 * (c1 - c0) ? (2u << kPhaseNarrowJ) - 1u : (1u << 2) | (1u << 3);
+      double sms = 0;  // that the wide chains take
+      for (int i = 0; i <= nside; ++i) {
+        const int n = cls[i + 1] - cls[i];
+        most = std::max(most, n);
+        sms += 2.0 * n / phase_chains_per_sm(class_of(order[cls[i]]), false);
+      }
+      if (4 * most >= 3 * (c1 - c0)) narrow = (2u << kPhaseNarrowJ) - 1u;
+      else if (sms > sm_count) narrow = (1u << 2) | (1u << 3);
     }
     int lrc = GP_OK;
     for (int i = 0; i <= nside && lrc == GP_OK; ++i) {

@@ -337,7 +337,7 @@ __device__ __forceinline__ void het_update(f2 (&prob)[NS][4], const uint32_t (&w
 }
 
 template <int J, int V>
-__global__ void __launch_bounds__(256 / V, V == 4 ? (J <= 3 ? 6 : 4) : J <= 2 ? 5 : J <= 4 ? 4 : J <= 5 ? 3 : 2)
+__global__ void __launch_bounds__(256 / V, phase_chains_per_sm(J, V == 4))
     k_phase_chain(const int32_t* __restrict__ tsel, const int32_t* __restrict__ nstates,
                   const int32_t* __restrict__ npoly, const uint32_t* __restrict__ hvar, int WB, int Kp, PhaseVars P,
                   PhaseStore S, ModelConst mc) {

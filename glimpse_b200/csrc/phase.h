@@ -64,6 +64,10 @@ void launch_var_records(const int32_t* tsel, int nb, const int32_t* poly, int L,
 // 256 (J - 1) < K <= 256 J states (S.order may point into a longer order). narrow:
 // two warps a chain instead of four, for J <= kPhaseNarrowJ.
 constexpr int kPhaseNarrowJ = 5;
+// Chains of class J that are resident on an SM together (their registers are bounded to that).
+constexpr int phase_chains_per_sm(int J, bool narrow) {
+  return narrow ? (J <= 3 ? 6 : 4) : J <= 2 ? 5 : J <= 4 ? 4 : J <= 5 ? 3 : 2;
+}
 int launch_phase_chain(int J, bool narrow, const int32_t* tsel, int nb, const int32_t* nstates, const uint32_t* hvar,
                        int WB, int Kp, const int32_t* npoly, PhaseVars P, PhaseStore S, const ModelConst& mc,
                        cudaStream_t s);
