@@ -213,19 +213,25 @@ def default_subset(threads):
     return max(1, min(threads, 32))
 
 
+def reference_unavailable(native_rng=False):
+    """Why the reference's library cannot be run here, or None."""
+    try:
+        from oracle import oracle as O
+        if O.ref_available(native_rng=native_rng):
+            return None
+    except Exception as e:  # pragma: no cover
+        return f"oracle import failed: {e}"
+    return f"oracle/_ref/libglimpse_ref{'_native' if native_rng else ''}.so not built"
+
+
 def run_reference(args):
     rank, world, _ = env_rank()
     if rank != 0:
         return 0
-    try:
-        from oracle import oracle as O
-        native = getattr(args, "ref_rng", "replay") == "native"
-        if not O.ref_available(native_rng=native):
-            lib = "libglimpse_ref_native.so" if native else "libglimpse_ref.so"
-            print(json.dumps({"impl": "reference", "unavailable": f"oracle/_ref/{lib} not built"}))
-            return 0
-    except Exception as e:  # pragma: no cover
-        print(json.dumps({"impl": "reference", "unavailable": f"oracle import failed: {e}"}))
+    native = getattr(args, "ref_rng", "replay") == "native"
+    why = reference_unavailable(native)
+    if why:
+        print(json.dumps({"impl": "reference", "unavailable": why}))
         return 0
     w = synth.workload(args.config, seed=1)
     threads = 1 if native else (os.cpu_count() or 1)
@@ -381,7 +387,10 @@ def run_ours(args):
             "selection": select,
             "e2e": {"value": e2e_value, "unit": "samples/s", "h2d_bytes_per_step": int(h2d),
                     "d2h_bytes_per_step": int(d2h)}}
-    if rank == 0 and world == 1 and not args.no_cpu_baseline:
+    why = reference_unavailable()
+    if why:
+        line["cpu_baseline"] = {"unavailable": why}
+    elif rank == 0 and world == 1 and not args.no_cpu_baseline:
         # The same fixed subset on both sides: a complete run of the first
         # targets, on the GPU (device time) and on the host cores (reference).
         threads = os.cpu_count() or 1
