@@ -260,7 +260,7 @@ Context::~Context() {
   tune_tarhap.release();
   stage.release();
   list_off.release(); list_ids.release(); merged_states.release();
-  ckpt.release(); ckpt_sum.release(); loglik.release();
+  ckpt_sum.release(); loglik.release();
   for (DevBuf* b : learned.all()) b->release();
   if (phase_err_host) cudaFreeHost(phase_err_host);
   for (SideStream& x : side) {
@@ -388,7 +388,6 @@ int Context::run_impute(const float* d_hl, const uint8_t* d_flat, float* d_hp) {
   // The checkpointed modes (kernels_impute_ckpt.cu): chains of their own, the same blocks.
   const bool ck = precision_mode != GP_PRECISION_FULL, bf16 = precision_mode == GP_PRECISION_CKPT_BF16;
   if (ck) {
-    if (bf16 && (e = ckpt.ensure((size_t)2 * n * w.WB * w.Kp * 2)) != cudaSuccess) return cuda_fail(e, "alloc ckpt");
     if ((e = ckpt_sum.ensure((size_t)n * w.WB * 32 * 4)) != cudaSuccess) return cuda_fail(e, "alloc ckpt");
     if ((e = loglik.ensure((size_t)n * 8)) != cudaSuccess) return cuda_fail(e, "alloc loglik");
   }
@@ -397,8 +396,25 @@ int Context::run_impute(const float* d_hl, const uint8_t* d_flat, float* d_hp) {
   std::vector<int32_t> order(n);
   for (int i = 0; i < n; ++i) order[i] = i;
   std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return impute_np[x] > impute_np[y]; });
+  // Windows of the checkpointed modes: as few as keep the batch within 1/8 byte per cell (site of a set, state of
+  // the largest) in BF16 mode and 1/4 in FP32, at most 16 (the rows of two are then 1/16 and 1/32), of 16 blocks
+  // and more in either half. Blocks beside chains slow them: 32 haplotypes at K 400-1,200 18.4 ms with 16, 17.9
+  // with one.
+  int windows = 1;
+  if (ck) {
+    int np_max = 0;
+    for (int i = 0; i < n; ++i) np_max = std::max(np_max, impute_np[i]);
+    auto total = [&](int wins) {
+      int64_t b = 0;
+      for (int i = 0; i < n; ++i) b += ckpt_layout(impute_np[i], host_nstates[i], bf16, wins).total * 4;
+      return b;
+    };
+    while (windows < 16 && windows * 2 <= np_max / 1024 && total(windows) > (int64_t)n * w.WB * 32 * w.Kp / (bf16 ? 8 : 4))
+      windows *= 2;
+  }
   // chunks of the order whose kept rows (two per kRowSites sites) fit the budget
   auto row_bytes = [&](int i) {
+    if (ck) return ckpt_layout(impute_np[i], host_nstates[i], bf16, windows).total * 4;
     return (int64_t)2 * ((impute_np[i] + kRowSites - 1) / kRowSites) * 128 * impute_groups(host_nstates[i]) * 4;
   };
   size_t need_all = 0;
@@ -436,35 +452,63 @@ int Context::run_impute(const float* d_hl, const uint8_t* d_flat, float* d_hp) {
   // each followed on its stream by the class's blocks (not when the chains are timed).
   // Chains wait on latency and the lighter classes end early, so their blocks, which
   // want issue slots, fill the SMs beside the heavier chains (256 haplotypes
-  // at K 400-1,200: 21.9 ms a call, 24.6 with all blocks after all chains).
+  // at K 400-1,200: 21.9 ms a call, 24.6 with all blocks after all chains). In the checkpointed
+  // modes each stream takes its class's own halves and then window by window, with the blocks.
   auto run_chains = [&](size_t c, int cpc, bool blocks) -> int {
     const int c0 = chunk_start[c], c1 = chunk_start[c + 1];
     std::vector<int> cls(1, c0);
     for (int j = c0 + 1; j < c1; ++j)
       if (class_of(order[j]) != class_of(order[j - 1])) cls.push_back(j);
     cls.push_back(c1);
-    const int nc = (int)cls.size() - 1, nside = std::min(nc - 1, kMaxSideStreams);
+    // streams of the classes' chains; in the checkpointed modes the heaviest classes have another for their blocks
+    const int nc = (int)cls.size() - 1, nchain = std::min(nc, 1 + kMaxSideStreams);
+    const int nblock = ck ? std::min(nc, 1 + kMaxSideStreams - nchain) : 0, nside = nchain - 1 + nblock;
     if (fork_streams(nside) != cudaSuccess) return GP_E_CUDA;
-    auto stream_of = [&](int i) { return i % (nside + 1) == 0 ? stream : side[i % (nside + 1) - 1].s; };
+    auto stream_of = [&](int i) { return i % nchain == 0 ? stream : side[i % nchain - 1].s; };
     auto np_of = [&](int i) {
       int m = 0;
       for (int j = cls[i]; j < cls[i + 1]; ++j) m = std::max(m, impute_np[order[j]]);
       return m;
     };
     int rc = GP_OK;
-    for (int i = 0; i < nc && rc == GP_OK; ++i) {
-      const int J = class_of(order[cls[i]]), cnt = cls[i + 1] - cls[i];
-      if (ck) {
-        rc = launch_impute_ckpt(J, bf16, np_of(i), w, ckpt.ptr, ckpt_sum.as<float>(), stream_of(i), cls[i], cnt);
-        prof.kernel_launches += bf16 ? 2 : 1;
-        continue;
+    if (ck) {
+      std::vector<int> wlen(nc, 0);  // longest window of a class
+      for (int i = 0; i < nc; ++i)
+        for (int j = cls[i]; j < cls[i + 1]; ++j) {
+          const CkptLayout lay = ckpt_layout(impute_np[order[j]], host_nstates[order[j]], bf16, windows);
+          wlen[i] = std::max({wlen[i], lay.wlen0, lay.wlen1});
+        }
+      for (int win = -1; win < windows; ++win)
+        for (int i = 0; i < nc && rc == GP_OK; ++i) {
+          const int J = class_of(order[cls[i]]), cnt = cls[i + 1] - cls[i];
+          const cudaStream_t s = stream_of(i);
+          rc = launch_ckpt_chain(J, bf16, windows, win, w, ckpt_sum.as<float>(), s, cls[i], cnt);
+          prof.kernel_launches += 1;
+          if (win < 0 || rc != GP_OK) continue;
+          cudaStream_t sb = s;
+          if (i < nblock) {
+            // the window's blocks follow its chains; the chains after next, its rows' next user, follow the blocks
+            const SideStream& x = side[nchain - 1 + i];
+            const cudaEvent_t chained = i == 0 ? fork_event : side[i - 1].done;
+            sb = x.s;
+            if (cudaEventRecord(chained, s) != cudaSuccess || cudaStreamWaitEvent(sb, chained, 0) != cudaSuccess ||
+                (win > 0 && cudaStreamWaitEvent(s, x.done, 0) != cudaSuccess))
+              rc = GP_E_CUDA;
+          }
+          if (rc == GP_OK)
+            rc = launch_ckpt_window(J, bf16, windows, win, wlen[i], w, d_hp, sb, cls[i], cnt);
+          if (rc == GP_OK && i < nblock && cudaEventRecord(side[nchain - 1 + i].done, sb) != cudaSuccess) rc = GP_E_CUDA;
+          prof.kernel_launches += bf16 ? 2 : 1;
+        }
+    } else {
+      for (int i = 0; i < nc && rc == GP_OK; ++i) {
+        rc = launch_impute_chain(class_of(order[cls[i]]), w, stream_of(i), cls[i], cls[i + 1] - cls[i], cpc);
+        prof.kernel_launches += 1;
       }
-      rc = launch_impute_chain(J, w, stream_of(i), cls[i], cnt, cpc);
-      prof.kernel_launches += 1;
-    }
-    for (int i = 0; i < nc && rc == GP_OK && blocks; ++i) {
-      rc = launch_impute_block(ck, np_of(i), w, d_hp, stream_of(i), cls[i], cls[i + 1] - cls[i]);
-      prof.kernel_launches += 1;
+      for (int i = 0; i < nc && rc == GP_OK && blocks; ++i) {
+        rc = launch_impute_block(np_of(i), w, d_hp, stream_of(i), cls[i], cls[i + 1] - cls[i]);
+        prof.kernel_launches += 1;
+      }
     }
     if (join_streams(nside) != cudaSuccess) return GP_E_CUDA;
     return rc;

@@ -112,7 +112,7 @@ struct Context {
   int run_impute(const float* d_hl, const uint8_t* d_flat, float* d_hp);
   size_t store_budget(size_t held, size_t need);
   int precision_mode = GP_PRECISION_FULL;
-  DevBuf ckpt, ckpt_sum, loglik;  // checkpointed imputation: BF16 rows, AlphaSums, log-likelihoods
+  DevBuf ckpt_sum, loglik;  // checkpointed imputation: AlphaSums, log-likelihoods
   int loglik_n = 0;                             // entries of the last checkpointed imputation call
   int impute_chunks = 0;  // launches pairs of the last run_impute (1 when the whole batch fit)
   int phase_chunks = 0;   // chunks of the last run_phase

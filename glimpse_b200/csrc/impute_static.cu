@@ -187,7 +187,7 @@ extern "C" int gp_impute_one_static(gp_ctx* ctx, int32_t k, const uint32_t* stat
   cudaMemcpyAsync(w.row_off.ptr, &zero64, 8, cudaMemcpyHostToDevice, s);
   gp::launch_site_records(c.panel, c.mc, w, w.hl.as<float>(), w.flat.as<uint8_t>(), s);
   int lrc = gp::launch_impute_chain(gp::impute_groups(k), w, s);
-  if (lrc == GP_OK) lrc = gp::launch_impute_block(false, np, w, w.hp.as<float>(), s);
+  if (lrc == GP_OK) lrc = gp::launch_impute_block(np, w, w.hp.as<float>(), s);
   if (lrc != GP_OK) return finish((c.fail(GP_E_ARG, "impute_one_static: too many states"), GP_E_ARG));
   gp::launch_impute_finish(c.panel, c.mc, w, w.hl.as<float>(), w.flat.as<uint8_t>(), w.hp.as<float>(), s);
   c.prof.kernel_launches += 9;

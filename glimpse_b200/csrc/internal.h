@@ -157,15 +157,76 @@ constexpr int kRowSites = 16;
 int launch_impute_chain(int J, ImputeWork& w, cudaStream_t s, int first = 0, int count = -1, int cpc = 1);
 // After the chains, for haplotypes of any K with at most max_poly polymorphic
 // sites: prob_hid of every site into hp.
-int launch_impute_block(bool ck, int max_poly, ImputeWork& w, float* hp, cudaStream_t s, int first = 0, int count = -1);
+int launch_impute_block(int max_poly, ImputeWork& w, float* hp, cudaStream_t s, int first = 0, int count = -1);
 // Rows of 128 states that a chain of K states runs (the J of launch_impute_chain).
 int impute_groups(int K);
-// The chains of the checkpointed modes (kernels_impute_ckpt.cu) for the haplotypes
-// order[first .. first + count), all with 256 (J - 1) < K <= 256 J and at most
-// max_poly polymorphic sites; launch_impute_block follows. ckpt: [2][n][WB][Kp] BF16
-// rows (bf16 only); asum: [n][32 WB].
-int launch_impute_ckpt(int J, bool bf16, int max_poly, ImputeWork& w, void* ckpt, float* asum, cudaStream_t s,
+
+// The checkpointed modes (kernels_impute_ckpt.cu). A haplotype is split at site M = 32 mblk,
+// about np / 2. Both chains first run their own half ([0, M) forward, [M, np) backward) and
+// keep checkpoints of it: a row per 16 sites (FP32), or one per 32 rounded to BF16. Then they
+// run the other's half in windows, whose posteriors are formed window by window, beside the
+// chains of the next one: only two windows' rows exist at a time. All of a haplotype's rows
+// lie together, of Ks states each.
+struct CkptLayout {
+  int nrow, nblk, mblk;  // blocks of 16 and of 32 sites, blocks of 32 before M
+  int Ks;                // row stride: states rounded up to 128
+  // blocks of 32 of a window, and its rows' place (floats) for even windows; odd ones lie behind: in
+  // [M, np), run forward, and in [0, M), run backward
+  int wlen0, wlen1, wrows0, wrows1;
+  int64_t win0, win1;
+  int64_t state, total;  // floats: the chains' states between launches (row and sum, two rows each), all
+};
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline CkptLayout ckpt_layout(int np, int K, bool bf16, int windows) {
+  CkptLayout a;
+  a.nrow = (np + 15) / 16;
+  a.nblk = (np + 31) / 32;
+  a.mblk = np / 64;
+  a.Ks = (K + 127) / 128 * 128;
+  a.wlen0 = (a.nblk - a.mblk + windows - 1) / windows;
+  a.wlen1 = (a.mblk + windows - 1) / windows;
+  a.state = (int64_t)(bf16 ? (a.nblk + 1) / 2 : a.nrow) * a.Ks;
+  // a window's rows: those of the chain, and in BF16 mode the recomputed ones of the other direction
+  a.wrows0 = (bf16 ? 4 : 2) * a.wlen0;
+  a.wrows1 = (bf16 ? 4 : 2) * a.wlen1;
+  a.win0 = a.state + 4 * a.Ks;
+  const int kept = windows > 1 ? 2 : 1;
+  a.win1 = a.win0 + (int64_t)kept * a.wrows0 * a.Ks;
+  a.total = a.win1 + (int64_t)kept * a.wrows1 * a.Ks;
+  return a;
+}
+// The rows (floats) of window w in half 0 or 1.
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline int64_t ckpt_window_rows(const CkptLayout& a, int half, int w) {
+  return half == 0 ? a.win0 + (w & 1 ? (int64_t)a.wrows0 * a.Ks : 0) : a.win1 + (w & 1 ? (int64_t)a.wrows1 * a.Ks : 0);
+}
+// The blocks [lo, hi) of 32 sites of window w in [M, np) (half 0) or [0, M) (half 1).
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline void ckpt_window(const CkptLayout& a, int half, int w, int& lo, int& hi) {
+  if (half == 0) {
+    lo = a.mblk + w * a.wlen0;
+    hi = lo + a.wlen0 < a.nblk ? lo + a.wlen0 : a.nblk;
+  } else {
+    hi = a.mblk - w * a.wlen1;
+    lo = hi - a.wlen1 > 0 ? hi - a.wlen1 : 0;
+  }
+}
+// For the haplotypes order[first .. first + count), all with 256 (J - 1) < K <= 256 J: the
+// chains over their own halves (win < 0) or window win; asum: [n][32 WB]. Then the
+// posteriors of a window of at most wlen blocks of 32 in either half (launch_ckpt_posteriors
+// after the rows that BF16 mode recomputes).
+int launch_ckpt_chain(int J, bool bf16, int windows, int win, ImputeWork& w, float* asum, cudaStream_t s, int first,
+                      int count);
+int launch_ckpt_window(int J, bool bf16, int windows, int win, int wlen, ImputeWork& w, float* hp, cudaStream_t s,
                        int first, int count);
+int launch_ckpt_posteriors(bool bf16, int windows, int win, int wlen, ImputeWork& w, float* hp, cudaStream_t s,
+                           int first, int count);
 // The FP64 log-likelihood of every haplotype from its AlphaSums.
 void launch_ckpt_loglik(ImputeWork& w, const float* asum, double* loglik, cudaStream_t s);
 void launch_impute_finish(const DevPanel& P, const ModelConst& mc, ImputeWork& w, const float* hl,

@@ -5,20 +5,24 @@
 // precision path (kernels_impute_warp.cu, after imputation_hmm.cpp:80-353):
 // sequential chains keep the scaling factor of every site and a row per kRowSites
 // sites, and k_impute_block forms the posteriors. What differs:
+//   - The memory. Each haplotype is split at M (a multiple of 32, about np / 2). Both
+//     chains run their own halves and keep checkpoints of them, then the other's half in
+//     windows, each followed by its posteriors (ckpt_layout): 1/4 byte per site and state
+//     in FP32, 1/16 in BF16, and the rows of two windows, against 1/2 for all rows. The
+//     chains run as many sites one after another as without windows.
 //   - The sums over states have another fixed tree (state k: lane k % 32 of virtual
 //     warp (k / 32) % 8; j in order, lanes at distances 16 .. 1, virtual warps at 1,
 //     2, 4), that of the AlphaSums whose logarithms make up the log-likelihood.
-//   - With BF16 checkpoints, each haplotype is split at M (a multiple of 32, about
-//     np / 2). On [0, M) the forward messages, and on [M, np) the backward ones, are
-//     those recomputed from a row rounded to BF16 at the start of each block of 32
-//     sites (k_ckpt_block, one CTA per block: its factors and rows replace the
+//   - With BF16 checkpoints, the forward messages on [0, M) and the backward ones on
+//     [M, np) are those recomputed from a row rounded to BF16 at the start of each
+//     block of 32 sites (k_ckpt_block, one CTA per block: its factors replace the
 //     chain's there), and either chain goes on from a rounded row at M.
 //     Either kernel is bound by its chain of dependent steps: a site per step, of which
 //     the sum over 256 J states, its barrier and its five shuffles are most. A chain has
 //     two warps, so that a lane's states are independent work within a step and the
 //     barrier joins two warps only; with 256 threads and both half passes in sequence,
 //     each a chain of its own, 32 haplotypes (400 - 1,200 states) at 150,000 sites took
-//     65 ms a call, against 27.
+//     65 ms a call, against 26.
 //   - The FP64 chunk log-likelihood sum_l log AlphaSum_l (the reference keeps no such
 //     value), from the AlphaSum of every site, off the chain.
 #include <cuda_bf16.h>
@@ -33,7 +37,6 @@ namespace {
 constexpr int kCkptThreads = 64;
 
 struct CkptArgs {
-  int count;                // haplotypes of the launch
   const int32_t* __restrict__ order;
   const int32_t* __restrict__ npoly;
   const int32_t* __restrict__ nstates;
@@ -42,11 +45,11 @@ struct CkptArgs {
   const float2* __restrict__ tr;
   const uint8_t* __restrict__ fl;
   const int64_t* __restrict__ row_off;
-  float* __restrict__ rows;  // as k_impute_block reads them: front-padded to 128 ceil(K / 128)
+  float* __restrict__ rows;  // per haplotype as ckpt_layout says, its states at the end of each row
   float* __restrict__ fac;   // [2][n][32 WB]
   float* __restrict__ asum;  // [n][32 WB] AlphaSum of every site
-  __nv_bfloat16* __restrict__ ckpt;  // [2][n][WB][Kp] rows entering a block, forward and backward
   int n, L, WB, Kp;
+  int windows, win;          // win < 0: the chains' own halves
 };
 
 // Partial sums: virtual warp v's lane at 32 v + 8 (lane & 3) + (lane >> 2), so that
@@ -57,23 +60,25 @@ struct CkptSmem {
   float4 rec[1 + 4 * 32 + 1];  // emission of allele 0 and 1, t / K and 1 - t into the site
 };
 
-// Steps through the blocks b_first .. b_last (in the direction of the chain).
+// Steps through the blocks b_first .. b_last (in the direction of the chain). Rows
+// entering blocks of 16 go to `out`, the one of block r0 first; in the chain's own half
+// (OWN) in BF16 mode, rows entering blocks of 32 to the checkpoints instead.
 // SEG: one block, from its BF16 checkpoint. J: 256 (J - 1) < K <= 256 J.
-template <int J, bool FWD, bool SEG, bool BF16>
-__device__ __forceinline__ void ckpt_run(const CkptArgs& A, CkptSmem& S, int t, int b_first, int b_last) {
+template <int J, bool FWD, bool SEG, bool BF16, bool OWN>
+__device__ __forceinline__ void ckpt_run(const CkptArgs& A, CkptSmem& S, const CkptLayout& lay, int t, int b_first,
+                                         int b_last, float* out, int r0) {
   constexpr int NP = 2 * J;  // packed pairs of states: virtual warps (0, 1) and (2, 3) of the warp, per j
   const int np = A.npoly[t], K = A.nstates[t];
   const int tid = threadIdx.x, lane = tid & 31, wi = tid >> 5;
-  const int mblk = ((np / 2) & ~31) >> 5;  // M = 32 mblk
-  const int nrow = (np + kRowSites - 1) / kRowSites;
-  const int Ks = (K + 127) / 128 * 128;
+  const int Ks = lay.Ks;
   // state of pair p: 256 (p / 2) + k0 + 64 (p & 1) (+ 32)
   const int k0 = 128 * wi + lane;
   auto state = [&](int p, int h) { return 256 * (p >> 1) + k0 + 64 * (p & 1) + 32 * h; };
-  float* rows = A.rows + A.row_off[t] + (FWD ? 0 : (size_t)nrow * Ks) + (Ks - K);
+  out += Ks - K;
+  float* const saved = A.rows + A.row_off[t] + lay.state + (FWD ? 0 : 2 * Ks);  // the chain's row and sum
   float* fac = A.fac + ((size_t)(FWD ? 0 : A.n) + t) * 32 * A.WB;
   const uint32_t* hv = A.hvar + (size_t)t * A.WB * A.Kp;
-  __nv_bfloat16* ck = A.ckpt + ((size_t)(FWD ? 0 : A.n) + t) * A.WB * A.Kp;
+  __nv_bfloat16* ck = reinterpret_cast<__nv_bfloat16*>(A.rows + A.row_off[t]);
   const float4* E = A.em + (size_t)t * A.L;
   const float2* T = A.tr + (size_t)t * A.L;
   const uint8_t* F = A.fl + (size_t)t * A.L;
@@ -110,7 +115,7 @@ __device__ __forceinline__ void ckpt_run(const CkptArgs& A, CkptSmem& S, int t, 
       f2_unpack(x[p], v[0], v[1]);
 #pragma unroll
       for (int h = 0; h < 2; ++h)
-        if (has(p, h)) rows[(size_t)i * Ks + state(p, h)] = v[h];
+        if (has(p, h)) out[(size_t)(i - r0) * Ks + state(p, h)] = v[h];
     }
   };
   auto round_row = [&]() {
@@ -130,14 +135,14 @@ __device__ __forceinline__ void ckpt_run(const CkptArgs& A, CkptSmem& S, int t, 
 #pragma unroll
   for (int p = 0; p < NP; ++p) {
     float v[2] = {0.f, 0.f};
-    if (SEG && !init) {
+    if (!init) {
 #pragma unroll
       for (int h = 0; h < 2; ++h)
-        if (has(p, h)) v[h] = __bfloat162float(ck[(size_t)b_first * A.Kp + state(p, h)]);
+        if (has(p, h)) v[h] = SEG ? __bfloat162float(ck[(size_t)b_first * Ks + state(p, h)]) : saved[state(p, h)];
     }
     x[p] = f2_pack(v[0], v[1]);
   }
-  float acc = 1.f;
+  float acc = SEG || init ? 1.f : saved[Ks];
   __syncthreads();
   const int wofs = 8 * (lane & 3) + (lane >> 2);
   const ulonglong2* const rin = reinterpret_cast<const ulonglong2*>(&S.red[0][8 * lane]);
@@ -196,28 +201,31 @@ __device__ __forceinline__ void ckpt_run(const CkptArgs& A, CkptSmem& S, int t, 
       load_recs(b + dir);
       load_words(b + dir);
     }
-    // Whether this block's rows are recomputed from its checkpoint (then only that is kept here).
-    const bool again = BF16 && !SEG && (FWD ? b < mblk : b >= mblk);
-    if (BF16 && !SEG && b != b_first) {
-      if (again) {
+    if (BF16 && !SEG && !(init && b == b_first)) {
+      if (OWN) {
 #pragma unroll
         for (int p = 0; p < NP; ++p) {
           float v[2];
           f2_unpack(x[p], v[0], v[1]);
 #pragma unroll
           for (int h = 0; h < 2; ++h)
-            if (has(p, h)) ck[(size_t)b * A.Kp + state(p, h)] = __float2bfloat16_rn(v[h]);
+            if (has(p, h)) ck[(size_t)b * Ks + state(p, h)] = __float2bfloat16_rn(v[h]);
         }
+      } else if (FWD ? b == lay.mblk : b == lay.mblk - 1) {
+        round_row();
       }
-      if (FWD ? b == mblk : b == mblk - 1) round_row();
     }
     if (b == b_first && init) step(std::integral_constant<bool, true>());
     const int end = FWD ? min(np - (b << 5), 32) : -1;
     while (i != end) {
       const int part = i / kRowSites;
-      if (!again && (FWD ? i == part * kRowSites : i == (part + 1) * kRowSites - 1))
+      if (!(BF16 && OWN) && (FWD ? i == part * kRowSites : i == (part + 1) * kRowSites - 1))
         store_row(b * (32 / kRowSites) + part);
       const int stop = FWD ? min(end, (part + 1) * kRowSites) : part * kRowSites - 1;
+      // A step is latency; unrolled, its loop's own instructions go (one haplotype, K = 600:
+      // 11.7 -> 11.4 ms). Not with many states, where mixed classes then slow one another (128
+      // haplotypes, K 1,000-2,048: 12.6 ms, 16.4 unrolled).
+#pragma unroll (J <= 5 ? 4 : 1)
       while (i != stop) step(std::integral_constant<bool, false>());
     }
     if (wi == 0) {
@@ -230,28 +238,55 @@ __device__ __forceinline__ void ckpt_run(const CkptArgs& A, CkptSmem& S, int t, 
     m = FWD ? 1u : 1u << 31;
     __syncthreads();
   }
+  if (!SEG && (FWD ? b_last < lay.nblk - 1 : b_last > 0)) {  // the next launch goes on from here
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+      float v[2];
+      f2_unpack(x[p], v[0], v[1]);
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        if (has(p, h)) saved[state(p, h)] = v[h];
+    }
+    if (tid == 0) saved[Ks] = acc;
+  }
 }
 
-// Both chains of every haplotype: CTA 2 c forward, 2 c + 1 backward.
-template <int J, bool BF16>
+// Both chains of every haplotype, over their own halves or a window of the other's: CTA
+// 2 c forward, 2 c + 1 backward.
+template <int J, bool BF16, bool OWN>
 __global__ void __launch_bounds__(kCkptThreads, 1) k_ckpt_chain(CkptArgs A) {
   __shared__ CkptSmem S;
   const int t = A.order[blockIdx.x >> 1];
-  const int nblk = (A.npoly[t] + 31) >> 5;
-  if (nblk == 0 || A.nstates[t] == 0) return;
-  if ((blockIdx.x & 1) == 0) ckpt_run<J, true, false, BF16>(A, S, t, 0, nblk - 1);
-  else ckpt_run<J, false, false, BF16>(A, S, t, nblk - 1, 0);
+  const bool fwd = (blockIdx.x & 1) == 0;
+  if (A.npoly[t] == 0 || A.nstates[t] == 0) return;
+  const CkptLayout lay = ckpt_layout(A.npoly[t], A.nstates[t], BF16, A.windows);
+  int lo = fwd ? 0 : lay.mblk, hi = fwd ? lay.mblk : lay.nblk;
+  if (!OWN) ckpt_window(lay, fwd ? 0 : 1, A.win, lo, hi);
+  if (lo >= hi) return;
+  float* out = A.rows + A.row_off[t] + (OWN ? 0 : ckpt_window_rows(lay, fwd ? 0 : 1, A.win));
+  const int r0 = OWN ? 0 : lo * (32 / kRowSites);
+  if (fwd) ckpt_run<J, true, false, BF16, OWN>(A, S, lay, t, lo, hi - 1, out, r0);
+  else ckpt_run<J, false, false, BF16, OWN>(A, S, lay, t, hi - 1, lo, out, r0);
 }
 
-// The recomputed block blockIdx.x of haplotype order[blockIdx.y].
+// The rows of the other direction for one block of the window, from its BF16 checkpoint.
+// blockIdx.x: the blocks in [M, np), then as many in [0, M); haplotype order[blockIdx.y].
 template <int J>
 __global__ void __launch_bounds__(kCkptThreads, 1) k_ckpt_block(CkptArgs A) {
   __shared__ CkptSmem S;
-  const int t = A.order[blockIdx.y], b = blockIdx.x;
-  const int np = A.npoly[t];
-  if (b >= (np + 31) >> 5 || A.nstates[t] == 0) return;
-  if (b < ((np / 2) & ~31) >> 5) ckpt_run<J, true, true, true>(A, S, t, b, b);
-  else ckpt_run<J, false, true, true>(A, S, t, b, b);
+  const int t = A.order[blockIdx.y];
+  if (A.npoly[t] == 0 || A.nstates[t] == 0) return;
+  const CkptLayout lay = ckpt_layout(A.npoly[t], A.nstates[t], true, A.windows);
+  const int per = gridDim.x / 2, half = (int)blockIdx.x >= per;
+  int lo, hi;
+  ckpt_window(lay, half, A.win, lo, hi);
+  const int b = lo + (int)blockIdx.x - half * per;
+  if (b >= hi) return;
+  const int r0 = lo * (32 / kRowSites);
+  float* out = A.rows + A.row_off[t] + ckpt_window_rows(lay, half, A.win) +
+               (int64_t)(half ? lay.wlen1 : lay.wlen0) * (32 / kRowSites) * lay.Ks;
+  if (half) ckpt_run<J, true, true, true, false>(A, S, lay, t, b, b, out, r0);
+  else ckpt_run<J, false, true, true, false>(A, S, lay, t, b, b, out, r0);
 }
 
 // Sum of log AlphaSum over the sites of haplotype blockIdx.x, in FP64.
@@ -272,10 +307,8 @@ __global__ void __launch_bounds__(256) k_ckpt_loglik(const float* __restrict__ a
 
 }  // namespace
 
-int launch_impute_ckpt(int J, bool bf16, int max_poly, ImputeWork& w, void* ckpt, float* asum, cudaStream_t s,
-                       int first, int count) {
+static CkptArgs ckpt_args(ImputeWork& w, int windows, int win, float* asum, int first) {
   CkptArgs a;
-  a.count = count;
   a.order = w.order.as<int32_t>() + first;
   a.npoly = w.npoly.as<int32_t>();
   a.nstates = w.nstates.as<int32_t>();
@@ -287,26 +320,49 @@ int launch_impute_ckpt(int J, bool bf16, int max_poly, ImputeWork& w, void* ckpt
   a.rows = w.rows.as<float>();
   a.fac = w.fac.as<float>();
   a.asum = asum;
-  a.ckpt = static_cast<__nv_bfloat16*>(ckpt);
   a.n = w.n;
   a.L = w.L;
   a.WB = w.WB;
   a.Kp = w.Kp;
-  const dim3 blocks((max_poly + 31) / 32, count);
-#define GP_CK(JJ)                                                       \
-  case JJ:                                                              \
-    if (!bf16) k_ckpt_chain<JJ, false><<<2 * count, kCkptThreads, 0, s>>>(a); \
-    else {                                                              \
-      k_ckpt_chain<JJ, true><<<2 * count, kCkptThreads, 0, s>>>(a);     \
-      if (blocks.x > 0) k_ckpt_block<JJ><<<blocks, kCkptThreads, 0, s>>>(a); \
-    }                                                                   \
+  a.windows = windows;
+  a.win = win;
+  return a;
+}
+
+#define GP_EACH_J(M) M(1) M(2) M(3) M(4) M(5) M(6) M(7) M(8)
+
+int launch_ckpt_chain(int J, bool bf16, int windows, int win, ImputeWork& w, float* asum, cudaStream_t s, int first,
+                      int count) {
+  const CkptArgs a = ckpt_args(w, windows, win, asum, first);
+#define GP_CK(JJ)                                                                                \
+  case JJ:                                                                                       \
+    if (bf16 && win < 0) k_ckpt_chain<JJ, true, true><<<2 * count, kCkptThreads, 0, s>>>(a);     \
+    else if (bf16) k_ckpt_chain<JJ, true, false><<<2 * count, kCkptThreads, 0, s>>>(a);          \
+    else if (win < 0) k_ckpt_chain<JJ, false, true><<<2 * count, kCkptThreads, 0, s>>>(a);       \
+    else k_ckpt_chain<JJ, false, false><<<2 * count, kCkptThreads, 0, s>>>(a);                   \
     return GP_OK;
   switch (J) {
-    GP_CK(1) GP_CK(2) GP_CK(3) GP_CK(4) GP_CK(5) GP_CK(6) GP_CK(7) GP_CK(8)
+    GP_EACH_J(GP_CK)
     default: return GP_E_ARG;
   }
 #undef GP_CK
 }
+
+int launch_ckpt_window(int J, bool bf16, int windows, int win, int wlen, ImputeWork& w, float* hp, cudaStream_t s,
+                       int first, int count) {
+  if (bf16 && wlen > 0) {
+    const CkptArgs a = ckpt_args(w, windows, win, nullptr, first);
+#define GP_CK(JJ) \
+  case JJ: k_ckpt_block<JJ><<<dim3(2 * wlen, count), kCkptThreads, 0, s>>>(a); break;
+    switch (J) {
+      GP_EACH_J(GP_CK)
+      default: return GP_E_ARG;
+    }
+#undef GP_CK
+  }
+  return launch_ckpt_posteriors(bf16, windows, win, wlen, w, hp, s, first, count);
+}
+#undef GP_EACH_J
 
 void launch_ckpt_loglik(ImputeWork& w, const float* asum, double* loglik, cudaStream_t s) {
   k_ckpt_loglik<<<w.n, 256, 0, s>>>(asum, w.npoly.as<int32_t>(), w.WB, loglik);

@@ -245,9 +245,14 @@ __global__ void __launch_bounds__(SOLO ? kChainThreads : kChainThreads * kMaxCha
 //
 // CK, for the checkpointed modes: the same with 256 threads, thread tid taking the
 // states 256 j + tid, without padding (only the last pair has absent states), and the
-// sums of those modes: lanes at distances 16 .. 1, then warps at 1, 2, 4.
+// sums of those modes: lanes at distances 16 .. 1, then warps at 1, 2, 4. It takes the
+// blocks of one window (blockIdx.z: in which half).
 // ---------------------------------------------------------------------------
 constexpr int RS = kRowSites;
+
+struct WindowArgs {
+  int bf16, windows, win;  // see ckpt_layout
+};
 
 template <bool CK>
 struct BlockSmem {
@@ -307,19 +312,35 @@ __device__ __forceinline__ void block_pair(unsigned fwd, unsigned bwd, unsigned 
 }
 
 template <bool CK>
-__global__ void __launch_bounds__(CK ? 256 : 128, CK ? 2 : 4) k_impute_block(ChainArgs A, int blocks_per) {
+__global__ void __launch_bounds__(CK ? 256 : 128, CK ? 2 : 4) k_impute_block(ChainArgs A, int blocks_per,
+                                                                                   WindowArgs W) {
   constexpr int NT = CK ? 256 : 128;  // threads, states of a row
   __shared__ BlockSmem<CK> S;
   const int t = A.order ? A.order[blockIdx.y] : blockIdx.y;
   const int np = A.npoly[t], K = A.nstates[t];
   const int nrow = (np + RS - 1) / RS;
-  int b = blockIdx.x * blocks_per;
-  const int bend = min(nrow, b + blocks_per);
+  int b = blockIdx.x * blocks_per, rend = nrow;
+  int64_t row0 = 0;  // CK: offset of forward row 0
+  int to_bwd = 0;    // rows from a forward row to the backward one
+  if constexpr (CK) {
+    const CkptLayout lay = ckpt_layout(np, K, W.bf16, W.windows);
+    const int half = blockIdx.z;
+    int lo, hi;
+    ckpt_window(lay, half, W.win, lo, hi);
+    b += lo * (32 / RS);
+    rend = min(nrow, hi * (32 / RS));
+    // the window's rows of its chain; the other direction's beside them or among the checkpoints
+    const int chain = (int)(ckpt_window_rows(lay, half, W.win) / lay.Ks) - lo * (32 / RS);
+    const int other = W.bf16 ? chain + (half ? lay.wlen1 : lay.wlen0) * (32 / RS) : 0;
+    row0 = (int64_t)(half == 0 ? chain : other) * lay.Ks + lay.Ks - K;
+    to_bwd = half == 0 ? other - chain : chain - other;
+  }
+  const int bend = min(rend, b + blocks_per);
   if (b >= bend || K == 0) return;
   const int J = (K + NT - 1) >> (CK ? 8 : 7), Ks = CK ? (K + 127) & ~127 : 128 * J;
   const int pad = CK ? 0 : Ks - K;  // in front of row 0
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const float* base = A.rows + A.row_off[t] + (CK ? Ks - K : 0);
+  const float* base = A.rows + A.row_off[t] + (CK ? row0 : 0);
   const uint32_t* hvt = A.hvar + (size_t)t * A.WB * A.Kp - pad;
 
   // Rows j and j + 1 of this thread in block b: words and the kept values entering from both
@@ -336,7 +357,7 @@ __global__ void __launch_bounds__(CK ? 256 : 128, CK ? 2 : 4) k_impute_block(Cha
     const int o0 = CK ? min(o, K - 1) : max(o, pad), o1 = CK ? min(o + NT, K - 1) : max(o + NT, pad);
     const uint32_t* hv = hvt + (size_t)((b * RS) >> 5) * A.Kp;
     const float* ar = base + (size_t)b * Ks;
-    const float* br = ar + (size_t)nrow * Ks;
+    const float* br = ar + (int64_t)(CK ? to_bwd : nrow) * Ks;
     const bool left = b > 0, right = b < nrow - 1;
     p.w0 = hv[o0];
     p.w1 = hv[o1];
@@ -525,17 +546,27 @@ int launch_impute_chain(int J, ImputeWork& w, cudaStream_t s, int first, int cou
 
 static_assert(2 * kRowSites == 32, "k_impute_block: one lane per sum of a block");
 
-int launch_impute_block(bool ck, int max_poly, ImputeWork& w, float* hp, cudaStream_t s, int first, int count) {
+// Blocks per CTA: enough to hide the loads of each, while some eight CTAs per SM are left.
+static int blocks_per_cta(long long total) { return (int)std::max(1ll, std::min(16ll, total / (8 * 148))); }
+
+int launch_impute_block(int max_poly, ImputeWork& w, float* hp, cudaStream_t s, int first, int count) {
   ChainArgs a;
   if (chain_args(w, hp, first, count, a) != GP_OK) return GP_E_ARG;
   const int blocks = (max_poly + kRowSites - 1) / kRowSites;
   if (a.count == 0 || blocks == 0) return GP_OK;
-  // Blocks per CTA: enough to hide the loads of each, while some eight CTAs per SM are left.
-  const long long total = (long long)blocks * a.count;
-  const int per = (int)std::max(1ll, std::min(16ll, total / (8 * 148)));
-  const dim3 g((blocks + per - 1) / per, a.count);
-  if (ck) k_impute_block<true><<<g, 256, 0, s>>>(a, per);
-  else k_impute_block<false><<<g, 128, 0, s>>>(a, per);
+  const int per = blocks_per_cta((long long)blocks * a.count);
+  k_impute_block<false><<<dim3((blocks + per - 1) / per, a.count), 128, 0, s>>>(a, per, {});
+  return GP_OK;
+}
+
+int launch_ckpt_posteriors(bool bf16, int windows, int win, int wlen, ImputeWork& w, float* hp, cudaStream_t s,
+                           int first, int count) {
+  ChainArgs a;
+  if (chain_args(w, hp, first, count, a) != GP_OK) return GP_E_ARG;
+  const int blocks = wlen * (32 / kRowSites);
+  if (a.count == 0 || blocks == 0) return GP_OK;
+  const int per = blocks_per_cta(2ll * blocks * a.count);
+  k_impute_block<true><<<dim3((blocks + per - 1) / per, a.count, 2), 256, 0, s>>>(a, per, {bf16, windows, win});
   return GP_OK;
 }
 

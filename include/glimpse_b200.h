@@ -228,9 +228,11 @@ int gp_impute_one_static(gp_ctx* ctx, int32_t k, const uint32_t* states, const f
  * the chunk log-likelihood sum_l log AlphaSum_l in FP64 (gp_loglik_get). With FP32
  * checkpoints the posteriors are those of the same recursion; with BF16 ones, the
  * messages of one direction per half are recomputed in FP32 from a row rounded to
- * BF16 every 32 polymorphic sites, at a small posterior error. Each mode keeps a row
- * of either direction every 16 sites (half a byte per site and state, in chunks of
- * haplotypes that fit); BF16 adds 1/8 byte per site and state for all haplotypes. */
+ * BF16 every 32 polymorphic sites, at a small posterior error. What is kept per
+ * polymorphic site and state (in chunks of haplotypes that fit the device): half a
+ * byte in full precision; with checkpoints as little as 1/4 + 1/32 byte in FP32 and
+ * 1/16 + 1/16 in BF16, and more only where uneven sets stay within 1/4 and 1/8 byte
+ * per site of the panel (or of the largest set in a run) and state of the largest set. */
 int gp_set_precision(gp_ctx* ctx, int32_t mode);
 
 /* The FP64 chunk log-likelihood of each haplotype of the last imputation call

@@ -243,3 +243,37 @@ def test_confident_likelihoods_against_all_states():
                     assert abs(ctx.loglik(len(Ks))[i] - llr) <= 1e-6 * L + ll_tol, (m, Ks[i])
     finally:
         ctx.close()
+
+
+@pytest.mark.gpu
+def test_checkpointed_modes_need_less_memory():
+    """Device memory of a context after one call of 12 sets of 2,000 states (rows of
+    2,048) over 40,000 sites, all polymorphic. Full precision keeps half a byte per cell
+    (site, state), in a buffer with 1/8 to spare; the modes share all else but 4 bytes
+    per site. FP32 checkpoints: 1/4 byte and windows of 1/32; BF16: 1/16 and windows of
+    1/16; each with 1/8 to spare and 1/100 for what is not per cell."""
+    import torch
+    from glimpse_b200 import native, synth
+    L, n = 40000, 12
+    w = synth.make_panel_and_targets(2048, L, 1.3, 0.0, 2, ("uniform", 0.5, 2.0), ("fixed", 200), seed=53)
+    P, T = w.panel, w.targets
+    rng = np.random.default_rng(1)
+    states = [np.sort(rng.choice(2048, size=2000, replace=False)).astype(np.uint32) for _ in range(n)]
+    hls = np.stack([init_hl(T.gl[i % 2], T.flat[i % 2]) for i in range(n)])
+    flats = np.stack([T.flat[i % 2] for i in range(n)])
+    modes = (native.PRECISION_FULL, native.PRECISION_CKPT_F32, native.PRECISION_CKPT_BF16)
+    taken = {}
+    for _ in range(2):  # the first pass loads the kernels
+        for m in modes:
+            before = torch.cuda.mem_get_info()[0]
+            ctx = native.Context(P)
+            try:
+                ctx.set_precision(m)
+                ctx.impute_batch(states, hls, flats)
+                taken[m] = before - torch.cuda.mem_get_info()[0]
+            finally:
+                ctx.close()
+    cells = n * L * 2048
+    shared = taken[modes[0]] - 0.5 * 9 / 8 * cells
+    assert taken[modes[1]] - shared <= ((1 / 4 + 1 / 32) * 9 / 8 + 1 / 100) * cells
+    assert taken[modes[2]] - shared <= ((1 / 16 + 1 / 16) * 9 / 8 + 1 / 100) * cells
