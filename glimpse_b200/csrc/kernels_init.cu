@@ -135,10 +135,11 @@ __global__ void k_init_select(InitSelArgs a) {
           const int m = (int)min(a.cref[v], a.calt[v]);
           if (m != mac) continue;
           const int64_t o = a.svar_off[v], sz = a.svar_off[v + 1] - o;
-          int picked[5];
-          int np = 0;
-          std_sample(g, sz, 5, [&](int64_t i) { picked[np++] = (int)i; });
-          for (int i = 0; i < np && set.count < k_init8; ++i) set.insert((uint32_t)a.svar_haps[o + picked[i]]);
+          // no array of the positions in between: one indexed by a running count ended in an
+          // address-space error on the device
+          std_sample(g, sz, 5, [&](int64_t i) {
+            if (set.count < k_init8) set.insert((uint32_t)a.svar_haps[o + i]);
+          });
         }
       }
     } else {

@@ -424,8 +424,8 @@ def restate_state_post(panel, states, HL, flat, ne=100000, err_imp=1e-12):
     return mass.reshape(nwin, K), ns
 
 
-def stream_floats(seed, purpose, iteration, target, n):
-    """The first n words of a random stream (replay_rng.h) as floats in [0, 1)."""
+def stream_words(seed, purpose, iteration, target, n):
+    """The first n words of a random stream (replay_rng.h)."""
     lo, s32 = np.uint64(0xFFFFFFFF), np.uint64(32)
     q = np.arange((n + 3) // 4, dtype=np.uint64)
     c = [q, np.full_like(q, target), np.full_like(q, iteration), np.full_like(q, purpose)]
@@ -434,8 +434,85 @@ def stream_floats(seed, purpose, iteration, target, n):
         p0, p1 = c[0] * np.uint64(0xD2511F53), c[2] * np.uint64(0xCD9E8D57)
         c = [(p1 >> s32) ^ c[1] ^ np.uint64(k0), p1 & lo, (p0 >> s32) ^ c[3] ^ np.uint64(k1), p0 & lo]
         k0, k1 = (k0 + 0x9E3779B9) & 0xFFFFFFFF, (k1 + 0xBB67AE85) & 0xFFFFFFFF
-    w = np.stack(c, 1).ravel()[:n].astype(np.float32) * np.float32(2.0 ** -32)
+    return np.stack(c, 1).ravel()[:n]
+
+
+def stream_floats(seed, purpose, iteration, target, n):
+    """Those words as floats in [0, 1)."""
+    w = stream_words(seed, purpose, iteration, target, n).astype(np.float32) * np.float32(2.0 ** -32)
     return np.minimum(w, np.nextafter(np.float32(1), np.float32(0)))
+
+
+def _sample(words, size, n):
+    """std::sample over size positions on an iterator of words: the positions picked, in order."""
+    def draw(bound):  # uniform in [0, bound)
+        while True:
+            p = int(next(words)) * bound
+            if (p & 0xFFFFFFFF) >= (2 ** 32 - bound) % bound:
+                return p >> 32
+    out, left, idx = [], size, 0
+    n = min(n, left)
+    if left and 0xFFFFFFFF // left >= left:
+        while n and left >= 2:
+            x, d = draw(left * (left - 1)), left - 1
+            for p in (x // d, x % d):
+                left -= 1
+                if p < n:
+                    out.append(idx)
+                    n -= 1
+                idx += 1
+                if not n:
+                    break
+    while n:
+        left -= 1
+        if draw(left + 1) < n:
+            out.append(idx)
+            n -= 1
+        idx += 1
+    return out
+
+
+def restate_init_select(panel, targets, t, kinit, seed=15052011, iteration=0):
+    """haplotype_set::performSelection_RARE_INIT_GL (haplotype_set.cpp:775-833) for diploid target t: the sorted
+    states, and the number of rare sites where its likelihoods call a carrier (haplotype_set.cpp:108-169)."""
+    f = np.float32
+    unphred = np.array([float("%.6e" % (10.0 ** (-i / 10.0))) for i in range(256)], f)
+    N = panel.n_ref_haps
+    s = np.flatnonzero((panel.flag_common == 0) & (targets.flat[t] == 0) & (panel.lq == 0))
+    g, k, mg = targets.gl[t][s].astype(int), np.arange(s.size), 2 * panel.major[s].astype(int)
+    call = (g[:, 1] <= g[k, mg]) | (g[k, 2 - mg] <= g[k, mg])
+    p = unphred[g].T
+    p = p / ((p[0] + p[1]) + p[2])
+    af = (panel.calt[s].astype(np.float64) / N).astype(f)
+    q = f(1) - af
+    p = np.stack([p[0] * (q * q), p[1] * ((f(2) * af) * q), p[2] * (af * af)])
+    p = p / ((p[0] + p[1]) + p[2])
+    sites = s[call & (p[1] + p[2 - mg, k] > p[mg, k])]
+    carriers = {int(v): [] for v in sites}
+    for h in range(N):
+        for v in panel.shap_sites[panel.shap_off[h]:panel.shap_off[h + 1]]:
+            if int(v) in carriers:
+                carriers[int(v)].append(h)
+    words = iter(stream_words(seed, 5, iteration, t, 1 << 20))
+    k8, picked = int(np.floor(f(kinit) * f(0.8))), set()
+    if len(sites) > k8:
+        mac = np.minimum(panel.cref, panel.calt)
+        for v in sites[np.argsort(mac[sites], kind="stable")]:
+            if len(picked) >= k8:
+                break
+            for i in _sample(words, len(carriers[int(v)]), 5):
+                if len(picked) < k8:
+                    picked.add(carriers[int(v)][i])
+    elif len(sites):
+        for v in sites:
+            for i in _sample(words, len(carriers[int(v)]), max(k8 // len(sites), 1)):
+                if len(picked) < k8:
+                    picked.add(carriers[int(v)][i])
+    if len(picked) < kinit:
+        for i in _sample(words, N, kinit):
+            if len(picked) < kinit:
+                picked.add(i)
+    return np.array(sorted(picked), np.uint32), len(sites)
 
 
 def restate_rephase(panel, states, h0, h1, flat, iteration, target, seed=15052011, ne=100000, err_phase=1e-4):

@@ -239,3 +239,27 @@ def test_deep_lists_on_a_panel_without_staged_rows():
         finally:
             ctx.close()
     assert got[0] == got[1] and got[2] == got[3] and all(0 < len(s) <= 90 for g in got for s in g)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kinit", [1, 2, 20, 78, 93])
+def test_init_selection_matches_restatement(kinit):
+    """The init selection of targets that carry more rare alleles than the share of
+    Kinit for them (by minor-allele count, five carriers a site), and of targets with
+    fewer (all sites), against a restatement on the same streams."""
+    from glimpse_b200 import native, synth
+    from oracle import oracle as O
+    w = synth.make_panel_and_targets(94, 8075, 0.215, 0.3, 4, ("uniform", 0.2, 12.0), ("fixed", 60), seed=1005,
+                                     sparse_maf=3.5 / 94)
+    ctx = native.Context(w.panel, kinit=kinit, kpbwt=11)
+    try:
+        ctx.set_targets(w.targets, kpbwt=w.targets.kpbwt)
+        ctx.select(O.STAGE_INIT, 0)
+        many = []
+        for t in range(w.targets.n):
+            want, sites = O.restate_init_select(w.panel, w.targets, t, kinit)
+            many.append(sites > int(0.8 * kinit))
+            assert want.tolist() == ctx.states(t).tolist(), t
+        assert any(many)
+    finally:
+        ctx.close()
