@@ -398,8 +398,8 @@ int Context::run_impute(const float* d_hl, const uint8_t* d_flat, float* d_hp) {
   std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return impute_np[x] > impute_np[y]; });
   // Windows of the checkpointed modes: as few as keep the batch within 1/8 byte per cell (site of a set, state of
   // the largest) in BF16 mode and 1/4 in FP32, at most 16 (the rows of two are then 1/16 and 1/32), of 16 blocks
-  // and more in either half. Blocks beside chains slow them: 32 haplotypes at K 400-1,200 18.4 ms with 16, 17.9
-  // with one.
+  // and more in either half. Blocks beside chains slow them where SMs are free: 32 haplotypes at K 400-1,200 18.5 ms
+  // with 16, 18.2 with one; 256 31.0 and 32.4.
   int windows = 1;
   if (ck) {
     int np_max = 0;

@@ -222,10 +222,9 @@ __device__ __forceinline__ void ckpt_run(const CkptArgs& A, CkptSmem& S, const C
       if (!(BF16 && OWN) && (FWD ? i == part * kRowSites : i == (part + 1) * kRowSites - 1))
         store_row(b * (32 / kRowSites) + part);
       const int stop = FWD ? min(end, (part + 1) * kRowSites) : part * kRowSites - 1;
-      // A step is latency; unrolled, its loop's own instructions go (one haplotype, K = 600:
-      // 11.7 -> 11.4 ms). Not with many states, where mixed classes then slow one another (128
-      // haplotypes, K 1,000-2,048: 12.6 ms, 16.4 unrolled).
-#pragma unroll (J <= 5 ? 4 : 1)
+      // Not unrolled: by four it took a single haplotype from 11.7 to 11.4 ms, but many chains of
+      // mixed classes from 27 to 36 (256 haplotypes at K 400-1,200).
+#pragma unroll 1
       while (i != stop) step(std::integral_constant<bool, false>());
     }
     if (wi == 0) {
