@@ -224,8 +224,8 @@ __device__ __forceinline__ float transition(const double* __restrict__ cm, int p
 //    with register moves, cost a quarter of the instructions.
 // Measured, whole phasing per iteration: 11 targets of a 2,503 x 30,011 panel at
 // K 130-900 28.1 -> 8.0 ms; 256 targets of a 10,000 x 150,000 panel at K 400-1,200
-// 116 -> 56 ms (both passes in one 256-thread CTA before). 235 warp instructions a
-// site at J = 2; two warps of one virtual warp each instead of one of two: slower
+// 116 -> 46 ms (both passes in one 256-thread CTA before). 243 warp instructions a
+// site at J = 2, 313 at J = 4; two warps of one virtual warp each instead of one of two: slower
 // at 11 targets (16.1 against 14.2 ms, first version) and at 256.
 // ---------------------------------------------------------------------------
 // V virtual warps per warp: 8 / V warps, 256 / V threads a chain.

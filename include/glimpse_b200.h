@@ -242,7 +242,10 @@ int gp_loglik_get(gp_ctx* ctx, int32_t n, double* out);
 
 /* phasing_hmm::rephaseHaplotypes(H0, H1, flat) (phasing_hmm.h:136) for n
  * diploid targets with explicit conditioning sets; h0/h1 updated in place
- * (n x L). Target t draws from stream (RNG_PHASE, iteration, target_ids[t]). */
+ * (n x L). Target t draws from stream (RNG_PHASE, iteration, target_ids[t]).
+ * Device memory, here and in the iterations: 64 bytes per state and segment (of
+ * three peak hets) or flat het of a target, in chunks of targets that fit; one
+ * target's must fit the device. */
 int gp_rephase_batch(gp_ctx* ctx, int32_t n, const int64_t* states_off, const uint32_t* states, uint8_t* h0,
                      uint8_t* h1, const uint8_t* flat, int32_t iteration, const int32_t* target_ids);
 
