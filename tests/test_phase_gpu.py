@@ -237,3 +237,31 @@ def test_small_sets_on_long_chunks_match_restatement(K):
         r0, r1, invalid = O.restate_rephase(P, s, h0, h1, flat, 3, t)
         assert not invalid
         assert np.array_equal(g0[t], r0) and np.array_equal(g1[t], r1), t
+
+
+@pytest.mark.gpu
+def test_small_sets_in_a_large_batch_match_restatement():
+    """The same for two-warp chains, whose unused slots are most of a warp: 240 targets
+    with 2 states each, all of one class."""
+    from oracle import oracle as O
+    from glimpse_b200 import native, synth
+    w = synth.make_panel_and_targets(1000, 12000, 0.3, 0.0, 3, ("uniform", 0.5, 2.0), ("fixed", 100), seed=83,
+                                     sparse_maf=0.005, alt_major_frac=0.1)
+    P, T = w.panel, w.targets
+    rng = np.random.default_rng(2)
+    n = 240
+    sets = [np.sort(rng.choice(P.n_ref_haps, size=2, replace=False)).astype(np.uint32) for _ in range(n)]
+    h0 = np.stack([_noisy_haps(rng, T.truth[i % 3, 0]) for i in range(n)])
+    h1 = np.stack([_noisy_haps(rng, T.truth[i % 3, 1]) for i in range(n)])
+    for i, s in enumerate(sets):
+        alt = np.flatnonzero(P.flag_common)[((P.hvar[:, s >> 3] >> (7 - (s & 7)).astype(np.uint8)) & 1).all(axis=1)]
+        h0[i, alt] = h1[i, alt] = 0
+    flat = np.stack([T.flat[i % 3] for i in range(n)])
+    ctx = native.Context(P)
+    try:
+        g0, g1 = ctx.rephase_batch(sets, h0, h1, flat, 5)
+    finally:
+        ctx.close()
+    for i in range(0, n, 7):
+        r0, r1, invalid = O.restate_rephase(P, sets[i], h0[i], h1[i], flat[i], 5, i)
+        assert not invalid and np.array_equal(g0[i], r0) and np.array_equal(g1[i], r1), i

@@ -277,3 +277,38 @@ def test_checkpointed_modes_need_less_memory():
     shared = taken[modes[0]] - 0.5 * 9 / 8 * cells
     assert taken[modes[1]] - shared <= ((1 / 4 + 1 / 32) * 9 / 8 + 1 / 100) * cells
     assert taken[modes[2]] - shared <= ((1 / 16 + 1 / 16) * 9 / 8 + 1 / 100) * cells
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", [1, 2])
+def test_windows_chunks_and_classes_give_the_same_bits(mode, monkeypatch):
+    """The number of windows follows the batch, and with more than four classes of 256
+    states some run their blocks behind their chains on one stream: eight classes in
+    one call, four, each set alone, and in chunks under a budget of 4 MB must give the
+    same posteriors and log-likelihoods, bit for bit."""
+    from glimpse_b200 import native, synth
+    w = synth.make_panel_and_targets(2100, 9000, 0.3, 0.3, 2, ("uniform", 0.5, 2.0), ("fixed", 200), seed=57,
+                                     sparse_maf=0.005)
+    P, T = w.panel, w.targets
+    rng = np.random.default_rng(mode)
+    Ks = [2, 300, 600, 900, 1100, 1400, 1700, 2048]
+    states = [np.sort(rng.choice(2100, size=K, replace=False)).astype(np.uint32) for K in Ks]
+    hls = np.stack([init_hl(T.gl[i % 2], T.flat[i % 2]) for i in range(len(Ks))])
+    flats = np.stack([T.flat[i % 2] for i in range(len(Ks))])
+    ctx = native.Context(P)
+
+    def run(idx):
+        hp = ctx.impute_batch([states[i] for i in idx], hls[idx], flats[idx])
+        return hp, np.asarray(ctx.loglik(len(idx)))
+
+    try:
+        ctx.set_precision(mode)
+        hp, ll = run(list(range(8)))
+        monkeypatch.setenv("GLIMPSE_B200_STORE_BUDGET_MB", "4")
+        parts = [(list(range(8)), run(list(range(8))))]
+        monkeypatch.delenv("GLIMPSE_B200_STORE_BUDGET_MB")
+        parts += [(idx, run(idx)) for idx in [[0, 1, 2, 3], [4, 5, 6, 7]] + [[i] for i in range(8)]]
+        for idx, (h, l) in parts:
+            assert np.array_equal(h, hp[idx]) and np.array_equal(l, ll[idx]), idx
+    finally:
+        ctx.close()
