@@ -482,7 +482,7 @@ int Context::run_impute(const float* d_hl, const uint8_t* d_flat, float* d_hp) {
         for (int i = 0; i < nc && rc == GP_OK; ++i) {
           const int J = class_of(order[cls[i]]), cnt = cls[i + 1] - cls[i];
           const cudaStream_t s = stream_of(i);
-          rc = launch_ckpt_chain(J, bf16, windows, win, w, ckpt_sum.as<float>(), s, cls[i], cnt);
+          rc = launch_ckpt_chain(J, bf16, 2 * (c1 - c0) <= sm_count, windows, win, w, ckpt_sum.as<float>(), s, cls[i], cnt);
           prof.kernel_launches += 1;
           if (win < 0 || rc != GP_OK) continue;
           cudaStream_t sb = s;

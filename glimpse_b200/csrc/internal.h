@@ -221,8 +221,8 @@ inline void ckpt_window(const CkptLayout& a, int half, int w, int& lo, int& hi) 
 // chains over their own halves (win < 0) or window win; asum: [n][32 WB]. Then the
 // posteriors of a window of at most wlen blocks of 32 in either half (launch_ckpt_posteriors
 // after the rows that BF16 mode recomputes).
-int launch_ckpt_chain(int J, bool bf16, int windows, int win, ImputeWork& w, float* asum, cudaStream_t s, int first,
-                      int count);
+int launch_ckpt_chain(int J, bool bf16, bool few, int windows, int win, ImputeWork& w, float* asum, cudaStream_t s,
+                      int first, int count);
 int launch_ckpt_window(int J, bool bf16, int windows, int win, int wlen, ImputeWork& w, float* hp, cudaStream_t s,
                        int first, int count);
 int launch_ckpt_posteriors(bool bf16, int windows, int win, int wlen, ImputeWork& w, float* hp, cudaStream_t s,

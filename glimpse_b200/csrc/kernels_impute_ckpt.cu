@@ -63,8 +63,8 @@ struct CkptSmem {
 // Steps through the blocks b_first .. b_last (in the direction of the chain). Rows
 // entering blocks of 16 go to `out`, the one of block r0 first; in the chain's own half
 // (OWN) in BF16 mode, rows entering blocks of 32 to the checkpoints instead.
-// SEG: one block, from its BF16 checkpoint. J: 256 (J - 1) < K <= 256 J.
-template <int J, bool FWD, bool SEG, bool BF16, bool OWN>
+// SEG: one block, from its BF16 checkpoint. J: 256 (J - 1) < K <= 256 J. U: steps unrolled.
+template <int J, bool FWD, bool SEG, bool BF16, bool OWN, int U>
 __device__ __forceinline__ void ckpt_run(const CkptArgs& A, CkptSmem& S, const CkptLayout& lay, int t, int b_first,
                                          int b_last, float* out, int r0) {
   constexpr int NP = 2 * J;  // packed pairs of states: virtual warps (0, 1) and (2, 3) of the warp, per j
@@ -222,9 +222,7 @@ __device__ __forceinline__ void ckpt_run(const CkptArgs& A, CkptSmem& S, const C
       if (!(BF16 && OWN) && (FWD ? i == part * kRowSites : i == (part + 1) * kRowSites - 1))
         store_row(b * (32 / kRowSites) + part);
       const int stop = FWD ? min(end, (part + 1) * kRowSites) : part * kRowSites - 1;
-      // Not unrolled: by four it took a single haplotype from 11.7 to 11.4 ms, but many chains of
-      // mixed classes from 27 to 36 (256 haplotypes at K 400-1,200).
-#pragma unroll 1
+#pragma unroll U
       while (i != stop) step(std::integral_constant<bool, false>());
     }
     if (wi == 0) {
@@ -252,7 +250,7 @@ __device__ __forceinline__ void ckpt_run(const CkptArgs& A, CkptSmem& S, const C
 
 // Both chains of every haplotype, over their own halves or a window of the other's: CTA
 // 2 c forward, 2 c + 1 backward.
-template <int J, bool BF16, bool OWN>
+template <int J, bool BF16, bool OWN, int U>
 __global__ void __launch_bounds__(kCkptThreads, 1) k_ckpt_chain(CkptArgs A) {
   __shared__ CkptSmem S;
   const int t = A.order[blockIdx.x >> 1];
@@ -264,8 +262,8 @@ __global__ void __launch_bounds__(kCkptThreads, 1) k_ckpt_chain(CkptArgs A) {
   if (lo >= hi) return;
   float* out = A.rows + A.row_off[t] + (OWN ? 0 : ckpt_window_rows(lay, fwd ? 0 : 1, A.win));
   const int r0 = OWN ? 0 : lo * (32 / kRowSites);
-  if (fwd) ckpt_run<J, true, false, BF16, OWN>(A, S, lay, t, lo, hi - 1, out, r0);
-  else ckpt_run<J, false, false, BF16, OWN>(A, S, lay, t, hi - 1, lo, out, r0);
+  if (fwd) ckpt_run<J, true, false, BF16, OWN, U>(A, S, lay, t, lo, hi - 1, out, r0);
+  else ckpt_run<J, false, false, BF16, OWN, U>(A, S, lay, t, hi - 1, lo, out, r0);
 }
 
 // The rows of the other direction for one block of the window, from its BF16 checkpoint.
@@ -284,8 +282,8 @@ __global__ void __launch_bounds__(kCkptThreads, 1) k_ckpt_block(CkptArgs A) {
   const int r0 = lo * (32 / kRowSites);
   float* out = A.rows + A.row_off[t] + ckpt_window_rows(lay, half, A.win) +
                (int64_t)(half ? lay.wlen1 : lay.wlen0) * (32 / kRowSites) * lay.Ks;
-  if (half) ckpt_run<J, true, true, true, false>(A, S, lay, t, b, b, out, r0);
-  else ckpt_run<J, false, true, true, false>(A, S, lay, t, b, b, out, r0);
+  if (half) ckpt_run<J, true, true, true, false, 1>(A, S, lay, t, b, b, out, r0);
+  else ckpt_run<J, false, true, true, false, 1>(A, S, lay, t, b, b, out, r0);
 }
 
 // Sum of log AlphaSum over the sites of haplotype blockIdx.x, in FP64.
@@ -330,21 +328,31 @@ static CkptArgs ckpt_args(ImputeWork& w, int windows, int win, float* asum, int 
 
 #define GP_EACH_J(M) M(1) M(2) M(3) M(4) M(5) M(6) M(7) M(8)
 
-int launch_ckpt_chain(int J, bool bf16, int windows, int win, ImputeWork& w, float* asum, cudaStream_t s, int first,
-                      int count) {
+// few: the batch's chains have an SM each. Their steps are then unrolled by four: a step is latency, and the loop's own
+// instructions go (one haplotype at K = 600 11.6 -> 11.3 ms, 32 at K 400-1,200 18.3 -> 17.9). Where chains of
+// mixed classes share SMs it costs a third (256: 31 -> 41 ms).
+int launch_ckpt_chain(int J, bool bf16, bool few, int windows, int win, ImputeWork& w, float* asum, cudaStream_t s,
+                      int first, int count) {
   const CkptArgs a = ckpt_args(w, windows, win, asum, first);
-#define GP_CK(JJ)                                                                                \
-  case JJ:                                                                                       \
-    if (bf16 && win < 0) k_ckpt_chain<JJ, true, true><<<2 * count, kCkptThreads, 0, s>>>(a);     \
-    else if (bf16) k_ckpt_chain<JJ, true, false><<<2 * count, kCkptThreads, 0, s>>>(a);          \
-    else if (win < 0) k_ckpt_chain<JJ, false, true><<<2 * count, kCkptThreads, 0, s>>>(a);       \
-    else k_ckpt_chain<JJ, false, false><<<2 * count, kCkptThreads, 0, s>>>(a);                   \
+#define GP_CK1(JJ, UU)                                                                           \
+  if (bf16 && win < 0) k_ckpt_chain<JJ, true, true, UU><<<2 * count, kCkptThreads, 0, s>>>(a);   \
+  else if (bf16) k_ckpt_chain<JJ, true, false, UU><<<2 * count, kCkptThreads, 0, s>>>(a);        \
+  else if (win < 0) k_ckpt_chain<JJ, false, true, UU><<<2 * count, kCkptThreads, 0, s>>>(a);     \
+  else k_ckpt_chain<JJ, false, false, UU><<<2 * count, kCkptThreads, 0, s>>>(a);
+#define GP_CK(JJ)         \
+  case JJ:                \
+    if (few) {            \
+      GP_CK1(JJ, 4)       \
+    } else {              \
+      GP_CK1(JJ, 1)       \
+    }                     \
     return GP_OK;
   switch (J) {
     GP_EACH_J(GP_CK)
     default: return GP_E_ARG;
   }
 #undef GP_CK
+#undef GP_CK1
 }
 
 int launch_ckpt_window(int J, bool bf16, int windows, int win, int wlen, ImputeWork& w, float* hp, cudaStream_t s,
